@@ -112,119 +112,308 @@ forward_simt_kernel(SimtNet net, const MlpLayerPointers* __restrict__ lp, const 
     for (int j = 0; j < od; ++j) outputs[int64_t(tid) * od + j] = o[j];
 }
 
-// learnGradient, generic.  Phase A (per thread): forward, loss, backward; every layer's input vector
-// a_l and output gradient dz_l stay in the per-thread arrays.  Phase B (per block): for each layer the
-// block stages `group` samples' (dz_l, a_l) in shared memory and each thread owns a strided set of
-// parameters, summing its terms over the staged samples in ascending order before one atomic add per
-// parameter per group.  With MLP_FLAG_SEQUENTIAL_SUM the per-sample vectors go to a global scratch
-// area instead and a second kernel adds them one sample at a time.
-__global__ void __launch_bounds__(256)
-learn_gradient_simt_kernel(SimtNet net, const MlpLayerPointers* __restrict__ lp, uint32_t* lossBuffer,
-                           const void* __restrict__ inputs, const void* __restrict__ targets, uint32_t count,
-                           int group, float* __restrict__ seq_scratch, float* __restrict__ input_grads)
+// learnGradient, generic.  A CTA walks tiles of 32 samples with the LANES on the samples and the warps on the
+// output features: every vector of a tile (layer inputs, pre-activations, output gradients) is a shared-memory row
+// of 32 floats per feature, a weight is one broadcast read shared by the 32 samples, and each sum runs over its
+// terms in ascending order exactly as simt_forward does.  Parameters are summed over the tile in ascending sample
+// order, over the CTA's tiles in shared memory where it has room, and leave through one atomic add per parameter
+// per CTA.  With MLP_FLAG_SEQUENTIAL_SUM the per-sample vectors go to a global scratch area instead and a second
+// kernel adds them one sample at a time.
+//
+// Bound: the latency of the layer chain at small batches (a tile is 2 NL + 2 barriers), fp32 issue at large ones.
+// One thread per sample with its vectors in local memory, which this replaces, put 4096 samples on 16 of the 148
+// SMs and walked every sum behind local-memory loads.
+constexpr int kTile = 32;                   // samples per tile, one per lane
+constexpr int kRow = kTile + 4;             // floats per feature row: 16-byte reads of eight consecutive rows hit distinct banks
+constexpr int kSimtThreads = 512;
+constexpr int kSimtWarps = kSimtThreads / 32;
+constexpr size_t kSimtSmemMax = 227 * 1024;
+
+// Shared-memory map of a network, in floats: feature rows of a_0 .. a_{nl-1} and the outputs (a_off[l] * kRow), then
+// of z_1 .. z_nl, then biases, and where there is room the weights (rows padded to multiples of four) and the
+// gradient sums of the CTA's tiles.
+struct SimtSmem {
+    int z, bias, total;
+    int w;                                  // -1: weights are read from global memory
+    int grads;                              // -1: sums leave after every tile
+    int w_off[MLP_MAX_LAYERS], b_off[MLP_MAX_LAYERS], g_off[MLP_MAX_LAYERS];   // inside their regions
+};
+
+// Four consecutive weights of output j, from shared memory (staged) or from the parameters.
+template <bool STAGED>
+struct WeightRows {
+    const MlpConfig& c;
+    const void* W;
+    const float* s_w;
+    int in, out, stride;
+    __device__ __forceinline__ float one(int j, int i) const
+    {
+        return STAGED ? s_w[j * stride + i] : load_weight(c, W, weight_index(c.param_layout, in, out, j, i));
+    }
+    __device__ __forceinline__ float4 four(int j, int i) const
+    {
+        if constexpr (STAGED) return *reinterpret_cast<const float4*>(s_w + j * stride + i);
+        return make_float4(one(j, i), i + 1 < in ? one(j, i + 1) : 0.0f, i + 2 < in ? one(j, i + 2) : 0.0f, i + 3 < in ? one(j, i + 3) : 0.0f);
+    }
+};
+
+// z and a of J outputs from j0 on for this lane's sample.
+template <int J, bool STAGED>
+__device__ __forceinline__ void tile_layer_forward(const MlpConfig& c, const WeightRows<STAGED>& w, const float* s_bias, const float* ain,
+                                                   float* z, float* aout, int j0, int act, bool round_act, bool fused)
 {
-    extern __shared__ float smem[];
+    float r[J];
+    int jr[J];
+#pragma unroll
+    for (int u = 0; u < J; ++u) {
+        jr[u] = min(j0 + u, w.out - 1);
+        r[u] = fused ? s_bias[jr[u]] : 0.0f;
+    }
+    int i = 0;
+    for (; i + 4 <= w.in; i += 4) {
+        const float a0 = ain[i * kRow], a1 = ain[(i + 1) * kRow], a2 = ain[(i + 2) * kRow], a3 = ain[(i + 3) * kRow];
+#pragma unroll
+        for (int u = 0; u < J; ++u) {
+            const float4 v = w.four(jr[u], i);
+            r[u] = mac(v.w, a3, mac(v.z, a2, mac(v.y, a1, mac(v.x, a0, r[u], fused), fused), fused), fused);
+        }
+    }
+    for (; i < w.in; ++i) {
+        const float a0 = ain[i * kRow];
+#pragma unroll
+        for (int u = 0; u < J; ++u) r[u] = mac(w.one(jr[u], i), a0, r[u], fused);
+    }
+#pragma unroll
+    for (int u = 0; u < J; ++u) {
+        if (j0 + u >= w.out) break;
+        const float zs = round_to(c.dtype, fused ? r[u] : r[u] + s_bias[j0 + u]);
+        const float v = act_value(act, c.act_alpha, zs);
+        z[(j0 + u) * kRow] = zs;
+        aout[(j0 + u) * kRow] = round_act ? round_to(operand_type(c), v) : v;
+    }
+}
+
+// r[u] = sum over j of W[j][i0 + u] dz[j], four inputs at a time (i0 a multiple of four).
+template <bool STAGED>
+__device__ __forceinline__ void tile_layer_backward(const WeightRows<STAGED>& w, const float* dz, int i0, float (&r)[4], bool fused)
+{
+#pragma unroll
+    for (int u = 0; u < 4; ++u) r[u] = 0.0f;
+    for (int j = 0; j < w.out; ++j) {
+        const float d = dz[j * kRow];
+        const float4 v = w.four(j, i0);
+        r[0] = mac(v.x, d, r[0], fused);
+        r[1] = mac(v.y, d, r[1], fused);
+        r[2] = mac(v.z, d, r[2], fused);
+        r[3] = mac(v.w, d, r[3], fused);
+    }
+}
+
+template <bool STAGED>
+__global__ void __launch_bounds__(kSimtThreads)
+learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_constant__ SimtSmem map, const MlpLayerPointers* __restrict__ lp,
+                           uint32_t* lossBuffer, const void* __restrict__ inputs, const void* __restrict__ targets, uint32_t count,
+                           uint32_t n_tiles, float* __restrict__ seq_scratch, float* __restrict__ input_grads)
+{
+    extern __shared__ __align__(16) float smem[];
     const MlpConfig& c = net.cfg;
     const int nl = c.n_layers;
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = tid < count;
-    float a[kMaxActFloats];   // inputs of every layer; outputs in the last slot
-    float zd[kMaxActFloats];  // pre-activations going forward, overwritten by dz going backward
-    float loss = 0.0f;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int od = c.dims[nl];
     const bool fused = c.sum_order == MLP_SUM_BIAS_FIRST_FUSED;
-    if (valid) {
-        simt_forward(net, lp, inputs, tid, a, zd);
-        const float scale = (c.loss == MLP_LOSS_MSE_MEAN) ? 1.0f / float(od) : 1.0f;
-        const float* o = a + net.a_off[nl];
-        float* dzl = zd + net.a_off[nl] - net.a_off[1];
-        for (int j = 0; j < od; ++j) {
-            const float t = load_as_f32(c.target_dtype, targets, int64_t(tid) * od + j);
-            const float diff = o[j] - t;
-            loss = fmaf(diff * scale, diff, loss);
-            const float dout = (2.0f * scale) * diff;
-            const float d = act_deriv(c.output_act, c.act_alpha, dzl[j]);
-            dzl[j] = round_to(operand_type(c), dout * d);
-        }
-        for (int l = nl - 1; l >= 1; --l) {
-            const int in = c.dims[l], out = c.dims[l + 1];
-            const float* dz = zd + net.a_off[l + 1] - net.a_off[1];
-            float* zprev = zd + net.a_off[l] - net.a_off[1];
-            const void* W = (const void*)lp[l].weights;
-            for (int i = 0; i < in; ++i) {
-                float r = 0.0f;
-                for (int j = 0; j < out; ++j) r = mac(load_weight(c, W, weight_index(c.param_layout, in, out, j, i)), dz[j], r, fused);
-                const float d = round_to(operand_type(c), act_deriv(c.hidden_act, c.act_alpha, zprev[i]));
-                zprev[i] = round_to(operand_type(c), r * d);
+    const int opd = operand_type(c);
+    const bool once = gridDim.x == n_tiles;       // one tile per CTA: its sums leave directly
+    float* const s_z = smem + map.z;              // z rows, later dz: layer l's outputs from row a_off[l + 1] - a_off[1]
+    auto z_rows = [&](int l) { return s_z + (net.a_off[l] - net.a_off[1]) * kRow; };   // of the vector leaving layer l - 1
+
+    for (int l = 0; l < nl; ++l) {
+        const int in = c.dims[l], out = c.dims[l + 1];
+        const MlpLayerPointers ptr = lp[l];
+        for (int j = threadIdx.x; j < out; j += kSimtThreads) smem[map.bias + map.b_off[l] + j] = load_as_f32(c.dtype, (const void*)ptr.biases, j);
+        if constexpr (STAGED) {
+            const int stride = (in + 3) & ~3;
+            for (int idx = threadIdx.x; idx < out * stride; idx += kSimtThreads) {
+                const int j = idx / stride, i = idx - j * stride;
+                smem[map.w + map.w_off[l] + idx] =
+                    i < in ? load_weight(c, (const void*)ptr.weights, weight_index(c.param_layout, in, out, j, i)) : 0.0f;
             }
+        }
+    }
+    auto weights = [&](int l) {
+        return WeightRows<STAGED>{c, STAGED ? nullptr : (const void*)lp[l].weights, STAGED ? smem + map.w + map.w_off[l] : nullptr,
+                                  c.dims[l], c.dims[l + 1], (c.dims[l] + 3) & ~3};
+    };
+
+    float run_max = 0.0f, run_sum = 0.0f;         // warp 0: this lane's samples
+    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const uint32_t s0 = tile * kTile;
+        const int n_here = min(kTile, (int)(count - s0));
+        const bool valid = lane < n_here;
+        // ---- inputs; rows past the batch are zero ----
+        for (int idx = threadIdx.x; idx < kTile * c.dims[0]; idx += kSimtThreads) {
+            const int s = idx / c.dims[0], i = idx - s * c.dims[0];
+            float v = 0.0f;
+            if (s < n_here) {
+                if (c.encoding == MLP_ENC_FREQ2D) {
+                    const float x = load_as_f32(c.input_dtype, inputs, int64_t(s0 + s) * 2 + (i >> 4));
+                    const float arg = ldexpf(3.14159265358979323846f, (i & 15) >> 1) * x;
+                    v = (i & 1) ? cosf(arg) : sinf(arg);
+                } else {
+                    v = load_as_f32(c.input_dtype, inputs, int64_t(s0) * c.dims[0] + idx);
+                }
+                v = round_to(opd, v);
+            }
+            smem[i * kRow + s] = v;
+        }
+        __syncthreads();
+        // ---- forward ----
+        for (int l = 0; l < nl; ++l) {
+            const WeightRows<STAGED> w = weights(l);
+            const bool last = l == nl - 1;
+            const float* ain = smem + net.a_off[l] * kRow + lane;
+            float* aout = smem + net.a_off[l + 1] * kRow + lane;
+            float* z = z_rows(l + 1) + lane;
+            const float* s_bias = smem + map.bias + map.b_off[l];
+            const int act = last ? c.output_act : c.hidden_act;
+            if (w.out <= kSimtWarps) {
+                if (warp < w.out) tile_layer_forward<1, STAGED>(c, w, s_bias, ain, z, aout, warp, act, !last, fused);
+            } else if (w.out <= 2 * kSimtWarps) {
+                if (2 * warp < w.out) tile_layer_forward<2, STAGED>(c, w, s_bias, ain, z, aout, 2 * warp, act, !last, fused);
+            } else {
+                for (int j0 = 4 * warp; j0 < w.out; j0 += 4 * kSimtWarps)
+                    tile_layer_forward<4, STAGED>(c, w, s_bias, ain, z, aout, j0, act, !last, fused);
+            }
+            __syncthreads();
+        }
+        // ---- loss (warp 0, a sample per lane, outputs in ascending order) and dz of the last layer (every warp) ----
+        {
+            const float scale = (c.loss == MLP_LOSS_MSE_MEAN) ? 1.0f / float(od) : 1.0f;
+            const float* o = smem + net.a_off[nl] * kRow + lane;
+            float* dz = z_rows(nl) + lane;
+            for (int j = warp; j < od; j += kSimtWarps) {
+                float g = 0.0f;
+                if (valid) {
+                    const float diff = o[j * kRow] - load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j);
+                    g = round_to(opd, ((2.0f * scale) * diff) * act_deriv(c.output_act, c.act_alpha, dz[j * kRow]));
+                }
+                dz[j * kRow] = g;
+            }
+            if (warp == 0 && valid) {
+                float loss = 0.0f;
+                for (int j = 0; j < od; ++j) {
+                    const float diff = o[j * kRow] - load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j);
+                    loss = fmaf(diff * scale, diff, loss);
+                }
+                run_max = fmaxf(run_max, loss);
+                run_sum += loss;
+            }
+        }
+        __syncthreads();
+        // ---- backward: dz of the layer before replaces its z; rows past the batch stay zero because dz is zero ----
+        for (int l = nl - 1; l >= 1; --l) {
+            const WeightRows<STAGED> w = weights(l);
+            const float* dz = z_rows(l + 1) + lane;
+            float* zprev = z_rows(l) + lane;
+            for (int i0 = 4 * warp; i0 < w.in; i0 += 4 * kSimtWarps) {
+                float r[4];
+                tile_layer_backward<STAGED>(w, dz, i0, r, fused);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (i0 + u >= w.in) break;
+                    const float d = round_to(opd, act_deriv(c.hidden_act, c.act_alpha, zprev[(i0 + u) * kRow]));
+                    zprev[(i0 + u) * kRow] = valid ? round_to(opd, r[u] * d) : 0.0f;
+                }
+            }
+            __syncthreads();
         }
         if (input_grads) {
             // dx = W_0^T dz_0: dead in the example (its inputs are no_diff), wanted by an encoder in front
-            const int in = c.dims[0], out = c.dims[1];
-            const float* dz = zd;
-            const void* W = (const void*)lp[0].weights;
-            for (int i = 0; i < in; ++i) {
-                float r = 0.0f;
-                for (int j = 0; j < out; ++j) r = mac(load_weight(c, W, weight_index(c.param_layout, in, out, j, i)), dz[j], r, fused);
-                input_grads[int64_t(tid) * in + i] = round_to(c.dtype, r);
+            const WeightRows<STAGED> w = weights(0);
+            for (int i0 = 4 * warp; i0 < w.in; i0 += 4 * kSimtWarps) {
+                float r[4];
+                tile_layer_backward<STAGED>(w, z_rows(1) + lane, i0, r, fused);
+                for (int u = 0; u < 4 && i0 + u < w.in; ++u)
+                    if (valid) input_grads[int64_t(s0 + lane) * w.in + i0 + u] = round_to(c.dtype, r[u]);
             }
         }
-    }
-
-    // Loss words: wave max folded in by the first lane; block sum added once.
-    {
-        float m = loss;
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        float sum = loss;
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if ((threadIdx.x & 31) == 0) {
-            if (blockIdx.x * blockDim.x + (threadIdx.x & ~31u) < count) atomicMax(lossBuffer, __float_as_uint(m));
-            atomicAdd((float*)(lossBuffer + 1), sum);
-        }
-    }
-
-    if (seq_scratch) {
-        // Layout per sample: [a of all layers (a_off[nl] floats)][dz of all layers (a_off[nl+1]-a_off[1] floats)].
-        if (valid) {
-            const int na = net.a_off[nl], nz = net.a_off[nl + 1] - net.a_off[1];
-            float* dst = seq_scratch + int64_t(tid) * (na + nz);
-            for (int i = 0; i < na; ++i) dst[i] = a[i];
-            for (int i = 0; i < nz; ++i) dst[na + i] = zd[i];
-        }
-        return;
-    }
-
-    const int first = blockIdx.x * blockDim.x;
-    const int n_block = count > (uint32_t)first ? min((int)blockDim.x, (int)(count - first)) : 0;
-    for (int l = 0; l < nl; ++l) {
-        const int in = c.dims[l], out = c.dims[l + 1];
-        const float* al = a + net.a_off[l];
-        const float* dz = zd + net.a_off[l + 1] - net.a_off[1];
-        float* dW = (float*)lp[l].weightsGrad;
-        float* dB = (float*)lp[l].biasesGrad;
-        const int stride = in + out;
-        for (int g0 = 0; g0 < n_block; g0 += group) {
-            const int gn = min(group, n_block - g0);
-            __syncthreads();
-            const int local = (int)threadIdx.x - g0;
-            if (local >= 0 && local < gn) {
-                float* row = smem + local * stride;
-                for (int i = 0; i < in; ++i) row[i] = al[i];
-                for (int j = 0; j < out; ++j) row[in + j] = dz[j];
+        if (seq_scratch) {
+            // Per sample: [a of all layers (a_off[nl] floats)][dz of all layers (a_off[nl + 1] - a_off[1] floats)].
+            const int na = net.a_off[nl], n = na + net.a_off[nl + 1] - net.a_off[1];
+            for (int idx = threadIdx.x; idx < n_here * n; idx += kSimtThreads) {
+                const int s = idx / n, k = idx - s * n;
+                seq_scratch[int64_t(s0 + s) * n + k] = k < na ? smem[k * kRow + s] : s_z[(k - na) * kRow + s];
             }
             __syncthreads();
-            for (int p = threadIdx.x; p < in * out + out; p += blockDim.x) {
-                float acc = 0.0f;
-                if (p < in * out) {
-                    const int j = p / in, i = p % in;
-                    for (int s = 0; s < gn; ++s) acc = mac(smem[s * stride + in + j], smem[s * stride + i], acc, fused);
-                    atomicAdd(dW + weight_index(c.param_layout, in, out, j, i), acc);
+            continue;
+        }
+        // ---- parameter sums of the tile: a thread takes one output and up to four inputs (the bias rides as one more) ----
+        for (int l = 0; l < nl; ++l) {
+            const int in = c.dims[l], out = c.dims[l + 1];
+            const float* al = smem + net.a_off[l] * kRow;
+            const float* dz = z_rows(l + 1);
+            const int blocks = in / 4 + (in & 3) + 1;   // fours, then the remaining inputs one by one, then the bias
+            for (int item = threadIdx.x; item < out * blocks; item += kSimtThreads) {
+                const int j = item / blocks, b = item - j * blocks;
+                const float* dzj = dz + j * kRow;
+                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                int i0, n;
+                if (b == blocks - 1) {
+                    i0 = in; n = 1;
+                    for (int s = 0; s < n_here; ++s) acc[0] += dzj[s];
+                } else if (b < in / 4) {
+                    i0 = b * 4; n = 4;
+                    // rows past the batch: dz is zero there, a_l need not be finite
+                    if (n_here < kTile) {
+                        for (int s = 0; s < n_here; ++s)
+                            for (int u = 0; u < 4; ++u) acc[u] = mac(dzj[s], al[(i0 + u) * kRow + s], acc[u], fused);
+                    } else
+#pragma unroll
+                    for (int s = 0; s < kTile; s += 4) {
+                        const float4 d = *reinterpret_cast<const float4*>(dzj + s);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const float4 v = *reinterpret_cast<const float4*>(al + (i0 + u) * kRow + s);
+                            acc[u] = mac(d.w, v.w, mac(d.z, v.z, mac(d.y, v.y, mac(d.x, v.x, acc[u], fused), fused), fused), fused);
+                        }
+                    }
                 } else {
-                    const int j = p - in * out;
-                    for (int s = 0; s < gn; ++s) acc += smem[s * stride + in + j];
-                    atomicAdd(dB + j, acc);
+                    i0 = in / 4 * 4 + (b - in / 4); n = 1;
+                    for (int s = 0; s < n_here; ++s) acc[0] = mac(dzj[s], al[i0 * kRow + s], acc[0], fused);
+                }
+                if (!once && map.grads >= 0) {
+                    float* g = smem + map.grads + map.g_off[l] + j * (in + 1) + i0;
+                    for (int u = 0; u < n; ++u) g[u] = tile == blockIdx.x ? acc[u] : g[u] + acc[u];
+                } else if (i0 == in) {
+                    atomicAdd((float*)lp[l].biasesGrad + j, acc[0]);
+                } else {
+                    for (int u = 0; u < n; ++u) atomicAdd((float*)lp[l].weightsGrad + weight_index(c.param_layout, in, out, j, i0 + u), acc[u]);
                 }
             }
+        }
+        __syncthreads();   // the next tile overwrites the rows
+    }
+    if (!seq_scratch && !once && map.grads >= 0) {
+        for (int l = 0; l < nl; ++l) {
+            const int in = c.dims[l], out = c.dims[l + 1];
+            float* dW = (float*)lp[l].weightsGrad;
+            float* dB = (float*)lp[l].biasesGrad;
+            for (int item = threadIdx.x; item < out * (in + 1); item += kSimtThreads) {
+                const int j = item / (in + 1), i = item - j * (in + 1);
+                const float g = smem[map.grads + map.g_off[l] + item];
+                if (i == in) atomicAdd(dB + j, g);
+                else atomicAdd(dW + weight_index(c.param_layout, in, out, j, i), g);
+            }
+        }
+    }
+    // Loss words: the largest per-sample loss, and the sum added once per CTA.
+    if (warp == 0) {
+        for (int o = 16; o > 0; o >>= 1) {
+            run_max = fmaxf(run_max, __shfl_xor_sync(0xffffffffu, run_max, o));
+            run_sum += __shfl_xor_sync(0xffffffffu, run_sum, o);
+        }
+        if (lane == 0) {
+            atomicMax(lossBuffer, __float_as_uint(run_max));
+            atomicAdd((float*)(lossBuffer + 1), run_sum);
         }
     }
 }
@@ -342,28 +531,42 @@ cudaError_t launch_learn_gradient_simt(cudaStream_t st, const MlpConfig& c, cons
     SimtNet net;
     if (!make_simt_net(c, &net, err)) return cudaErrorInvalidValue;
     if (a.count == 0) return cudaSuccess;
-    int max_stride = 0;
-    for (int l = 0; l < c.n_layers; ++l) max_stride = std::max(max_stride, c.dims[l] + c.dims[l + 1]);
-    const int budget = 96 * 1024;
-    int group = budget / (max_stride * 4);
-    group = std::min(256, group / 32 * 32);
-    if (group < 32) {
-        if (err) *err = "layer too wide for the one-thread-per-sample kernel's staging buffer";
-        return cudaErrorInvalidValue;
-    }
-    const size_t smem = size_t(group) * max_stride * 4;
-    {
-        cudaError_t e = cudaFuncSetAttribute(learn_gradient_simt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
-        if (e != cudaSuccess) return e;
-    }
-    const uint32_t grid = (a.count + 255) / 256;
     const bool seq = (a.flags & MLP_FLAG_SEQUENTIAL_SUM) != 0;
-    learn_gradient_simt_kernel<<<grid, 256, smem, st>>>(net, (const MlpLayerPointers*)a.networkBuffer,
-                                                        (uint32_t*)a.lossBuffer, (const void*)a.inputs,
-                                                        (const void*)a.targets, a.count, group,
-                                                        seq ? seq_scratch : nullptr, input_grads);
+    SimtSmem map{};
+    int floats = net.a_off[c.n_layers + 1] * kRow;
+    map.z = floats;
+    floats += (net.a_off[c.n_layers + 1] - net.a_off[1]) * kRow;
+    map.bias = floats;
+    int nb = 0, nw = 0, ng = 0;
+    for (int l = 0; l < c.n_layers; ++l) {
+        map.b_off[l] = nb; nb += c.dims[l + 1];
+        map.w_off[l] = nw; nw += c.dims[l + 1] * ((c.dims[l] + 3) & ~3);
+        map.g_off[l] = ng; ng += c.dims[l + 1] * (c.dims[l] + 1);
+    }
+    floats += (nb + 3) & ~3;
+    // Weights first (every tile reads them twice), then the gradient sums.
+    const int room = int(kSimtSmemMax / 4);
+    map.w = map.grads = -1;
+    if (floats + nw <= room) { map.w = floats; floats += nw; }
+    if (!seq && floats + ng <= room) { map.grads = floats; floats += ng; }
+    map.total = floats;
+    const size_t smem = size_t(floats) * 4;
+    static_assert((2 * kMaxActFloats * kRow + kMaxActFloats + 3) * 4 <= kSimtSmemMax, "the vectors of every accepted network fit");
+    auto kern = map.w >= 0 ? learn_gradient_simt_kernel<true> : learn_gradient_simt_kernel<false>;
+    int device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSimtSmemMax));
+    if (e != cudaSuccess) return e;
+    // As many CTAs as are resident at once (512 threads each), each walking its share of the tiles.
+    const uint32_t tiles = (a.count + kTile - 1) / kTile;
+    const uint32_t per_sm = uint32_t(std::max<size_t>(1, std::min<size_t>(2, kSimtSmemMax / (smem + 1024))));
+    const uint32_t grid = std::min(tiles, per_sm * uint32_t(sms));
+    kern<<<grid, kSimtThreads, smem, st>>>(net, map, (const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer,
+                                           (const void*)a.inputs, (const void*)a.targets, a.count, tiles, seq ? seq_scratch : nullptr,
+                                           input_grads);
     *launches += 1;
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess || !seq) return e;
     for (int l = 0; l < c.n_layers; ++l) {
         const int np = c.dims[l] * c.dims[l + 1] + c.dims[l + 1];
