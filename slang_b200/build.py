@@ -28,7 +28,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
 
 # (object name, source, extra flags).  The one-thread-per-sample kernels must not contract a*b+c into
 # an fma on their own: their fp32 results are compared bit for bit with a sequential CPU.  The padded
-# tensor-core kernel is instantiated some fifty times; its source is compiled in eight parts, the wide
+# tensor-core kernels are instantiated some two hundred times; their source is compiled in ten parts, the wide
 # kernel's in three (training builds, forward-only builds, training builds with the optional outputs).
 UNITS = [
     ("abi", "abi.cu", []),
@@ -43,7 +43,7 @@ UNITS = [
     ("permuto", "permuto.cu", ["-fmad=false"]),
     ("selftest", "selftest.cu", []),
     ("tile_mma", "tile_mma.cu", []),
-] + [("tc_train_narrow_%d" % i, "tc_train_narrow.cu", ["-DMLPB200_NARROW_PART=%d" % i]) for i in range(8)]
+] + [("tc_narrow_%d" % i, "tc_narrow.cu", ["-DMLPB200_NARROW_PART=%d" % i]) for i in range(10)]
 
 
 def _nvcc():
