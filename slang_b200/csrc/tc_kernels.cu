@@ -82,8 +82,14 @@ constexpr uint32_t kLossPart = kBias + 5 * 128 * 4;  // fp32 [8 feature groups][
 constexpr uint32_t kBars = kLossPart + 8 * 64 * 4;   // mbarriers: x_full[2], t_full, acc_full[2], acc_free[2], out_full, out_free
 constexpr uint32_t kTmemPtr = kBars + 12 * 8;
 constexpr uint32_t kAbort = kTmemPtr + 4;
-constexpr uint32_t kSmemBytes = kAbort + 4;   // the dynamic shared-memory base must be 1024-byte aligned (checked at run time)
+constexpr uint32_t kNet = (kAbort + 4 + 15u) & ~15u;   // MlpLayerPointers [5]
+constexpr uint32_t kSmemBytes = kNet + 5 * 32;   // the dynamic shared-memory base must be 1024-byte aligned (checked at run time)
 static_assert(kSmemBytes <= 232448, "shared-memory map exceeds the per-CTA limit");
+
+// The gradients on their way out, over the operand buffers: rows padded by 16 bytes, so that eight lanes' 16-byte
+// stores down a column of rows meet distinct banks.
+constexpr uint32_t kOutRow = H + 4, kOutRow0 = D0 + 4;   // floats
+static_assert(3 * H * kOutRow * 4 <= kBias, "three layers of outgoing gradients fit the operand buffers");
 
 // Tensor-memory columns.
 constexpr uint32_t kColDW1 = 0, kColDW4T = 384, kColAcc = 448, kTmemCols = 512;
@@ -203,6 +209,85 @@ struct WideTrainParams {
     unsigned long long* timing;  // trace builds only: time stamps written by CTA 0
 };
 
+// Adds the CTA's weight gradients: dW_0 from shared memory, where the epilogue threads have put their sums, the others from
+// their accumulators.  An accumulator holds a parameter row per lane: written out from there every reduction touched 32
+// rows.  The rows go through shared memory (the operand buffers, free by now) and leave as consecutive 16-byte
+// reductions (42.1 to 32.8 us a step of 20011 samples through 32-128-128-3).  A function of its own, called by the 512
+// epilogue threads: inlined, it took registers from the tile loop (60.2 to 63.9 ms at 2^26 samples).
+template <int NL, bool XTRA>
+__device__ __noinline__ void wide_write_out(const WideTrainParams& p, bool ok)
+{
+    using namespace wide;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = smem_raw;
+    const uint32_t tmem_base = *(volatile uint32_t*)(smem + kTmemPtr);
+    constexpr int kEpiThreads = 32 * kEpiWarps;
+    const int t = (int)threadIdx.x - 64, warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+    const int q = warp & 3, e = (warp - 2) >> 2, f = q * 32 + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
+    const MlpLayerPointers* net = (const MlpLayerPointers*)(smem + kNet);
+    volatile uint32_t* abort_flag = (volatile uint32_t*)(smem + kAbort);
+    // rows [out][in] at `s` (`stride` floats apart) into the gradients, in the layout the parameters have
+    auto add_rows = [&](const float* s, int stride, int in, int out, float* g) {
+        if (XTRA && p.param_layout != MLP_PARAMS_ROW_MAJOR) {
+            // tiled parameters: the gradient of weight (o, i) goes where the weight itself lies
+            for (int i = t; i < out * in; i += kEpiThreads) {
+                const int o = i / in, k = i - o * in;
+                atomicAdd(g + weight_index(p.param_layout, in, out, o, k), s[o * stride + k]);
+            }
+        } else if ((in & 3) == 0) {
+            const int n = in >> 2;   // four parameters per reduction (16-byte aligned: rows are multiples of 16 bytes)
+            for (int i = t; i < out * n; i += kEpiThreads) {
+                const int o = i / n, k = i - o * n;
+                atomicAdd((float4*)g + i, *(const float4*)(s + o * stride + 4 * k));
+            }
+        } else {
+            for (int i = t; i < out * in; i += kEpiThreads) {
+                const int o = i / in, k = i - o * in;
+                atomicAdd(g + i, s[o * stride + k]);
+            }
+        }
+    };
+    tc_fence_after();
+    named_bar_sync(1, kEpiThreads);
+    ok = ok && !*abort_flag;
+    if (ok) {
+        add_rows((const float*)smem, kOutRow0, p.dims[0], p.dims[1], (float*)net[0].weightsGrad);
+        // dW of the output layer, transposed: lane = input feature, column = output feature: consecutive as it stands
+        const int in = p.dims[NL - 1], out = p.dims[NL];
+        float* dW = (float*)net[NL - 1].weightsGrad;
+        uint32_t v[16];
+        tmem_ld_cols(lane_base + kColDW4T + (uint32_t)(e * 16), v);
+        tmem_ld_wait();
+        if (f < in) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (e * 16 + i < out) atomicAdd(dW + (XTRA ? weight_index(p.param_layout, in, out, e * 16 + i, f) : (int64_t)(e * 16 + i) * in + f), __uint_as_float(v[i]));
+        }
+    }
+    if constexpr (NL > 2) {
+        named_bar_sync(1, kEpiThreads);
+        if (ok) {
+#pragma unroll
+            for (int l = 1; l <= NL - 2; ++l) {
+                uint32_t v[32];
+                tmem_ld_cols(lane_base + kColDW1 + (uint32_t)(l - 1) * 128u + (uint32_t)(e * 32), v);
+                tmem_ld_wait();
+                float4* row = (float4*)((float*)smem + ((l - 1) * H + f) * kOutRow + e * 32);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    row[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+            }
+        }
+        named_bar_sync(1, kEpiThreads);
+        if (ok) {
+#pragma unroll 1
+            for (int l = 1; l <= NL - 2; ++l)
+                add_rows((const float*)smem + (l - 1) * H * kOutRow, kOutRow, p.dims[l], p.dims[l + 1], (float*)net[l].weightsGrad);
+        }
+    }
+}
+
 // FWD builds stop after the output layer and write the network outputs (the "forward" entry point of the same
 // shapes): no targets, no derivatives, no gradient products.
 // F32S: fp32 parameter storage with 16-bit operands (weights converted while they are staged, pre-activations and
@@ -213,7 +298,7 @@ struct WideTrainParams {
 template <int FMT, int ACT, int NL, bool FWD, bool F32S = false, bool XTRA = false>
 __global__ void __launch_bounds__(wide::kThreads, 1)
 learn_gradient_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_t,
-                           const WideTrainParams p)
+                           const __grid_constant__ WideTrainParams p)
 {
     using namespace wide;
     using E = Elem<FMT>;
@@ -259,6 +344,8 @@ learn_gradient_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
         tmem_alloc(tmem_ptr, kTmemCols);
         tmem_relinquish();
     }
+    MlpLayerPointers* s_net = (MlpLayerPointers*)(smem + kNet);   // the layers' addresses, for the write-out
+    if (threadIdx.x < NL * 4) ((uint64_t*)s_net)[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
     for (int l = 0; l < NL; ++l) {
         // Real widths in x out, padded to inp x outp with zeros (padded rows, columns and biases are zero, so
         // padded features carry no signal forward and receive no gradient).
@@ -866,77 +953,13 @@ learn_gradient_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
 
         // ---- one add per parameter per CTA ----
         if (!FWD && ok && !*abort_flag && n_my_tiles > 0) {
-            tc_fence_after();
-            // Only real rows and columns leave; the gradients are row-major [out][in] with the network's own widths.
-#pragma unroll
-            for (int l = 1; l <= NL - 2; ++l) {
-                const int in = p.dims[l], out = p.dims[l + 1];
-                float* dW = (float*)p.net[l].weightsGrad + (size_t)f * in;
-                const int col = e * 32;
-                uint32_t v[32];
-                tmem_ld_cols(lane_base + kColDW1 + (uint32_t)(l - 1) * 128u + (uint32_t)col, v);
-                tmem_ld_wait();
-                if (f < out) {
-                    if (XTRA && p.param_layout != MLP_PARAMS_ROW_MAJOR) {
-                        // tiled parameters: the gradient of weight (f, i) goes where the weight itself lies
-                        float* gW = (float*)p.net[l].weightsGrad;
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col + i < in) atomicAdd(gW + weight_index(p.param_layout, in, out, f, col + i), __uint_as_float(v[i]));
-                    } else if ((in & 3) == 0) {
-                        // four parameters per reduction (16-byte aligned: rows are multiples of 16 bytes)
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            if (col + i < in)
-                                atomicAdd((float4*)(dW + col + i), make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]),
-                                                                               __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col + i < in) atomicAdd(dW + col + i, __uint_as_float(v[i]));
-                    }
-                }
-            }
-            {
-                // dW of the output layer, transposed: lane = input feature, column = output feature.
-                const int in = p.dims[NL - 1], out = p.dims[NL];
-                float* dW = (float*)p.net[NL - 1].weightsGrad;
-                uint32_t v[16];
-                tmem_ld_cols(lane_base + kColDW4T + (uint32_t)(e * 16), v);
-                tmem_ld_wait();
-                if (f < in) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (e * 16 + i < out) atomicAdd(dW + (XTRA ? weight_index(p.param_layout, in, out, e * 16 + i, f) : (int64_t)(e * 16 + i) * in + f), __uint_as_float(v[i]));
-                }
-            }
-            {
-                const int in = p.dims[0], out = p.dims[1];
-                float* dW = (float*)p.net[0].weightsGrad + (size_t)f * in + e * 16;
-                if (f < out) {
-                    if (XTRA && p.param_layout != MLP_PARAMS_ROW_MAJOR) {
-                        float* gW = (float*)p.net[0].weightsGrad;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (e * 16 + i < in) atomicAdd(gW + weight_index(p.param_layout, in, out, f, e * 16 + i), dw0[i]);
-                    } else if ((in & 3) == 0) {
-#pragma unroll
-                        for (int i = 0; i < 16; i += 4)
-                            if (e * 16 + i < in) atomicAdd((float4*)(dW + i), make_float4(dw0[i], dw0[i + 1], dw0[i + 2], dw0[i + 3]));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (e * 16 + i < in) atomicAdd(dW + i, dw0[i]);
-                    }
-                }
-            }
 #pragma unroll
             for (int l = 0; l < NL - 1; ++l)
-                if (f < p.dims[l + 1]) atomicAdd((float*)p.net[l].biasesGrad + f, db[l]);
+                if (f < p.dims[l + 1]) atomicAdd((float*)s_net[l].biasesGrad + f, db[l]);
             if ((lane & 3) == 0) {
                 const int j = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
                 const int feat = (q >> 1) * 32 + e * 8 + j;
-                if (feat < p.dims[NL]) atomicAdd((float*)p.net[NL - 1].biasesGrad + feat, db_out);
+                if (feat < p.dims[NL]) atomicAdd((float*)s_net[NL - 1].biasesGrad + feat, db_out);
             }
             if (e == 0 && q < 2) {
                 float mx = run_max, tot = run_sum;
@@ -951,13 +974,22 @@ learn_gradient_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
                 }
             }
         }
+        if constexpr (!FWD) {
+            const bool out_ok = ok && n_my_tiles > 0;
+            if (out_ok) {   // every product has completed: dW_0 was the last
+                float4* row = (float4*)((float*)smem + f * kOutRow0 + e * 16);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) row[i] = make_float4(dw0[4 * i], dw0[4 * i + 1], dw0[4 * i + 2], dw0[4 * i + 3]);
+            }
+            wide_write_out<NL, XTRA>(p, out_ok);   // last: nothing lives across the call
+        }
     }
 
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, wide::kTmemCols);
+        tmem_dealloc(*(volatile uint32_t*)tmem_ptr, wide::kTmemCols);
     }
 }
 
