@@ -451,28 +451,52 @@ sequential_sum_kernel(SimtNet net, const MlpLayerPointers* __restrict__ lp, cons
 
 // adjustParameters, fp32 state (examples/mlp-training/adam.slang:21-37 widened to float):
 // NaN gradient -> zero it and skip; +-inf -> +-10000; eps inside the square root; gradient zeroed.
+// A thread takes E elements a block apart, their loads issued together, and takes the bias corrections, two powers by
+// squaring, once for elements of the same iteration (nearly always all of them).  Bound: HBM at E = 4.
+template <int E>
 __global__ void __launch_bounds__(256)
-adjust_parameters_kernel(MlpConfig c, MlpAdamState* __restrict__ states, void* __restrict__ params,
+adjust_parameters_kernel(const __grid_constant__ MlpConfig c, MlpAdamState* __restrict__ states, void* __restrict__ params,
                          float* __restrict__ grads, uint32_t count)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float g = grads[i];
-    if (isnan(g)) { grads[i] = 0.0f; return; }
-    float4 raw = reinterpret_cast<float4*>(states)[i];
-    float mean = raw.x, var = raw.y;
-    int32_t it = __float_as_int(raw.z) + 1;
-    if (isinf(g)) g = g > 0.0f ? 10000.0f : -10000.0f;
-    mean = c.beta1 * mean + (1.0f - c.beta1) * g;
-    var = c.beta2 * var + ((1.0f - c.beta2) * g) * g;
-    const float mean_hat = __fdiv_rn(mean, 1.0f - pow_int(c.beta1, it));
-    const float var_hat = __fdiv_rn(var, 1.0f - pow_int(c.beta2, it));
-    float p = c.adam_master ? raw.w : load_as_f32(c.dtype, params, i);
-    const float denom = __fsqrt_rn(fmaxf(0.0f, var_hat) + c.eps);
-    p = p - __fdiv_rn(c.lr * mean_hat, denom);
-    reinterpret_cast<float4*>(states)[i] = make_float4(mean, var, __int_as_float(it), p);
-    store_from_f32(c.dtype, params, i, p);
-    grads[i] = 0.0f;
+    const uint32_t first = blockIdx.x * (256u * E) + threadIdx.x;
+    float g[E], p[E];
+    float4 raw[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const uint32_t i = first + 256u * k;
+        g[k] = __int_as_float(0x7fffffff);
+        if (i < count) {
+            g[k] = grads[i];
+            raw[k] = __ldcs(reinterpret_cast<const float4*>(states) + i);
+            p[k] = c.adam_master ? raw[k].w : load_as_f32(c.dtype, params, i);
+        }
+    }
+    int32_t known = -1;
+    float c1 = 0.0f, c2 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const uint32_t i = first + 256u * k;
+        if (i >= count) break;
+        grads[i] = 0.0f;
+        float gk = g[k];
+        if (isnan(gk)) continue;
+        float mean = raw[k].x, var = raw[k].y;
+        const int32_t it = __float_as_int(raw[k].z) + 1;
+        if (isinf(gk)) gk = gk > 0.0f ? 10000.0f : -10000.0f;
+        mean = c.beta1 * mean + (1.0f - c.beta1) * gk;
+        var = c.beta2 * var + ((1.0f - c.beta2) * gk) * gk;
+        if (k == 0 || it != known) {
+            known = it;
+            c1 = 1.0f - pow_int(c.beta1, it);
+            c2 = 1.0f - pow_int(c.beta2, it);
+        }
+        const float mean_hat = __fdiv_rn(mean, c1);
+        const float var_hat = __fdiv_rn(var, c2);
+        const float denom = __fsqrt_rn(fmaxf(0.0f, var_hat) + c.eps);
+        const float v = p[k] - __fdiv_rn(c.lr * mean_hat, denom);
+        __stcs(reinterpret_cast<float4*>(states) + i, make_float4(mean, var, __int_as_float(it), v));
+        store_from_f32(c.dtype, params, i, v);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -587,8 +611,12 @@ size_t sequential_scratch_floats_per_sample(const MlpConfig& c)
 cudaError_t launch_adjust_parameters(cudaStream_t st, const MlpConfig& c, const MlpAdjustParamsParams& a, int* launches)
 {
     if (a.count == 0) return cudaSuccess;
-    adjust_parameters_kernel<<<(a.count + 255) / 256, 256, 0, st>>>(c, (MlpAdamState*)a.adamStates, (void*)a.params,
-                                                                   (float*)a.gradients, a.count);
+    // Four elements a thread once that still leaves every SM eight blocks of 256 (an encoder's table); one below, where the
+    // launch is all there is (a network's parameters).
+    constexpr uint32_t kMany = 148u * 8u * 1024u;
+    MlpAdamState* states = (MlpAdamState*)a.adamStates;
+    if (a.count >= kMany) adjust_parameters_kernel<4><<<(a.count + 1023) / 1024, 256, 0, st>>>(c, states, (void*)a.params, (float*)a.gradients, a.count);
+    else adjust_parameters_kernel<1><<<(a.count + 255) / 256, 256, 0, st>>>(c, states, (void*)a.params, (float*)a.gradients, a.count);
     *launches += 1;
     return cudaGetLastError();
 }
