@@ -11,6 +11,9 @@ import torch
 
 from . import config as C
 
+# Bytes of inputs and targets from which a piece's copy runs at the link's rate (its launch is lost in it).
+_PIECE_BYTES = 8 << 20
+
 _TORCH_DTYPE = {C.F32: torch.float32, C.F16: torch.float16, C.BF16: torch.bfloat16}
 
 
@@ -52,10 +55,15 @@ class HostStepper:
         self.h2d_bytes = x_host.numel() * x_host.element_size()
         if self.teacher is None:
             self.h2d_bytes += t_host.numel() * t_host.element_size()
-        n_chunks = (count + self.chunk - 1) // self.chunk
+        # What runs after the last copy has arrived is one piece's kernels, so a batch that would fit a few pieces is cut
+        # into up to sixteen: a step of 2^20 samples of 256 bytes waits for 1/16 of its kernels instead of all of them.
+        per_sample = self.h2d_bytes // max(count, 1)
+        piece = max(-(-count // 16), _PIECE_BYTES // max(per_sample, 1), 1)
+        piece = min(self.chunk, (piece + 127) // 128 * 128)   # whole tiles
+        n_chunks = (count + piece - 1) // piece
         for i in range(n_chunks):
             b = i & 1
-            i0, i1 = i * self.chunk, min(count, (i + 1) * self.chunk)
+            i0, i1 = i * piece, min(count, (i + 1) * piece)
             n = i1 - i0
             if i >= 2:
                 self.copy_stream.wait_event(self.compute_done[b])
