@@ -1,0 +1,33 @@
+// Launches that overlap the end of the kernel before them on the stream (programmatic dependent launch).
+//
+// A kernel launched with launch_after() may start while its predecessor is still running, so it calls grid_wait() before
+// its first access to global memory; that returns when the predecessor has completed and its writes are visible.  Because
+// every such kernel waits before it completes, completion stays in stream order.  grid_release() lets the successor's
+// blocks start as soon as every block of this kernel has been placed; they hold no work back, they only wait.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace mlpb200 {
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_after(cudaStream_t st, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+}  // namespace mlpb200

@@ -24,6 +24,7 @@
 
 #include <string>
 
+#include "launch_pdl.cuh"
 #include "launchers.h"
 #include "mlp_common.cuh"
 #include "tc_host.h"
@@ -158,35 +159,61 @@ forward_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         prefetch_tmap(&tmap_x);
         prefetch_tmap(&tmap_out);
     }
+    grid_release();
+    grid_wait();
+    if (threadIdx.x == 0) {
+        // the chains' first tiles: on their way while the weights are staged
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            if ((uint32_t)c < n_my_tiles) {
+                const uint32_t tile = blockIdx.x + (uint32_t)c * gridDim.x;
+                mbar_expect_tx(&x_full[c], kXBytes);
+#pragma unroll
+                for (int pn = 0; pn < DIN / panel_w(DIN); ++pn)
+                    tma_load_2d(smem + G::kAct + c * G::kActBytes + pn * (128 * row_bytes(DIN)), &tmap_x, pn * panel_w(DIN),
+                                (int32_t)(tile * 128u), &x_full[c]);
+            }
+        }
+    }
     if (warp == 1) {
         tmem_alloc(tmem_ptr, G::kTmemCols);
         tmem_relinquish();
     }
-    // Weights into shared memory, row-major rows re-cut into swizzled panels; biases as fp32.
+    // Weights into shared memory, row-major rows re-cut into swizzled panels; biases as fp32.  Every layer's addresses are
+    // read at once and every layer's copies are in flight together: one layer after the other, each behind its own
+    // dependent reads, was most of the time of a call of a thousand samples.
+    uint64_t w_addr[NL], b_addr[NL];
+#pragma unroll
+    for (int l = 0; l < NL; ++l) { w_addr[l] = p.net[l].weights; b_addr[l] = p.net[l].biases; }
+#pragma unroll
     for (int l = 0; l < NL; ++l) {
         const int in = G::in_dim(l), out = G::out_dim(l);
-        const uint4* src = (const uint4*)p.net[l].weights;
-        const uint16_t* src16 = (const uint16_t*)p.net[l].weights;
+        const uint4* src = (const uint4*)w_addr[l];
+        const uint16_t* src16 = (const uint16_t*)w_addr[l];
         const int cpr = in / 8;
         for (int idx = threadIdx.x; idx < out * cpr; idx += G::kThreads) {
             const int o = idx / cpr, j = idx % cpr;
-            const uint32_t off = (l == 0) ? chunk_offset<DIN>(out, o, j) : chunk_offset<DH>(out, o, j);
-            uint4 v;
+            const uint32_t off = G::w_off(l) + ((l == 0) ? chunk_offset<DIN>(out, o, j) : chunk_offset<DH>(out, o, j));
             if (p.param_layout == MLP_PARAMS_ROW_MAJOR) {
-                v = src[idx];
+                cp_async_16(sbase + off, src + idx);
             } else {
                 // OptimalLayout: the eight inputs of a chunk are four pairs inside one 16x16 tile
                 uint16_t hw[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) hw[e] = src16[weight_index(MLP_PARAMS_OPTIMAL, in, out, o, j * 8 + e)];
-                v = make_uint4(hw[0] | ((uint32_t)hw[1] << 16), hw[2] | ((uint32_t)hw[3] << 16), hw[4] | ((uint32_t)hw[5] << 16),
-                               hw[6] | ((uint32_t)hw[7] << 16));
+                *(uint4*)(smem + off) = make_uint4(hw[0] | ((uint32_t)hw[1] << 16), hw[2] | ((uint32_t)hw[3] << 16), hw[4] | ((uint32_t)hw[5] << 16),
+                                                   hw[6] | ((uint32_t)hw[7] << 16));
             }
-            *(uint4*)(smem + G::w_off(l) + off) = v;
         }
-        for (int j = threadIdx.x; j < 128; j += G::kThreads)
-            s_bias[l * 128 + j] = j < out ? load_as_f32(FMT, (const void*)p.net[l].biases, j) : 0.0f;
     }
+    for (int idx = threadIdx.x; idx < NL * 128; idx += G::kThreads) {
+        const int l = idx >> 7, j = idx & 127;
+        uint64_t b = 0;
+#pragma unroll
+        for (int i = 0; i < NL; ++i) b = i == l ? b_addr[i] : b;
+        s_bias[idx] = j < G::out_dim(l) ? load_as_f32(FMT, (const void*)b, j) : 0.0f;
+    }
+    cp_async_wait_all();
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -208,19 +235,6 @@ forward_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             uint32_t steps[NCH];  // products issued so far per chain
 #pragma unroll
             for (int c = 0; c < NCH; ++c) steps[c] = 0;
-            if (leader) {
-#pragma unroll
-                for (int c = 0; c < NCH; ++c) {
-                    if (c % NCW == cw && (uint32_t)c < n_my_tiles) {
-                        const uint32_t tile = blockIdx.x + (uint32_t)c * gridDim.x;
-                        mbar_expect_tx(&x_full[c], kXBytes);
-#pragma unroll
-                        for (int pn = 0; pn < DIN / panel_w(DIN); ++pn)
-                            tma_load_2d(smem + G::kAct + c * G::kActBytes + pn * (128 * row_bytes(DIN)), &tmap_x, pn * panel_w(DIN),
-                                        (int32_t)(tile * 128u), &x_full[c]);
-                    }
-                }
-            }
             const uint32_t rounds = (n_my_tiles + NCH - 1) / NCH;
             for (uint32_t j = 0; j < rounds && ok; ++j) {
 #pragma unroll
@@ -463,8 +477,7 @@ static cudaError_t launch_fwd(cudaStream_t st, TcWorkspace* ws, const MlpConfig&
     if (e != cudaSuccess) return e;
     const uint32_t slots = (uint32_t)ws->sm_count * (uint32_t)CPS;
     const uint32_t grid = p.n_tiles < slots ? p.n_tiles : slots;
-    kern<<<grid, G::kThreads, G::kSmemBytes, st>>>(mx, mo, p);
-    return cudaGetLastError();
+    return launch_after(st, kern, grid, G::kThreads, G::kSmemBytes, mx, mo, p);
 }
 
 cudaError_t launch_forward_tc(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpForwardParams& a, int* launches,

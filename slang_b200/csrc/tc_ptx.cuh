@@ -88,6 +88,13 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity)
 
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// 16 bytes from global to shared memory without passing through registers.
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // 2-D tiled TMA load into this CTA's shared memory, completion counted in bytes on an mbarrier.
 // A plain per-CTA load: every CTA fetches its own tile.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int32_t c0, int32_t c1, uint64_t* bar)
