@@ -13,6 +13,7 @@
 #include <string>
 
 #include "mlp_common.cuh"
+#include "launch_pdl.cuh"
 #include "launchers.h"
 
 #include "example_kernels.cuh"
@@ -222,6 +223,8 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
     const int od = c.dims[nl];
     const bool fused = c.sum_order == MLP_SUM_BIAS_FIRST_FUSED;
     const int opd = operand_type(c);
+    grid_release();
+    grid_wait();
     const bool once = gridDim.x == n_tiles;       // one tile per CTA: its sums leave directly
     float* const s_z = smem + map.z;              // z rows, later dz: layer l's outputs from row a_off[l + 1] - a_off[1]
     auto z_rows = [&](int l) { return s_z + (net.a_off[l] - net.a_off[1]) * kRow; };   // of the vector leaving layer l - 1
@@ -459,6 +462,8 @@ adjust_parameters_kernel(const __grid_constant__ MlpConfig c, MlpAdamState* __re
                          float* __restrict__ grads, uint32_t count)
 {
     const uint32_t first = blockIdx.x * (256u * E) + threadIdx.x;
+    grid_release();
+    grid_wait();
     float g[E], p[E];
     float4 raw[E];
 #pragma unroll
@@ -586,11 +591,9 @@ cudaError_t launch_learn_gradient_simt(cudaStream_t st, const MlpConfig& c, cons
     const uint32_t tiles = (a.count + kTile - 1) / kTile;
     const uint32_t per_sm = uint32_t(std::max<size_t>(1, std::min<size_t>(2, kSimtSmemMax / (smem + 1024))));
     const uint32_t grid = std::min(tiles, per_sm * uint32_t(sms));
-    kern<<<grid, kSimtThreads, smem, st>>>(net, map, (const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer,
-                                           (const void*)a.inputs, (const void*)a.targets, a.count, tiles, seq ? seq_scratch : nullptr,
-                                           input_grads);
+    e = launch_after(st, kern, grid, kSimtThreads, smem, net, map, (const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer,
+                     (const void*)a.inputs, (const void*)a.targets, a.count, tiles, seq ? seq_scratch : nullptr, input_grads);
     *launches += 1;
-    e = cudaGetLastError();
     if (e != cudaSuccess || !seq) return e;
     for (int l = 0; l < c.n_layers; ++l) {
         const int np = c.dims[l] * c.dims[l + 1] + c.dims[l + 1];
@@ -615,10 +618,11 @@ cudaError_t launch_adjust_parameters(cudaStream_t st, const MlpConfig& c, const 
     // launch is all there is (a network's parameters).
     constexpr uint32_t kMany = 148u * 8u * 1024u;
     MlpAdamState* states = (MlpAdamState*)a.adamStates;
-    if (a.count >= kMany) adjust_parameters_kernel<4><<<(a.count + 1023) / 1024, 256, 0, st>>>(c, states, (void*)a.params, (float*)a.gradients, a.count);
-    else adjust_parameters_kernel<1><<<(a.count + 255) / 256, 256, 0, st>>>(c, states, (void*)a.params, (float*)a.gradients, a.count);
+    const cudaError_t e = a.count >= kMany
+        ? launch_after(st, adjust_parameters_kernel<4>, (a.count + 1023) / 1024, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count)
+        : launch_after(st, adjust_parameters_kernel<1>, (a.count + 255) / 256, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count);
     *launches += 1;
-    return cudaGetLastError();
+    return e;
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -23,6 +23,7 @@
 #include <string>
 #include <type_traits>
 
+#include "launch_pdl.cuh"
 #include "launchers.h"
 #include "tc_host.h"
 #include "tc_narrow.cuh"
@@ -64,7 +65,8 @@ struct TrainMap {
     static constexpr uint32_t kBars = kLoss + kWarps * 8;                // full and empty [group][slot], done
     static constexpr uint32_t kTmemPtr = kBars + (2 * NG * kNumSlots + 1) * 8;
     static constexpr uint32_t kAbort = kTmemPtr + 4;
-    static constexpr uint32_t kSmemBytes = kAbort + 4 + 1024;
+    static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;           // MlpLayerPointers [NL]
+    static constexpr uint32_t kSmemBytes = kNet + NL * 32 + 1024;
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
     // tensor memory: W + 16 columns per layer (dW_l, then db_l)
     static constexpr uint32_t kDwCols = W + 16;
@@ -116,21 +118,34 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
             ((uint32_t*)(smem + M::kOnes))[i] = (word >> 2) == (row & 7) && (word & 3) == 0 ? (C::kOnes & 0xffffu) : 0u;
         }
     }
-#pragma unroll 1
-    for (int l = 0; l < NL; ++l) {
-        const int in = cfg.dims[l], out = cfg.dims[l + 1];
-        const MlpLayerPointers ptr = p.net[l];
-        const int ki = l == 0 ? ikind : kEights, ko = l == NL - 1 ? okind : kEights;
-        const int nt = l == NL - 1 ? OT : NT;
-        stage_panel<FMT>(smem + M::kForward + l * M::kPanel, cfg, ptr, in, out, ki, ko, false, M::kQ, nt, threadIdx.x, kThreads);
-        if (l > 0 || p.input_grads)
-            stage_panel<FMT>(smem + M::kReverse + l * M::kPanel, cfg, ptr, in, out, ki, ko, true, l == NL - 1 ? (OK + 1) / 2 : M::kQ, NT, threadIdx.x, kThreads);
-        for (int j = threadIdx.x; j < nt * 8; j += kThreads) {
-            const int f = feature_of(ko, j >> 3, j & 7);
-            // features past the real width: below zero for ReLU, so that no derivative there is the one at zero
-            float* b = (float*)(smem + M::kBias) + l * W * 2 + (j >> 1) * 4 + (j & 1);
-            b[0] = b[2] = f < out ? load_as_f32(cfg.dtype, (const void*)ptr.biases, f) : (HACT == MLP_ACT_RELU && l < NL - 1 ? -1.0f : 0.0f);
-        }
+    grid_release();
+    grid_wait();
+    const MlpLayerPointers* s_net = (const MlpLayerPointers*)(smem + M::kNet);
+    if (threadIdx.x < NL * 4) ((uint64_t*)(smem + M::kNet))[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
+    __syncthreads();
+    // forward panels, then reverse panels from the last layer down (layer 0's only for the input gradients)
+    stage_panels<FMT, M::kQ * NT * 32>(smem, cfg, p.input_grads ? 2 * NL : 2 * NL - 1, [&](int which, int* chunks) {
+        const bool rev = which >= NL;
+        const int l = rev ? 2 * NL - 1 - which : which;
+        const bool last = l == NL - 1;
+        Panel d;
+        d.weights = (const void*)s_net[l].weights;
+        d.in = cfg.dims[l]; d.out = cfg.dims[l + 1];
+        d.in_kind = l == 0 ? ikind : kEights;
+        d.out_kind = last ? okind : kEights;
+        d.transposed = rev;
+        d.tiles = !rev && last ? OT : NT;
+        d.dst = (rev ? M::kReverse : M::kForward) + (uint32_t)l * M::kPanel;
+        *chunks = (rev && last ? (OK + 1) / 2 : M::kQ) * d.tiles * 32;
+        return d;
+    }, threadIdx.x, kThreads);
+    for (int i = threadIdx.x; i < NL * W; i += kThreads) {
+        const int l = i / W, j = i % W;
+        if (l == NL - 1 && j >= OT * 8) continue;
+        // features past the real width: below zero for ReLU, so that no derivative there is the one at zero
+        const int f = feature_of(l == NL - 1 ? okind : kEights, j >> 3, j & 7);
+        float* b = (float*)(smem + M::kBias) + l * W * 2 + (j >> 1) * 4 + (j & 1);
+        b[0] = b[2] = f < cfg.dims[l + 1] ? load_as_f32(cfg.dtype, (const void*)s_net[l].biases, f) : (HACT == MLP_ACT_RELU && l < NL - 1 ? -1.0f : 0.0f);
     }
     fence_async_smem();
     tc_fence_before();
@@ -565,8 +580,8 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
         for (int l = 0; l < NL; ++l) {
             const int in = cfg.dims[l], out = cfg.dims[l + 1];
             const int ki = l == 0 ? ikind : kEights, ko = l == NL - 1 ? okind : kEights;
-            float* dW = (float*)p.net[l].weightsGrad;
-            float* dB = (float*)p.net[l].biasesGrad;
+            float* dW = (float*)s_net[l].weightsGrad;
+            float* dB = (float*)s_net[l].biasesGrad;
             for (int i = threadIdx.x; i < W * (W + 1); i += kThreads) {
                 // position -> feature, in rows and columns
                 const int r = i / (W + 1), k = i - r * (W + 1);
@@ -603,7 +618,7 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
     constexpr int NT = W / 8, KS = W / 16, kQ = (W + 31) / 32;
     constexpr int HK = tile_kind(NT);                    // how hidden vectors are dealt to the lanes
     constexpr uint32_t kPanel = kQ * NT * 512;
-    extern __shared__ __align__(128) uint8_t smem[];     // [n_layers] panels, then fp32 biases [n_layers][W / 2 pairs][twice]
+    extern __shared__ __align__(128) uint8_t smem[];     // [n_layers] panels, then fp32 biases [n_layers][W / 2 pairs][twice], addresses
     const uint32_t sbase = smem_u32(smem);
     const MlpConfig& cfg = p.cfg;
     const int nl = cfg.n_layers, od = cfg.dims[nl];
@@ -612,18 +627,29 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
     const int ikind = input_kind(cfg.dims[0]);
     constexpr int okind = tile_kind(OT);
     float* s_bias_w = (float*)(smem + (uint32_t)nl * kPanel);
-#pragma unroll 1
-    for (int l = 0; l < nl; ++l) {
-        const int in = cfg.dims[l], out = cfg.dims[l + 1];
-        const MlpLayerPointers ptr = p.net[l];
-        const int ki = l == 0 ? ikind : HK, ko = l == nl - 1 ? okind : HK;
-        const int nt = l == nl - 1 ? OT : NT;
-        stage_panel<FMT>(smem + (uint32_t)l * kPanel, cfg, ptr, in, out, ki, ko, false, kQ, nt, threadIdx.x, 32 * kForwardWarps);
-        for (int j = threadIdx.x; j < nt * 8; j += 32 * kForwardWarps) {
-            const int f = feature_of(ko, j >> 3, j & 7);
-            float* b = s_bias_w + l * W * 2 + (j >> 1) * 4 + (j & 1);
-            b[0] = b[2] = f < out ? load_as_f32(cfg.dtype, (const void*)ptr.biases, f) : 0.0f;
-        }
+    MlpLayerPointers* s_net = (MlpLayerPointers*)(s_bias_w + nl * W * 2);
+    grid_release();
+    grid_wait();
+    if (threadIdx.x < nl * 4) ((uint64_t*)s_net)[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
+    __syncthreads();
+    stage_panels<FMT, kQ * NT * 32>(smem, cfg, nl, [&](int l, int* chunks) {
+        Panel d;
+        d.weights = (const void*)s_net[l].weights;
+        d.in = cfg.dims[l]; d.out = cfg.dims[l + 1];
+        d.in_kind = l == 0 ? ikind : HK;
+        d.out_kind = l == nl - 1 ? okind : HK;
+        d.transposed = false;
+        d.tiles = l == nl - 1 ? OT : NT;
+        d.dst = (uint32_t)l * kPanel;
+        *chunks = kQ * d.tiles * 32;
+        return d;
+    }, threadIdx.x, 32 * kForwardWarps);
+    for (int i = threadIdx.x; i < nl * W; i += 32 * kForwardWarps) {
+        const int l = i / W, j = i % W;
+        if (l == nl - 1 && j >= OT * 8) continue;
+        const int f = feature_of(l == nl - 1 ? okind : HK, j >> 3, j & 7);
+        float* b = s_bias_w + l * W * 2 + (j >> 1) * 4 + (j & 1);
+        b[0] = b[2] = f < cfg.dims[l + 1] ? load_as_f32(cfg.dtype, (const void*)s_net[l].biases, f) : 0.0f;
     }
     __syncthreads();
     const uint32_t panel0 = sbase + (uint32_t)lane * 16u;
@@ -751,8 +777,7 @@ static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params
     if (e != cudaSuccess) return e;
     p.n_tiles = (uint32_t)(((uint64_t)p.count + M::kRows - 1) / M::kRows);
     const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
-    kern<<<grid, M::kThreads, M::kSmemBytes, st>>>(p);
-    return cudaGetLastError();
+    return launch_after(st, kern, grid, M::kThreads, M::kSmemBytes, p);
 }
 
 template <int W, int NL, int FMT, int OT>
@@ -783,14 +808,13 @@ static cudaError_t launch_forward(cudaStream_t st, TcWorkspace* ws, narrow::Para
 {
     constexpr int MT = 2;
     auto kern = narrow::forward_narrow_kernel<W, FMT, HACT, OT, MT>;
-    const size_t smem = (size_t)p.cfg.n_layers * ((W + 31) / 32 * (W / 8) * 512 + W * 8);
+    const size_t smem = (size_t)p.cfg.n_layers * ((W + 31) / 32 * (W / 8) * 512 + W * 8 + 32);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     constexpr uint32_t per_tile = narrow::kForwardWarps * 16 * MT;
     p.n_tiles = (uint32_t)(((uint64_t)p.count + per_tile - 1) / per_tile);
     const uint32_t slots = 2u * (uint32_t)ws->sm_count;
-    kern<<<p.n_tiles < slots ? p.n_tiles : slots, 32 * narrow::kForwardWarps, smem, st>>>(p);
-    return cudaGetLastError();
+    return launch_after(st, kern, p.n_tiles < slots ? p.n_tiles : slots, 32 * narrow::kForwardWarps, smem, p);
 }
 
 template <int W, int FMT, int OT>

@@ -157,40 +157,70 @@ __device__ __forceinline__ void store_fragment(uint32_t addr, const uint32_t (&a
     asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
 }
 
-// One weight panel: QN groups of 32 K slots x TN tiles x 32 lanes x 16 bytes.  TRANSPOSED: the columns are the
-// layer's inputs and K its outputs (the reverse products), else columns are outputs and K inputs.
+// What a staging loop needs to know about one weight panel: QN groups of 32 K slots x TN tiles x 32 lanes x 16 bytes.
+// `transposed`: the columns are the layer's inputs and K its outputs (the reverse products), else columns are outputs and
+// K inputs.
+struct Panel {
+    const void* weights;
+    uint32_t dst;        // byte offset
+    int in, out, in_kind, out_kind, tiles;
+    bool transposed;
+};
+
+// Chunk `idx` (16 bytes: lane idx % 32 of a tile) of a panel.
 template <int FMT>
-__device__ __forceinline__ void stage_panel(uint8_t* dst, const MlpConfig& c, const MlpLayerPointers& ptr, int in, int out, int in_kind, int out_kind,
-                                            bool transposed, int qn, int tn, int tid, int nthreads)
+__device__ __forceinline__ uint4 panel_chunk(const MlpConfig& c, const Panel& p, int idx)
 {
     using C = Cvt<FMT>;
-    const uint16_t* w16 = (const uint16_t*)ptr.weights;
-    const float* w32 = (const float*)ptr.weights;
-    const bool whole = !transposed && in_kind == kEights && (in & 7) == 0 && (ptr.weights & 15u) == 0 && c.param_layout == MLP_PARAMS_ROW_MAJOR &&
-                       c.dtype != MLP_F32;
-    for (int idx = tid; idx < qn * tn * 32; idx += nthreads) {
-        const int lane = idx & 31, t = (idx >> 5) % tn, q = (idx >> 5) / tn;
-        const int g = lane >> 2, cc = lane & 3;
-        const int n = feature_of(transposed ? in_kind : out_kind, t, g);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (whole) {
-            const int k = 32 * q + 8 * cc;
-            if (n < out && k < in) v = *(const uint4*)(w16 + (size_t)n * in + k);
-        } else {
-            uint16_t h[8];
+    const uint16_t* w16 = (const uint16_t*)p.weights;
+    const float* w32 = (const float*)p.weights;
+    const int lane = idx & 31, tt = idx >> 5, q = tt / p.tiles, t = tt - q * p.tiles;
+    const int g = lane >> 2, cc = lane & 3;
+    const int n = feature_of(p.transposed ? p.in_kind : p.out_kind, t, g);
+    if (!p.transposed && p.in_kind == kEights && (p.in & 7) == 0 && ((uint64_t)p.weights & 15u) == 0 && c.param_layout == MLP_PARAMS_ROW_MAJOR &&
+        c.dtype != MLP_F32) {
+        const int k = 32 * q + 8 * cc;
+        return n < p.out && k < p.in ? __ldg((const uint4*)(w16 + (size_t)n * p.in + k)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint16_t h[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int k = feature_of(transposed ? out_kind : in_kind, 4 * q + (r >> 1), 2 * cc + (r & 1));
-                const int o = transposed ? k : n, i = transposed ? n : k;
-                h[r] = 0;
-                if (o < out && i < in) {
-                    const int64_t wi = weight_index(c.param_layout, in, out, o, i);
-                    h[r] = c.dtype == MLP_F32 ? (uint16_t)(C::pack2(w32[wi], 0.0f) & 0xffffu) : w16[wi];
-                }
-            }
-            v = make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
+    for (int r = 0; r < 8; ++r) {
+        const int k = feature_of(p.transposed ? p.out_kind : p.in_kind, 4 * q + (r >> 1), 2 * cc + (r & 1));
+        const int o = p.transposed ? k : n, i = p.transposed ? n : k;
+        h[r] = 0;
+        if (o < p.out && i < p.in) {
+            const int64_t wi = weight_index(c.param_layout, p.in, p.out, o, i);
+            h[r] = c.dtype == MLP_F32 ? (uint16_t)(C::pack2(__ldg(w32 + wi), 0.0f) & 0xffffu) : __ldg(w16 + wi);
         }
-        *(uint4*)(dst + (size_t)idx * 16) = v;
+    }
+    return make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
+}
+
+// Stages every panel of a network: `panel(i)` describes panel i, whose chunks number at most PC.  Two chunks a thread are
+// read before either is stored, and nothing waits between panels: staged one layer after the other, each behind its own
+// address, the weights were most of the time of a step of one tile.
+template <int FMT, int PC, class F>
+__device__ __forceinline__ void stage_panels(uint8_t* smem, const MlpConfig& c, int n_panels, F panel, int tid, int nthreads)
+{
+#pragma unroll 1
+    for (int base = tid; base < n_panels * PC; base += 2 * nthreads) {
+        uint4 v[2];
+        uint32_t at[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = base + u * nthreads;
+            at[u] = 0xffffffffu;
+            if (i >= n_panels * PC) continue;
+            const int which = i / PC, idx = i % PC;
+            int chunks;
+            const Panel p = panel(which, &chunks);
+            if (idx >= chunks) continue;
+            v[u] = panel_chunk<FMT>(c, p, idx);
+            at[u] = p.dst + (uint32_t)idx * 16u;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (at[u] != 0xffffffffu) *(uint4*)(smem + at[u]) = v[u];
     }
 }
 
