@@ -45,7 +45,7 @@ struct TrainMap {
     static constexpr bool kSlots = W == 64;
     static constexpr int kWarps = NG * GW;                               // warps with samples; one more issues where there are slots
     static constexpr int kThreads = 32 * (kWarps + (kSlots ? 1 : 0));
-    static constexpr int kRows = 16 * kWarps;                            // samples of a tile
+    static constexpr int kUnit = GW * 16;                                // samples a group takes at a time
     static constexpr int kQ = W / 32, kT = W / 8;
     static constexpr uint32_t kPanel = kQ * kT * 512;                    // one weight matrix in fragment order
     static constexpr uint32_t kTile = GW * 16 * W * 2;                   // [samples of a group][W] operand tile
@@ -57,7 +57,7 @@ struct TrainMap {
     static constexpr uint32_t kForward = kOnes + (kSlots ? 2048 : 0);
     static constexpr uint32_t kReverse = kForward + NL * kPanel;
     // [NL][W rows][W + 1]; one copy per warp where the warps keep their own sums
-    static constexpr uint32_t kSumFloats = NL * W * (W + 1);
+    static constexpr uint32_t kSumRow = W + 1, kSumFloats = NL * W * kSumRow;
     static constexpr uint32_t kSumBytes = kSumFloats * 4 * (kSlots ? 1 : kWarps);
     static constexpr uint32_t kPanelsEnd = kReverse + NL * kPanel;
     static constexpr uint32_t kBias = kPanelsEnd > kSumBytes ? kPanelsEnd : ((kSumBytes + 15) & ~15u);   // fp32 [NL][W / 2 pairs][twice]
@@ -65,8 +65,10 @@ struct TrainMap {
     static constexpr uint32_t kBars = kLoss + kWarps * 8;                // full and empty [group][slot], done
     static constexpr uint32_t kTmemPtr = kBars + (2 * NG * kNumSlots + 1) * 8;
     static constexpr uint32_t kAbort = kTmemPtr + 4;
-    static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;           // MlpLayerPointers [NL]
-    static constexpr uint32_t kSmemBytes = kNet + NL * 32 + 1024;
+    static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;           // MlpLayerPointers [NL], then where the weights are cut from
+    static constexpr uint32_t kSmemBytes = kNet + NL * 40 + 1024;
+    // the stored weights during set-up: where the slots, or the sums past the panels, will be
+    static constexpr uint32_t kStored = kSlots ? kSlot0 : kPanelsEnd, kStoredEnd = kSlots ? kOnes : kBias;
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
     // tensor memory: W + 16 columns per layer (dW_l, then db_l)
     static constexpr uint32_t kDwCols = W + 16;
@@ -123,13 +125,25 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
     const MlpLayerPointers* s_net = (const MlpLayerPointers*)(smem + M::kNet);
     if (threadIdx.x < NL * 4) ((uint64_t*)(smem + M::kNet))[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
     __syncthreads();
+    const void** s_from = (const void**)(smem + M::kNet + NL * 32);
+    copy_weights<NL>(smem + M::kStored, M::kStoredEnd - M::kStored, cfg, s_net, s_from, threadIdx.x, kThreads);
+    for (int i = threadIdx.x; i < NL * W; i += kThreads) {
+        const int l = i / W, j = i % W;
+        if (l == NL - 1 && j >= OT * 8) continue;
+        // features past the real width: below zero for ReLU, so that no derivative there is the one at zero
+        const int f = feature_of(l == NL - 1 ? okind : kEights, j >> 3, j & 7);
+        float* b = (float*)(smem + M::kBias) + l * W * 2 + (j >> 1) * 4 + (j & 1);
+        b[0] = b[2] = f < cfg.dims[l + 1] ? load_as_f32(cfg.dtype, (const void*)s_net[l].biases, f) : (HACT == MLP_ACT_RELU && l < NL - 1 ? -1.0f : 0.0f);
+    }
+    cp_async_wait_all();
+    __syncthreads();
     // forward panels, then reverse panels from the last layer down (layer 0's only for the input gradients)
-    stage_panels<FMT, M::kQ * NT * 32>(smem, cfg, p.input_grads ? 2 * NL : 2 * NL - 1, [&](int which, int* chunks) {
+    cut_panels<FMT, M::kQ * NT * 32>(smem, cfg, p.input_grads ? 2 * NL : 2 * NL - 1, [&](int which, int* chunks) {
         const bool rev = which >= NL;
         const int l = rev ? 2 * NL - 1 - which : which;
         const bool last = l == NL - 1;
         Panel d;
-        d.weights = (const void*)s_net[l].weights;
+        d.weights = s_from[l];
         d.in = cfg.dims[l]; d.out = cfg.dims[l + 1];
         d.in_kind = l == 0 ? ikind : kEights;
         d.out_kind = last ? okind : kEights;
@@ -139,14 +153,6 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
         *chunks = (rev && last ? (OK + 1) / 2 : M::kQ) * d.tiles * 32;
         return d;
     }, threadIdx.x, kThreads);
-    for (int i = threadIdx.x; i < NL * W; i += kThreads) {
-        const int l = i / W, j = i % W;
-        if (l == NL - 1 && j >= OT * 8) continue;
-        // features past the real width: below zero for ReLU, so that no derivative there is the one at zero
-        const int f = feature_of(l == NL - 1 ? okind : kEights, j >> 3, j & 7);
-        float* b = (float*)(smem + M::kBias) + l * W * 2 + (j >> 1) * 4 + (j & 1);
-        b[0] = b[2] = f < cfg.dims[l + 1] ? load_as_f32(cfg.dtype, (const void*)s_net[l].biases, f) : (HACT == MLP_ACT_RELU && l < NL - 1 ? -1.0f : 0.0f);
-    }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -185,7 +191,9 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
         // even tile, then of the odd one), and its 16-byte chunk's swizzle: chunk 2 k + (block / 2), moved with the row.
         const uint32_t slot_row = sbase + M::kSlot0 + (uint32_t)((warp % GW) * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * 128u;
         const uint32_t slot_chunk = (uint32_t)(lane >> 4) ^ (uint32_t)(lane & 7);
-        uint32_t tile = blockIdx.x;
+        // unit u of the batch goes to CTA u % grid, group (u / grid) % NG: small batches spread over SMs first
+        const uint32_t stride = gridDim.x * NG, in_unit = (uint32_t)((warp % GW) * 16 + g);
+        uint32_t unit = blockIdx.x + gridDim.x * (uint32_t)(warp / GW);
 
         // dW_l | db_l of this warp's samples from dZ_l and A_l (operand fragments)
         auto gradients = [&](auto layer, const uint32_t (&dz)[kTrainBlocks][W / 16][4], const uint32_t (&a)[kTrainBlocks][W / 16][4]) {
@@ -231,16 +239,16 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
         };
 
         RawInputs<MT> raw;
-        fetch_raw(raw, p, (uint64_t)tile * (uint64_t)M::kRows + (uint64_t)(warp * 16 * MT + g), 16u, c);
-        for (; tile < p.n_tiles && ok; tile += gridDim.x) {
+        fetch_raw(raw, p, (uint64_t)unit * (uint64_t)M::kUnit + in_unit, 16u, c);
+        for (; unit < p.n_tiles && ok; unit += stride) {
             // block m of this warp: samples base + 16 m + {0, 8}
-            const uint64_t base = (uint64_t)tile * (uint64_t)M::kRows + (uint64_t)(warp * 16 * MT + g);
+            const uint64_t base = (uint64_t)unit * (uint64_t)M::kUnit + in_unit;
             uint32_t A[NL][MT][KS][4];                              // every layer's input
             uint32_t D[kKeepD ? NL - 1 : 1][MT][KS][4];             // derivatives of the hidden activations
             uint32_t zero_seen[NL - 1] = {};                        // ReLU: whether any pre-activation of the layer was exactly zero
             {
                 // the next tile's input and target rows: start them on their way into L2
-                const uint64_t ns = base + (uint64_t)gridDim.x * (uint64_t)M::kRows + (uint64_t)((c & 1) * 8) + (MT == 2 && (c & 2) ? 16u : 0u);
+                const uint64_t ns = base + (uint64_t)stride * (uint64_t)M::kUnit + (uint64_t)((c & 1) * 8) + (MT == 2 && (c & 2) ? 16u : 0u);
                 if (ns < p.count && (MT == 2 || c < 2)) {
                     if (!raw_inputs(cfg))
                         asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p.inputs + ns * (uint64_t)cfg.dims[0] * (cfg.input_dtype == MLP_F32 ? 4u : 2u)));
@@ -249,7 +257,7 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
             }
 #pragma unroll
             for (int m = 0; m < MT; ++m) load_inputs<FMT, KS>(A[0][m], p, raw.v[m], base + 16u * (uint64_t)m, c);
-            fetch_raw(raw, p, base + (uint64_t)gridDim.x * (uint64_t)M::kRows, 16u, c);
+            fetch_raw(raw, p, base + (uint64_t)stride * (uint64_t)M::kUnit, 16u, c);
             // few targets per lane are fetched here, a forward pass ahead of their use (as stored: a conversion would wait)
             uint32_t tgt[MT][2][OT <= 2 ? OT * 2 : 1];
             if constexpr (OT <= 2) {
@@ -483,18 +491,23 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
         constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29);              // 8-row groups 1024 bytes apart, 128-byte swizzle
         constexpr uint32_t kIdesc = umma_idesc(C::kUmmaFmt, 1, 1, 64, W + 16);        // dZ^T (MN, 64 rows) x [A | ones] (MN)
         const uint32_t lo = (sbase & 0x3FFFFu) >> 4;
-        const uint32_t fills = ((p.n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x) * NL;
-        uint32_t done[NG];
+        const uint32_t stride = gridDim.x * NG;
+        uint32_t done[NG], fills[NG];
+        uint32_t left = 0, idle = 0;
 #pragma unroll
-        for (int j = 0; j < NG; ++j) done[j] = 0;
+        for (int j = 0; j < NG; ++j) {
+            const uint32_t first = blockIdx.x + gridDim.x * (uint32_t)j;
+            done[j] = 0;
+            fills[j] = first < p.n_tiles ? ((p.n_tiles - first + stride - 1) / stride) * NL : 0u;
+            left += fills[j];
+        }
         uint32_t started = 0;    // layers whose accumulator has been written
-        uint32_t left = fills * NG, idle = 0;
         while (left > 0 && ok) {
             bool any = false;
 #pragma unroll
             for (int j = 0; j < NG; ++j) {
                 const uint32_t slot = (uint32_t)j * M::kNumSlots + done[j] % M::kNumSlots;
-                if (done[j] < fills && mbar_test_wait(&slot_full[slot], (done[j] / M::kNumSlots) & 1u)) {
+                if (done[j] < fills[j] && mbar_test_wait(&slot_full[slot], (done[j] / M::kNumSlots) & 1u)) {
                     tc_fence_after();
                     const uint32_t l = NL - 1 - done[j] % NL;
                     if (leader) {
@@ -574,26 +587,37 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
     }
     __syncthreads();
     if (!*abort_flag) {
+        // Real parameters in the order they are stored, the layers one after the other over the threads; four to a reduction
+        // where rows are whole 16-byte pieces.  (Walking the padded matrices instead, one parameter to a reduction, took
+        // 7 us.)
         constexpr int kCopies = kSlots ? 1 : NW;
         const float* sums = (const float*)(smem + M::kSums);
+        int i = threadIdx.x;
 #pragma unroll 1
         for (int l = 0; l < NL; ++l) {
             const int in = cfg.dims[l], out = cfg.dims[l + 1];
             const int ki = l == 0 ? ikind : kEights, ko = l == NL - 1 ? okind : kEights;
             float* dW = (float*)s_net[l].weightsGrad;
             float* dB = (float*)s_net[l].biasesGrad;
-            for (int i = threadIdx.x; i < W * (W + 1); i += kThreads) {
-                // position -> feature, in rows and columns
-                const int r = i / (W + 1), k = i - r * (W + 1);
-                const int o = feature_of(ko, r >> 3, r & 7);
-                const int f = k == W ? in : feature_of(ki, k >> 3, k & 7);
-                if (o >= out || (k < W && f >= in)) continue;
+            auto total = [&](int o, int column) {
+                const float* at = sums + (l * W + position_of(ko, o)) * M::kSumRow + column;
                 float v = 0.0f;
 #pragma unroll
-                for (int w = 0; w < kCopies; ++w) v += sums[w * M::kSumFloats + l * W * (W + 1) + i];
-                if (k == W) atomicAdd(dB + o, v);
-                else atomicAdd(dW + weight_index(cfg.param_layout, in, out, o, f), v);
+                for (int w = 0; w < kCopies; ++w) v += at[w * M::kSumFloats];
+                return v;
+            };
+            const bool fours = (in & 3) == 0 && cfg.param_layout == MLP_PARAMS_ROW_MAJOR && ((uint64_t)dW & 15u) == 0;
+            const int per_row = fours ? in >> 2 : in;
+            for (; i < out * per_row; i += kThreads) {
+                const int o = i / per_row, k = i - o * per_row;
+                if (fours)
+                    atomicAdd((float4*)dW + i, make_float4(total(o, position_of(ki, 4 * k)), total(o, position_of(ki, 4 * k + 1)),
+                                                           total(o, position_of(ki, 4 * k + 2)), total(o, position_of(ki, 4 * k + 3))));
+                else atomicAdd(dW + weight_index(cfg.param_layout, in, out, o, k), total(o, position_of(ki, k)));
             }
+            i -= out * per_row;
+            for (; i < out; i += kThreads) atomicAdd(dB + i, total(i, W));
+            i -= out;
         }
         if (threadIdx.x == 0) {
             const float* part = (const float*)(smem + M::kLoss);
@@ -618,7 +642,7 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
     constexpr int NT = W / 8, KS = W / 16, kQ = (W + 31) / 32;
     constexpr int HK = tile_kind(NT);                    // how hidden vectors are dealt to the lanes
     constexpr uint32_t kPanel = kQ * NT * 512;
-    extern __shared__ __align__(128) uint8_t smem[];     // [n_layers] panels, then fp32 biases [n_layers][W / 2 pairs][twice], addresses
+    extern __shared__ __align__(128) uint8_t smem[];     // [n_layers] panels, then fp32 biases [n_layers][W / 2 pairs][twice], addresses, stored weights
     const uint32_t sbase = smem_u32(smem);
     const MlpConfig& cfg = p.cfg;
     const int nl = cfg.n_layers, od = cfg.dims[nl];
@@ -632,9 +656,20 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
     grid_wait();
     if (threadIdx.x < nl * 4) ((uint64_t*)s_net)[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
     __syncthreads();
-    stage_panels<FMT, kQ * NT * 32>(smem, cfg, nl, [&](int l, int* chunks) {
+    const void** s_from = (const void**)(s_net + nl);
+    copy_weights<5>((uint8_t*)(s_from + 6), (uint32_t)p.raw_bytes, cfg, s_net, s_from, threadIdx.x, 32 * kForwardWarps);
+    for (int i = threadIdx.x; i < nl * W; i += 32 * kForwardWarps) {
+        const int l = i / W, j = i % W;
+        if (l == nl - 1 && j >= OT * 8) continue;
+        const int f = feature_of(l == nl - 1 ? okind : HK, j >> 3, j & 7);
+        float* b = s_bias_w + l * W * 2 + (j >> 1) * 4 + (j & 1);
+        b[0] = b[2] = f < cfg.dims[l + 1] ? load_as_f32(cfg.dtype, (const void*)s_net[l].biases, f) : 0.0f;
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    cut_panels<FMT, kQ * NT * 32>(smem, cfg, nl, [&](int l, int* chunks) {
         Panel d;
-        d.weights = (const void*)s_net[l].weights;
+        d.weights = s_from[l];
         d.in = cfg.dims[l]; d.out = cfg.dims[l + 1];
         d.in_kind = l == 0 ? ikind : HK;
         d.out_kind = l == nl - 1 ? okind : HK;
@@ -644,13 +679,6 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
         *chunks = kQ * d.tiles * 32;
         return d;
     }, threadIdx.x, 32 * kForwardWarps);
-    for (int i = threadIdx.x; i < nl * W; i += 32 * kForwardWarps) {
-        const int l = i / W, j = i % W;
-        if (l == nl - 1 && j >= OT * 8) continue;
-        const int f = feature_of(l == nl - 1 ? okind : HK, j >> 3, j & 7);
-        float* b = s_bias_w + l * W * 2 + (j >> 1) * 4 + (j & 1);
-        b[0] = b[2] = f < cfg.dims[l + 1] ? load_as_f32(cfg.dtype, (const void*)s_net[l].biases, f) : 0.0f;
-    }
     __syncthreads();
     const uint32_t panel0 = sbase + (uint32_t)lane * 16u;
     const uint32_t s_bias = sbase + (uint32_t)nl * kPanel + (uint32_t)c * 16u;
@@ -775,7 +803,7 @@ static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params
     auto kern = narrow::learn_gradient_narrow_kernel<W, NL, FMT, HACT, OT, NG, GW>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kSmemBytes);
     if (e != cudaSuccess) return e;
-    p.n_tiles = (uint32_t)(((uint64_t)p.count + M::kRows - 1) / M::kRows);
+    p.n_tiles = (uint32_t)(((uint64_t)p.count + M::kUnit - 1) / M::kUnit);
     const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
     return launch_after(st, kern, grid, M::kThreads, M::kSmemBytes, p);
 }
@@ -808,7 +836,9 @@ static cudaError_t launch_forward(cudaStream_t st, TcWorkspace* ws, narrow::Para
 {
     constexpr int MT = 2;
     auto kern = narrow::forward_narrow_kernel<W, FMT, HACT, OT, MT>;
-    const size_t smem = (size_t)p.cfg.n_layers * ((W + 31) / 32 * (W / 8) * 512 + W * 8 + 32);
+    p.raw_bytes = 0;
+    for (int l = 0; l < p.cfg.n_layers; ++l) p.raw_bytes += (int)((narrow::stored_weight_bytes(p.cfg, l) + 15u) & ~15u);
+    const size_t smem = (size_t)p.cfg.n_layers * ((W + 31) / 32 * (W / 8) * 512 + W * 8 + 32) + 48 + (size_t)p.raw_bytes;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     constexpr uint32_t per_tile = narrow::kForwardWarps * 16 * MT;

@@ -22,6 +22,7 @@
 #include <stdint.h>
 
 #include "mlp_common.cuh"
+#include "tc_layout.cuh"
 #include "tc_ptx.cuh"
 
 namespace mlpb200 {
@@ -52,7 +53,8 @@ struct Params {
     float* input_grads;   // training, optional: [count][dims[0]] gradient with respect to the (unencoded) inputs
     float* outputs;       // forward: fp32 [count][dims[n_layers]]
     uint32_t count;
-    uint32_t n_tiles;
+    uint32_t n_tiles;     // units of work
+    int raw_bytes;        // forward: shared memory for the stored weights
     int vec_in, vec_tgt, vec_out, vec_dx;   // rows may be read / written as whole 16-byte pieces (widths and addresses allow it)
 };
 
@@ -157,12 +159,23 @@ __device__ __forceinline__ void store_fragment(uint32_t addr, const uint32_t (&a
     asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
 }
 
-// What a staging loop needs to know about one weight panel: QN groups of 32 K slots x TN tiles x 32 lanes x 16 bytes.
-// `transposed`: the columns are the layer's inputs and K its outputs (the reverse products), else columns are outputs and
-// K inputs.
+// Where the 16-byte chunk `chunk` of row `row` of a [rows][W] operand tile lies inside its row (W 32 or 64).
+template <int W>
+__device__ __forceinline__ int swizzled_chunk(int row, int chunk) { return chunk ^ ((row >> layout::swz_shift(W)) & layout::swz_mask(W)); }
+
+// Where feature f of a vector lies: 8 * tile + column.
+__host__ __device__ constexpr int position_of(int kind, int f)
+{
+    return kind == kEights ? 32 * (f >> 5) + 8 * ((f & 7) >> 1) + 2 * ((f >> 3) & 3) + (f & 1)
+         : kind == kFours  ? 8 * ((f >> 1) & 1) + 2 * (f >> 2) + (f & 1)
+                           : f;
+}
+
+// One weight panel: groups of 32 K slots x `tiles` tiles x 32 lanes x 16 bytes.  `transposed`: the columns are the layer's
+// inputs and K its outputs (the reverse products), else columns are outputs and K inputs.
 struct Panel {
-    const void* weights;
-    uint32_t dst;        // byte offset
+    const void* weights;   // the parameters, or their copy in shared memory
+    uint32_t dst;          // byte offset
     int in, out, in_kind, out_kind, tiles;
     bool transposed;
 };
@@ -177,50 +190,71 @@ __device__ __forceinline__ uint4 panel_chunk(const MlpConfig& c, const Panel& p,
     const int lane = idx & 31, tt = idx >> 5, q = tt / p.tiles, t = tt - q * p.tiles;
     const int g = lane >> 2, cc = lane & 3;
     const int n = feature_of(p.transposed ? p.in_kind : p.out_kind, t, g);
-    if (!p.transposed && p.in_kind == kEights && (p.in & 7) == 0 && ((uint64_t)p.weights & 15u) == 0 && c.param_layout == MLP_PARAMS_ROW_MAJOR &&
-        c.dtype != MLP_F32) {
-        const int k = 32 * q + 8 * cc;
-        return n < p.out && k < p.in ? __ldg((const uint4*)(w16 + (size_t)n * p.in + k)) : make_uint4(0u, 0u, 0u, 0u);
-    }
     uint16_t h[8];
+    if ((p.transposed ? p.out_kind : p.in_kind) == kEights && c.param_layout == MLP_PARAMS_ROW_MAJOR && c.dtype != MLP_F32) {
+        // the usual case: eight consecutive K features, along a stored row or down a stored column
+        const int k0 = 32 * q + 8 * cc, limit = n < (p.transposed ? p.in : p.out) ? (p.transposed ? p.out : p.in) - k0 : 0;
+        if (!p.transposed && (p.in & 7) == 0 && ((uint64_t)w16 & 15u) == 0) return limit > 0 ? *(const uint4*)(w16 + n * p.in + k0) : make_uint4(0u, 0u, 0u, 0u);
+        const uint16_t* w = p.transposed ? w16 + k0 * p.in + n : w16 + n * p.in + k0;
+        const int step = p.transposed ? p.in : 1;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) h[r] = r < limit ? w[r * step] : (uint16_t)0;
+        return make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
+    }
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int k = feature_of(p.transposed ? p.out_kind : p.in_kind, 4 * q + (r >> 1), 2 * cc + (r & 1));
         const int o = p.transposed ? k : n, i = p.transposed ? n : k;
         h[r] = 0;
         if (o < p.out && i < p.in) {
-            const int64_t wi = weight_index(c.param_layout, p.in, p.out, o, i);
-            h[r] = c.dtype == MLP_F32 ? (uint16_t)(C::pack2(__ldg(w32 + wi), 0.0f) & 0xffffu) : __ldg(w16 + wi);
+            const int wi = (int)weight_index(c.param_layout, p.in, p.out, o, i);
+            h[r] = c.dtype == MLP_F32 ? (uint16_t)(C::pack2(w32[wi], 0.0f) & 0xffffu) : w16[wi];
         }
     }
     return make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
 }
 
-// Stages every panel of a network: `panel(i)` describes panel i, whose chunks number at most PC.  Two chunks a thread are
-// read before either is stored, and nothing waits between panels: staged one layer after the other, each behind its own
-// address, the weights were most of the time of a step of one tile.
-template <int FMT, int PC, class F>
-__device__ __forceinline__ void stage_panels(uint8_t* smem, const MlpConfig& c, int n_panels, F panel, int tid, int nthreads)
+// Bytes of a layer's weights as they are stored.
+__host__ __device__ inline uint32_t stored_weight_bytes(const MlpConfig& c, int l)
 {
-#pragma unroll 1
-    for (int base = tid; base < n_panels * PC; base += 2 * nthreads) {
-        uint4 v[2];
-        uint32_t at[2];
+    uint32_t in = (uint32_t)c.dims[l], out = (uint32_t)c.dims[l + 1];
+    if (c.param_layout == MLP_PARAMS_OPTIMAL) { in = (in + 15u) & ~15u; out = (out + 15u) & ~15u; }
+    return in * out * (c.dtype == MLP_F32 ? 4u : 2u);
+}
+
+// Copies the stored weights of all layers to shared memory, all copies in flight together; copied[l] is where layer l's
+// lie, or its own address where they do not fit `room` bytes or do not start on a 16-byte boundary.  Each panel is then
+// cut from there.  Cut straight from global memory, value by value, the panels took 4 of the 20 us of a step of 128
+// samples.  cp_async_wait_all() and a barrier are still to come.
+template <int NLMAX>
+__device__ __forceinline__ void copy_weights(uint8_t* raw, uint32_t room, const MlpConfig& c, const MlpLayerPointers* net, const void** copied, int tid, int nthreads)
+{
+    uint32_t at = 0;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int i = base + u * nthreads;
-            at[u] = 0xffffffffu;
-            if (i >= n_panels * PC) continue;
-            const int which = i / PC, idx = i % PC;
-            int chunks;
-            const Panel p = panel(which, &chunks);
-            if (idx >= chunks) continue;
-            v[u] = panel_chunk<FMT>(c, p, idx);
-            at[u] = p.dst + (uint32_t)idx * 16u;
+    for (int l = 0; l < NLMAX; ++l) {
+        if (l >= c.n_layers) break;
+        const uint32_t bytes = stored_weight_bytes(c, l), whole = bytes & ~15u;
+        const uint8_t* src = (const uint8_t*)net[l].weights;
+        const bool fits = at + bytes <= room && ((uint64_t)src & 15u) == 0;
+        if (fits) {
+            const uint32_t dst = ptx::smem_u32(raw + at);
+            for (uint32_t i = (uint32_t)tid * 16u; i < whole; i += (uint32_t)nthreads * 16u) ptx::cp_async_16(dst + i, src + i);
+            if ((uint32_t)tid < (bytes - whole) / 2u) ((uint16_t*)(raw + at + whole))[tid] = ((const uint16_t*)(src + whole))[tid];
         }
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-            if (at[u] != 0xffffffffu) *(uint4*)(smem + at[u]) = v[u];
+        if (tid == 0) copied[l] = fits ? (const void*)(raw + at) : (const void*)src;
+        at += (bytes + 15u) & ~15u;
+    }
+}
+
+// Cuts every panel of a network: `panel(i)` describes panel i, whose chunks number at most PC.
+template <int FMT, int PC, class F>
+__device__ __forceinline__ void cut_panels(uint8_t* smem, const MlpConfig& c, int n_panels, F panel, int tid, int nthreads)
+{
+#pragma unroll 2
+    for (int i = tid; i < n_panels * PC; i += nthreads) {
+        int chunks;
+        const Panel p = panel(i / PC, &chunks);
+        if (i % PC < chunks) *(uint4*)(smem + p.dst + (uint32_t)(i % PC) * 16u) = panel_chunk<FMT>(c, p, i % PC);
     }
 }
 
