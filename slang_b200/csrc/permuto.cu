@@ -266,13 +266,15 @@ permuto_encode_kernel(const __grid_constant__ MlpPermutoConfig c, const float* _
 
 // The level-0 thread of a position adds the level threads' position-gradient terms in ascending level
 // order: by warp shuffles when a warp holds whole positions (L divides 32), through shared memory otherwise.
-template <int D, int F, typename T>
+// POS: the position gradients are wanted.  Only they need the table's features: without them the gathers, half of the
+// kernel's memory requests, are left out (an encoder with fixed positions).
+template <int D, int F, typename T, bool POS>
 __global__ void __launch_bounds__(256)
 permuto_backward_kernel(const __grid_constant__ MlpPermutoConfig c, const float* __restrict__ positions,
                         const T* __restrict__ table, const T* __restrict__ d_out, T* __restrict__ d_table,
                         float* __restrict__ d_positions, uint32_t count)
 {
-    __shared__ float s_dpos[256 * D];
+    __shared__ float s_dpos[POS ? 256 * D : 1];
     __shared__ MlpPermutoLevelInfo s_levels[MLP_PERMUTO_MAX_LEVELS];
     const uint32_t L = uint32_t(c.n_levels);
     const uint32_t per_block = 256u / L;
@@ -307,19 +309,20 @@ permuto_backward_kernel(const __grid_constant__ MlpPermutoConfig c, const float*
 #pragma unroll
             for (int k = 0; k <= D; ++k) {
                 const uint32_t idx = vertex_index<D, F>(s, k, li);
-                const Vec<F, T> feat = load_vec<F, T>(table + idx);
                 const T w = Elem<T>::from(s.bary[k]);
                 T term[F];
-                float dw = 0.0f;
 #pragma unroll
-                for (int f = 0; f < F; ++f) {
-                    term[f] = Elem<T>::mul(w, dy.v[f]);
-                    dw += Elem<T>::to_float(Elem<T>::mul(feat.v[f], dy.v[f]));
+                for (int f = 0; f < F; ++f) term[f] = Elem<T>::mul(w, dy.v[f]);
+                if constexpr (POS) {
+                    const Vec<F, T> feat = load_vec<F, T>(table + idx);
+                    float dw = 0.0f;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) dw += Elem<T>::to_float(Elem<T>::mul(feat.v[f], dy.v[f]));
+                    dbary[k] = dw;
                 }
                 red_add<F>(d_table + idx, term);
-                dbary[k] = dw;
             }
-            if (d_positions) {
+            if constexpr (POS) {
                 dbary[D + 1] = dbary[0];
                 constexpr float inv = 1.0f / float(D + 1);
                 float de[D + 1];
@@ -340,7 +343,7 @@ permuto_backward_kernel(const __grid_constant__ MlpPermutoConfig c, const float*
                 }
             }
         }
-        if (d_positions) {   // uniform over the block
+        if constexpr (POS) {
             if ((32u % L) == 0) {
                 // the level threads of a position sit in one warp: the level-0 lane pulls the others' terms
                 // in ascending level order (every lane runs the shuffles; lanes past the batch carry zeros)
@@ -401,7 +404,8 @@ cudaError_t run(bool backward, cudaStream_t st, const MlpPermutoConfig& c, uint6
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int resident = 0;   // blocks of this kernel that fit an SM at once
     if (!backward) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, permuto_encode_kernel<D, F, T>, 256, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, permuto_backward_kernel<D, F, T>, 256, 0);
+    else if (d_positions) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, permuto_backward_kernel<D, F, T, true>, 256, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, permuto_backward_kernel<D, F, T, false>, 256, 0);
     if (resident < 1) resident = 1;
     // encode: one wave of blocks that walk the positions; reverse: up to 64 waves of short blocks
     const unsigned grid = (unsigned)std::min<uint64_t>(groups, uint64_t(sms) * resident * (backward ? 64 : 1));
@@ -409,8 +413,8 @@ cudaError_t run(bool backward, cudaStream_t st, const MlpPermutoConfig& c, uint6
         permuto_encode_kernel<D, F, T><<<grid, 256, 0, st>>>(
             c, (const float*)positions, (const T*)table, (T*)out, count);
     } else {
-        permuto_backward_kernel<D, F, T><<<grid, 256, 0, st>>>(
-            c, (const float*)positions, (const T*)table, (const T*)out, (T*)d_table, (float*)d_positions, count);
+        auto kern = d_positions ? permuto_backward_kernel<D, F, T, true> : permuto_backward_kernel<D, F, T, false>;
+        kern<<<grid, 256, 0, st>>>(c, (const float*)positions, (const T*)table, (const T*)out, (T*)d_table, (float*)d_positions, count);
     }
     return cudaGetLastError();
 }
