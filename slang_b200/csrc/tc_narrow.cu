@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
             const uint64_t base = (uint64_t)unit * (uint64_t)M::kUnit + in_unit;
             uint32_t A[NL][MT][KS][4];                              // every layer's input
             uint32_t D[kKeepD ? NL - 1 : 1][MT][KS][4];             // derivatives of the hidden activations
-            uint32_t zero_seen[NL - 1] = {};                        // ReLU: whether any pre-activation of the layer was exactly zero
+            uint32_t zero_seen = 0;                                 // ReLU: whether any pre-activation was exactly zero
             {
                 // the next tile's input and target rows: start them on their way into L2
                 const uint64_t ns = base + (uint64_t)stride * (uint64_t)M::kUnit + (uint64_t)((c & 1) * 8) + (MT == 2 && (c & 2) ? 16u : 0u);
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
                                 // max(z, -0): below zero leaves a negative zero, so a z of exactly zero, whose derivative
                                 // is one half, is told apart by its positive one
                                 a = C::max2(C::pack2(z0, z1), 0x80008000u);
-                                zero_seen[l] |= (a - 0x00010001u) & ~a;   // bit 15 of a half: the half is +0
+                                zero_seen |= (a - 0x00010001u) & ~a;   // bit 15 of a half: the half is +0
                             } else if constexpr (HACT == MLP_ACT_LEAKY_RELU) {
                                 // max(z, alpha z) with 0 <= alpha < 1 (the launcher sees to it); the sign bit is "z < 0"
                                 const float2 az = __fmul2_rn(make_float2(z0, z1), make_float2(alpha, alpha));
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
                             }
                         }
                 if constexpr (HACT == MLP_ACT_RELU) {
-                    if (zero_seen[l - 1] & 0x80008000u) {   // some pre-activation was exactly zero: half of the gradient passes there
+                    if (zero_seen & 0x80008000u) {   // some pre-activation was exactly zero: half of the gradient passes there
 #pragma unroll
                         for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -798,7 +798,7 @@ static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params
     // for (16 with 128 each, 11 with 168, 8 with 255), one of them issuing.
     constexpr bool kept = HACT != MLP_ACT_RELU && HACT != MLP_ACT_LEAKY_RELU;
     constexpr int state = NL + (kept ? NL - 1 : 0);
-    constexpr int NG = W == 32 ? 8 : state <= 4 ? 5 : state <= 5 ? 5 : 7, GW = W == 32 ? 1 : state <= 4 ? 3 : state <= 5 ? 2 : 1;
+    constexpr int NG = W == 32 ? 8 : state <= 4 ? 3 : state <= 5 ? 5 : 7, GW = W == 32 ? 1 : state <= 4 ? 5 : state <= 5 ? 2 : 1;
     using M = narrow::TrainMap<W, NL, NG, GW>;
     auto kern = narrow::learn_gradient_narrow_kernel<W, NL, FMT, HACT, OT, NG, GW>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kSmemBytes);
