@@ -455,8 +455,11 @@ sequential_sum_kernel(SimtNet net, const MlpLayerPointers* __restrict__ lp, cons
 // adjustParameters, fp32 state (examples/mlp-training/adam.slang:21-37 widened to float):
 // NaN gradient -> zero it and skip; +-inf -> +-10000; eps inside the square root; gradient zeroed.
 // A thread takes E elements a block apart, their loads issued together, and takes the bias corrections, two powers by
-// squaring, once for elements of the same iteration (nearly always all of them).  Bound: HBM at E = 4.
-template <int E>
+// squaring, once for elements of the same iteration (nearly always all of them).  A parameter that no gradient has
+// reached yet (zero gradient, zero moments: the unused slots of a hash table) keeps its value exactly, so only its
+// iteration count moves; three divisions and a root per element are what the kernel issues otherwise.  PLAIN: fp32
+// parameters without a master copy.  Bound: HBM and instruction issue at E = 4.
+template <int E, bool PLAIN>
 __global__ void __launch_bounds__(256)
 adjust_parameters_kernel(const __grid_constant__ MlpConfig c, MlpAdamState* __restrict__ states, void* __restrict__ params,
                          float* __restrict__ grads, uint32_t count)
@@ -473,7 +476,8 @@ adjust_parameters_kernel(const __grid_constant__ MlpConfig c, MlpAdamState* __re
         if (i < count) {
             g[k] = grads[i];
             raw[k] = __ldcs(reinterpret_cast<const float4*>(states) + i);
-            p[k] = c.adam_master ? raw[k].w : load_as_f32(c.dtype, params, i);
+            if constexpr (PLAIN) p[k] = static_cast<const float*>(params)[i];
+            else p[k] = c.adam_master ? raw[k].w : load_as_f32(c.dtype, params, i);
         }
     }
     int32_t known = -1;
@@ -482,15 +486,20 @@ adjust_parameters_kernel(const __grid_constant__ MlpConfig c, MlpAdamState* __re
     for (int k = 0; k < E; ++k) {
         const uint32_t i = first + 256u * k;
         if (i >= count) break;
-        grads[i] = 0.0f;
         float gk = g[k];
+        const int32_t it = __float_as_int(raw[k].z) + 1;
+        if (gk == 0.0f && (__float_as_uint(raw[k].x) | __float_as_uint(raw[k].y)) == 0u && c.eps > 0.0f) {
+            __stcs(reinterpret_cast<float4*>(states) + i, make_float4(0.0f, 0.0f, __int_as_float(it), p[k]));
+            if (!PLAIN && c.adam_master) store_from_f32(c.dtype, params, i, p[k]);
+            continue;
+        }
+        grads[i] = 0.0f;
         if (isnan(gk)) continue;
         float mean = raw[k].x, var = raw[k].y;
-        const int32_t it = __float_as_int(raw[k].z) + 1;
         if (isinf(gk)) gk = gk > 0.0f ? 10000.0f : -10000.0f;
         mean = c.beta1 * mean + (1.0f - c.beta1) * gk;
         var = c.beta2 * var + ((1.0f - c.beta2) * gk) * gk;
-        if (k == 0 || it != known) {
+        if (it != known) {
             known = it;
             c1 = 1.0f - pow_int(c.beta1, it);
             c2 = 1.0f - pow_int(c.beta2, it);
@@ -500,7 +509,8 @@ adjust_parameters_kernel(const __grid_constant__ MlpConfig c, MlpAdamState* __re
         const float denom = __fsqrt_rn(fmaxf(0.0f, var_hat) + c.eps);
         const float v = p[k] - __fdiv_rn(c.lr * mean_hat, denom);
         __stcs(reinterpret_cast<float4*>(states) + i, make_float4(mean, var, __int_as_float(it), v));
-        store_from_f32(c.dtype, params, i, v);
+        if constexpr (PLAIN) static_cast<float*>(params)[i] = v;
+        else store_from_f32(c.dtype, params, i, v);
     }
 }
 
@@ -618,9 +628,10 @@ cudaError_t launch_adjust_parameters(cudaStream_t st, const MlpConfig& c, const 
     // launch is all there is (a network's parameters).
     constexpr uint32_t kMany = 148u * 8u * 1024u;
     MlpAdamState* states = (MlpAdamState*)a.adamStates;
+    const auto many = c.dtype == MLP_F32 && !c.adam_master ? adjust_parameters_kernel<4, true> : adjust_parameters_kernel<4, false>;
     const cudaError_t e = a.count >= kMany
-        ? launch_after(st, adjust_parameters_kernel<4>, (a.count + 1023) / 1024, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count)
-        : launch_after(st, adjust_parameters_kernel<1>, (a.count + 255) / 256, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count);
+        ? launch_after(st, many, (a.count + 1023) / 1024, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count)
+        : launch_after(st, adjust_parameters_kernel<1, false>, (a.count + 255) / 256, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count);
     *launches += 1;
     return e;
 }
