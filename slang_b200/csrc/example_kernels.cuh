@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "../../include/slang_b200_mlp_config.h"
+#include "launch_pdl.cuh"
 
 namespace mlpb200 {
 
@@ -19,19 +20,35 @@ namespace mlpb200 {
 // The literal example: 4 -> 16 -> 4 in half (examples/mlp-training/{kernels,network,mlp_sw,mlvec_sw}.slang).
 // Every half operation is rounded on its own, as IEEE half arithmetic does.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ __half hmul_(__half a, __half b) { return __float2half_rn(__half2float(a) * __half2float(b)); }
-__device__ __forceinline__ __half hadd_(__half a, __half b) { return __float2half_rn(__half2float(a) + __half2float(b)); }
-__device__ __forceinline__ __half hsub_(__half a, __half b) { return __float2half_rn(__half2float(a) - __half2float(b)); }
+__device__ __forceinline__ __half hmul_(__half a, __half b) { return __hmul_rn(a, b); }
+__device__ __forceinline__ __half hadd_(__half a, __half b) { return __hadd_rn(a, b); }
+__device__ __forceinline__ __half hsub_(__half a, __half b) { return __hsub_rn(a, b); }
 __device__ __forceinline__ __half hdiv_(__half a, __half b) { return __float2half_rn(__fdiv_rn(__half2float(a), __half2float(b))); }
 __device__ __forceinline__ bool hneg_(__half a) { return __half2float(a) < 0.0f; }
 
-template <int In, int Out>
-__device__ void ex_layer_eval(const MlpLayerPointers& lp, const __half* x, __half* y)
+// Both layers' parameters in shared memory, read from global memory once per block and all at the same time (every sample
+// reads every one of them).
+struct ExampleParams {
+    alignas(16) __half w1[64], w2[64];
+    alignas(16) __half b1[16], b2[4];
+};
+__device__ __forceinline__ void ex_stage(ExampleParams& s, const MlpLayerPointers& l1, const MlpLayerPointers& l2)
 {
-    const __half* W = (const __half*)lp.weights;
-    const __half* B = (const __half*)lp.biases;
+    const int t = (int)threadIdx.x;
+    if (t < 64) s.w1[t] = ((const __half*)l1.weights)[t];
+    else if (t < 128) s.w2[t - 64] = ((const __half*)l2.weights)[t - 64];
+    else if (t < 144) s.b1[t - 128] = ((const __half*)l1.biases)[t - 128];
+    else if (t < 148) s.b2[t - 144] = ((const __half*)l2.biases)[t - 144];
+    __syncthreads();
+}
+
+template <int In, int Out>
+__device__ void ex_layer_eval(const __half* W, const __half* B, const __half* x, __half* y)
+{
+#pragma unroll
     for (int i = 0; i < Out; ++i) {
         __half r = B[i];
+#pragma unroll
         for (int j = 0; j < In; ++j) r = hadd_(r, hmul_(W[i * In + j], x[j]));
         y[i] = r;
     }
@@ -40,19 +57,24 @@ __device__ void ex_layer_eval(const MlpLayerPointers& lp, const __half* x, __hal
         if (hneg_(y[i])) y[i] = hmul_(y[i], slope);
 }
 
-// Backward of one layer for one sample.  The per-sample weight- and bias-gradient terms are left in
-// shared memory (g and x) for the ordered block-level sum; dx = W^T g.
-template <int In, int Out>
-__device__ void ex_layer_bwd(const MlpLayerPointers& lp, const __half* x, __half* g, __half* dx)
+// Backward of one layer for one sample, given the outputs y its forward pass left (the reference evaluates the layer again:
+// the same operations on the same values).  The per-sample weight- and bias-gradient terms are left in shared memory (g
+// and x) for the ordered block-level sum; dx = W^T g.
+template <int Out>
+__device__ void ex_activation_bwd(const __half* y, __half* g)
 {
-    __half fwd[Out];
-    ex_layer_eval<In, Out>(lp, x, fwd);
     const __half slope = __float2half_rn(0.01f);
+#pragma unroll
     for (int i = 0; i < Out; ++i)
-        if (hneg_(fwd[i])) g[i] = hmul_(g[i], slope);
-    const __half* W = (const __half*)lp.weights;
+        if (hneg_(y[i])) g[i] = hmul_(g[i], slope);
+}
+template <int In, int Out>
+__device__ void ex_input_bwd(const __half* W, const __half* g, __half* dx)
+{
+#pragma unroll
     for (int i = 0; i < In; ++i) {
         __half r = __float2half_rn(0.0f);
+#pragma unroll
         for (int j = 0; j < Out; ++j) r = hadd_(r, hmul_(W[j * In + i], g[j]));
         dx[i] = r;
     }
@@ -78,14 +100,16 @@ __device__ inline void atomic_add_half(__half* addr, __half v)
 // Ordered sum over the block's samples of g[s][i] * x[s][j] (half, one rounding per multiply and per
 // add, ascending sample order), then one atomic per element per block.  With a single block (the
 // example runs 16 samples) the result is what a sequential machine produces.
-template <int In, int Out>
+// FIRST: the thread the layer's parameters start at, so that the two layers' sums run side by side.
+template <int In, int Out, int FIRST>
 __device__ void ex_accumulate(const MlpLayerPointers& lp, const __half* sg, const __half* sx, int n_valid, int gstride,
                               int xstride)
 {
     __half* dW = (__half*)lp.weightsGrad;
     __half* dB = (__half*)lp.biasesGrad;
     const bool single = gridDim.x == 1;
-    for (int p = threadIdx.x; p < In * Out + Out; p += blockDim.x) {
+    const int p = (int)threadIdx.x - FIRST;
+    if (p >= 0 && p < In * Out + Out) {
         const bool is_w = p < In * Out;
         const int i = is_w ? p / In : p - In * Out, j = is_w ? p % In : 0;
         __half* dst = is_w ? dW + p : dB + i;
@@ -115,15 +139,19 @@ learnGradient(const MlpLayerPointers* __restrict__ network, uint32_t* lossBuffer
 
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = tid < count;
+    grid_release();
+    grid_wait();
     const MlpLayerPointers L1 = network[0], L2 = network[1];
+    __shared__ ExampleParams s_p;
+    ex_stage(s_p, L1, L2);
     float this_loss = 0.0f;
     if (valid) {
         const float2 in = inputs[tid];
         const __half x = __float2half_rn(in.x), y = __float2half_rn(in.y);
         __half enc[4] = {x, y, hmul_(x, x), hmul_(y, y)};
-        __half h1[16], out[4], g2[4], g1[16], dead[4];
-        ex_layer_eval<4, 16>(L1, enc, h1);
-        ex_layer_eval<16, 4>(L2, h1, out);
+        __half h1[16], out[4], g2[4], g1[16];
+        ex_layer_eval<4, 16>(s_p.w1, s_p.b1, enc, h1);
+        ex_layer_eval<16, 4>(s_p.w2, s_p.b2, h1, out);
         const __half one = __float2half_rn(1.0f), half_ = __float2half_rn(0.5f);
         __half gt[4];
         gt[0] = hdiv_(hadd_(x, y), hadd_(one, hmul_(y, y)));
@@ -137,16 +165,17 @@ learnGradient(const MlpLayerPointers* __restrict__ network, uint32_t* lossBuffer
             l = hadd_(l, hmul_(d, d));
         }
         this_loss = __half2float(l);
-        ex_layer_bwd<16, 4>(L2, h1, g2, g1);
-        ex_layer_bwd<4, 16>(L1, enc, g1, dead);
+        ex_activation_bwd<4>(out, g2);
+        ex_input_bwd<16, 4>(s_p.w2, g2, g1);
+        ex_activation_bwd<16>(h1, g1);
         for (int k = 0; k < 4; ++k) { s_enc[threadIdx.x * 4 + k] = enc[k]; s_g2[threadIdx.x * 4 + k] = g2[k]; }
         for (int k = 0; k < 16; ++k) { s_h1[threadIdx.x * 16 + k] = h1[k]; s_g1[threadIdx.x * 16 + k] = g1[k]; }
     }
     __syncthreads();
     const int first = blockIdx.x * blockDim.x;
     const int n_valid = count > (uint32_t)first ? min((int)blockDim.x, (int)(count - first)) : 0;
-    ex_accumulate<16, 4>(L2, s_g2, s_h1, n_valid, 4, 16);
-    ex_accumulate<4, 16>(L1, s_g1, s_enc, n_valid, 16, 4);
+    ex_accumulate<16, 4, 0>(L2, s_g2, s_h1, n_valid, 4, 16);
+    ex_accumulate<4, 16, 96>(L1, s_g1, s_enc, n_valid, 16, 4);
 
     // WaveActiveMax, then the first lane folds the wave's value into the loss word.
     float m = this_loss;
@@ -167,12 +196,12 @@ learnGradient(const MlpLayerPointers* __restrict__ network, uint32_t* lossBuffer
 // row-major gradient segment (coopVecReduceSumAccumulate, hlsl.meta.slang:33344-33351).
 // ------------------------------------------------------------------------------------------------
 template <int In, int Out>
-__device__ void cv_layer_sums(const MlpLayerPointers& lp, const __half* x, __half* o)
+__device__ void cv_layer_sums(const __half* W, const __half* B, const __half* x, __half* o)
 {
-    const __half* W = (const __half*)lp.weights;
-    const __half* B = (const __half*)lp.biases;
+#pragma unroll
     for (int i = 0; i < Out; ++i) {
         __half r = __float2half_rn(0.0f);
+#pragma unroll
         for (int j = 0; j < In; ++j) r = hadd_(r, hmul_(W[i * In + j], x[j]));
         o[i] = hadd_(r, B[i]);
     }
@@ -188,34 +217,30 @@ __device__ void cv_activation(const __half* o, __half* y)
     }
 }
 
-// g <- gradient with respect to the pre-activation sums o; dx = W^T g with sums starting from zero.
-template <int In, int Out>
-__device__ void cv_layer_bwd(const MlpLayerPointers& lp, const __half* o, __half* g, __half* dx)
+// g <- gradient with respect to the pre-activation sums o (dx = W^T g, from zero, is ex_input_bwd's).
+template <int Out>
+__device__ void cv_activation_bwd(const __half* o, __half* g)
 {
     const __half slope = __float2half_rn(0.001f), half_ = __float2half_rn(0.5f);
+#pragma unroll
     for (int i = 0; i < Out; ++i) {
         const float a = __half2float(o[i]), b = __half2float(hmul_(o[i], slope));
         if (a > b) { /* whole gradient to the first argument */ }
         else if (a < b) g[i] = hmul_(g[i], slope);
         else { const __half h = hmul_(half_, g[i]); g[i] = hadd_(h, hmul_(h, slope)); }
     }
-    const __half* W = (const __half*)lp.weights;
-    for (int i = 0; i < In; ++i) {
-        __half r = __float2half_rn(0.0f);
-        for (int j = 0; j < Out; ++j) r = hadd_(r, hmul_(W[j * In + i], g[j]));
-        dx[i] = r;
-    }
 }
 
 // Like ex_accumulate, with the weight gradient in the one-tile training-optimal layout.
-template <int In, int Out>
+template <int In, int Out, int FIRST>
 __device__ void cv_accumulate(const MlpLayerPointers& lp, const __half* sg, const __half* sx, int n_valid, int gstride,
                               int xstride)
 {
     __half* dW = (__half*)lp.weightsGrad;
     __half* dB = (__half*)lp.biasesGrad;
     const bool single = gridDim.x == 1;
-    for (int p = threadIdx.x; p < In * Out + Out; p += blockDim.x) {
+    const int p = (int)threadIdx.x - FIRST;
+    if (p >= 0 && p < In * Out + Out) {
         const bool is_w = p < In * Out;
         const int i = is_w ? p / In : p - In * Out, j = is_w ? p % In : 0;
         __half* dst = is_w ? dW + i * 16 + j : dB + i;
@@ -242,16 +267,20 @@ learnGradient_coopvec(const MlpLayerPointers* __restrict__ network, uint32_t* lo
 
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = tid < count;
+    grid_release();
+    grid_wait();
     const MlpLayerPointers L1 = network[0], L2 = network[1];
+    __shared__ ExampleParams s_p;
+    ex_stage(s_p, L1, L2);
     float this_loss = 0.0f;
     if (valid) {
         const float2 in = inputs[tid];
         const __half x = __float2half_rn(in.x), y = __float2half_rn(in.y);
         __half enc[4] = {x, y, hmul_(x, x), hmul_(y, y)};
-        __half o1[16], h1[16], o2[4], out[4], g2[4], g1[16], dead[4];
-        cv_layer_sums<4, 16>(L1, enc, o1);
+        __half o1[16], h1[16], o2[4], out[4], g2[4], g1[16];
+        cv_layer_sums<4, 16>(s_p.w1, s_p.b1, enc, o1);
         cv_activation<16>(o1, h1);
-        cv_layer_sums<16, 4>(L2, h1, o2);
+        cv_layer_sums<16, 4>(s_p.w2, s_p.b2, h1, o2);
         cv_activation<4>(o2, out);
         const __half one = __float2half_rn(1.0f), half_ = __float2half_rn(0.5f);
         __half gt[4];
@@ -266,16 +295,17 @@ learnGradient_coopvec(const MlpLayerPointers* __restrict__ network, uint32_t* lo
             l = hadd_(l, hmul_(d, d));
         }
         this_loss = __half2float(l);
-        cv_layer_bwd<16, 4>(L2, o2, g2, g1);
-        cv_layer_bwd<4, 16>(L1, o1, g1, dead);
+        cv_activation_bwd<4>(o2, g2);
+        ex_input_bwd<16, 4>(s_p.w2, g2, g1);
+        cv_activation_bwd<16>(o1, g1);
         for (int k = 0; k < 4; ++k) { s_enc[threadIdx.x * 4 + k] = enc[k]; s_g2[threadIdx.x * 4 + k] = g2[k]; }
         for (int k = 0; k < 16; ++k) { s_h1[threadIdx.x * 16 + k] = h1[k]; s_g1[threadIdx.x * 16 + k] = g1[k]; }
     }
     __syncthreads();
     const int first = blockIdx.x * blockDim.x;
     const int n_valid = count > (uint32_t)first ? min((int)blockDim.x, (int)(count - first)) : 0;
-    cv_accumulate<16, 4>(L2, s_g2, s_h1, n_valid, 4, 16);
-    cv_accumulate<4, 16>(L1, s_g1, s_enc, n_valid, 16, 4);
+    cv_accumulate<16, 4, 0>(L2, s_g2, s_h1, n_valid, 4, 16);
+    cv_accumulate<4, 16, 96>(L1, s_g1, s_enc, n_valid, 16, 4);
 
     float m = this_loss;
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -286,12 +316,15 @@ extern "C" __global__ void __launch_bounds__(256)
 adjustParameters(MlpExampleAdamState* states, __half* params, __half* gradients, uint32_t count)
 {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_release();
+    grid_wait();
     if (tid >= count) return;
     __half g = gradients[tid];
+    MlpExampleAdamState st = states[tid];
+    __half p = params[tid];
     if (__hisnan(g)) { gradients[tid] = __float2half_rn(0.0f); return; }
     const __half beta1 = __float2half_rn(0.9f), beta2 = __float2half_rn(0.999f);
     const __half eps = __float2half_rn(1e-7f), lr = __float2half_rn(0.01f), one = __float2half_rn(1.0f);
-    MlpExampleAdamState st = states[tid];
     st.iteration++;
     if (__hisinf(g)) g = __float2half_rn(__half2float(g) > 0.0f ? 10000.0f : -10000.0f);
     __half m = __ushort_as_half(st.mean), v = __ushort_as_half(st.variance);
@@ -304,7 +337,6 @@ adjustParameters(MlpExampleAdamState* states, __half* params, __half* gradients,
     const __half var_hat = hdiv_(v, hsub_(one, p2));
     const __half mx = __half2float(var_hat) > 0.0f ? var_hat : __float2half_rn(0.0f);
     const __half den = __float2half_rn(__fsqrt_rn(__half2float(hadd_(mx, eps))));
-    __half p = params[tid];
     p = hsub_(p, hdiv_(hmul_(lr, mean_hat), den));
     params[tid] = p;
     st.mean = __half_as_ushort(m);

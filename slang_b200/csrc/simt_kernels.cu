@@ -532,23 +532,17 @@ static bool make_simt_net(const MlpConfig& c, SimtNet* net, std::string* err)
 
 cudaError_t launch_example_learn_gradient(cudaStream_t st, const MlpLearnGradParams& a, uint32_t grid)
 {
-    learnGradient<<<grid, 256, 0, st>>>((const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer,
-                                        (const float2*)a.inputs, a.count);
-    return cudaGetLastError();
+    return launch_after(st, learnGradient, grid, 256, 0, (const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer, (const float2*)a.inputs, a.count);
 }
 
 cudaError_t launch_example_learn_gradient_coopvec(cudaStream_t st, const MlpLearnGradParams& a, uint32_t grid)
 {
-    learnGradient_coopvec<<<grid, 256, 0, st>>>((const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer,
-                                                (const float2*)a.inputs, a.count);
-    return cudaGetLastError();
+    return launch_after(st, learnGradient_coopvec, grid, 256, 0, (const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer, (const float2*)a.inputs, a.count);
 }
 
 cudaError_t launch_example_adjust_parameters(cudaStream_t st, const MlpAdjustParamsParams& a, uint32_t grid)
 {
-    adjustParameters<<<grid, 256, 0, st>>>((MlpExampleAdamState*)a.adamStates, (__half*)a.params, (__half*)a.gradients,
-                                           a.count);
-    return cudaGetLastError();
+    return launch_after(st, adjustParameters, grid, 256, 0, (MlpExampleAdamState*)a.adamStates, (__half*)a.params, (__half*)a.gradients, a.count);
 }
 
 cudaError_t launch_forward_simt(cudaStream_t st, const MlpConfig& c, const MlpForwardParams& a, int* launches,
