@@ -13,6 +13,11 @@ import numpy as np
 from . import config as C
 from .lib import check, load
 
+try:
+    from . import _fastcall as _F   # the per-step calls; bound when the library is loaded
+except ImportError:                 # not built yet: load() says so
+    _F = None
+
 
 class LearnGradParams(ctypes.Structure):
     _fields_ = [("networkBuffer", ctypes.c_uint64), ("lossBuffer", ctypes.c_uint64),
@@ -47,10 +52,13 @@ FLAG_INPUT_GRADIENT = 4
 class Buffer:
     def __init__(self, device, handle, size):
         self.device, self.handle, self.size = device, handle, size
+        self._h = handle.value
         self.address = load().mlp_buffer_address(handle)
 
     def clear(self, offset=0, size=None):
-        check(load().mlp_buffer_clear(self.device.handle, self.handle, offset, self.size - offset if size is None else size))
+        rc = _F.clear(self.device._h, self._h, offset, self.size - offset if size is None else size)
+        if rc:
+            check(rc)
 
     def read(self, dtype=np.uint8, offset=0, size=None):
         size = self.size - offset if size is None else size
@@ -66,16 +74,19 @@ class Buffer:
     def destroy(self):
         if self.handle:
             load().mlp_buffer_destroy(self.handle)
-            self.handle = None
+            self.handle, self._h = None, 0
 
 
 class Kernel:
     def __init__(self, device, handle):
         self.device, self.handle = device, handle
+        self._h = handle.value
         self.implementation = load().mlp_kernel_implementation(handle).decode()
 
     def dispatch(self, args, groups):
-        check(load().mlp_dispatch(self.device.handle, self.handle, ctypes.byref(args), ctypes.sizeof(args), groups, 1, 1))
+        rc = _F.dispatch(self.device._h, self._h, args, groups)
+        if rc:
+            check(rc)
 
 
 class Device:
@@ -87,6 +98,7 @@ class Device:
             # `stream` is a cudaStream_t as an integer (0 = the legacy default stream)
             check(load().mlp_device_create_on_stream(ordinal, ctypes.c_void_p(stream), ctypes.byref(h)))
         self.handle = h
+        self._h = h.value
         self.ordinal = ordinal
         # the cudaStream_t the kernels run on when the caller supplied it; None when the library
         # created its own stream, which a caller cannot order other work against
@@ -144,7 +156,7 @@ class Device:
     def destroy(self):
         if self.handle:
             load().mlp_device_destroy(self.handle)
-            self.handle = None
+            self.handle, self._h = None, 0
 
 
 def groups_for(count):
@@ -250,19 +262,24 @@ class Trainer:
         input_grads_address the gradient with respect to the inputs ([count][dims[0]] fp32) is written too."""
         if clear_loss:
             self.loss.clear()
-        args = LearnGradParamsEx(self.network.address, self.loss.address, inputs_address, targets_address, count, flags)
         if input_grads_address:
-            args.flags |= FLAG_INPUT_GRADIENT
-            args = LearnGradParamsEx2(args, input_grads_address)
-        self.k_learn.dispatch(args, groups_for(count))
+            flags |= FLAG_INPUT_GRADIENT
+        rc = _F.learn(self.device._h, self.k_learn._h, self.network.address, self.loss.address, inputs_address, targets_address, count, flags,
+                      input_grads_address, (count + 255) // 256)
+        if rc:
+            check(rc)
 
     def adjust_parameters(self):
-        args = AdjustParamsParams(self.states.address, self.params.address, self.grads.address, self.total)
-        self.k_adjust.dispatch(args, groups_for(self.total))
+        rc = _F.adjust(self.device._h, self.k_adjust._h, self.states.address, self.params.address, self.grads.address, self.total,
+                       (self.total + 255) // 256)
+        if rc:
+            check(rc)
 
     def forward(self, inputs_address, outputs_address, count, flags=0):
-        args = ForwardParams(self.network.address, inputs_address, outputs_address, count, flags)
-        self.k_forward.dispatch(args, groups_for(count))
+        rc = _F.forward(self.device._h, self.k_forward._h, self.network.address, inputs_address, outputs_address, count, flags,
+                        (count + 255) // 256)
+        if rc:
+            check(rc)
 
     def read_loss(self):
         """(largest per-sample loss, sum of per-sample losses) of the last learnGradient."""

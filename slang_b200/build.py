@@ -4,7 +4,8 @@
 
 Each translation unit is compiled to an object with its own flags (stale units side by side, one nvcc
 process each) and the objects are linked into slang_b200/libslang_b200_mlp.so; the literal example
-entry points are also built into a stand-alone device module, slang_b200/mlp_training_kernels.cubin.
+entry points are also built into a stand-alone device module, slang_b200/mlp_training_kernels.cubin, and the
+per-step calls of Python hosts into a small extension, slang_b200/_fastcall.so.
 A unit is stale when its source, or any header its last compile read (nvcc -MD), is newer than its
 object.  The CUDA runtime is linked statically so the library has no dependency beyond the driver.
 """
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -21,6 +23,9 @@ OBJDIR = os.path.join(HERE, "build")
 # Stand-alone device module holding the literal example entry points (for cuModuleLoadData hosts).
 CUBIN = os.path.join(HERE, "mlp_training_kernels.cubin")
 CUBIN_SRC = "example_module.cu"
+# The per-step calls for Python hosts (CPython extension).
+FASTCALL = os.path.join(HERE, "_fastcall.so")
+FASTCALL_SRC = "fastcall.c"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
@@ -134,6 +139,13 @@ def build(force=False, verbose=False, jobs=None, without=(), out=None):
     cd = os.path.join(OBJDIR, "example_module.d")
     if force or _stale(CUBIN, cs, cd):
         cmd = [nvcc, "-arch=sm_100a", "-cubin", "-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-MD", "-MF", cd, cs, "-o", CUBIN]
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.check_call(cmd)
+    fs = os.path.join(CSRC, FASTCALL_SRC)
+    fd = os.path.join(OBJDIR, "fastcall.d")
+    if force or _stale(FASTCALL, fs, fd):
+        cmd = ["gcc", "-O2", "-std=c11", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-MD", "-MF", fd, fs, "-o", FASTCALL]
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.check_call(cmd)

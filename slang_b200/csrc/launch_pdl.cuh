@@ -9,10 +9,26 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace mlpb200 {
 
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A kernel's dynamic shared-memory limit, raised once per device instead of on every launch (one static object per kernel;
+// the attribute outlives the call, and raising it twice from two threads does no harm).
+struct SmemLimit {
+    std::atomic<uint64_t> raised{0};   // bit d: device d
+    cudaError_t raise(const void* kernel, int device, size_t bytes)
+    {
+        const uint64_t bit = device >= 0 && device < 64 ? uint64_t(1) << device : 0;
+        if (raised.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess) raised.fetch_or(bit, std::memory_order_relaxed);
+        return e;
+    }
+};
 
 template <class... P, class... A>
 inline cudaError_t launch_after(cudaStream_t st, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, A&&... args)

@@ -589,7 +589,8 @@ cudaError_t launch_learn_gradient_simt(cudaStream_t st, const MlpConfig& c, cons
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSimtSmemMax));
+    static SmemLimit limit[2];   // one per build
+    if (e == cudaSuccess) e = limit[map.w >= 0].raise((const void*)kern, device, kSimtSmemMax);
     if (e != cudaSuccess) return e;
     // As many CTAs as are resident at once (512 threads each), each walking its share of the tiles.
     const uint32_t tiles = (a.count + kTile - 1) / kTile;

@@ -473,7 +473,8 @@ static cudaError_t launch_fwd(cudaStream_t st, TcWorkspace* ws, const MlpConfig&
     p.act_alpha = c.act_alpha;
     p.out_storage = (a.flags & MLP_FLAG_OUTPUT_STORAGE_TYPE) ? 1u : 0u;
     auto kern = fwd::forward_tc_kernel<DIN, DH, DOUT, NL, FMT, ACT, OUT_ACT, NCH, CS, CPS, NCW>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmemBytes);
+    static SmemLimit limit;
+    const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, G::kSmemBytes);
     if (e != cudaSuccess) return e;
     const uint32_t slots = (uint32_t)ws->sm_count * (uint32_t)CPS;
     const uint32_t grid = p.n_tiles < slots ? p.n_tiles : slots;

@@ -32,6 +32,7 @@
 
 #include <string>
 
+#include "launch_pdl.cuh"
 #include "launchers.h"
 #include "mlp_common.cuh"
 #include "tc_host.h"
@@ -1142,10 +1143,11 @@ static cudaError_t launch_wide(cudaStream_t st, TcWorkspace* ws, const CUtensorM
                                const WideTrainParams& p)
 {
     auto kern = learn_gradient_wide_kernel<FMT, ACT, NL, FWD, F32S, XTRA>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide::kSmemBytes);
+    static SmemLimit limit;
+    const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, wide::kSmemBytes);
     if (e != cudaSuccess) return e;
     const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
-    kern<<<grid, wide::kThreads, wide::kSmemBytes, st>>>(mx, mt, p);
+    kern<<<grid, wide::kThreads, wide::kSmemBytes, st>>>(mx, mt, p);   // (launched to overlap its predecessor it was 2 us slower)
     return cudaGetLastError();
 }
 

@@ -801,7 +801,8 @@ static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params
     constexpr int NG = W == 32 ? 8 : state <= 4 ? 3 : state <= 5 ? 5 : 7, GW = W == 32 ? 1 : state <= 4 ? 5 : state <= 5 ? 2 : 1;
     using M = narrow::TrainMap<W, NL, NG, GW>;
     auto kern = narrow::learn_gradient_narrow_kernel<W, NL, FMT, HACT, OT, NG, GW>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::kSmemBytes);
+    static SmemLimit limit;
+    const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, M::kSmemBytes);
     if (e != cudaSuccess) return e;
     p.n_tiles = (uint32_t)(((uint64_t)p.count + M::kUnit - 1) / M::kUnit);
     const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
@@ -839,7 +840,8 @@ static cudaError_t launch_forward(cudaStream_t st, TcWorkspace* ws, narrow::Para
     p.raw_bytes = 0;
     for (int l = 0; l < p.cfg.n_layers; ++l) p.raw_bytes += (int)((narrow::stored_weight_bytes(p.cfg, l) + 15u) & ~15u);
     const size_t smem = (size_t)p.cfg.n_layers * ((W + 31) / 32 * (W / 8) * 512 + W * 8 + 32) + 48 + (size_t)p.raw_bytes;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit limit;   // (of the largest network, whatever this one needs)
+    const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, 5 * ((W + 31) / 32 * (W / 8) * 512 + W * 8 + 32) + 48 + 5 * W * W * 4);
     if (e != cudaSuccess) return e;
     constexpr uint32_t per_tile = narrow::kForwardWarps * 16 * MT;
     p.n_tiles = (uint32_t)(((uint64_t)p.count + per_tile - 1) / per_tile);

@@ -93,6 +93,8 @@ def load():
         fn = getattr(L, name)
         if fn.restype is ctypes.c_int:
             fn.restype = i32
+    from . import _fastcall
+    _fastcall.bind(ctypes.cast(L.mlp_dispatch, ctypes.c_void_p).value, ctypes.cast(L.mlp_buffer_clear, ctypes.c_void_p).value)
     _lib = L
     return L
 

@@ -21,6 +21,8 @@ class TorchTrainer:
             raise RuntimeError("a CUDA device is required (the library has no CPU fallback)")
         idx = torch.cuda.current_device() if device_index is None else device_index
         self.cfg = cfg
+        self.in_width, self.out_width = int(cfg.input_width), int(cfg.out_dim)
+        self.in_dtype, self.target_dtype = TORCH_DTYPE[cfg.input_dtype], TORCH_DTYPE[cfg.target_dtype]
         self.stream = torch.cuda.current_stream(idx)
         self.device = Device(idx, self.stream.cuda_stream)
         _, _, total = C.param_layout(cfg)
@@ -33,15 +35,15 @@ class TorchTrainer:
         """The tensor as dense rows.  The kernels read dense [count, width] rows; a strided view (a column
         slice, a transposed or stepped view: what the reference's TensorView reads through its strides,
         bindless-storage.slang:247-336) is packed by one strided copy on the same stream first."""
-        if not (t.is_cuda and t.dim() == 2 and t.shape[1] == width and t.dtype == TORCH_DTYPE[dtype]):
-            raise ValueError("%s must be a CUDA tensor [count, %d] of %s" % (what, width, TORCH_DTYPE[dtype]))
+        if not (t.is_cuda and t.dim() == 2 and t.shape[1] == width and t.dtype == dtype):
+            raise ValueError("%s must be a CUDA tensor [count, %d] of %s" % (what, width, dtype))
         if t.device.index != self.device.ordinal:
             raise ValueError("%s lives on another device" % what)
         return t if t.is_contiguous() else t.contiguous()
 
     def learn_gradient(self, inputs, targets, flags=0):
-        inputs = self._rows(inputs, self.cfg.input_width, self.cfg.input_dtype, "inputs")
-        targets = self._rows(targets, self.cfg.out_dim, self.cfg.target_dtype, "targets")
+        inputs = self._rows(inputs, self.in_width, self.in_dtype, "inputs")
+        targets = self._rows(targets, self.out_width, self.target_dtype, "targets")
         if inputs.shape[0] != targets.shape[0]:
             raise ValueError("inputs and targets disagree on the sample count")
         self.trainer.learn_gradient(inputs.data_ptr(), targets.data_ptr(), inputs.shape[0], flags)
@@ -52,13 +54,11 @@ class TorchTrainer:
     def forward(self, inputs, out=None):
         """Network outputs as fp32 [count, out_dim]; `out` may be any fp32 view of that shape (a strided one is
         filled through a dense temporary)."""
-        inputs = self._rows(inputs, self.cfg.input_width, self.cfg.input_dtype, "inputs")
-        dense = torch.empty((inputs.shape[0], self.cfg.out_dim), dtype=torch.float32, device=inputs.device)
-        if out is not None:
-            if not (out.is_cuda and out.dtype == torch.float32 and tuple(out.shape) == tuple(dense.shape)):
-                raise ValueError("out must be a CUDA fp32 tensor [count, %d]" % self.cfg.out_dim)
-            if out.is_contiguous():
-                dense = out
+        inputs = self._rows(inputs, self.in_width, self.in_dtype, "inputs")
+        shape = (inputs.shape[0], self.out_width)
+        if out is not None and not (out.is_cuda and out.dtype == torch.float32 and tuple(out.shape) == shape):
+            raise ValueError("out must be a CUDA fp32 tensor [count, %d]" % self.out_width)
+        dense = out if out is not None and out.is_contiguous() else inputs.new_empty(shape, dtype=torch.float32)
         self.trainer.forward(inputs.data_ptr(), dense.data_ptr(), inputs.shape[0])
         if out is not None and dense is not out:
             out.copy_(dense)
