@@ -128,7 +128,7 @@ constexpr int kTile = 32;                   // samples per tile, one per lane
 constexpr int kRow = kTile + 4;             // floats per feature row: 16-byte reads of eight consecutive rows hit distinct banks
 constexpr int kSimtThreads = 512;
 constexpr int kSimtWarps = kSimtThreads / 32;
-constexpr size_t kSimtSmemMax = 227 * 1024;
+constexpr size_t kSimtSmemMax = 226 * 1024;   // (beside the layer addresses)
 
 // Shared-memory map of a network, in floats: feature rows of a_0 .. a_{nl-1} and the outputs (a_off[l] * kRow), then
 // of z_1 .. z_nl, then biases, and where there is room the weights (rows padded to multiples of four) and the
@@ -229,21 +229,32 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
     float* const s_z = smem + map.z;              // z rows, later dz: layer l's outputs from row a_off[l + 1] - a_off[1]
     auto z_rows = [&](int l) { return s_z + (net.a_off[l] - net.a_off[1]) * kRow; };   // of the vector leaving layer l - 1
 
-    for (int l = 0; l < nl; ++l) {
-        const int in = c.dims[l], out = c.dims[l + 1];
-        const MlpLayerPointers ptr = lp[l];
-        for (int j = threadIdx.x; j < out; j += kSimtThreads) smem[map.bias + map.b_off[l] + j] = load_as_f32(c.dtype, (const void*)ptr.biases, j);
+    // Addresses first, then every layer's parameters without waiting in between.
+    __shared__ MlpLayerPointers s_net[MLP_MAX_LAYERS];
+    if (threadIdx.x < nl * 4) reinterpret_cast<uint64_t*>(s_net)[threadIdx.x] = reinterpret_cast<const uint64_t*>(lp)[threadIdx.x];
+    __syncthreads();
+    {
+        int i = threadIdx.x;
+        for (int l = 0; l < nl; ++l) {
+            const int out = c.dims[l + 1];
+            for (; i < out; i += kSimtThreads) smem[map.bias + map.b_off[l] + i] = load_as_f32(c.dtype, (const void*)s_net[l].biases, i);
+            i -= out;
+        }
         if constexpr (STAGED) {
-            const int stride = (in + 3) & ~3;
-            for (int idx = threadIdx.x; idx < out * stride; idx += kSimtThreads) {
-                const int j = idx / stride, i = idx - j * stride;
-                smem[map.w + map.w_off[l] + idx] =
-                    i < in ? load_weight(c, (const void*)ptr.weights, weight_index(c.param_layout, in, out, j, i)) : 0.0f;
+            for (int l = 0; l < nl; ++l) {
+                const int in = c.dims[l], out = c.dims[l + 1], stride = (in + 3) & ~3;
+#pragma unroll 4
+                for (; i < out * stride; i += kSimtThreads) {
+                    const int j = i / stride, k = i - j * stride;
+                    smem[map.w + map.w_off[l] + i] =
+                        k < in ? load_weight(c, (const void*)s_net[l].weights, weight_index(c.param_layout, in, out, j, k)) : 0.0f;
+                }
+                i -= out * stride;
             }
         }
     }
     auto weights = [&](int l) {
-        return WeightRows<STAGED>{c, STAGED ? nullptr : (const void*)lp[l].weights, STAGED ? smem + map.w + map.w_off[l] : nullptr,
+        return WeightRows<STAGED>{c, STAGED ? nullptr : (const void*)s_net[l].weights, STAGED ? smem + map.w + map.w_off[l] : nullptr,
                                   c.dims[l], c.dims[l + 1], (c.dims[l] + 3) & ~3};
     };
 
@@ -268,6 +279,9 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
             }
             smem[i * kRow + s] = v;
         }
+        // up to sixteen targets of a sample, a warp each, are fetched a forward pass ahead of their use
+        float target = 0.0f;
+        if (warp < od && valid) target = load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + warp);
         __syncthreads();
         // ---- forward ----
         for (int l = 0; l < nl; ++l) {
@@ -296,7 +310,7 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
             for (int j = warp; j < od; j += kSimtWarps) {
                 float g = 0.0f;
                 if (valid) {
-                    const float diff = o[j * kRow] - load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j);
+                    const float diff = o[j * kRow] - (j == warp ? target : load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j));
                     g = round_to(opd, ((2.0f * scale) * diff) * act_deriv(c.output_act, c.act_alpha, dz[j * kRow]));
                 }
                 dz[j * kRow] = g;
@@ -304,7 +318,7 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
             if (warp == 0 && valid) {
                 float loss = 0.0f;
                 for (int j = 0; j < od; ++j) {
-                    const float diff = o[j * kRow] - load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j);
+                    const float diff = o[j * kRow] - (j == 0 ? target : load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j));
                     loss = fmaf(diff * scale, diff, loss);
                 }
                 run_max = fmaxf(run_max, loss);
@@ -387,9 +401,9 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
                     float* g = smem + map.grads + map.g_off[l] + j * (in + 1) + i0;
                     for (int u = 0; u < n; ++u) g[u] = tile == blockIdx.x ? acc[u] : g[u] + acc[u];
                 } else if (i0 == in) {
-                    atomicAdd((float*)lp[l].biasesGrad + j, acc[0]);
+                    atomicAdd((float*)s_net[l].biasesGrad + j, acc[0]);
                 } else {
-                    for (int u = 0; u < n; ++u) atomicAdd((float*)lp[l].weightsGrad + weight_index(c.param_layout, in, out, j, i0 + u), acc[u]);
+                    for (int u = 0; u < n; ++u) atomicAdd((float*)s_net[l].weightsGrad + weight_index(c.param_layout, in, out, j, i0 + u), acc[u]);
                 }
             }
         }
@@ -398,8 +412,8 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
     if (!seq_scratch && !once && map.grads >= 0) {
         for (int l = 0; l < nl; ++l) {
             const int in = c.dims[l], out = c.dims[l + 1];
-            float* dW = (float*)lp[l].weightsGrad;
-            float* dB = (float*)lp[l].biasesGrad;
+            float* dW = (float*)s_net[l].weightsGrad;
+            float* dB = (float*)s_net[l].biasesGrad;
             for (int item = threadIdx.x; item < out * (in + 1); item += kSimtThreads) {
                 const int j = item / (in + 1), i = item - j * (in + 1);
                 const float g = smem[map.grads + map.g_off[l] + item];
