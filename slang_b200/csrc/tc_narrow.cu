@@ -299,9 +299,13 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
                                 a = C::max2(C::pack2(z0, z1), 0x80008000u);
                                 zero_seen |= (a - 0x00010001u) & ~a;   // bit 15 of a half: the half is +0
                             } else if constexpr (HACT == MLP_ACT_LEAKY_RELU) {
-                                // max(z, alpha z) with 0 <= alpha < 1 (the launcher sees to it); the sign bit is "z < 0"
-                                const float2 az = __fmul2_rn(make_float2(z0, z1), make_float2(alpha, alpha));
-                                a = C::max2(C::pack2(z0, z1), C::pack2(az.x, az.y));
+                                // max(z, alpha z) with 0 < alpha < 1 (the launcher sees to it), from the rounded z where
+                                // z is rounded.  The sign bit is "z < 0": adding +0 to alpha z makes a zero z of either
+                                // sign a positive zero, while an alpha z that only rounds to zero keeps its sign.
+                                const uint32_t zp = C::pack2(z0, z1);
+                                if (!f32s) { z0 = C::lo(zp); z1 = C::hi(zp); }
+                                const float2 az = __ffma2_rn(make_float2(z0, z1), make_float2(alpha, alpha), make_float2(0.0f, 0.0f));
+                                a = C::max2(zp, C::pack2(az.x, az.y));
                             } else {
                                 if (!f32s) {
                                     const uint32_t zp = C::pack2(z0, z1);
@@ -713,12 +717,12 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
                     if constexpr (HACT == MLP_ACT_RELU) {
                         a = C::relu2(zp);
                     } else {
+                        if (!f32s) { z0 = C::lo(zp); z1 = C::hi(zp); }
                         if constexpr (HACT == MLP_ACT_LEAKY_RELU) {
                             const float2 az = __fmul2_rn(make_float2(z0, z1), make_float2(alpha, alpha));
                             a = C::max2(zp, C::pack2(az.x, az.y));
                             continue;
                         }
-                        if (!f32s) { z0 = C::lo(zp); z1 = C::hi(zp); }
                         if constexpr (HACT == MLP_ACT_GELU_TANH) {
                             a = C::pack2(act_value(MLP_ACT_GELU_TANH, alpha, z0), act_value(MLP_ACT_GELU_TANH, alpha, z1));
                         } else {

@@ -483,10 +483,11 @@ __device__ __forceinline__ void activate_any(int act, float alpha, float (&v)[N]
     }
 }
 
-// The hidden activation a network's build is chosen by: leaky ReLU as max(z, alpha z) needs 0 <= alpha < 1.
+// The hidden activation a network's build is chosen by: leaky ReLU as max(z, alpha z) needs 0 < alpha < 1 (at zero, an
+// infinite z would not give the NaN that alpha z is).
 inline int built_activation(const MlpConfig& c)
 {
-    if (c.hidden_act == MLP_ACT_LEAKY_RELU && !(c.act_alpha >= 0.0f && c.act_alpha < 1.0f)) return -1;
+    if (c.hidden_act == MLP_ACT_LEAKY_RELU && !(c.act_alpha > 0.0f && c.act_alpha < 1.0f)) return -1;
     return c.hidden_act;
 }
 

@@ -1,0 +1,102 @@
+"""The arithmetic of hidden activations in the kernels for widths up to 64, where it shows: the activation takes the
+pre-activation as it is rounded to the storage type, and a pre-activation that rounds to zero, from either side, is a
+zero (with fp32 storage it is not rounded and keeps its side)."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from slang_b200 import config as C
+
+from mlp_testlib import layer_rel_errs, rel_err
+
+pytestmark = pytest.mark.gpu
+
+STORAGE = {"f16": (C.F16, 0), "bf16": (C.BF16, 0), "f32-f16": (C.F32, C.F16)}
+
+
+@pytest.fixture(scope="module")
+def device():
+    from slang_b200.api import Device
+    d = Device(0)
+    yield d
+    d.destroy()
+
+
+def _config(dims, storage, act, **more):
+    dtype, operand = STORAGE[storage]
+    return C.make_config(dims, dtype, act, input_dtype=C.F32, target_dtype=C.F32, adam_master=0 if dtype == C.F32 else 1,
+                         operand_dtype=operand, **more)
+
+
+@pytest.mark.parametrize("alpha", [0.01, 0.3])
+@pytest.mark.parametrize("storage", list(STORAGE))
+@pytest.mark.parametrize("width", [12, 24, 40])
+def test_leaky_relu_takes_the_rounded_preactivation(device, width, storage, alpha):
+    """One sample through 2-width-width whose every sum is exact in fp32 and whose second layer is the identity: outputs
+    and gradients have to equal the oracle's bit for bit."""
+    from slang_b200.api import Trainer
+    cfg = _config([2, width, width], storage, C.ACT_LEAKY_RELU, act_alpha=alpha)
+    rng = np.random.default_rng(width)
+    w_off, b_off, total = C.param_layout(cfg)
+    p = np.zeros(total, dtype=np.float32)
+    w0 = np.empty((width, 2), dtype=np.float32)
+    w0[:, 0] = -rng.integers(64, 128, width) / 128.0    # times x_0: eleven bits, and a few more below them from x_1
+    w0[:, 1] = rng.integers(-7, 8, width) / 8192.0
+    p[w_off[0]:w_off[0] + 2 * width] = w0.ravel()
+    p[w_off[1]:w_off[1] + width * width] = np.eye(width, dtype=np.float32).ravel()
+    params = C.to_storage(p, cfg.dtype)
+    x = np.array([[13.0 / 16.0, 1.0]], dtype=np.float32)
+    t = rng.uniform(-1, 1, (1, width)).astype(np.float32)
+    tr = Trainer(device, cfg, params)
+    xb, tb, yb = device.create_buffer(x.nbytes, x), device.create_buffer(t.nbytes, t), device.create_buffer(4 * width)
+    tr.forward(xb.address, yb.address, 1)
+    assert np.array_equal(yb.read(np.float32), np.asarray(oracle.forward(cfg, params, x, 1), dtype=np.float32).ravel())
+    want = np.zeros(total, dtype=np.float32)
+    oracle.learn_gradient(cfg, params, want, x, t, 1)
+    tr.learn_gradient(xb.address, tb.address, 1)
+    assert np.array_equal(tr.read_grads(), want)
+
+
+def _around_zero(device, dims, storage, act):
+    """Three samples in four have one input, the smallest half above zero: every first-layer pre-activation is a product
+    of less than half of it (biases are zero), of either sign.  Gradients, input gradients and loss against the oracle."""
+    from slang_b200.api import Trainer
+    cfg = _config(dims, storage, act, act_alpha=0.02)
+    count = 500
+    rng = np.random.default_rng(sum(dims))
+    params = C.init_params(cfg, seed=4, scheme="xavier")
+    p = C.from_storage(params, cfg.dtype).copy()
+    w_off, b_off, total = C.param_layout(cfg)
+    w0 = p[w_off[0]:w_off[0] + dims[0] * dims[1]]
+    w0 *= 0.45 / np.abs(w0).max()
+    for l in range(1, len(dims) - 1):
+        p[b_off[l]:b_off[l] + dims[l + 1]] = rng.uniform(-0.5, 0.5, dims[l + 1])
+    params = C.to_storage(p, cfg.dtype)
+    x = rng.uniform(-1, 1, (count, dims[0])).astype(np.float32)
+    small = np.arange(count) % 4 != 0
+    x[small] = 0.0
+    x[small, rng.integers(0, dims[0], count)[small]] = np.float32(2.0 ** -24)
+    t = rng.uniform(-1, 1, (count, dims[-1])).astype(np.float32)
+    want, words = np.zeros(total, dtype=np.float32), np.zeros(2, dtype=np.uint32)
+    want_dx = oracle.learn_gradient_inputs(cfg, params, want, x, t, count, words)
+    tr = Trainer(device, cfg, params)
+    xb, tb = device.create_buffer(x.nbytes, x), device.create_buffer(t.nbytes, t)
+    dxb = device.create_buffer(want_dx.nbytes)
+    tr.learn_gradient(xb.address, tb.address, count, input_grads_address=dxb.address)
+    # 1e-2: the bar of 16-bit gradients in these tests; a derivative of 0, 1/2, alpha or 1 in another's place is 0.1 to 1
+    assert max(layer_rel_errs(cfg, tr.read_grads(), want)) < 1e-2
+    dx = dxb.read(np.float32).reshape(want_dx.shape)
+    assert rel_err(dx, want_dx) < 1e-2
+    assert rel_err(dx[small], want_dx[small]) < 1e-2
+    largest, total_loss = tr.read_loss()
+    ref = words.view(np.float32)
+    assert abs(largest - ref[0]) <= 1e-3 * ref[0] and abs(total_loss - ref[1]) <= 1e-3 * ref[1]
+
+
+AROUND_ZERO = [[4, 32, 32, 4], [32, 24, 3], [6, 64, 48, 64, 3], [40, 64, 20]]
+
+
+@pytest.mark.parametrize("storage", ["f16", "f32-f16"])
+@pytest.mark.parametrize("dims", AROUND_ZERO, ids=lambda d: "-".join(map(str, d)))
+def test_leaky_relu_around_zero(device, dims, storage):
+    _around_zero(device, dims, storage, C.ACT_LEAKY_RELU)
