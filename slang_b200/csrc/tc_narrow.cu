@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
             const uint64_t base = (uint64_t)unit * (uint64_t)M::kUnit + in_unit;
             uint32_t A[NL][MT][KS][4];                              // every layer's input
             uint32_t D[kKeepD ? NL - 1 : 1][MT][KS][4];             // derivatives of the hidden activations
-            uint32_t zero_seen = 0;                                 // ReLU: whether any pre-activation was exactly zero
+            bool zero_seen = false;                                 // ReLU: whether any pre-activation was zero
             {
                 // the next tile's input and target rows: start them on their way into L2
                 const uint64_t ns = base + (uint64_t)stride * (uint64_t)M::kUnit + (uint64_t)((c & 1) * 8) + (MT == 2 && (c & 2) ? 16u : 0u);
@@ -285,56 +285,86 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
                 if (l > 0 || in_steps == KS) layer_product<FMT, true, MT, NT, KS>(acc, A[l], fwd_panel + (uint32_t)l * M::kPanel, NT * 512u, start);
                 else if (in_steps == 2) layer_product<FMT, true, MT, NT, 2>(acc, A[l], fwd_panel, NT * 512u, start);
                 else layer_product<FMT, true, MT, NT, 1>(acc, A[l], fwd_panel, NT * 512u, start);
+                if constexpr (HACT == MLP_ACT_RELU) {
+                    // The backward pass recovers the derivative from the activation: one above zero, zero at +0, one half at
+                    // the -0 that marks a zero pre-activation (one that rounds to a zero of either sign).  Few fragments
+                    // hold one: the smallest magnitude is watched, one three-operand minimum for two values, and the marks
+                    // are set only where it calls for them (2^24 texels: 3.80 ms a step; with the sign of every value
+                    // settled in 16-bit arithmetic instead, 3.97 to 4.06).  Not rounded (fp32 storage), only a zero is
+                    // zero, and what lies above it stays there.
+                    if (f32s) {
 #pragma unroll
-                for (int m = 0; m < MT; ++m) {
+                        for (int i = 0; i < MT * NT * 4; ++i) {
+                            float& z = acc[i / (NT * 4)][i / 4 % NT][i & 3];
+                            z = z > 0.0f ? fmaxf(z, C::kSmallest) : z;
+                        }
+                    }
+                    const float tiny = f32s ? 0.0f : 0.5f * C::kSmallest;   // the largest magnitude that rounds to zero
+                    float least = 1.0f;
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) {
+                    for (int i = 0; i < MT * NT * 2; ++i) {
+                        const int m = i / (NT * 2), t = (i >> 1) % NT, h = i & 1;
+                        const float z0 = acc[m][t][2 * h], z1 = acc[m][t][2 * h + 1];
+                        A[l + 1][m][t >> 1][(t & 1) * 2 + h] = C::relu2(C::pack2(z0, z1));
+                        least = fminf(fminf(fabsf(z0), fabsf(z1)), least);
+                    }
+                    if (least <= tiny) {
+                        zero_seen = true;
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float z0 = acc[m][t][2 * h], z1 = acc[m][t][2 * h + 1];
+                        for (int i = 0; i < MT * NT * 2; ++i) {
+                            const int m = i / (NT * 2), t = (i >> 1) % NT, h = i & 1;
                             uint32_t& a = A[l + 1][m][t >> 1][(t & 1) * 2 + h];
-                            if constexpr (HACT == MLP_ACT_RELU) {
-                                // max(z, -0): below zero leaves a negative zero, so a z of exactly zero, whose derivative
-                                // is one half, is told apart by its positive one
-                                a = C::max2(C::pack2(z0, z1), 0x80008000u);
-                                zero_seen |= (a - 0x00010001u) & ~a;   // bit 15 of a half: the half is +0
-                            } else if constexpr (HACT == MLP_ACT_LEAKY_RELU) {
-                                // max(z, alpha z) with 0 < alpha < 1 (the launcher sees to it), from the rounded z where
-                                // z is rounded.  The sign bit is "z < 0": adding +0 to alpha z makes a zero z of either
-                                // sign a positive zero, while an alpha z that only rounds to zero keeps its sign.
-                                const uint32_t zp = C::pack2(z0, z1);
-                                if (!f32s) { z0 = C::lo(zp); z1 = C::hi(zp); }
-                                const float2 az = __ffma2_rn(make_float2(z0, z1), make_float2(alpha, alpha), make_float2(0.0f, 0.0f));
-                                a = C::max2(zp, C::pack2(az.x, az.y));
-                            } else {
-                                if (!f32s) {
+                            if (fabsf(acc[m][t][2 * h]) <= tiny) a |= 0x8000u;
+                            if (fabsf(acc[m][t][2 * h + 1]) <= tiny) a |= 0x80000000u;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+#pragma unroll
+                        for (int t = 0; t < NT; ++t) {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                float z0 = acc[m][t][2 * h], z1 = acc[m][t][2 * h + 1];
+                                uint32_t& a = A[l + 1][m][t >> 1][(t & 1) * 2 + h];
+                                if constexpr (HACT == MLP_ACT_LEAKY_RELU) {
+                                    // max(z, alpha z) with 0 < alpha < 1 (the launcher sees to it), from the rounded z where
+                                    // z is rounded.  The sign bit is "z < 0": adding +0 to alpha z makes a zero z of either
+                                    // sign a positive zero, while an alpha z that only rounds to zero keeps its sign.
                                     const uint32_t zp = C::pack2(z0, z1);
-                                    z0 = C::lo(zp);
-                                    z1 = C::hi(zp);
-                                }
-                                if constexpr (HACT == MLP_ACT_GELU_TANH) {
-                                    float v[2], d[2];
-                                    gelu_pair(z0, v[0], d[0]);
-                                    gelu_pair(z1, v[1], d[1]);
-                                    a = C::pack2(v[0], v[1]);
-                                    D[l][m][t >> 1][(t & 1) * 2 + h] = C::pack2(d[0], d[1]);
+                                    if (!f32s) { z0 = C::lo(zp); z1 = C::hi(zp); }
+                                    const float2 az = __ffma2_rn(make_float2(z0, z1), make_float2(alpha, alpha), make_float2(0.0f, 0.0f));
+                                    a = C::max2(zp, C::pack2(az.x, az.y));
                                 } else {
-                                    acc[m][t][2 * h] = z0;
-                                    acc[m][t][2 * h + 1] = z1;
+                                    if (!f32s) {
+                                        const uint32_t zp = C::pack2(z0, z1);
+                                        z0 = C::lo(zp);
+                                        z1 = C::hi(zp);
+                                    }
+                                    if constexpr (HACT == MLP_ACT_GELU_TANH) {
+                                        float v[2], d[2];
+                                        gelu_pair(z0, v[0], d[0]);
+                                        gelu_pair(z1, v[1], d[1]);
+                                        a = C::pack2(v[0], v[1]);
+                                        D[l][m][t >> 1][(t & 1) * 2 + h] = C::pack2(d[0], d[1]);
+                                    } else {
+                                        acc[m][t][2 * h] = z0;
+                                        acc[m][t][2 * h + 1] = z1;
+                                    }
                                 }
                             }
                         }
-                    }
-                    if constexpr (HACT < 0) {
-                        float v[NT * 4], d[NT * 4];
+                        if constexpr (HACT < 0) {
+                            float v[NT * 4], d[NT * 4];
 #pragma unroll
-                        for (int i = 0; i < NT * 4; ++i) v[i] = acc[m][i >> 2][i & 3];
-                        activate_any(cfg.hidden_act, alpha, v, d, true);
+                            for (int i = 0; i < NT * 4; ++i) v[i] = acc[m][i >> 2][i & 3];
+                            activate_any(cfg.hidden_act, alpha, v, d, true);
 #pragma unroll
-                        for (int i = 0; i < NT * 2; ++i) {
-                            const int t = i >> 1, h = i & 1;
-                            A[l + 1][m][t >> 1][(t & 1) * 2 + h] = C::pack2(v[t * 4 + 2 * h], v[t * 4 + 2 * h + 1]);
-                            D[l][m][t >> 1][(t & 1) * 2 + h] = C::pack2(d[t * 4 + 2 * h], d[t * 4 + 2 * h + 1]);
+                            for (int i = 0; i < NT * 2; ++i) {
+                                const int t = i >> 1, h = i & 1;
+                                A[l + 1][m][t >> 1][(t & 1) * 2 + h] = C::pack2(v[t * 4 + 2 * h], v[t * 4 + 2 * h + 1]);
+                                D[l][m][t >> 1][(t & 1) * 2 + h] = C::pack2(d[t * 4 + 2 * h], d[t * 4 + 2 * h + 1]);
+                            }
                         }
                     }
                 }
@@ -424,14 +454,14 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
                             }
                         }
                 if constexpr (HACT == MLP_ACT_RELU) {
-                    if (zero_seen & 0x80008000u) {   // some pre-activation was exactly zero: half of the gradient passes there
+                    if (zero_seen) {   // some pre-activation was zero: half of the gradient passes there
 #pragma unroll
                         for (int m = 0; m < MT; ++m)
 #pragma unroll
                             for (int i = 0; i < NT * 2; ++i) {
                                 const int t = i >> 1, h = i & 1;
                                 const uint32_t a = A[l][m][t >> 1][(t & 1) * 2 + h];
-                                const uint32_t zero = C::zero_mask(a) & ~sign_mask(a);
+                                const uint32_t zero = sign_mask(a);
                                 dz[m][t >> 1][(t & 1) * 2 + h] |= C::pack2(0.5f * acc[m][t][2 * h], 0.5f * acc[m][t][2 * h + 1]) & zero;
                             }
                     }

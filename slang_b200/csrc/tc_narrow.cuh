@@ -62,6 +62,7 @@ template <int FMT> struct Cvt;
 template <> struct Cvt<MLP_BF16> {
     static constexpr uint32_t kUmmaFmt = 1;
     static constexpr uint32_t kOnes = 0x3F803F80u;
+    static constexpr float kSmallest = 0x1p-133f;   // the smallest number above zero
     __device__ static __forceinline__ float round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
     __device__ static __forceinline__ uint32_t pack2(float lo, float hi)
     {
@@ -80,8 +81,7 @@ template <> struct Cvt<MLP_BF16> {
         const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
         return *reinterpret_cast<const uint32_t*>(&r);
     }
-    // 0xffff in the halves that are zero / above zero
-    __device__ static __forceinline__ uint32_t zero_mask(uint32_t z2) { return __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&z2), __floats2bfloat162_rn(0.0f, 0.0f)); }
+    // 0xffff in the halves that are above zero
     __device__ static __forceinline__ uint32_t positive_mask(uint32_t a2) { return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&a2), __floats2bfloat162_rn(0.0f, 0.0f)); }
     __device__ static __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
     {
@@ -99,6 +99,7 @@ template <> struct Cvt<MLP_BF16> {
 template <> struct Cvt<MLP_F16> {
     static constexpr uint32_t kUmmaFmt = 0;
     static constexpr uint32_t kOnes = 0x3C003C00u;
+    static constexpr float kSmallest = 0x1p-24f;
     __device__ static __forceinline__ float round(float v) { return __half2float(__float2half_rn(v)); }
     __device__ static __forceinline__ uint32_t pack2(float lo, float hi)
     {
@@ -117,7 +118,6 @@ template <> struct Cvt<MLP_F16> {
         const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
         return *reinterpret_cast<const uint32_t*>(&r);
     }
-    __device__ static __forceinline__ uint32_t zero_mask(uint32_t z2) { return __heq2_mask(*reinterpret_cast<const __half2*>(&z2), __floats2half2_rn(0.0f, 0.0f)); }
     __device__ static __forceinline__ uint32_t positive_mask(uint32_t a2) { return __hgt2_mask(*reinterpret_cast<const __half2*>(&a2), __floats2half2_rn(0.0f, 0.0f)); }
     __device__ static __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
     {

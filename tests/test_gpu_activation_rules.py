@@ -100,3 +100,10 @@ AROUND_ZERO = [[4, 32, 32, 4], [32, 24, 3], [6, 64, 48, 64, 3], [40, 64, 20]]
 @pytest.mark.parametrize("dims", AROUND_ZERO, ids=lambda d: "-".join(map(str, d)))
 def test_leaky_relu_around_zero(device, dims, storage):
     _around_zero(device, dims, storage, C.ACT_LEAKY_RELU)
+
+
+@pytest.mark.parametrize("storage", ["f16", "f32-f16"])
+@pytest.mark.parametrize("dims", AROUND_ZERO, ids=lambda d: "-".join(map(str, d)))
+def test_relu_around_zero(device, dims, storage):
+    """The derivative at zero is one half, from whichever side the pre-activation was rounded."""
+    _around_zero(device, dims, storage, C.ACT_RELU)
