@@ -779,6 +779,21 @@ __global__ void __launch_bounds__(32 * kForwardWarps, 2) forward_narrow_kernel(c
             float o[OT * 4], d[OT * 4];
 #pragma unroll
             for (int i = 0; i < OT * 4; ++i) o[i] = f32s ? acc[m][i >> 2][i & 3] : C::round(acc[m][i >> 2][i & 3]);
+            if (OT == 1 && od <= 4) {
+                // half of the tile's columns are padding: the lanes that hold them take the second row of those that do not
+                // (1920 x 1080 view with three outputs: 146.5 -> 142.1 us)
+                const float z0 = __shfl_xor_sync(0xffffffffu, o[2], 2), z1 = __shfl_xor_sync(0xffffffffu, o[3], 2);
+                float v[2] = {c < 2 ? o[0] : z0, c < 2 ? o[1] : z1}, dv[2];
+                activate_outputs(cfg.output_act, alpha, v, dv, false);
+                const uint64_t row = base + 16u * (uint64_t)m + 8u * (uint64_t)(c >> 1);
+                const int f = 2 * (c & 1);
+                if (row < p.count) {
+                    float* dst = p.outputs + row * (uint64_t)od;
+                    if (f < od) dst[f] = v[0];
+                    if (f + 1 < od) dst[f + 1] = v[1];
+                }
+                continue;
+            }
             activate_outputs(cfg.output_act, alpha, o, d, false);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {

@@ -107,3 +107,25 @@ def test_leaky_relu_around_zero(device, dims, storage):
 def test_relu_around_zero(device, dims, storage):
     """The derivative at zero is one half, from whichever side the pre-activation was rounded."""
     _around_zero(device, dims, storage, C.ACT_RELU)
+
+
+@pytest.mark.parametrize("dims", [[1, 32, 3], [1, 40, 8], [1, 16, 1], [1, 24, 2], [1, 64, 4], [1, 33, 5]], ids=lambda d: "-".join(map(str, d)))
+def test_output_sigmoid_is_as_exact_as_one_thread_per_sample(device, dims):
+    """Outputs are returned in fp32, so the sigmoid is that of the general kernels bit for bit (the output layer copies
+    the one input, so both kernels give it the same pre-activation)."""
+    from slang_b200.api import Trainer
+    cfg = _config(dims, "f16", C.ACT_RELU, output_act=C.ACT_SIGMOID)
+    w_off, _, total = C.param_layout(cfg)
+    p = np.zeros(total, dtype=np.float32)
+    p[w_off[0]], p[w_off[0] + 1] = 1.0, -1.0                # x above zero, and -x above zero
+    for o in range(dims[2]):
+        p[w_off[1] + o * dims[1]:w_off[1] + o * dims[1] + 2] = [1.0, -1.0]
+    params = C.to_storage(p, cfg.dtype)
+    x = np.linspace(-12, 12, 5001, dtype=np.float32).reshape(-1, 1)
+    xb, yb = device.create_buffer(x.nbytes, x), device.create_buffer(4 * x.size * dims[2])
+    outputs = []
+    for entry in ("forward", "forward_simt"):
+        tr = Trainer(device, cfg, params, forward_entry=entry)
+        tr.forward(xb.address, yb.address, x.size)
+        outputs.append(yb.read(np.float32).copy())
+    assert np.array_equal(outputs[0], outputs[1])
