@@ -4,6 +4,10 @@
 // its first access to global memory; that returns when the predecessor has completed and its writes are visible.  Because
 // every such kernel waits before it completes, completion stays in stream order.  grid_release() lets the successor's
 // blocks start as soon as every block of this kernel has been placed; they hold no work back, they only wait.
+//
+// Tensor memory is taken after grid_wait() and the successor released after that, by the warp that took it (one thread's
+// release counts for its block).  A block that held tensor memory while it waits could keep a block of its predecessor on
+// the same SM from ever getting its own, and a block that has yet to take some must not let in a successor that does so first.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -159,8 +159,12 @@ forward_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         prefetch_tmap(&tmap_x);
         prefetch_tmap(&tmap_out);
     }
-    grid_release();
     grid_wait();
+    if (warp == 1) {
+        tmem_alloc(tmem_ptr, G::kTmemCols);
+        tmem_relinquish();
+        grid_release();
+    }
     if (threadIdx.x == 0) {
         // the chains' first tiles: on their way while the weights are staged
 #pragma unroll
@@ -174,10 +178,6 @@ forward_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                                 (int32_t)(tile * 128u), &x_full[c]);
             }
         }
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_ptr, G::kTmemCols);
-        tmem_relinquish();
     }
     // Weights into shared memory, row-major rows re-cut into swizzled panels; biases as fp32.  Every layer's addresses are
     // read at once and every layer's copies are in flight together: one layer after the other, each behind its own

@@ -110,18 +110,21 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
         fence_mbar_init();
     }
     if constexpr (kSlots) {
-        if (warp == NW) {
-            tmem_alloc((uint32_t*)(smem + M::kTmemPtr), 512);
-            tmem_relinquish();
-        }
         // 16 rows of 128 bytes, the first 16-bit element of each one; the swizzle moves the 16-byte chunk with the row
         for (int i = threadIdx.x; i < 512; i += kThreads) {
             const int row = i >> 5, word = i & 31;
             ((uint32_t*)(smem + M::kOnes))[i] = (word >> 2) == (row & 7) && (word & 3) == 0 ? (C::kOnes & 0xffffu) : 0u;
         }
     }
-    grid_release();
+    if constexpr (!kSlots) grid_release();
     grid_wait();
+    if constexpr (kSlots) {
+        if (warp == NW) {
+            tmem_alloc((uint32_t*)(smem + M::kTmemPtr), 512);
+            tmem_relinquish();
+            grid_release();
+        }
+    }
     const MlpLayerPointers* s_net = (const MlpLayerPointers*)(smem + M::kNet);
     if (threadIdx.x < NL * 4) ((uint64_t*)(smem + M::kNet))[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
     __syncthreads();

@@ -64,3 +64,34 @@ def test_adam_over_large_segments_is_bit_exact(device, count):
     got = sb.read(np.uint8).view(C.ADAM_STATE_DTYPE)
     assert all(np.array_equal(got[f], st[f]) for f in ("mean", "variance", "iteration"))
     assert not gb.read(np.float32).any()
+
+
+@pytest.mark.parametrize("train", [[64, 64, 64, 64], [8, 24, 24, 4]], ids=["tensor-memory", "registers"])
+@pytest.mark.parametrize("width", [16, 64, 128])
+def test_inference_and_training_steps_back_to_back(device, width, train):
+    """A forward pass and a training step of another network, each launched to overlap the one before: what they compute
+    is what they compute with a wait in between."""
+    from slang_b200.api import Trainer
+    fcfg = C.make_config([width] * 5, C.F16, C.ACT_RELU, input_dtype=C.F16, target_dtype=C.F32)
+    tcfg = C.make_config(train, C.F16, C.ACT_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
+    count = 40000
+    rng = np.random.default_rng(width)
+    fx = device.create_buffer(2 * count * width, C.to_storage(rng.uniform(-1, 1, (count, width)), C.F16))
+    fy = device.create_buffer(4 * count * width)
+    x = device.create_buffer(4 * count * train[0], rng.uniform(-1, 1, (count, train[0])).astype(np.float32))
+    t = device.create_buffer(4 * count * train[-1], rng.uniform(-1, 1, (count, train[-1])).astype(np.float32))
+    ftr = Trainer(device, fcfg, C.init_params(fcfg, seed=1, scheme="kaiming"))
+    ttr = Trainer(device, tcfg, C.init_params(tcfg, seed=2, scheme="kaiming"))
+    results = []
+    for wait in (True, False):
+        ttr.grads.clear()
+        for _ in range(20):
+            for call in (lambda: ftr.forward(fx.address, fy.address, count),
+                         lambda: ttr.learn_gradient(x.address, t.address, count, clear_loss=False)):
+                call()
+                if wait:
+                    device.wait()
+        results.append((ttr.read_grads(), fy.read(np.uint32).copy()))
+        fy.clear()
+    assert rel_err(results[1][0], results[0][0]) < 1e-5   # fp32 sums of the CTAs in another order
+    assert np.array_equal(results[0][1], results[1][1])
