@@ -261,7 +261,7 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
     float run_max = 0.0f, run_sum = 0.0f;         // warp 0: this lane's samples
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const uint32_t s0 = tile * kTile;
-        const int n_here = min(kTile, (int)(count - s0));
+        const int n_here = (int)min((uint32_t)kTile, count - s0);
         const bool valid = lane < n_here;
         // ---- inputs; rows past the batch are zero ----
         for (int idx = threadIdx.x; idx < kTile * c.dims[0]; idx += kSimtThreads) {
@@ -607,7 +607,7 @@ cudaError_t launch_learn_gradient_simt(cudaStream_t st, const MlpConfig& c, cons
     if (e == cudaSuccess) e = limit[map.w >= 0].raise((const void*)kern, device, kSimtSmemMax);
     if (e != cudaSuccess) return e;
     // As many CTAs as are resident at once (512 threads each), each walking its share of the tiles.
-    const uint32_t tiles = (a.count + kTile - 1) / kTile;
+    const uint32_t tiles = (uint32_t)((uint64_t(a.count) + kTile - 1) / kTile);
     const uint32_t per_sm = uint32_t(std::max<size_t>(1, std::min<size_t>(2, kSimtSmemMax / (smem + 1024))));
     const uint32_t grid = std::min(tiles, per_sm * uint32_t(sms));
     e = launch_after(st, kern, grid, kSimtThreads, smem, net, map, (const MlpLayerPointers*)a.networkBuffer, (uint32_t*)a.lossBuffer,
@@ -634,11 +634,11 @@ cudaError_t launch_adjust_parameters(cudaStream_t st, const MlpConfig& c, const 
 {
     if (a.count == 0) return cudaSuccess;
     // Four elements a thread once that still leaves every SM eight blocks of 256 (an encoder's table); one below, where the
-    // launch is all there is (a network's parameters).
+    // launch is all there is (a network's parameters), and for the last counts whose indices four apart would not fit 32 bits.
     constexpr uint32_t kMany = 148u * 8u * 1024u;
     MlpAdamState* states = (MlpAdamState*)a.adamStates;
     const auto many = c.dtype == MLP_F32 && !c.adam_master ? adjust_parameters_kernel<4, true> : adjust_parameters_kernel<4, false>;
-    const cudaError_t e = a.count >= kMany
+    const cudaError_t e = a.count >= kMany && a.count <= 0xffffffffu - 1023u
         ? launch_after(st, many, (a.count + 1023) / 1024, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count)
         : launch_after(st, adjust_parameters_kernel<1, false>, (a.count + 255) / 256, 256, 0, c, states, (void*)a.params, (float*)a.gradients, a.count);
     *launches += 1;

@@ -299,3 +299,24 @@ def test_argument_errors(device):
     b = device.create_buffer(16)
     with pytest.raises(MlpError):
         b.clear(8, 16)
+
+
+def test_three_times_2_30_samples(device):
+    """Sample counts are 32-bit numbers without a sign.  A network of zeros with targets of one: every sample has loss 1,
+    bias gradient -2 and weight gradient -2 x."""
+    import torch
+    from slang_b200.api import Trainer
+    cfg = C.make_config([1, 1], C.F32, C.ACT_RELU, input_dtype=C.F16, target_dtype=C.F16)
+    count = 3 * (1 << 30) + 33
+    w_off, b_off, total = C.param_layout(cfg)
+    x = torch.full((count,), 0.5, dtype=torch.float16, device="cuda")
+    t = torch.ones(count, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    tr = Trainer(device, cfg, np.zeros(total, dtype=np.float32))
+    tr.learn_gradient(x.data_ptr(), t.data_ptr(), count)
+    g, (largest, loss) = tr.read_grads(), tr.read_loss()
+    del x, t
+    torch.cuda.empty_cache()
+    # fp32 sums of 3 * 2^30 equal terms in a few thousand parts: 1e-4 is a thousand roundings
+    assert largest == 1.0 and abs(loss / count - 1.0) < 1e-4
+    assert abs(g[b_off[0]] / (-2.0 * count) - 1.0) < 1e-4 and abs(g[w_off[0]] / (-1.0 * count) - 1.0) < 1e-4
