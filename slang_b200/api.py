@@ -11,12 +11,10 @@ import ctypes
 import numpy as np
 
 from . import config as C
+from . import lib as _lib
 from .lib import check, load
 
-try:
-    from . import _fastcall as _F   # the per-step calls; bound when the library is loaded
-except ImportError:                 # not built yet: load() says so
-    _F = None
+_F = _lib.fastcall   # the per-step calls: load() sets it, here too, when it has bound them
 
 
 class LearnGradParams(ctypes.Structure):

@@ -5,7 +5,7 @@
 Each translation unit is compiled to an object with its own flags (stale units side by side, one nvcc
 process each) and the objects are linked into slang_b200/libslang_b200_mlp.so; the literal example
 entry points are also built into a stand-alone device module, slang_b200/mlp_training_kernels.cubin, and the
-per-step calls of Python hosts into a small extension, slang_b200/_fastcall.so.
+per-step calls of Python hosts into a small extension, slang_b200/_fastcall (one per Python version).
 A unit is stale when its source, or any header its last compile read (nvcc -MD), is newer than its
 object.  The CUDA runtime is linked statically so the library has no dependency beyond the driver.
 """
@@ -24,7 +24,7 @@ OBJDIR = os.path.join(HERE, "build")
 CUBIN = os.path.join(HERE, "mlp_training_kernels.cubin")
 CUBIN_SRC = "example_module.cu"
 # The per-step calls for Python hosts (CPython extension).
-FASTCALL = os.path.join(HERE, "_fastcall.so")
+FASTCALL = os.path.join(HERE, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 FASTCALL_SRC = "fastcall.c"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -143,7 +143,7 @@ def build(force=False, verbose=False, jobs=None, without=(), out=None):
             print(" ".join(cmd), flush=True)
         subprocess.check_call(cmd)
     fs = os.path.join(CSRC, FASTCALL_SRC)
-    fd = os.path.join(OBJDIR, "fastcall.d")
+    fd = os.path.join(OBJDIR, os.path.basename(FASTCALL) + ".d")
     if force or _stale(FASTCALL, fs, fd):
         cmd = ["gcc", "-O2", "-std=c11", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-MD", "-MF", fd, fs, "-o", FASTCALL]
         if verbose:

@@ -5,6 +5,7 @@ handle is requested, the caller gets an exception.
 """
 import ctypes
 import os
+import sys
 
 from .config import MlpConfig
 
@@ -29,6 +30,7 @@ EXPORTS = [
 CUBIN_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "mlp_training_kernels.cubin")
 
 _lib = None
+fastcall = None   # the extension with the per-step calls, once load() has bound it
 
 
 class MlpError(RuntimeError):
@@ -38,7 +40,7 @@ class MlpError(RuntimeError):
 
 
 def load():
-    global _lib
+    global _lib, fastcall
     if _lib is not None:
         return _lib
     if not os.path.exists(LIB_PATH):
@@ -95,6 +97,10 @@ def load():
             fn.restype = i32
     from . import _fastcall
     _fastcall.bind(ctypes.cast(L.mlp_dispatch, ctypes.c_void_p).value, ctypes.cast(L.mlp_buffer_clear, ctypes.c_void_p).value)
+    fastcall = _fastcall
+    api = sys.modules.get(__package__ + ".api")
+    if api is not None:   # imported before the library was loaded (or built)
+        api._F = _fastcall
     _lib = L
     return L
 
