@@ -263,7 +263,7 @@ class Trainer:
         if input_grads_address:
             flags |= FLAG_INPUT_GRADIENT
         rc = _F.learn(self.device._h, self.k_learn._h, self.network.address, self.loss.address, inputs_address, targets_address, count, flags,
-                      input_grads_address, (count + 255) // 256)
+                      input_grads_address or 0, (count + 255) // 256)
         if rc:
             check(rc)
 

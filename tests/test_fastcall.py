@@ -5,6 +5,8 @@ import subprocess
 import sys
 import sysconfig
 
+import pytest
+
 from slang_b200 import lib
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -32,3 +34,17 @@ except lib.MlpError as e:
 def test_the_extension_is_named_for_its_python():
     lib.load()
     assert lib.fastcall.__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+@pytest.mark.parametrize("input_grads", [None, 0])
+def test_no_input_gradients_may_be_none(input_grads):
+    from slang_b200 import api
+    lib.load()
+
+    class Handle:
+        _h = address = 0
+
+    trainer = api.Trainer.__new__(api.Trainer)
+    trainer.device = trainer.k_learn = trainer.network = trainer.loss = Handle()
+    with pytest.raises(lib.MlpError):
+        trainer.learn_gradient(0, 0, 16, clear_loss=False, input_grads_address=input_grads)
