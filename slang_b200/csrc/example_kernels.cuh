@@ -27,18 +27,20 @@ __device__ __forceinline__ __half hdiv_(__half a, __half b) { return __float2hal
 __device__ __forceinline__ bool hneg_(__half a) { return __half2float(a) < 0.0f; }
 
 // Both layers' parameters in shared memory, read from global memory once per block and all at the same time (every sample
-// reads every one of them).
+// reads every one of them).  The example's blocks have 256 threads; a host that loads the module may launch any number up
+// to that, so these loops and those of the sums take what a block has.
 struct ExampleParams {
     alignas(16) __half w1[64], w2[64];
     alignas(16) __half b1[16], b2[4];
 };
 __device__ __forceinline__ void ex_stage(ExampleParams& s, const MlpLayerPointers& l1, const MlpLayerPointers& l2)
 {
-    const int t = (int)threadIdx.x;
-    if (t < 64) s.w1[t] = ((const __half*)l1.weights)[t];
-    else if (t < 128) s.w2[t - 64] = ((const __half*)l2.weights)[t - 64];
-    else if (t < 144) s.b1[t - 128] = ((const __half*)l1.biases)[t - 128];
-    else if (t < 148) s.b2[t - 144] = ((const __half*)l2.biases)[t - 144];
+    for (int t = (int)threadIdx.x; t < 148; t += (int)blockDim.x) {
+        if (t < 64) s.w1[t] = ((const __half*)l1.weights)[t];
+        else if (t < 128) s.w2[t - 64] = ((const __half*)l2.weights)[t - 64];
+        else if (t < 144) s.b1[t - 128] = ((const __half*)l1.biases)[t - 128];
+        else s.b2[t - 144] = ((const __half*)l2.biases)[t - 144];
+    }
     __syncthreads();
 }
 
@@ -108,8 +110,8 @@ __device__ void ex_accumulate(const MlpLayerPointers& lp, const __half* sg, cons
     __half* dW = (__half*)lp.weightsGrad;
     __half* dB = (__half*)lp.biasesGrad;
     const bool single = gridDim.x == 1;
-    const int p = (int)threadIdx.x - FIRST;
-    if (p >= 0 && p < In * Out + Out) {
+    for (int p = (int)threadIdx.x - FIRST; p < In * Out + Out; p += (int)blockDim.x) {
+        if (p < 0) continue;
         const bool is_w = p < In * Out;
         const int i = is_w ? p / In : p - In * Out, j = is_w ? p % In : 0;
         __half* dst = is_w ? dW + p : dB + i;
@@ -239,8 +241,8 @@ __device__ void cv_accumulate(const MlpLayerPointers& lp, const __half* sg, cons
     __half* dW = (__half*)lp.weightsGrad;
     __half* dB = (__half*)lp.biasesGrad;
     const bool single = gridDim.x == 1;
-    const int p = (int)threadIdx.x - FIRST;
-    if (p >= 0 && p < In * Out + Out) {
+    for (int p = (int)threadIdx.x - FIRST; p < In * Out + Out; p += (int)blockDim.x) {
+        if (p < 0) continue;
         const bool is_w = p < In * Out;
         const int i = is_w ? p / In : p - In * Out, j = is_w ? p % In : 0;
         __half* dst = is_w ? dW + i * 16 + j : dB + i;
