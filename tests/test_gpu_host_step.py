@@ -6,6 +6,8 @@ import pytest
 
 from slang_b200 import config as C
 
+from mlp_testlib import rel_err
+
 pytestmark = pytest.mark.gpu
 
 
@@ -53,6 +55,37 @@ def test_host_step_matches_resident_step(with_teacher):
         assert abs(mean * count - l_ref[1]) <= 1e-4 * abs(l_ref[1]) and mx == l_ref[0]
         assert stepper.h2d_bytes == count * 128 * (1 if with_teacher else 2) and stepper.d2h_bytes == 8
         tr.adjust_parameters = orig_adjust
+    finally:
+        device.destroy()
+
+
+def test_host_step_cuts_a_batch_that_would_fit_one_piece(monkeypatch):
+    """Up to sixteen pieces of whole tiles, here of 1280 samples with a ragged last one, below the stepper's chunk."""
+    import torch
+    from slang_b200 import host_step
+    from slang_b200.api import Device, Trainer
+    monkeypatch.setattr(host_step, "_PIECE_BYTES", 1 << 16)
+    torch.cuda.set_device(0)
+    device = Device(0, torch.cuda.current_stream().cuda_stream)
+    try:
+        cfg, count = C.named_config("c4"), 20011
+        p0 = C.init_params(cfg, seed=4, scheme="xavier")
+        gen = torch.Generator(device="cuda"); gen.manual_seed(9)
+        x = torch.randn((count, 64), device="cuda", generator=gen).to(torch.bfloat16)
+        t = (torch.randn((count, 64), device="cuda", generator=gen) * 0.3).to(torch.bfloat16)
+        ref = Trainer(device, cfg, p0)
+        ref.learn_gradient(x.data_ptr(), t.data_ptr(), count)
+        g_ref, l_ref = ref.read_grads(), ref.read_loss()
+        tr = Trainer(device, cfg, p0)
+        xh, th = x.cpu().pin_memory(), t.cpu().pin_memory()
+        pieces, grads = [], {}
+        learn = tr.learn_gradient
+        tr.learn_gradient = lambda xa, ta, n, **more: (pieces.append(n), learn(xa, ta, n, **more))
+        tr.adjust_parameters = lambda: grads.setdefault("g", tr.read_grads())
+        mx, mean = host_step.HostStepper(tr).step(xh, th)
+        assert pieces == [1280] * 15 + [20011 - 15 * 1280]
+        assert rel_err(grads["g"], g_ref) <= 1e-4      # pieces add in a different order than one launch
+        assert abs(mean * count - l_ref[1]) <= 1e-4 * abs(l_ref[1]) and mx == l_ref[0]
     finally:
         device.destroy()
 
