@@ -267,7 +267,7 @@ def measure_narrow(torch, device, dev_t, name, count, warmup, steps):
         # the CPU-runnable parity configuration: a launch-bound step (4096 samples), reported as ms per step
         x = (torch.rand((count, 2), device=dev_t, generator=gen) * 2 - 1).contiguous()
         t = (torch.sin(np.pi * x[:, 0]) * torch.cos(np.pi * x[:, 1])).reshape(count, 1).contiguous()
-        workload = "fp32 MLP 2-16-16-16-1 ReLU, MSE, Adam lr 1e-3 (one thread per sample)"
+        workload = "fp32 MLP 2-16-16-16-1 ReLU, MSE, Adam lr 1e-3 (general kernels, fp32)"
     elif name == "c2":
         x = torch.rand((count, 4), device=dev_t, generator=gen)
         w = torch.from_numpy(C.unit_vectors(1234, 4, 4)).to(dev_t)
@@ -354,7 +354,7 @@ def measure_narrow(torch, device, dev_t, name, count, warmup, steps):
 
 def measure_other_widths(torch, device, dev_t):
     """Networks that are neither a benchmark configuration nor at most 64 wide: learnGradient + adjustParameters
-    on 2^20 samples through the shape's fastest kernel and, for scale, through the one-thread-per-sample kernel
+    on 2^20 samples through the shape's fastest kernel and, for scale, through the general kernel without tensor cores
     (2^17 samples)."""
     from slang_b200 import config as C
     from slang_b200.api import Trainer
@@ -772,8 +772,8 @@ def main():
             r, n, dt = oracle_rate(cfg, args.config, threads, 12.0)
             line["cpu_baseline"] = {"value": r, "unit": UNIT, "cores": threads, "kind": "port",
                                     "sample": "%d samples, learnGradient + adjustParameters once, %.1f s" % (n, dt)}
-            # The structure of the reference's example kernels on the same GPU: one thread per sample,
-            # scalar fused multiply-adds, block-level sums and atomics (learnGradient_simt), on a bounded sample.
+            # The general kernel on the same GPU: no tensor cores, scalar multiply-adds, sums of 32-sample tiles and
+            # atomics (learnGradient_simt), on a bounded sample.
             n_simt = min(count, 1 << 18)
             tr_simt = Trainer(device, cfg, p0, learn_entry="learnGradient_simt")
             for _ in range(2):
@@ -786,7 +786,7 @@ def main():
             e1.record()
             torch.cuda.synchronize()
             line["gpu_baseline"] = {"value": n_simt / (e0.elapsed_time(e1) * 1e-3), "unit": UNIT,
-                                    "kind": "one thread per sample on the same GPU (the example kernels' structure, this library's learnGradient_simt)",
+                                    "kind": "this library's general kernel without tensor cores on the same GPU (learnGradient_simt)",
                                     "sample": "%d samples, learnGradient + adjustParameters once" % n_simt}
         if world == 1 and not args.no_sub:
             # The other configurations under the same clock, in this process: configurations 1, 2 and 3

@@ -95,7 +95,7 @@ typedef struct MlpForwardParams {
 /* forward: write the outputs rounded to the network's storage type (tensor-core path only). */
 #define MLP_FLAG_OUTPUT_STORAGE_TYPE 2u
 /* learnGradient with MlpLearnGradParamsEx2: also write the input gradients (networks without an input
- * encoding; on the tensor cores wherever learnGradient itself runs there, else one thread per sample). */
+ * encoding; on the tensor cores wherever learnGradient itself runs there, else on the general kernels). */
 #define MLP_FLAG_INPUT_GRADIENT 4u
 
 /* ---- device ------------------------------------------------------------------------------- */
@@ -206,14 +206,15 @@ int32_t mlp_kernel_load(MlpDevice* device, const void* image, size_t image_size,
 /* The same entry points specialised for a problem description, the way the reference specialises
  * FeedForwardLayer<In, Out> at compile time.  entry_point is one of
  *   "learnGradient"      args MlpLearnGradParamsEx   (fastest implementation for the shape)
- *   "learnGradient_simt" args MlpLearnGradParamsEx   (one thread per sample, any shape)
+ *   "learnGradient_simt" args MlpLearnGradParamsEx   (no tensor cores, any shape)
  *   "adjustParameters"   args MlpAdjustParamsParams  (MlpAdamState per element, fp32 gradients)
  *   "forward"            args MlpForwardParams
  *   "forward_simt"       args MlpForwardParams */
 int32_t mlp_kernel_get_for_config(MlpDevice* device, const MlpConfig* config, const char* entry_point,
                                   MlpKernel** out_kernel);
 int32_t mlp_kernel_destroy(MlpKernel* kernel);
-/* Name of the implementation a kernel handle resolved to ("simt", "tcgen05", ...). */
+/* Name of the implementation a kernel handle resolved to: "tcgen05" for the tensor-core kernels (those for widths up to
+ * 64 also, or only, issue mma.sync), "simt" for the general ones, "module" for a loaded one. */
 const char* mlp_kernel_implementation(const MlpKernel* kernel);
 
 /* dispatchKernel (mlp-training.cpp:252-268): bind, setData(offset 0, &args, size), dispatchCompute.

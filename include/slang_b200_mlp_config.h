@@ -88,7 +88,7 @@ typedef struct MlpConfig {
     int32_t input_width;               /* values per sample in the inputs buffer (2 for FREQ2D, else dims[0]) */
     float lr, beta1, beta2, eps;       /* Adam constants (adam.slang:15-19) */
     int32_t adam_master;               /* 1: Adam keeps an fp32 copy of each parameter in its state */
-    int32_t sum_order;                 /* MlpSumOrder of the one-thread-per-sample kernels */
+    int32_t sum_order;                 /* MlpSumOrder of the general kernels */
     int32_t param_layout;              /* MlpParamLayout of the weights and of their gradients */
     int32_t operand_dtype;             /* 0: products read the storage type.  MLP_F16 / MLP_BF16 with dtype = MLP_F32:
                                           the neural module's T = float on its tensor-core path, whose matrix

@@ -31,7 +31,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
           "--expt-relaxed-constexpr"]
 
-# (object name, source, extra flags).  The one-thread-per-sample kernels must not contract a*b+c into
+# (object name, source, extra flags).  The general kernels must not contract a*b+c into
 # an fma on their own: their fp32 results are compared bit for bit with a sequential CPU.  The padded
 # tensor-core kernels are instantiated some two hundred times; their source is compiled in ten parts, the wide
 # kernel's in three (training builds, forward-only builds, training builds with the optional outputs).

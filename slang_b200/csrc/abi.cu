@@ -285,7 +285,7 @@ int32_t mlp_kernel_get_for_config(MlpDevice* d, const MlpConfig* config, const c
     if (!config_ok(config, &why)) return fail(MLP_E_INVALID_ARG, "bad config: %s", why.c_str());
     MlpKernel* k = new MlpKernel();
     k->cfg = *config;
-    k->impl = "simt";
+    k->impl = "simt";   // or "tcgen05": the tensor-core kernels, whichever instructions they issue
     if (!std::strcmp(entry_point, "learnGradient")) {
         if (tc_train_supported(*config)) { k->entry = Entry::Learn; k->impl = "tcgen05"; }
         else k->entry = Entry::LearnSimt;

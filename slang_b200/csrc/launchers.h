@@ -53,7 +53,7 @@ cudaError_t launch_forward_wide(cudaStream_t st, TcWorkspace* ws, const MlpConfi
 cudaError_t launch_learn_gradient_narrow(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c,
                                          const MlpLearnGradParamsEx& a, int* launches, std::string* err,
                                          float* input_grads = nullptr);
-// Forward pass of the same padded kernel (any widths up to 64, any activation, input conversion or the
+// Forward pass for the same networks (any widths up to 64, any activation, input conversion or the
 // frequency encoding); fp32 outputs.
 cudaError_t launch_forward_narrow(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpForwardParams& a,
                                   int* launches, std::string* err);

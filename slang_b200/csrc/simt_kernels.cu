@@ -1,8 +1,8 @@
-// One-thread-per-sample kernels: the literal example entry points and the shape-generic path.
+// General kernels without tensor cores: the literal example entry points and the shape-generic path.
 //
-// These keep the reference's dispatch contract exactly: [numthreads(256,1,1)], thread id =
-// blockIdx.x * blockDim.x + threadIdx.x, grid = ceil(count / 256)
-// (examples/mlp-training/kernels.slang:8-41, examples/mlp-training/mlp-training.cpp:181-204).
+// The callers keep the reference's dispatch contract: [numthreads(256,1,1)], grid = ceil(count / 256)
+// (examples/mlp-training/kernels.slang:8-41, examples/mlp-training/mlp-training.cpp:181-204).  The example kernels
+// and the forward pass run a thread per sample, learnGradient a CTA per tiles of 32 samples.
 // They serve every shape and number format; the tensor-core kernels take over for the shapes they
 // are built for.  This file is compiled with -fmad=false: every multiply and add is separately
 // rounded unless fmaf is written out, so fp32 results match a sequential CPU bit for bit.
@@ -21,9 +21,9 @@
 namespace mlpb200 {
 
 // ------------------------------------------------------------------------------------------------
-// Shape-generic path: any MlpConfig within the scratch limits, one thread per sample.
+// Shape-generic path: any MlpConfig whose layer widths sum to at most kMaxActFloats.
 // ------------------------------------------------------------------------------------------------
-constexpr int kMaxActFloats = 768;  // sum of all layer widths a thread may hold
+constexpr int kMaxActFloats = 768;  // sum of all layer widths (a forward thread's arrays, a tile's shared memory)
 
 struct SimtNet {
     MlpConfig cfg;
@@ -118,7 +118,8 @@ forward_simt_kernel(SimtNet net, const MlpLayerPointers* __restrict__ lp, const 
 // of 32 floats per feature, a weight is one broadcast read shared by the 32 samples, and each sum runs over its
 // terms in ascending order exactly as simt_forward does.  Parameters are summed over the tile in ascending sample
 // order, over the CTA's tiles in shared memory where it has room, and leave through one atomic add per parameter
-// per CTA.  With MLP_FLAG_SEQUENTIAL_SUM the per-sample vectors go to a global scratch area instead and a second
+// per CTA; where it has none (fp32 64-128-128-128-128-64), per tile, with weights it has no room for read from global
+// memory (65536 samples of that network: 12.2 ms; a thread per sample with its vectors in local memory: 29.2).  With MLP_FLAG_SEQUENTIAL_SUM the per-sample vectors go to a global scratch area instead and a second
 // kernel adds them one sample at a time.
 //
 // Bound: the latency of the layer chain at small batches (a tile is 2 NL + 2 barriers), fp32 issue at large ones.
@@ -538,7 +539,7 @@ static bool make_simt_net(const MlpConfig& c, SimtNet* net, std::string* err)
     for (int l = 0; l <= c.n_layers; ++l) { net->a_off[l] = off; off += c.dims[l]; }
     net->a_off[c.n_layers + 1] = off;
     if (off > kMaxActFloats) {
-        if (err) *err = "sum of layer widths exceeds the per-thread limit of the one-thread-per-sample kernels";
+        if (err) *err = "sum of layer widths exceeds the limit of the general kernels";
         return false;
     }
     return true;
@@ -633,8 +634,10 @@ size_t sequential_scratch_floats_per_sample(const MlpConfig& c)
 cudaError_t launch_adjust_parameters(cudaStream_t st, const MlpConfig& c, const MlpAdjustParamsParams& a, int* launches)
 {
     if (a.count == 0) return cudaSuccess;
-    // Four elements a thread once that still leaves every SM eight blocks of 256 (an encoder's table); one below, where the
-    // launch is all there is (a network's parameters), and for the last counts whose indices four apart would not fit 32 bits.
+    // Four elements a thread once that still leaves every one of a B200's 148 SMs eight blocks of 256 (an encoder's table);
+    // one below, where the launch is all there is (a network's parameters).  fp32, one against four: 2^18 4.2 / 4.4 us,
+    // 2^19 5.3 / 5.1, 2^20 9.3 / 6.7, 1.5 M 12.9 / 8.8, 2^23 70.5 / 55.7.  One also for the
+    // last counts, whose indices four apart would not fit 32 bits.
     constexpr uint32_t kMany = 148u * 8u * 1024u;
     MlpAdamState* states = (MlpAdamState*)a.adamStates;
     const auto many = c.dtype == MLP_F32 && !c.adam_master ? adjust_parameters_kernel<4, true> : adjust_parameters_kernel<4, false>;

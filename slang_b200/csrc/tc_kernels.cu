@@ -1004,7 +1004,7 @@ learn_gradient_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
 #endif
 // fp32 input rows -> the operand type, for networks whose inputs arrive as fp32 (an encoder in front of the
 // network writes fp32 features): the wide kernel takes its input tile by TMA in the operand type, so the rows
-// are rounded once by this launch, exactly as the epilogue-built input rows of the padded kernel are.
+// are rounded once by this launch, exactly as the kernel for narrower networks rounds its input rows.
 template <int FMT>
 __global__ void convert_input_rows_kernel(const float4* __restrict__ src, uint2* __restrict__ dst, size_t n4)
 {
@@ -1043,7 +1043,7 @@ static cudaError_t converted_input_rows(cudaStream_t st, TcWorkspace* ws, int op
 static bool wide_supported(const MlpConfig& c)
 {
     // Two to five layers; inputs and outputs up to 64 wide, hidden layers up to 128; at least one width
-    // above 64 (narrower networks run the padded 64-wide kernel); 16-bit storage with inputs in the same
+    // above 64 (narrower networks run the kernel for widths up to 64); 16-bit storage with inputs in the same
     // format and rows that start on 16-byte boundaries (the input tile arrives by TMA); identity output.
     const int nl = c.n_layers;
     if (nl < 2 || nl > wide::kMaxLayers) return false;

@@ -1,8 +1,8 @@
 // learnGradient and forward for networks of widths up to 64 (the fp16 CoopVec-style network 4-32-32-32-32-4, the
 // neural-texture network enc(2->32)-64-64-64-3, anything in between), 16-bit operands.
 //
-// A warp carries 16 or 32 samples through every layer in registers (tc_narrow.cuh) and never waits for another warp
-// on the way down or back up.  What contracts over samples, the weight and bias gradients, is done
+// A warp carries 16 samples (training) or 32 (forward) through every layer in registers (tc_narrow.cuh) and never waits
+// for another warp on the way down or back up.  What contracts over samples, the weight and bias gradients, is done
 //   at padded width 32: in registers as well.  The layer inputs and the output gradients of the warp's samples are
 //     transposed 8x8 blocks at a time (movmatrix) and multiplied with mma.sync into accumulators the warp keeps for
 //     the whole launch (NL x 32 x 32 fp32 over 32 lanes); the warps' sums meet in shared memory once, at the end.
@@ -10,8 +10,8 @@
 //     its samples' dZ_l and A_l rows into a slot of shared memory ([samples][64 features] tiles, 128-byte
 //     swizzle), one warp issues dW_l | db_l [64 x 80] += dZ_l^T . [A_l | 1] (contraction over the slot's rows) into
 //     tensor memory, and the slot is free again when that product has completed.  Slots belong to groups of one to
-//     three warps: with one slot for all sixteen the warps ran in step, products against products and epilogues
-//     against epilogues, and a 2^24-sample step took 5.3 ms instead of 3.8.
+//     five warps: with one slot for all fifteen the warps ran in step, products against products and epilogues
+//     against epilogues, and a 2^24-sample step took 5.3 ms instead of 3.9 (3.83 now).
 // Either way each parameter receives one atomic add per CTA at the end.
 //
 // What the reference does instead: one thread per sample with per-element global atomics
@@ -37,7 +37,9 @@ namespace narrow {
 enum : uint32_t { kStatusSlot = 0x2000u };
 
 constexpr int kForwardWarps = 8;
-constexpr int kTrainBlocks = 1;   // 16-sample blocks a training warp carries at a time
+// 16-sample blocks a training warp carries at a time: one (the fragment helpers shared with the forward kernel take more,
+// what follows a layer's products here does not).
+constexpr int kTrainBlocks = 1;
 
 // Shared-memory map of the training kernel (bytes from a 1024-aligned base).  NG groups of GW warps carry samples.
 template <int W, int NL, int NG, int GW>
@@ -251,8 +253,8 @@ __global__ void __launch_bounds__(32 * (NG * GW + (W == 64 ? 1 : 0)), 1) learn_g
             bool zero_seen = false;                                 // ReLU: whether any pre-activation was zero
             {
                 // the next tile's input and target rows: start them on their way into L2
-                const uint64_t ns = base + (uint64_t)stride * (uint64_t)M::kUnit + (uint64_t)((c & 1) * 8) + (MT == 2 && (c & 2) ? 16u : 0u);
-                if (ns < p.count && (MT == 2 || c < 2)) {
+                const uint64_t ns = base + (uint64_t)stride * (uint64_t)M::kUnit + (uint64_t)((c & 1) * 8);
+                if (ns < p.count && c < 2) {
                     if (!raw_inputs(cfg))
                         asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p.inputs + ns * (uint64_t)cfg.dims[0] * (cfg.input_dtype == MLP_F32 ? 4u : 2u)));
                     asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p.targets + ns * (uint64_t)od * (cfg.target_dtype == MLP_F32 ? 4u : 2u)));
@@ -847,7 +849,10 @@ template <int W, int NL, int FMT, int HACT, int OT>
 static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
 {
     // Width 32: eight warps of 255 registers.  Width 64: as many warps as the state of a sample block leaves registers
-    // for (16 with 128 each, 11 with 168, 8 with 255), one of them issuing.
+    // for (16 with 128 each, 11 with 168, 8 with 255), one of them issuing.  Groups, fp16 learnGradient of 2^20 and of 20000
+    // samples: 5 x 2 warps 415 / 25.1 us against 10 x 1 421 / 27.3 (32-64-64-3, GELU) and 624 / 33.3 against 710 / 35.8
+    // (64 x 6, ReLU); 7 x 1 984 / 47.7 against 1 x 7 873 / 47.7 (64 x 5, GELU) and 1210 / 60.0 against 1146 / 62.4 (64 x 6,
+    // GELU), where the one group would be the better one for large batches.
     constexpr bool kept = HACT != MLP_ACT_RELU && HACT != MLP_ACT_LEAKY_RELU;
     constexpr int state = NL + (kept ? NL - 1 : 0);
     constexpr int NG = W == 32 ? 8 : state <= 4 ? 3 : state <= 5 ? 5 : 7, GW = W == 32 ? 1 : state <= 4 ? 5 : state <= 5 ? 2 : 1;

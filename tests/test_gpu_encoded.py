@@ -82,7 +82,7 @@ def test_input_gradients_from_the_wide_kernel(device, dims, dtype, act):
 @pytest.mark.parametrize("dtype,hidden", [(C.F32, 16), (C.F16, 16), (C.F16, 128)])
 def test_encoder_in_front_of_the_network_trains_like_the_oracle(device, dtype, hidden):
     """fp32 network: one thread per sample; fp16 networks: the tensor-core kernel that runs learnGradient writes
-    the input gradients (the padded 64-wide one; for 128 hidden units the wide one, whose fp32 feature rows
+    the input gradients (the one for widths up to 64; for 128 hidden units the wide one, whose fp32 feature rows
     are rounded to fp16 by a launch in front of it)."""
     from slang_b200.encoded import EncodedTrainer
     rng = np.random.default_rng(12)

@@ -1,4 +1,4 @@
-"""GPU parity of the forward kernels (tensor-core and one-thread-per-sample) against the CPU oracle."""
+"""GPU parity of the forward kernels (tensor-core and general) against the CPU oracle."""
 import numpy as np
 import pytest
 
@@ -101,7 +101,7 @@ def test_forward_output_in_storage_type(device):
 @pytest.mark.parametrize("count", [1, 130, 128 * 148 * 2 + 9])
 def test_narrow_network_forward_on_tensor_cores(device, case, count):
     """Networks of any widths up to 64 (any activation, input conversion or the frequency encoding) run
-    their forward pass through the padded tensor-core kernel; outputs against the oracle."""
+    their forward pass through the tensor-core kernel for them; outputs against the oracle."""
     rng = np.random.default_rng(count % 97 + len(case))
     if case in ("c2", "c3"):
         cfg = C.named_config(case)

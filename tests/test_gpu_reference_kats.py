@@ -5,7 +5,7 @@
   row, db = B for B = 32, 64, 128) through the tcgen05 entry point "learnGradient" in fp16 and bf16.
 * source/standard-modules/neural/activations.slang:27-228 (all nine activations) plus the two this
   library adds (GELU-tanh, the cooperative-vector example's max form): value and derivative through
-  "forward" and "learnGradient" on the one-thread-per-sample kernels and on the padded tcgen05 kernel,
+  "forward" and "learnGradient" on the general kernels and on the tensor-core kernel for widths up to 64,
   against the oracle, which tests/test_oracle_kat.py pins on activation-functions-test.slang:31-154.
 * config 2 at its stated 1000 steps on a reduced batch.
 """
@@ -111,7 +111,7 @@ def test_every_activation_one_thread_per_sample(device, act):
 @pytest.mark.parametrize("act", ALL_ACTS, ids=[ACT_NAME[a] for a in ALL_ACTS])
 def test_every_activation_on_the_padded_tensor_core_kernel(device, act, dtype):
     """16-bit storage, hidden and output activation both `act`, through "learnGradient" and "forward" of
-    the padded tcgen05 kernel: gradients per tensor within 1e-2, loss within 1e-2, outputs within one
+    the tensor-core kernel for widths up to 64: gradients per tensor within 1e-2, loss within 1e-2, outputs within one
     storage rounding step of the oracle."""
     from oracle import oracle
     from slang_b200.api import Trainer

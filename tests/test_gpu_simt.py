@@ -1,4 +1,4 @@
-"""GPU parity of the one-thread-per-sample kernels against the CPU oracle, through the C ABI."""
+"""GPU parity of the general kernels (no tensor cores) against the CPU oracle, through the C ABI."""
 import ctypes
 
 import numpy as np

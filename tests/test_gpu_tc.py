@@ -1,5 +1,5 @@
 """GPU parity of the tensor-core learnGradient (64-128-128-128-128-64) against the CPU oracle and
-against the one-thread-per-sample kernel, through the C ABI."""
+against the general kernel, through the C ABI."""
 import numpy as np
 import pytest
 
@@ -72,7 +72,7 @@ def test_c4_trajectory(device):
 
 def test_c4_tensor_core_matches_simt_on_large_batch(device):
     """2^17 samples: too many for the scalar oracle in a test, so the tensor-core kernel is checked
-    against the one-thread-per-sample kernel (itself pinned to the oracle), and the gradient of the
+    against the general kernel (itself pinned to the oracle), and the gradient of the
     whole batch against the sum of the gradients of its two halves."""
     from slang_b200.api import Trainer
     count = 1 << 17
@@ -107,7 +107,7 @@ def test_c4_tensor_core_matches_simt_on_large_batch(device):
 @pytest.mark.parametrize("count", [1, 127, 129, 1024, 128 * 148 * 2 + 5])
 def test_narrow_networks_on_tensor_cores(device, name, count):
     """fp16 4-32-32-32-32-4 (LeakyReLU) and enc(2->32)-64-64-64-3 (ReLU, sigmoid output, L2) through the
-    padded 64-wide tensor-core kernel: gradients per tensor within 1e-2, loss words within 1e-2."""
+    tensor-core kernel for widths up to 64: gradients per tensor within 1e-2, loss words within 1e-2."""
     cfg, p0, batches = make_problem(name, count, seed=17, steps=1)
     _, l_ref, g_ref, _ = oracle_trajectory(cfg, p0, batches, n_threads=8)
     _, l_gpu, g_gpu, _, tr = gpu_trajectory(device, cfg, p0, batches)
@@ -121,8 +121,7 @@ def test_narrow_networks_on_tensor_cores(device, name, count):
 
 @pytest.mark.parametrize("dims", [[8, 48, 24], [20, 64, 33, 40], [64, 64, 64, 64, 64, 64], [3, 16, 7]])
 def test_narrow_kernel_other_shapes(device, dims):
-    """Shapes that exercise each column split of the padded kernel's epilogue (output width <= 16, <= 32,
-    larger), odd widths, bf16, tanh hidden units."""
+    """Output widths in each of the kernel's builds (up to 8, up to 16, larger), odd widths, bf16, tanh hidden units."""
     from oracle import oracle
     rng = np.random.default_rng(sum(dims))
     cfg = C.make_config(dims, dtype=C.BF16, hidden_act=C.ACT_TANH, output_act=C.ACT_IDENTITY, adam_master=1)
@@ -142,8 +141,8 @@ def test_narrow_kernel_other_shapes(device, dims):
 
 @pytest.mark.parametrize("dims,dtype", [([32, 64, 64, 3], C.F16), ([10, 40, 12], C.BF16), ([64, 64, 64, 64, 32], C.BF16)])
 def test_narrow_kernel_two_tiles_in_flight(device, dims, dtype):
-    """ReLU networks of up to four layers run two tiles per CTA once there are more tiles than SMs; the
-    derivative is recovered from the stored activation (negative zero marks a zero pre-activation).  Inputs
+    """ReLU networks with more units of work than SMs: the derivative is recovered from the activation, whose negative
+    zero marks a zero pre-activation.  Inputs
     with many exact zeros exercise the tie: zero inputs and zero biases give zero pre-activations."""
     rng = np.random.default_rng(len(dims) * 7 + dims[0])
     cfg = C.make_config(dims, dtype=dtype, hidden_act=C.ACT_RELU, output_act=C.ACT_IDENTITY, adam_master=1)
@@ -267,7 +266,7 @@ def test_wide_kernel_other_shapes(device, dims, dtype, act, tdtype):
 
 
 @pytest.mark.parametrize("dims,op,act", [
-    ([16, 64, 64, 8], C.F16, C.ACT_RELU),                 # padded 64-wide kernel
+    ([16, 64, 64, 8], C.F16, C.ACT_RELU),                 # widths up to 64
     ([4, 32, 32, 32, 4], C.BF16, C.ACT_LEAKY_RELU),       # its 32-wide build
     ([64, 128, 128, 64], C.BF16, C.ACT_GELU_TANH),        # wide kernel (16-bit inputs)
     ([32, 96, 128, 10], C.F16, C.ACT_TANH),               # wide kernel, run-time activation, targets read directly

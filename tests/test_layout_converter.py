@@ -87,7 +87,7 @@ def test_fflayer_optimal_layout_envelope():
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims,dtype,entry", [
     ([4, 2], "f32", "forward_simt"),               # the tiled test's own layer: [39, 80]
-    ([4, 4, 2], "f16", "forward"),                 # padded 64-wide tensor-core kernel
+    ([4, 4, 2], "f16", "forward"),                 # kernel for widths up to 64
     ([64, 64, 64, 64, 64], "f16", "forward"),      # constant-width tensor-core kernel
     ([128, 128, 128, 128, 128], "bf16", "forward"),
     ([32, 128, 128, 3], "f16", "forward"),         # wide tensor-core kernel
@@ -156,7 +156,7 @@ def test_forward_reads_optimal_layout_in_place(dims, dtype, entry):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims,dtype,act,entry", [
     ([2, 16, 16, 1], "f32", C.ACT_RELU, "learnGradient"),                 # one thread per sample
-    ([20, 48, 64, 3], "f16", C.ACT_LEAKY_RELU, "learnGradient"),          # padded 64-wide tensor-core kernel, ragged tiles
+    ([20, 48, 64, 3], "f16", C.ACT_LEAKY_RELU, "learnGradient"),          # kernel for widths up to 64, ragged tiles
     ([4, 32, 32, 32, 32, 4], "f16", C.ACT_LEAKY_RELU, "learnGradient"),   # its 32-wide build
     ([64, 128, 128, 128, 128, 64], "bf16", C.ACT_GELU_TANH, "learnGradient"),  # wide tensor-core kernel
     ([32, 96, 128, 10], "f16", C.ACT_RELU, "learnGradient"),              # wide kernel, widths that are not tile multiples
