@@ -57,6 +57,13 @@ cudaError_t launch_learn_gradient_narrow(cudaStream_t st, TcWorkspace* ws, const
 // frequency encoding); fp32 outputs.
 cudaError_t launch_forward_narrow(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpForwardParams& a,
                                   int* launches, std::string* err);
+// The same for the networks and batches that whole tiles of 128 samples on tcgen05 suit better (tc_chain.cu).
+bool chain_train_suits(const MlpConfig& c, uint32_t count);
+bool chain_forward_suits(const MlpConfig& c, uint32_t count);
+cudaError_t launch_learn_gradient_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpLearnGradParamsEx& a,
+                                        int* launches, std::string* err, float* input_grads = nullptr);
+cudaError_t launch_forward_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpForwardParams& a,
+                                 int* launches, std::string* err);
 // Developer builds (-DMLPB200_TRACE) only: time stamps CTA 0 of the last wide learnGradient recorded.
 cudaError_t tc_read_timing(cudaStream_t st, TcWorkspace* ws, unsigned long long* out256);
 // Reads and clears the device status word (0 = no kernel gave up on a bounded wait).

@@ -1,0 +1,869 @@
+// learnGradient and forward for networks of widths up to 64, 16-bit storage, ReLU or leaky ReLU hidden layers: tcgen05
+// products over whole tiles of 128 samples, several tiles in flight per SM (tc_chain.cuh).  tc_narrow.cu has the other
+// networks and the smallest batches.
+//
+//   forward   Z_l [128 x H]    = 1 . b_l^T + A_l [128 x W] . W_l^T   A: A_l, K-major      B: W_l [out][in], K-major
+//   input     dA_l [128 x H]   = dZ_l [128 x H] . W_l                A: dZ_l, K-major     B: W_l, MN-major
+//   weights   dW_l | db_l [64 x (W + 8)] += dZ_l^T . [A_l | 1]       A: dZ_l, MN-major    B: A_l, then a tile whose first column is ones
+//
+// Bound by instruction issue and by the hand-offs between a chain's four warps and the tensor pipe; the chains' tiles fill
+// shared memory, so there are no more of them.  Against the register-chained kernels of tc_narrow.cu, us: texture network
+// (32-64-64-64-3) 2^24 samples a step 3830 -> 2400, width 32 (4-32-32-32-32-4, leaky ReLU) 2^20 samples 160 -> 132, 1920 x 1080 view of the
+// texture network 142 -> 96.  Counters of 2^20 samples of the texture network: issue slots 41 %, tensor pipe 31 %, LSU wavefronts 43 %.
+//
+// What the reference does instead: one thread per sample with per-element global atomics
+// (examples/mlp-training/mlp_sw.slang:28-58) or CoopVec calls whose CPU/CUDA fallback is scalar loops
+// (examples/mlp-training-coopvec/fflayer.slang:16-58, source/slang/hlsl.meta.slang:32835-32912).
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <string>
+
+#include "launch_pdl.cuh"
+#include "launchers.h"
+#include "tc_chain.cuh"
+#include "tc_host.h"
+
+namespace mlpb200 {
+
+using namespace ptx;
+
+namespace chain {
+
+enum : uint32_t { kStatusIssue = 0x4000u, kStatusRow = 0x8000u, kStatusGrad = 0x10000u };
+
+// Warps that issue gradient products: two (even and odd layers) beside four chains; with three, sixteen warps in all leave
+// each thread 128 registers and seventeen 96.
+__host__ __device__ constexpr int grad_warps(int chains) { return chains == 3 ? 1 : 2; }
+
+// Shared-memory map of the training kernel (bytes from a 1024-aligned base).  H: padded hidden width; IW: padded input
+// width; OW: padded output width; NCH: chains.
+template <int H, int NL, int IW, int OW, int NCH>
+struct TrainMap {
+    static constexpr int kWarps = 4 * NCH;                // with samples; one more per chain issues its layer products, one or two the gradient products
+    static constexpr int kGradWarps = grad_warps(NCH);
+    static constexpr int kThreads = 32 * (kWarps + NCH + kGradWarps);
+    static constexpr int kDzW = OW == 16 ? 32 : H;             // row width of the last layer's dZ
+    __host__ __device__ static constexpr int in_w(int l) { return l == 0 ? IW : H; }
+    __host__ __device__ static constexpr int out_w(int l) { return l == NL - 1 ? OW : H; }
+    static constexpr uint32_t kRowsIn = kTile * IW * 2, kRows = kTile * H * 2;
+    // a chain's tiles: A_0, A_1 .. A_{NL-1} (dZ_{l-1} replaces A_l), dZ_{NL-1}
+    __host__ __device__ static constexpr uint32_t a_off(int l) { return l == 0 ? 0u : kRowsIn + (uint32_t)(l - 1) * kRows; }
+    static constexpr uint32_t kDz = a_off(NL);
+    static constexpr uint32_t kChainBytes = kDz + kTile * kDzW * 2;
+    __host__ __device__ static constexpr uint32_t w_off(int l) { return l == 0 ? 0u : (uint32_t)H * IW * 2 + (uint32_t)(l - 1) * H * H * 2; }
+    static constexpr uint32_t kWeights = 0;
+    static constexpr uint32_t kChains = (w_off(NL - 1) + (uint32_t)OW * H * 2 + 1023) & ~1023u;
+    static constexpr uint32_t kOnesIn = kChains + NCH * kChainBytes;   // 16 rows whose first element is one, in the layout of A_0
+    static constexpr uint32_t kOnes = kOnesIn + (IW == H ? 0 : 16 * IW * 2);
+    static constexpr uint32_t kUnit = kOnes + 16 * H * 2;
+    static constexpr uint32_t kHiddenBias = kUnit + kUnitBytes;        // [NL - 1][H rows][16]
+    static constexpr uint32_t kBias = kHiddenBias + (NL - 1) * H * 32; // the output layer's, fp32 [OW]
+    static constexpr uint32_t kLoss = kBias + OW * 4;              // fp32 [kWarps][2]
+    static constexpr uint32_t kBars = kLoss + kWarps * 8;              // per chain: ready, acc_full, and for each gradient warp dz_ready, dw_done
+    static constexpr uint32_t kTmemPtr = kBars + (2 + 2 * kGradWarps) * NCH * 8;
+    static constexpr uint32_t kAbort = kTmemPtr + 4;
+    static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;
+    static constexpr uint32_t kSmemBytes = kNet + NL * 32 + 1024;
+    static constexpr uint32_t kSumRow = H + 1;                         // the outgoing gradients: fp32 [NL][H][H + 1], over the chains' tiles
+    static_assert(NL * H * kSumRow * 4 <= kOnesIn, "room for the sums");
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
+    // tensor memory: an accumulator per chain, then the gradients, which the chains share
+    __host__ __device__ static constexpr uint32_t dw_cols(int l) { return (uint32_t)in_w(l) + 16; }
+    __host__ __device__ static constexpr uint32_t dw_col(int l) { return NCH * (uint32_t)H + (l == 0 ? 0u : dw_cols(0) + (uint32_t)(l - 1) * (H + 16)); }
+    static_assert(dw_col(NL) <= 512, "tensor memory budget");
+};
+
+template <int H, int NL, int IW, int OW, int NCH, int FMT, int HACT>
+__global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gradient_chain_kernel(const __grid_constant__ Params p)
+{
+    using M = TrainMap<H, NL, IW, OW, NCH>;
+    using C = Cvt<FMT>;
+    constexpr int kThreads = M::kThreads, NW = M::kWarps, G = M::kGradWarps;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sbase = smem_u32(smem);
+    const MlpConfig& cfg = p.cfg;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    uint64_t* ready = (uint64_t*)(smem + M::kBars);   // the chain's operand rows are written and its accumulator is drained
+    uint64_t* acc_full = ready + NCH;                 // a layer product has completed
+    uint64_t* dz_ready = acc_full + NCH;              // [chain][layer % G]: a dZ is written
+    uint64_t* dw_done = dz_ready + G * NCH;           // [chain][layer % G]: a gradient product has completed
+    volatile uint32_t* abort_flag = (volatile uint32_t*)(smem + M::kAbort);
+    const int od = cfg.dims[NL];
+
+    // ---- set-up ----
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < NCH; ++c) {
+            mbar_init(&ready[c], 4);
+            mbar_init(&acc_full[c], 1);
+            for (int g = 0; g < G; ++g) {
+                mbar_init(&dz_ready[G * c + g], 4);
+                mbar_init(&dw_done[G * c + g], 1);
+            }
+        }
+        *abort_flag = 0u;
+        fence_mbar_init();
+    }
+    for (int i = threadIdx.x; i < 16 * H / 2; i += kThreads) {
+        const int row = i / (H / 2), word = i % (H / 2);
+        ((uint32_t*)(smem + M::kOnes))[i] = (uint32_t)(word * 4) == row_at<H>(row) - (uint32_t)row * H * 2 ? (C::kOnes & 0xffffu) : 0u;
+    }
+    if constexpr (IW != H) {
+        for (int i = threadIdx.x; i < 16 * IW / 2; i += kThreads) {
+            const int row = i / (IW / 2), word = i % (IW / 2);
+            ((uint32_t*)(smem + M::kOnesIn))[i] = (uint32_t)(word * 4) == row_at<IW>(row) - (uint32_t)row * IW * 2 ? (C::kOnes & 0xffffu) : 0u;
+        }
+    }
+    grid_wait();
+    if (warp == NW + NCH) {
+        tmem_alloc((uint32_t*)(smem + M::kTmemPtr), 512);
+        tmem_relinquish();
+        grid_release();
+    }
+    const MlpLayerPointers* s_net = (const MlpLayerPointers*)(smem + M::kNet);
+    if (threadIdx.x < NL * 4) ((uint64_t*)(smem + M::kNet))[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
+    __syncthreads();
+    stage_weights<IW>(smem + M::kWeights, cfg, (const void*)s_net[0].weights, H, cfg.dims[0], cfg.dims[1], threadIdx.x, kThreads);
+#pragma unroll 1
+    for (int l = 1; l < NL; ++l)
+        stage_weights<H>(smem + M::kWeights + M::w_off(1) + (uint32_t)(l - 1) * (H * H * 2), cfg, (const void*)s_net[l].weights, l == NL - 1 ? OW : H,
+                         cfg.dims[l], cfg.dims[l + 1], threadIdx.x, kThreads);
+    // hidden features past the real width: below zero for ReLU, so that no derivative there is the one at zero
+    first_column(smem + M::kUnit, 8, threadIdx.x, kThreads, [](int) { return C::kOnes; });
+    first_column(smem + M::kHiddenBias, (NL - 1) * H, threadIdx.x, kThreads, [&](int row) -> uint32_t {
+        const int l = row / H, f = row % H;
+        return f < cfg.dims[l + 1] ? ((const uint16_t*)s_net[l].biases)[f] : HACT == MLP_ACT_RELU ? C::kOnes | 0x8000u : 0u;
+    });
+    for (int i = threadIdx.x; i < OW; i += kThreads)
+        ((float*)(smem + M::kBias))[i] = i < od ? load_as_f32(cfg.dtype, (const void*)s_net[NL - 1].biases, i) : 0.0f;
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *(volatile uint32_t*)(smem + M::kTmemPtr);
+    const uint32_t stride = gridDim.x * NCH;
+    bool ok = true;
+
+    if (warp < NW) {
+        // =================================== samples ===============================================
+        const int ch = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+        const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ch * H);
+        const uint32_t cb = sbase + M::kChains + (uint32_t)ch * M::kChainBytes;
+        const uint32_t in_row = cb + row_at<IW>(r), own_row = cb + M::kRowsIn + row_at<H>(r), dz_row = cb + M::kDz + row_at<M::kDzW>(r);
+        const uint32_t s_bias = sbase + M::kBias;
+        const float scale = cfg.loss == MLP_LOSS_MSE_MEAN ? 1.0f / (float)od : 1.0f;
+        const float alpha = cfg.act_alpha, alpha_op = C::round(alpha);
+        constexpr float kTiny = 0.5f * C::kSmallest;   // the largest magnitude that rounds to zero
+        float run_max = 0.0f, run_sum = 0.0f;
+        uint32_t full = 0, done = 0;                   // phases seen of acc_full; bit g: parity of dw_done's g
+        auto wait_full = [&]() {
+            ok = ok && mbar_wait(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
+            ++full;
+            tc_fence_after();
+        };
+        auto wait_done = [&](int l) {
+            ok = ok && mbar_wait(&dw_done[G * ch + l % G], (done >> (l % G)) & 1u, abort_flag, p.status, kStatusRow);
+            done ^= 1u << (l % G);
+        };
+        // hands A_l over (gradient < 0), or dZ of layer `gradient`
+        auto release = [&](bool product, int gradient) {
+            tc_fence_before();
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                if (product) mbar_arrive(&ready[ch]);
+                if (gradient >= 0) mbar_arrive(&dz_ready[G * ch + gradient % G]);
+            }
+        };
+        RawRow raw;
+        uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch;
+        uint64_t sample = (uint64_t)tile * kTile + (uint64_t)r;
+        Rows in(p.inputs, stored_inputs(cfg), cfg.input_dtype, sample, stride * kTile), tgt(p.targets, od, cfg.target_dtype, sample, stride * kTile);
+        const bool wide_target = cfg.target_dtype == MLP_F32;
+        fetch_row(raw, p, in.at, sample < p.count);
+        bool first = true;
+        for (; tile < p.n_tiles && ok; tile += stride) {
+            const bool valid = sample < p.count;
+            bool zero_seen = false;
+            // ---- input row; stored when the gradient product of the chain's last tile has read A_0 ----
+            write_row<FMT, IW>(in_row, p, raw, in.at, valid, [&]() { if (!first) wait_done(0); });
+            first = false;
+            if (!ok) break;
+            release(true, -1);
+            // few targets are fetched a forward pass ahead of their use; the next tile's rows are started on their way
+            uint32_t t4[4];
+            if (od <= 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) t4[i] = load_bits(tgt.at, wide_target, i, valid && i < od);
+            }
+            const char* targets = tgt.at;
+            const uint64_t current = sample;
+            sample += (uint64_t)stride * kTile;
+            in.at += in.step;
+            tgt.at += tgt.step;
+            fetch_row(raw, p, in.at, sample < p.count);
+            if (sample < p.count) {
+                if (!short_row(cfg)) prefetch_row(in.at);
+                prefetch_row(tgt.at);
+            }
+            // ---- forward, hidden layers ----
+#pragma unroll 1
+            for (int l = 0; l < NL - 1; ++l) {
+                wait_full();
+                if (!ok) break;
+                const uint32_t dst = own_row + (uint32_t)l * M::kRows;   // A_{l + 1}
+                float least = 1.0f;
+                uint32_t v[H / 32][32];
+                tmem_ld_32x32(t_acc, v[0]);
+                wait_ld(v[0]);
+                if constexpr (H == 64) tmem_ld_32x32(t_acc + 32u, v[H / 32 - 1]);
+                hidden_columns<FMT, HACT>(v[0], dst, alpha, least);
+                if constexpr (H == 64) {
+                    wait_ld(v[H / 32 - 1]);
+                    hidden_columns<FMT, HACT>(v[H / 32 - 1], dst ^ 64u, alpha, least);
+                }
+                if (HACT == MLP_ACT_RELU && __any_sync(0xffffffffu, least <= 0.5f * C::kSmallest)) {   // one that rounds to zero
+                    zero_seen = true;
+                    marked_columns<FMT, H>(t_acc, dst);
+                }
+                release(true, -1);
+            }
+            // ---- output layer, loss, dZ of the last layer ----
+            wait_full();
+            if (!ok) break;
+            float loss = 0.0f;
+#pragma unroll 1
+            for (int f = 0; f < ((od + 15) & ~15); f += 4) {
+                uint32_t z0 = 0u, z1 = 0u;
+                if (f < od) {
+                    float o[4], d[4], t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, g[4];
+                    output_columns<FMT>(o, t_acc, s_bias, f);
+                    if (od <= 4) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) t[i] = bits_value(cfg.target_dtype, t4[i]);
+                    } else if (valid) {
+                        load_targets(t, p, targets, od, f);
+                    }
+                    activate_outputs(cfg.output_act, alpha, o, d);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool real = valid && f + i < od;
+                        const float diff = real ? o[i] - t[i] : 0.0f;
+                        loss = fmaf(diff * scale, diff, loss);
+                        g[i] = real ? ((2.0f * scale) * diff) * d[i] : 0.0f;
+                    }
+                    z0 = C::pack2(g[0], g[1]);
+                    z1 = C::pack2(g[2], g[3]);
+                }
+                sts64((dz_row ^ (uint32_t)(16 * (f >> 3))) + (uint32_t)(2 * (f & 4)), z0, z1);
+            }
+            run_max = fmaxf(run_max, loss);
+            run_sum += loss;
+            release(true, NL - 1);
+            // ---- backward: dA_l times the derivative is dZ_{l-1}, written over A_l once the gradient product has read it ----
+#pragma unroll 1
+            for (int l = NL - 1; l >= 1; --l) {
+                wait_full();
+                if (!ok) break;
+                const uint32_t at = own_row + (uint32_t)(l - 1) * M::kRows;   // A_l
+                if (HACT == MLP_ACT_RELU && zero_seen) {
+                    wait_done(l);
+                    if (!ok) break;
+                    reverse_marked_columns<FMT, H>(t_acc, at);
+                } else {
+                    uint32_t v[H / 32][32], z[H / 32][16];
+                    tmem_ld_32x32(t_acc, v[0]);
+                    wait_ld(v[0]);
+                    if constexpr (H == 64) tmem_ld_32x32(t_acc + 32u, v[H / 32 - 1]);
+                    reverse_columns<FMT, HACT>(z[0], v[0], at, alpha_op);
+                    if constexpr (H == 64) {
+                        wait_ld(v[H / 32 - 1]);
+                        reverse_columns<FMT, HACT>(z[H / 32 - 1], v[H / 32 - 1], at ^ 64u, alpha_op);
+                    }
+                    wait_done(l);
+                    if (!ok) break;
+#pragma unroll
+                    for (int j = 0; j < H / 8; ++j) {
+                        const uint32_t* w = &z[j >> 2][4 * (j & 3)];
+                        sts128(at ^ (uint32_t)(16 * j), w[0], w[1], w[2], w[3]);
+                    }
+                }
+                release(l > 1 || p.input_grads, l - 1);
+            }
+            // ---- optional: the input gradients dZ_0 . W_0, rounded to the storage type ----
+            if (p.input_grads) {
+                wait_full();
+                if (!ok) break;
+                const int in = cfg.dims[0];
+                float* row = p.input_grads + current * (uint64_t)in;
+#pragma unroll 1
+                for (int f = 0; f < in; f += 8) {
+                    uint32_t v[8];
+                    tmem_ld_32x8(t_acc + (uint32_t)f, v);
+                    tmem_ld_wait();
+                    float x[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) x[i] = C::round(__uint_as_float(v[i]));
+                    if (!valid) continue;
+                    if (p.vec_dx) {
+                        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(row + f), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]),
+                                     "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
+                                     : "memory");
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (f + i < in) row[f + i] = x[i];
+                    }
+                }
+                tc_fence_before();
+            }
+        }
+        if (!first) wait_done(0);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            run_max = fmaxf(run_max, __shfl_xor_sync(0xffffffffu, run_max, o));
+            run_sum += __shfl_xor_sync(0xffffffffu, run_sum, o);
+        }
+        if (lane == 0) {
+            ((float*)(smem + M::kLoss))[warp * 2] = run_max;
+            ((float*)(smem + M::kLoss))[warp * 2 + 1] = run_sum;
+        }
+    } else if (warp < NW + NCH) {
+        // =================================== layer products of one chain ===========================
+        const int ch = warp - NW;
+        const uint32_t lo = (sbase & 0x3FFFFu) >> 4;
+        const uint32_t cb = M::kChains + (uint32_t)ch * M::kChainBytes;
+        const uint32_t acc = tmem_base + (uint32_t)(ch * H);
+        const int in_steps = (cfg.dims[0] + 15) / 16, out_steps = (od + 15) / 16;
+        constexpr uint32_t F = C::kUmmaFmt;
+        uint32_t seen = 0;
+        auto wait_ready = [&]() {
+            ok = ok && mbar_wait(&ready[ch], seen & 1u, abort_flag, p.status, kStatusIssue);
+            ok = __all_sync(0xffffffffu, ok);
+            ++seen;
+            tc_fence_after();
+        };
+        for (uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch; tile < p.n_tiles && ok; tile += stride) {
+#pragma unroll
+            for (int l = 0; l < NL; ++l) {
+                wait_ready();
+                if (ok && elect_one()) {
+                    if (l < NL - 1) umma_f16(acc, desc_unit(lo, M::kUnit), desc_k<16>(lo, M::kHiddenBias + (uint32_t)l * H * 32, 0), umma_idesc(F, 0, 0, 128, H), 0u);
+                    if (l == 0) {
+#pragma unroll
+                        for (int k = 0; k < IW / 16; ++k)
+                            if (k < in_steps) umma_f16(acc, desc_k<IW>(lo, cb, k), desc_k<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 0, 128, H), 1u);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < H / 16; ++k)
+                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l), k), desc_k<H>(lo, M::kWeights + M::w_off(l), k), umma_idesc(F, 0, 0, 128, M::out_w(l)),
+                                     l < NL - 1 || k > 0);
+                    }
+                    umma_commit(&acc_full[ch]);
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int l = NL - 1; l >= 0; --l) {
+                if (l == 0 && !p.input_grads) break;
+                wait_ready();
+                if (ok && elect_one()) {
+                    if (l == NL - 1) {
+#pragma unroll
+                        for (int k = 0; k < OW / 16; ++k)
+                            if (k < out_steps)
+                                umma_f16(acc, desc_k<M::kDzW>(lo, cb + M::kDz, k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k), umma_idesc(F, 0, 1, 128, H), k > 0);
+                    } else if (l > 0) {
+#pragma unroll
+                        for (int k = 0; k < H / 16; ++k)
+                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l + 1), k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k), umma_idesc(F, 0, 1, 128, H), k > 0);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < H / 16; ++k)
+                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(1), k), desc_mn<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 1, 128, IW), k > 0);
+                    }
+                    umma_commit(&acc_full[ch]);
+                }
+                __syncwarp();
+            }
+        }
+    } else {
+        // =================================== gradient products of all chains =======================
+        // Warp g takes the layers g, g + G, .. of whichever chain has a dZ ready; one thread issues all
+        // products into one accumulator, so those are in order.  (The loop is kept small: with a copy of the code per chain and
+        // layer, its instructions were fetched anew each time.)
+        const int g = warp - NW - NCH;
+        const uint32_t lo = (sbase & 0x3FFFFu) >> 4;
+        constexpr uint32_t F = C::kUmmaFmt;
+        const uint32_t top = (uint32_t)(NL - 1 - (NL - 1 - g) % G);        // this warp's last layer; its first is g
+        uint32_t total = 0, idle = 0, started = 0, phase = 0, layers = 0;   // hand-overs to come; layers begun; four bits a chain: its layer
+        for (int c = 0; c < NCH; ++c) {
+            const uint32_t first = blockIdx.x + gridDim.x * (uint32_t)c;
+            layers |= top << (4 * c);
+            total += first < p.n_tiles ? ((p.n_tiles - first + stride - 1) / stride) * (top / G + 1) : 0u;
+        }
+        uint32_t c = 0;
+#pragma unroll 1
+        while (total > 0 && ok) {
+            if (__all_sync(0xffffffffu, mbar_test_wait(&dz_ready[G * c + g], (phase >> c) & 1u))) {
+                tc_fence_after();
+                const uint32_t l = (layers >> (4 * c)) & 15u, cb = M::kChains + c * M::kChainBytes;
+                const uint32_t a = l == 0 ? cb : cb + M::kRowsIn + (l - 1) * M::kRows;           // A_l
+                const uint32_t z = l == NL - 1 ? cb + M::kDz : cb + M::kRowsIn + l * M::kRows;   // dZ_l
+                const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16));
+                const uint32_t begun = (started >> l) & 1u;
+                auto gradient = [&](auto z_width, auto a_width, uint32_t ones) {
+                    constexpr int ZW = decltype(z_width)::value, AW = decltype(a_width)::value;
+#pragma unroll
+                    for (int k = 0; k < kTile / 16; ++k)
+                        umma_f16(d, desc_mn<ZW>(lo, z, k), desc_mn<AW>(lo, a, k, ones - a - (uint32_t)k * 16u * (uint32_t)layout::row_bytes(AW)),
+                                 umma_idesc(F, 1, 1, 64, AW + 8), k > 0 ? 1u : begun);
+                };
+                using WideT = std::integral_constant<int, H>;
+                if (elect_one()) {
+                    if (l == 0 && IW != H) gradient(WideT{}, std::integral_constant<int, IW>{}, M::kOnesIn);
+                    else if (l == NL - 1 && M::kDzW != H) gradient(std::integral_constant<int, M::kDzW>{}, WideT{}, M::kOnes);
+                    else gradient(WideT{}, WideT{}, M::kOnes);
+                    umma_commit(&dw_done[G * c + g]);
+                }
+                __syncwarp();
+                started |= 1u << l;
+                layers += (l < G ? top - l : 0u - G) << (4 * c);
+                phase ^= 1u << c;
+                --total;
+                idle = 0;
+            } else if (++idle > kMaxPolls || ((idle & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0u))) {
+                *abort_flag = 1u;
+                atomicOr(p.status, kStatusGrad);
+                ok = false;
+            }
+            c = c + 1 == NCH ? 0u : c + 1;
+        }
+    }
+
+    // ---- one add per parameter per CTA ----
+    tc_fence_before();
+    __syncthreads();   // every chain has seen its last gradient product completed (or the CTA is aborting)
+    tc_fence_after();
+    const bool good = !*abort_flag;
+    float* sums = (float*)smem;
+    if (good && warp < NW) {
+        // Row r of a 64-row accumulator sits on lane 32 (r / 16) + r % 16: the first 16 lanes of this warp's quarter hold rows
+        // 16 quarter + lane.  The warps of a quarter take the 16-column pieces in turn.
+        const int quarter = warp & 3, row = quarter * 16 + lane;
+#pragma unroll 1
+        for (int l = 0; l < NL; ++l) {
+            const int w = l == 0 ? IW : H;
+#pragma unroll 1
+            for (int piece = warp >> 2; piece <= w / 16; piece += NCH) {
+                uint32_t v[16];
+                tmem_ld_32x16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (uint32_t)(l - 1) * (H + 16)) + (uint32_t)piece * 16u, v);
+                wait_ld(v);
+                if (lane < 16 && row < H) {
+                    float* at = sums + (l * H + row) * (int)M::kSumRow;
+                    if (piece == w / 16) at[H] = __uint_as_float(v[0]);
+                    else
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) at[piece * 16 + i] = __uint_as_float(v[i]);
+                }
+            }
+        }
+        tc_fence_before();
+    }
+    __syncthreads();
+    if (good) {
+        // real parameters in the order they are stored, four to a reduction where rows are whole 16-byte pieces
+        int i = threadIdx.x;
+#pragma unroll 1
+        for (int l = 0; l < NL; ++l) {
+            const int in = cfg.dims[l], out = cfg.dims[l + 1];
+            float* dW = (float*)s_net[l].weightsGrad;
+            float* dB = (float*)s_net[l].biasesGrad;
+            const float* s = sums + l * H * (int)M::kSumRow;
+            const bool fours = (in & 3) == 0 && cfg.param_layout == MLP_PARAMS_ROW_MAJOR && ((uint64_t)dW & 15u) == 0;
+            const int per_row = fours ? in >> 2 : in;
+            for (; i < out * per_row; i += kThreads) {
+                const int o = i / per_row, k = i - o * per_row;
+                const float* at = s + o * (int)M::kSumRow;
+                if (fours) atomicAdd((float4*)dW + i, make_float4(at[4 * k], at[4 * k + 1], at[4 * k + 2], at[4 * k + 3]));
+                else atomicAdd(dW + weight_index(cfg.param_layout, in, out, o, k), at[k]);
+            }
+            i -= out * per_row;
+            for (; i < out; i += kThreads) atomicAdd(dB + i, s[i * (int)M::kSumRow + H]);
+            i -= out;
+        }
+        if (threadIdx.x == 0) {
+            const float* part = (const float*)(smem + M::kLoss);
+            float mx = part[0], sm = part[1];
+#pragma unroll
+            for (int w = 1; w < NW; ++w) { mx = fmaxf(mx, part[2 * w]); sm += part[2 * w + 1]; }
+            atomicMax(p.loss_words, __float_as_uint(mx));
+            atomicAdd((float*)(p.loss_words + 1), sm);
+        }
+    }
+    tc_fence_after();
+    if (warp == NW + NCH) tmem_dealloc(tmem_base, 512);
+}
+
+// Shared-memory map of the forward kernel.
+template <int H, int IW, int OW, int NCH>
+struct ForwardMap {
+    static constexpr int kThreads = 32 * 5 * NCH;
+    static constexpr int kMaxLayers = 5;
+    static constexpr uint32_t kChainBytes = kTile * (IW > H ? IW : H) * 2;   // the current layer's input rows
+    __host__ __device__ static constexpr uint32_t w_off(int l) { return l == 0 ? 0u : (uint32_t)H * IW * 2 + (uint32_t)(l - 1) * H * H * 2; }
+    static constexpr uint32_t kChains = (w_off(kMaxLayers - 1) + (uint32_t)H * H * 2 + 1023) & ~1023u;
+    static constexpr uint32_t kStageFloats = 32 * (OW + 1);                  // outputs of a warp's rows on their way out
+    static constexpr uint32_t kStage = kChains + NCH * kChainBytes;
+    static constexpr uint32_t kUnit = (kStage + 4 * NCH * kStageFloats * 4 + 255) & ~255u;
+    static constexpr uint32_t kHiddenBias = kUnit + kUnitBytes;              // [4][H rows][16]
+    static constexpr uint32_t kBias = kHiddenBias + (kMaxLayers - 1) * H * 32;   // the output layer's, fp32 [OW]
+    static constexpr uint32_t kBars = kBias + OW * 4;                        // per chain: ready, acc_full
+    static constexpr uint32_t kTmemPtr = kBars + 2 * NCH * 8;
+    static constexpr uint32_t kAbort = kTmemPtr + 4;
+    static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;
+    static constexpr uint32_t kSmemBytes = kNet + kMaxLayers * 32 + 1024;
+    static constexpr uint32_t kTmemCols = layout::pow2_at_least_32(NCH * H);
+    static_assert(kSmemBytes <= 227 * 1024 && kTmemCols <= 512, "shared and tensor memory budget");
+};
+
+template <int H, int IW, int OW, int NCH, int FMT, int HACT>
+__global__ void __launch_bounds__(32 * 5 * NCH, 1) forward_chain_kernel(const __grid_constant__ Params p)
+{
+    using M = ForwardMap<H, IW, OW, NCH>;
+    using C = Cvt<FMT>;
+    constexpr int kThreads = M::kThreads;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sbase = smem_u32(smem);
+    const MlpConfig& cfg = p.cfg;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int nl = cfg.n_layers, od = cfg.dims[nl];
+    uint64_t* ready = (uint64_t*)(smem + M::kBars);
+    uint64_t* acc_full = ready + NCH;
+    volatile uint32_t* abort_flag = (volatile uint32_t*)(smem + M::kAbort);
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < NCH; ++c) {
+            mbar_init(&ready[c], 4);
+            mbar_init(&acc_full[c], 1);
+        }
+        *abort_flag = 0u;
+        fence_mbar_init();
+    }
+    grid_wait();
+    if (warp == 4 * NCH) {
+        tmem_alloc((uint32_t*)(smem + M::kTmemPtr), M::kTmemCols);
+        tmem_relinquish();
+        grid_release();
+    }
+    const MlpLayerPointers* s_net = (const MlpLayerPointers*)(smem + M::kNet);
+    if (threadIdx.x < nl * 4) ((uint64_t*)(smem + M::kNet))[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
+    __syncthreads();
+    stage_weights<IW>(smem, cfg, (const void*)s_net[0].weights, H, cfg.dims[0], cfg.dims[1], threadIdx.x, kThreads);
+#pragma unroll 1
+    for (int l = 1; l < nl; ++l)
+        stage_weights<H>(smem + M::w_off(1) + (uint32_t)(l - 1) * (H * H * 2), cfg, (const void*)s_net[l].weights, l == nl - 1 ? OW : H, cfg.dims[l],
+                         cfg.dims[l + 1], threadIdx.x, kThreads);
+    first_column(smem + M::kUnit, 8, threadIdx.x, kThreads, [](int) { return C::kOnes; });
+    first_column(smem + M::kHiddenBias, (nl - 1) * H, threadIdx.x, kThreads, [&](int row) -> uint32_t {
+        const int l = row / H, f = row % H;
+        return f < cfg.dims[l + 1] ? ((const uint16_t*)s_net[l].biases)[f] : 0u;
+    });
+    for (int i = threadIdx.x; i < OW; i += kThreads)
+        ((float*)(smem + M::kBias))[i] = i < od ? load_as_f32(cfg.dtype, (const void*)s_net[nl - 1].biases, i) : 0.0f;
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *(volatile uint32_t*)(smem + M::kTmemPtr);
+    const uint32_t stride = gridDim.x * NCH;
+    bool ok = true;
+    if (warp < 4 * NCH) {
+        const int ch = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+        const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ch * H);
+        const uint32_t cb = sbase + M::kChains + (uint32_t)ch * M::kChainBytes;
+        const uint32_t in_row = cb + row_at<IW>(r), own_row = cb + row_at<H>(r);
+        const uint32_t s_bias = sbase + M::kBias;
+        const float alpha = cfg.act_alpha;
+        uint32_t full = 0;
+        auto wait_full = [&]() {
+            ok = ok && mbar_wait(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
+            ++full;
+            tc_fence_after();
+        };
+        auto release = [&]() {
+            tc_fence_before();
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[ch]);
+        };
+        RawRow raw;
+        uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch;
+        uint64_t sample = (uint64_t)tile * kTile + (uint64_t)r;
+        Rows in(p.inputs, stored_inputs(cfg), cfg.input_dtype, sample, stride * kTile), out(p.outputs, od, MLP_F32, sample, stride * kTile);
+        // Rows of more than four outputs leave through shared memory, a warp's 32 rows as one run (row by row from the threads that
+        // own them, 50 outputs of 2^20 samples took 353 us, 134 now).
+        const bool staged = od > 4;
+        const int od_odd = od | 1;
+        float* stage = (float*)(smem + M::kStage) + warp * M::kStageFloats;
+        const uint32_t od_inverse = ((1u << 20) + (uint32_t)od - 1u) / (uint32_t)od;   // (i * od_inverse) >> 20 is i / od for i < 32 od <= 2048
+        fetch_row(raw, p, in.at, sample < p.count);
+        for (; tile < p.n_tiles && ok; tile += stride) {
+            const bool valid = sample < p.count;
+            float* dst = (float*)out.at;
+            write_row<FMT, IW>(in_row, p, raw, in.at, valid, []() {});
+            release();
+            sample += (uint64_t)stride * kTile;
+            in.at += in.step;
+            out.at += out.step;
+            fetch_row(raw, p, in.at, sample < p.count);
+            if (sample < p.count && !short_row(cfg)) prefetch_row(in.at);
+#pragma unroll 1
+            for (int l = 0; l < nl - 1; ++l) {
+                wait_full();
+                if (!ok) break;
+                float least = 0.0f;
+                uint32_t v[H / 32][32];
+                tmem_ld_32x32(t_acc, v[0]);
+                wait_ld(v[0]);
+                if constexpr (H == 64) tmem_ld_32x32(t_acc + 32u, v[H / 32 - 1]);
+                hidden_columns<FMT, HACT>(v[0], own_row, alpha, least);
+                if constexpr (H == 64) {
+                    wait_ld(v[H / 32 - 1]);
+                    hidden_columns<FMT, HACT>(v[H / 32 - 1], own_row ^ 64u, alpha, least);
+                }
+                release();
+            }
+            wait_full();
+            if (!ok) break;
+#pragma unroll 1
+            for (int f = 0; f < od; f += 4) {
+                float o[4], d[4];
+                output_columns<FMT>(o, t_acc, s_bias, f);
+                activate_outputs(cfg.output_act, alpha, o, d);
+                if (staged) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (f + i < od) stage[lane * od_odd + f + i] = o[i];
+                } else if (valid) {
+                    if (p.vec_out) {
+                        *(float4*)dst = make_float4(o[0], o[1], o[2], o[3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (i < od) dst[i] = o[i];
+                    }
+                }
+            }
+            if (staged) {
+                __syncwarp();
+                float* rows = dst - lane * od;
+                const uint64_t first = (uint64_t)tile * kTile + (uint64_t)(quarter * 32);
+                const uint32_t n = first >= p.count ? 0u : (p.count - first < 32u ? (uint32_t)(p.count - first) : 32u) * (uint32_t)od;
+#pragma unroll 4
+                for (uint32_t i = lane; i < n; i += 32) rows[i] = stage[i + ((i * od_inverse) >> 20) * (uint32_t)(od_odd - od)];
+                __syncwarp();
+            }
+            tc_fence_before();
+        }
+    } else {
+        const int ch = warp - 4 * NCH;
+        const uint32_t lo = (sbase & 0x3FFFFu) >> 4;
+        const uint32_t cb = M::kChains + (uint32_t)ch * M::kChainBytes, acc = tmem_base + (uint32_t)(ch * H);
+        const int in_steps = (cfg.dims[0] + 15) / 16;
+        constexpr uint32_t F = C::kUmmaFmt;
+        uint32_t seen = 0;
+        for (uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch; tile < p.n_tiles && ok; tile += stride) {
+#pragma unroll 1
+            for (int l = 0; l < nl; ++l) {
+                ok = ok && mbar_wait(&ready[ch], seen & 1u, abort_flag, p.status, kStatusIssue);
+                ok = __all_sync(0xffffffffu, ok);
+                ++seen;
+                tc_fence_after();
+                if (ok && elect_one()) {
+                    if (l < nl - 1) umma_f16(acc, desc_unit(lo, M::kUnit), desc_k<16>(lo, M::kHiddenBias + (uint32_t)l * (H * 32), 0), umma_idesc(F, 0, 0, 128, H), 0u);
+                    if (l == 0) {
+#pragma unroll
+                        for (int k = 0; k < IW / 16; ++k)
+                            if (k < in_steps) umma_f16(acc, desc_k<IW>(lo, cb, k), desc_k<IW>(lo, 0u, k), umma_idesc(F, 0, 0, 128, H), 1u);
+                    } else {
+                        const uint32_t id = l == nl - 1 ? umma_idesc(F, 0, 0, 128, OW) : umma_idesc(F, 0, 0, 128, H);
+                        const uint32_t w = (uint32_t)H * IW * 2 + (uint32_t)(l - 1) * (H * H * 2);
+#pragma unroll
+                        for (int k = 0; k < H / 16; ++k) umma_f16(acc, desc_k<H>(lo, cb, k), desc_k<H>(lo, w, k), id, l < nl - 1 || k > 0);
+                    }
+                    umma_commit(&acc_full[ch]);
+                }
+                __syncwarp();
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 4 * NCH) tmem_dealloc(tmem_base, M::kTmemCols);
+}
+
+}  // namespace chain
+
+// ------------------------------------------------------------------------------------------------
+// Host side.  Compiled once per MLPB200_CHAIN_PART: 0 the entry points, 1 .. 4 the training builds of 2 .. 5 layers, 5 the
+// forward builds.
+// ------------------------------------------------------------------------------------------------
+#ifndef MLPB200_CHAIN_PART
+#error "compile with -DMLPB200_CHAIN_PART=0..5 (slang_b200/build.py does)"
+#endif
+
+template <int NL> cudaError_t launch_chain_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p);
+cudaError_t launch_chain_forward(cudaStream_t st, TcWorkspace* ws, narrow::Params& p);
+
+#if MLPB200_CHAIN_PART >= 1 && MLPB200_CHAIN_PART <= 4
+template <int H, int NL, int IW, int OW, int NCH, int FMT, int HACT>
+static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    using M = chain::TrainMap<H, NL, IW, OW, NCH>;
+    auto kern = chain::learn_gradient_chain_kernel<H, NL, IW, OW, NCH, FMT, HACT>;
+    static SmemLimit limit;
+    const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, M::kSmemBytes);
+    if (e != cudaSuccess) return e;
+    const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
+    return launch_after(st, kern, grid, M::kThreads, M::kSmemBytes, p);
+}
+
+template <int H, int NL, int IW, int OW, int NCH>
+static cudaError_t launch_shape(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    const bool relu = p.cfg.hidden_act == MLP_ACT_RELU;
+    if (p.cfg.dtype == MLP_BF16) return relu ? launch_train<H, NL, IW, OW, NCH, MLP_BF16, MLP_ACT_RELU>(st, ws, p) : launch_train<H, NL, IW, OW, NCH, MLP_BF16, MLP_ACT_LEAKY_RELU>(st, ws, p);
+    return relu ? launch_train<H, NL, IW, OW, NCH, MLP_F16, MLP_ACT_RELU>(st, ws, p) : launch_train<H, NL, IW, OW, NCH, MLP_F16, MLP_ACT_LEAKY_RELU>(st, ws, p);
+}
+
+template <int NL>
+cudaError_t launch_chain_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    bool fits32 = p.cfg.dims[NL] <= 16;
+    for (int l = 0; l <= NL; ++l) fits32 = fits32 && p.cfg.dims[l] <= 32;
+    if (fits32) return launch_shape<32, NL, 32, 16, 4>(st, ws, p);
+    // as many chains as shared and tensor memory hold, up to three
+    if (p.cfg.dims[0] <= 32 && p.cfg.dims[NL] <= 16) return launch_shape<64, NL, 32, 16, NL == 5 ? 2 : 3>(st, ws, p);
+    if constexpr (NL <= 4) return launch_shape<64, NL, 64, 64, NL == 4 ? 2 : 3>(st, ws, p);
+    return cudaErrorInvalidValue;
+}
+template cudaError_t launch_chain_train<1 + MLPB200_CHAIN_PART>(cudaStream_t, TcWorkspace*, narrow::Params&);
+#endif
+
+#if MLPB200_CHAIN_PART == 5
+template <int H, int IW, int OW, int NCH, int FMT, int HACT>
+static cudaError_t launch_forward(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    using M = chain::ForwardMap<H, IW, OW, NCH>;
+    auto kern = chain::forward_chain_kernel<H, IW, OW, NCH, FMT, HACT>;
+    static SmemLimit limit;
+    const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, M::kSmemBytes);
+    if (e != cudaSuccess) return e;
+    const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
+    return launch_after(st, kern, grid, M::kThreads, M::kSmemBytes, p);
+}
+
+template <int H, int IW, int OW, int NCH>
+static cudaError_t launch_shape(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    const bool relu = p.cfg.hidden_act == MLP_ACT_RELU;
+    if (p.cfg.dtype == MLP_BF16) return relu ? launch_forward<H, IW, OW, NCH, MLP_BF16, MLP_ACT_RELU>(st, ws, p) : launch_forward<H, IW, OW, NCH, MLP_BF16, MLP_ACT_LEAKY_RELU>(st, ws, p);
+    return relu ? launch_forward<H, IW, OW, NCH, MLP_F16, MLP_ACT_RELU>(st, ws, p) : launch_forward<H, IW, OW, NCH, MLP_F16, MLP_ACT_LEAKY_RELU>(st, ws, p);
+}
+
+cudaError_t launch_chain_forward(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    const int nl = p.cfg.n_layers;
+    int widest = 0;
+    for (int l = 0; l <= nl; ++l) widest = p.cfg.dims[l] > widest ? p.cfg.dims[l] : widest;
+    const bool few = p.cfg.dims[nl] <= 16;
+    if (widest <= 32) return few ? launch_shape<32, 32, 16, 6>(st, ws, p) : launch_shape<32, 32, 32, 6>(st, ws, p);
+    if (p.cfg.dims[0] <= 32 && few) return launch_shape<64, 32, 16, 6>(st, ws, p);
+    return launch_shape<64, 64, 64, 3>(st, ws, p);
+}
+#endif
+
+#if MLPB200_CHAIN_PART == 0
+// Rows of `width` values of `bytes` each from an address on whole pieces of `piece` bytes.
+static int pieces(uint64_t address, int width, int bytes, int piece) { return address % (uint64_t)piece == 0 && (width * bytes) % piece == 0; }
+
+static narrow::Params chain_params(TcWorkspace* ws, const MlpConfig& c, uint64_t network, uint64_t inputs, uint32_t count)
+{
+    narrow::Params p = {};
+    p.cfg = c;
+    p.net = (const MlpLayerPointers*)network;
+    p.status = ws->status;
+    p.inputs = (const void*)inputs;
+    p.count = count;
+    p.n_tiles = (uint32_t)(((uint64_t)count + chain::kTile - 1) / chain::kTile);
+    p.vec_in = pieces(inputs, c.dims[0], c.input_dtype == MLP_F32 ? 4 : 2, 16);
+    return p;
+}
+
+static bool chain_network(const MlpConfig& c)
+{
+    if (c.n_layers < 2 || c.n_layers > 5) return false;
+    if ((c.dtype != MLP_BF16 && c.dtype != MLP_F16) || (c.operand_dtype && c.operand_dtype != c.dtype)) return false;
+    const int act = narrow::built_activation(c);
+    if (act != MLP_ACT_RELU && act != MLP_ACT_LEAKY_RELU) return false;
+    for (int l = 0; l <= c.n_layers; ++l)
+        if (c.dims[l] > 64) return false;
+    return c.encoding != MLP_ENC_FREQ2D || c.dims[0] == 32;
+}
+
+// Batches from which the tiles are the better way, us against the kernels of tc_narrow.cu (which deal 16 samples at a time):
+// learnGradient and adjustParameters of the texture network, 600 samples 22.5 / 20.5, 16384: 26.7 / 20.6, 2^20: 267 / 174; width
+// 32, 16 samples 17.5 / 18.4, 600: 18.5 / 18.4, 2^20: 160 / 132; 16-32-3, 600: 12.9 / 12.6, 2^20: 113 / 55.
+constexpr uint32_t kTrainFrom = 1024;
+// forward, 20-48-48-3: 100 samples 6.5 / 9.3, 8192: 7.2 / 6.6, 2^20: 73.6 / 42.5; 4-32-32-32-32-4, 2000 samples 6.5 / 6.7, 16384: 9.3 /
+// 6.8, 2^20: 45.6 / 41.6; 64-64-64-50, 2^20: 214 / 134.
+constexpr uint32_t kForwardFrom = 4096;
+
+static bool chain_train_network(const MlpConfig& c)
+{
+    if (!chain_network(c)) return false;
+    if (c.n_layers < 5) return true;
+    // five layers of width 64 with wide inputs or outputs leave room for one chain only
+    return c.dims[0] <= 32 && c.dims[c.n_layers] <= 16;
+}
+
+bool chain_train_suits(const MlpConfig& c, uint32_t count) { return count >= kTrainFrom && chain_train_network(c); }
+bool chain_forward_suits(const MlpConfig& c, uint32_t count) { return count >= kForwardFrom && chain_network(c); }
+
+cudaError_t launch_learn_gradient_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpLearnGradParamsEx& a,
+                                        int* launches, std::string* err, float* input_grads)
+{
+    if (!chain_train_network(c)) { if (err) *err = "shape not built for tiles of samples"; return cudaErrorInvalidValue; }
+    narrow::Params p = chain_params(ws, c, a.networkBuffer, a.inputs, a.count);
+    p.loss_words = (uint32_t*)a.lossBuffer;
+    p.targets = (const void*)a.targets;
+    p.input_grads = input_grads;
+    const int tgt = c.target_dtype == MLP_F32 ? 4 : 2;
+    p.vec_tgt = pieces(a.targets, c.dims[c.n_layers], tgt, 4 * tgt);
+    p.vec_dx = pieces((uint64_t)input_grads, c.dims[0], 4, 32);
+    *launches += 1;
+    switch (c.n_layers) {
+    case 2: return launch_chain_train<2>(st, ws, p);
+    case 3: return launch_chain_train<3>(st, ws, p);
+    case 4: return launch_chain_train<4>(st, ws, p);
+    case 5: return launch_chain_train<5>(st, ws, p);
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_forward_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpForwardParams& a,
+                                 int* launches, std::string* err)
+{
+    if (!chain_network(c)) { if (err) *err = "shape not built for tiles of samples"; return cudaErrorInvalidValue; }
+    narrow::Params p = chain_params(ws, c, a.networkBuffer, a.inputs, a.count);
+    p.outputs = (float*)a.outputs;
+    p.vec_out = pieces(a.outputs, c.dims[c.n_layers], 4, 16);
+    *launches += 1;
+    return launch_chain_forward(st, ws, p);
+}
+#endif
+
+}  // namespace mlpb200

@@ -1,0 +1,396 @@
+// Networks of widths up to 64 on tcgen05 with whole tiles of 128 samples: what the kernels of tc_chain.cu share.
+//
+// A "chain" is four warps that carry one tile through the network: a thread owns one sample (one tensor-memory lane).  The
+// layer inputs A_l lie in shared memory as [128 samples][features] tiles, 16-bit, swizzled, so that one copy is the K-major
+// operand of the next layer's product and the MN-major operand of the weight-gradient product, and dZ_l replaces A_{l+1} where
+// it lay.  A fifth warp per chain issues its layer products and two warps the gradient products of all chains, so nothing
+// waits for another chain, and a chain's hand-offs (some 500 cycles each) are covered by the others' work.
+// Code that runs once per tile is kept small: the kernel is bound by instruction issue, and its loops have to stay in the
+// instruction cache (texture network, 2^24 texels: 2.5 ms a step with one copy of the gradient products' code, 2.6 with one
+// per layer and chain).
+#pragma once
+
+#include "tc_layout.cuh"
+#include "tc_narrow.cuh"
+
+namespace mlpb200 {
+namespace chain {
+
+using narrow::Cvt;
+using namespace ptx;
+using narrow::Params;
+
+constexpr int kTile = 128;   // samples of a tile
+
+// tcgen05.wait::ld that the loaded registers depend on
+__device__ __forceinline__ void wait_ld(uint32_t (&r)[32])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                   "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 ::"memory");
+}
+__device__ __forceinline__ void wait_ld(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 ::"memory");
+}
+
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b)
+{
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Byte offset of the first 16-byte chunk of row r of a [rows][W] operand tile (W 16, 32 or 64); chunk j is there ^ (16 j), as
+// tiles start on 1024-byte boundaries.
+template <int W>
+__device__ __forceinline__ uint32_t row_at(int r)
+{
+    return (uint32_t)r * (uint32_t)layout::row_bytes(W) + (uint32_t)(((r >> layout::swz_shift(W)) & layout::swz_mask(W)) << 4);
+}
+
+// Operand descriptors of a [rows][W] tile at byte offset `at` (lo: the base's address field).  K-major: step k is 16
+// features, 32 bytes inside the row.  MN-major: step k is 16 rows; `lbo` bytes lead from one row-wide block of the other
+// dimension to the next.
+template <int W>
+__device__ __forceinline__ uint64_t desc_k(uint32_t lo, uint32_t at, int k)
+{
+    constexpr uint32_t hi = ((8u * (uint32_t)layout::row_bytes(W)) >> 4) | (1u << 14) | (layout::layout_type(W) << 29);
+    return ((uint64_t)hi << 32) | (lo + ((at + (uint32_t)k * 32u) >> 4) + (1u << 16));
+}
+template <int W>
+__device__ __forceinline__ uint64_t desc_mn(uint32_t lo, uint32_t at, int k, uint32_t lbo = 16u)
+{
+    constexpr uint32_t hi = ((8u * (uint32_t)layout::row_bytes(W)) >> 4) | (1u << 14) | (layout::layout_type(W) << 29);
+    return ((uint64_t)hi << 32) | (lo + ((at + (uint32_t)k * 16u * (uint32_t)layout::row_bytes(W)) >> 4) + ((lbo >> 4) << 16));
+}
+
+// The biases of hidden layers enter as one more K step of the layer product, the first: a tile of rows (1, 0, .. 0) times rows
+// (bias, 0, .. 0), 16 wide.  The accumulator is then the pre-activation (one addition and half a shared-memory read per
+// pair of values less: 1920 x 1080 view 106 -> 95 us, texture step of 2^24 texels 2.52 -> 2.39 ms).  All groups of eight rows of the first are one.
+constexpr uint32_t kUnitBytes = 8 * 32;
+__device__ __forceinline__ uint64_t desc_unit(uint32_t lo, uint32_t at)
+{
+    constexpr uint32_t hi = (1u << 14) | (layout::layout_type(16) << 29);
+    return ((uint64_t)hi << 32) | (lo + (at >> 4) + (1u << 16));
+}
+// Rows whose first value is `value(row)` and the rest zero.
+template <class F>
+__device__ __forceinline__ void first_column(uint8_t* dst, int rows, int tid, int nthreads, F value)
+{
+    for (int i = tid; i < rows * 2; i += nthreads) {
+        const int row = i >> 1, chunk = i & 1;
+        *(uint4*)(dst + (row_at<16>(row) ^ (uint32_t)(16 * chunk))) = make_uint4(chunk == 0 ? value(row) & 0xffffu : 0u, 0u, 0u, 0u);
+    }
+}
+
+// A layer's weights as a zero-padded [rows][W] tile (rows: outputs), 16-bit storage.
+template <int W>
+__device__ __forceinline__ void stage_weights(uint8_t* dst, const MlpConfig& c, const void* weights, int rows, int in, int out, int tid, int nthreads)
+{
+    const uint16_t* w = (const uint16_t*)weights;
+    const bool whole = c.param_layout == MLP_PARAMS_ROW_MAJOR && (in & 7) == 0 && ((uint64_t)w & 15u) == 0;
+#pragma unroll 1
+    for (int i = tid; i < rows * (W / 8); i += nthreads) {
+        const int o = i / (W / 8), j = i % (W / 8);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (o < out && 8 * j < in) {
+            if (whole) {
+                v = *(const uint4*)(w + o * in + 8 * j);
+            } else {
+                uint16_t h[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) h[e] = 8 * j + e < in ? w[weight_index(c.param_layout, in, out, o, 8 * j + e)] : (uint16_t)0;
+                v = make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
+            }
+        }
+        *(uint4*)(dst + (row_at<W>(o) ^ (uint32_t)(16 * j))) = v;
+    }
+}
+
+// Value i of a row of fp32 or 16-bit values where `real`, else zero, without a branch; what is loaded is first touched by its use.
+__device__ __forceinline__ uint32_t load_bits(const char* row, bool wide, int i, bool real)
+{
+    uint32_t v;
+    if (wide)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.b32 %0, [%1];\n\t}" : "=r"(v) : "l"(row + 4 * i), "r"((int)real));
+    else
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.u16 %0, [%1];\n\t}" : "=r"(v) : "l"(row + 2 * i), "r"((int)real));
+    return v;
+}
+__device__ __forceinline__ float bits_value(int dtype, uint32_t b)
+{
+    return dtype == MLP_F32 ? __uint_as_float(b) : dtype == MLP_F16 ? __half2float(__ushort_as_half((uint16_t)b)) : __uint_as_float(b << 16);
+}
+
+// What a thread needs of its next sample's input before it can build the row: the two coordinates of the frequency
+// encoding, or the whole of a short row, as stored.
+struct RawRow { uint32_t v[8]; };
+
+__device__ __forceinline__ bool short_row(const MlpConfig& c) { return c.encoding == MLP_ENC_FREQ2D || c.dims[0] <= 8; }
+
+// Where a thread's input or target rows lie: one tile's to the next's.
+struct Rows {
+    const char* at;
+    uint64_t step;
+    __device__ __forceinline__ Rows(const void* base, int width, int dtype, uint64_t sample, uint32_t samples)
+        : at((const char*)base + sample * (uint64_t)(width * (dtype == MLP_F32 ? 4 : 2))), step((uint64_t)samples * (uint64_t)(width * (dtype == MLP_F32 ? 4 : 2))) {}
+};
+__device__ __forceinline__ int stored_inputs(const MlpConfig& c) { return c.encoding == MLP_ENC_FREQ2D ? 2 : c.dims[0]; }
+
+// 16 bytes where `real`, else zero, as load_bits().
+__device__ __forceinline__ void load_four(uint32_t* v, const char* at, bool real)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+                 "@q ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];\n\t}" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(at), "r"((int)real));
+}
+
+__device__ __forceinline__ void fetch_row(RawRow& raw, const Params& p, const char* row, bool real)
+{
+    const MlpConfig& c = p.cfg;
+    if (!short_row(c)) return;
+    const int width = stored_inputs(c);
+    const bool wide = c.input_dtype == MLP_F32;
+    if (wide && p.vec_in && c.encoding != MLP_ENC_FREQ2D) {   // four or eight values
+        load_four(raw.v, row, real);
+        if (width > 4) load_four(raw.v + 4, row + 16, real);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (i == 2 && width <= 2) break;
+        if (i == 4 && width <= 4) break;
+        raw.v[i] = load_bits(row, wide, i, real && i < width);
+    }
+}
+
+// Rows that are neither short nor whole 16-byte pieces of fp32 or operand-type values.
+template <int FMT>
+static __device__ __noinline__ void convert_row(uint32_t at, int dtype, const char* row, int width, bool real)
+{
+    for (int j = 0; j < (width + 15) / 16 * 2; ++j) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = real && 8 * j + i < width ? load_as_f32(dtype, row, 8 * j + i) : 0.0f;
+        using C = Cvt<FMT>;
+        sts128(at ^ (uint32_t)(16 * j), C::pack2(x[0], x[1]), C::pack2(x[2], x[3]), C::pack2(x[4], x[5]), C::pack2(x[6], x[7]));
+    }
+}
+
+// A thread's input row in operand format, up to the end of its last K step; `free()` is called before the first store.
+template <int FMT, int IW, class F>
+__device__ __forceinline__ void write_row(uint32_t at, const Params& p, const RawRow& raw, const char* src_row, bool real, F free)
+{
+    using C = Cvt<FMT>;
+    const MlpConfig& c = p.cfg;
+    const int width = c.dims[0], type = c.input_dtype;
+    if (c.encoding == MLP_ENC_FREQ2D) {
+        // chunks 0, 1: the first coordinate's octaves 0 to 3 and 4 to 7; chunks 2, 3: the second's
+        const float u = bits_value(type, raw.v[0]), v = bits_value(type, raw.v[1]);
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+            float2 x[8];
+            narrow::encode_octaves(u, v, 4 * k, x);
+            if (k == 0) free();
+            sts128(at ^ (uint32_t)(16 * k), C::pack2(x[0].x, x[1].x), C::pack2(x[2].x, x[3].x), C::pack2(x[4].x, x[5].x), C::pack2(x[6].x, x[7].x));
+            sts128(at ^ (uint32_t)(32 + 16 * k), C::pack2(x[0].y, x[1].y), C::pack2(x[2].y, x[3].y), C::pack2(x[4].y, x[5].y), C::pack2(x[6].y, x[7].y));
+        }
+    } else if (width <= 8) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = i < width ? bits_value(type, raw.v[i]) : 0.0f;
+        free();
+        sts128(at, C::pack2(x[0], x[1]), C::pack2(x[2], x[3]), C::pack2(x[4], x[5]), C::pack2(x[6], x[7]));
+        sts128(at ^ 16u, 0u, 0u, 0u, 0u);
+    } else if (p.vec_in && type == MLP_F32) {
+#pragma unroll 1
+        for (int h = 0; h < IW; h += 32) {
+            if (h >= width) break;
+            const float4* src = (const float4*)src_row + h / 4;
+            float4 x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = real && h + 4 * j < width ? __ldg(src + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (h == 0) free();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                sts128(at ^ (uint32_t)(2 * h + 16 * j), C::pack2(x[2 * j].x, x[2 * j].y), C::pack2(x[2 * j].z, x[2 * j].w), C::pack2(x[2 * j + 1].x, x[2 * j + 1].y),
+                       C::pack2(x[2 * j + 1].z, x[2 * j + 1].w));
+        }
+    } else if (p.vec_in && type == FMT) {
+        const uint4* src = (const uint4*)src_row;
+        uint4 x[IW / 8];
+#pragma unroll
+        for (int j = 0; j < IW / 8; ++j) x[j] = real && 8 * j < width ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+        free();
+#pragma unroll
+        for (int j = 0; j < IW / 8; ++j) sts128(at ^ (uint32_t)(16 * j), x[j].x, x[j].y, x[j].z, x[j].w);
+    } else {
+        free();
+        convert_row<FMT>(at, type, src_row, width, real);
+    }
+}
+
+// Starts a row on its way into L2.
+__device__ __forceinline__ void prefetch_row(const char* row) { asm volatile("prefetch.global.L2 [%0];" ::"l"(row)); }
+
+// Four values of a sample's target row from feature f on (f a multiple of four); zero past its width.
+__device__ __forceinline__ void load_targets(float (&t)[4], const Params& p, const char* row, int od, int f)
+{
+    const int dtype = p.cfg.target_dtype;
+    if (p.vec_tgt) {   // rows are whole pieces of four values
+        if (dtype == MLP_F32) {
+            const float4 x = __ldg((const float4*)((const float*)row + f));
+            t[0] = x.x; t[1] = x.y; t[2] = x.z; t[3] = x.w;
+        } else {
+            const uint2 x = __ldg((const uint2*)((const uint16_t*)row + f));
+            t[0] = bits_value(dtype, x.x & 0xffffu);
+            t[1] = bits_value(dtype, x.x >> 16);
+            t[2] = bits_value(dtype, x.y & 0xffffu);
+            t[3] = bits_value(dtype, x.y >> 16);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[i] = bits_value(dtype, load_bits(row, dtype == MLP_F32, f + i, f + i < od));
+    }
+}
+
+static __device__ __noinline__ float2 value_and_derivative(int act, float alpha, float z) { return make_float2(act_value(act, alpha, z), act_deriv(act, alpha, z)); }
+
+// The output activation of four values and its derivative.
+__device__ __forceinline__ void activate_outputs(int act, float alpha, float (&v)[4], float (&d)[4])
+{
+    if (act == MLP_ACT_IDENTITY) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = 1.0f;
+    } else if (act == MLP_ACT_SIGMOID) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float ex = expf(-fabsf(v[i]));
+            v[i] = narrow::divide_by_1_to_2(v[i] >= 0.0f ? 1.0f : ex, 1.0f + ex);
+            d[i] = v[i] * (1.0f - v[i]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 r = value_and_derivative(act, alpha, v[i]);
+            v[i] = r.x;
+            d[i] = r.y;
+        }
+    }
+}
+
+// Four output columns' accumulators plus bias, rounded, from output f on.
+template <int FMT>
+__device__ __forceinline__ void output_columns(float (&o)[4], uint32_t t_acc, uint32_t bias, int f)
+{
+    using C = Cvt<FMT>;
+    uint32_t v[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(t_acc + (uint32_t)f) : "memory");
+    const float4 b = narrow::lds_float4(bias + 4u * (uint32_t)f);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])::"memory");
+    o[0] = C::round(__uint_as_float(v[0]) + b.x);
+    o[1] = C::round(__uint_as_float(v[1]) + b.y);
+    o[2] = C::round(__uint_as_float(v[2]) + b.z);
+    o[3] = C::round(__uint_as_float(v[3]) + b.w);
+}
+
+// A row's hidden activations: 32 pre-activations rounded and activated, into the four chunks from `at` on (at: the first one's
+// address, a multiple of four chunks in the row).  ReLU: the smallest magnitude seen goes to `least`.
+template <int FMT, int HACT>
+__device__ __forceinline__ void hidden_columns(const uint32_t (&v)[32], uint32_t at, float alpha, float& least)
+{
+    using C = Cvt<FMT>;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        uint32_t a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float z0 = __uint_as_float(v[8 * j + 2 * i]), z1 = __uint_as_float(v[8 * j + 2 * i + 1]);
+            const uint32_t zp = C::pack2(z0, z1);
+            if constexpr (HACT == MLP_ACT_RELU) {
+                a[i] = C::relu2(zp);
+                least = fminf(fminf(fabsf(z0), fabsf(z1)), least);
+            } else {
+                const float2 az = __ffma2_rn(make_float2(C::lo(zp), C::hi(zp)), make_float2(alpha, alpha), make_float2(0.0f, 0.0f));
+                a[i] = C::max2(zp, C::pack2(az.x, az.y));
+            }
+        }
+        sts128(at ^ (uint32_t)(16 * j), a[0], a[1], a[2], a[3]);
+    }
+}
+
+// ReLU activations of a row in which a pre-activation rounds to zero, once more from the accumulator: those zeros are marked
+// by the sign.  Rare, so kept small.
+template <int FMT, int H>
+__device__ __forceinline__ void marked_columns(uint32_t t_acc, uint32_t row)
+{
+    using C = Cvt<FMT>;
+    constexpr float kTiny = 0.5f * C::kSmallest;   // the largest magnitude that rounds to zero
+#pragma unroll 1
+    for (int j = 0; j < H / 8; ++j) {
+        uint32_t v[8], a[4];
+        tmem_ld_32x8(t_acc + (uint32_t)(8 * j), v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float z0 = __uint_as_float(v[2 * i]), z1 = __uint_as_float(v[2 * i + 1]);
+            a[i] = C::relu2(C::pack2(z0, z1)) | (fabsf(z0) <= kTiny ? 0x8000u : 0u) | (fabsf(z1) <= kTiny ? 0x80000000u : 0u);
+        }
+        sts128(row ^ (uint32_t)(16 * j), a[0], a[1], a[2], a[3]);
+    }
+}
+
+// dZ = dA times the derivative, of the activations in the four chunks from `at` on.
+template <int FMT, int HACT>
+__device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_t (&v)[32], uint32_t at, float alpha_op)
+{
+    using C = Cvt<FMT>;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint4 act = narrow::lds128(at ^ (uint32_t)(16 * j));
+        const uint32_t a[4] = {act.x, act.y, act.z, act.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float g0 = __uint_as_float(v[8 * j + 2 * i]), g1 = __uint_as_float(v[8 * j + 2 * i + 1]);
+            if constexpr (HACT == MLP_ACT_RELU) {
+                z[4 * j + i] = C::pack2(g0, g1) & C::positive_mask(a[i]);
+            } else {
+                const uint32_t neg = narrow::sign_mask(a[i]);
+                const float2 ag = __fmul2_rn(make_float2(g0, g1), make_float2(alpha_op, alpha_op));
+                z[4 * j + i] = (C::pack2(ag.x, ag.y) & neg) | (C::pack2(g0, g1) & ~neg);
+            }
+        }
+    }
+}
+
+// The same over a whole row with marked zeros, where half of the gradient passes, in place.
+template <int FMT, int H>
+__device__ __forceinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row)
+{
+    using C = Cvt<FMT>;
+#pragma unroll 1
+    for (int j = 0; j < H / 8; ++j) {
+        uint32_t v[8], z[4];
+        tmem_ld_32x8(t_acc + (uint32_t)(8 * j), v);
+        const uint4 act = narrow::lds128(row ^ (uint32_t)(16 * j));
+        const uint32_t a[4] = {act.x, act.y, act.z, act.w};
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float g0 = __uint_as_float(v[2 * i]), g1 = __uint_as_float(v[2 * i + 1]);
+            z[i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | (C::pack2(0.5f * g0, 0.5f * g1) & narrow::sign_mask(a[i]));
+        }
+        sts128(row ^ (uint32_t)(16 * j), z[0], z[1], z[2], z[3]);
+    }
+}
+
+}  // namespace chain
+}  // namespace mlpb200

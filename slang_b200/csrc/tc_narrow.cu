@@ -980,6 +980,7 @@ cudaError_t launch_forward_narrow(cudaStream_t st, TcWorkspace* ws, const MlpCon
 {
     if (!tc_train_narrow_supported(c)) { if (err) *err = "shape not built for the narrow tensor-core path"; return cudaErrorInvalidValue; }
     if (a.count == 0) return cudaSuccess;
+    if (chain_forward_suits(c, a.count)) return launch_forward_chain(st, ws, c, a, launches, err);
     narrow::Params p = narrow_params(ws, c, a.networkBuffer, a.inputs, a.count);
     p.outputs = (float*)a.outputs;
     p.vec_out = whole_pieces(a.outputs, c.dims[c.n_layers], MLP_F32, 4);
@@ -992,6 +993,7 @@ cudaError_t launch_learn_gradient_narrow(cudaStream_t st, TcWorkspace* ws, const
 {
     if (!tc_train_narrow_supported(c)) { if (err) *err = "shape not built for the narrow tensor-core path"; return cudaErrorInvalidValue; }
     if (a.count == 0) return cudaSuccess;
+    if (chain_train_suits(c, a.count)) return launch_learn_gradient_chain(st, ws, c, a, launches, err, input_grads);
     narrow::Params p = narrow_params(ws, c, a.networkBuffer, a.inputs, a.count);
     p.loss_words = (uint32_t*)a.lossBuffer;
     p.targets = (const void*)a.targets;

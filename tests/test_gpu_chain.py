@@ -1,0 +1,122 @@
+"""Kernels that run whole tiles of 128 samples on the tensor pipe: samples around a tile and around the SMs' shares, every padded
+width and layer count, input rows of each kind, outputs that leave in each way, pre-activations that are zero."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from slang_b200 import config as C
+
+from mlp_testlib import layer_rel_errs, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    from slang_b200.api import Device
+    d = Device(0)
+    yield d
+    d.destroy()
+
+
+def _run(device, cfg, count, p0=None, x=None, t=None, input_grads=False):
+    """Gradients, loss, outputs and input gradients of the GPU and of the oracle."""
+    from slang_b200.api import Trainer
+    dims = cfg.layer_dims
+    rng = np.random.default_rng(sum(dims) + count)
+    width = 2 if cfg.encoding == C.ENC_FREQ2D else dims[0]
+    if x is None:
+        x = rng.uniform(0 if width == 2 else -1, 1, (count, width))
+    x = C.to_storage(x, cfg.input_dtype)
+    t = C.to_storage(rng.uniform(-1, 1, (count, dims[-1])) if t is None else t, cfg.target_dtype)
+    p0 = C.init_params(cfg, seed=3, scheme="xavier") if p0 is None else p0
+    tr = Trainer(device, cfg, p0)
+    xb, tb = device.create_buffer(x.nbytes, x), device.create_buffer(t.nbytes, t)
+    yb, gb = device.create_buffer(4 * count * dims[-1]), device.create_buffer(4 * count * dims[0])
+    tr.learn_gradient(xb.address, tb.address, count, input_grads_address=gb.address if input_grads else 0)
+    grads = np.zeros(tr.total, dtype=np.float32)
+    ref = oracle.learn_gradient(cfg, p0, grads, x, t, count, n_threads=8).view(np.float32)
+    loss = tr.read_loss()
+    got = tr.read_grads()
+    tr.forward(xb.address, yb.address, count)
+    want = np.asarray(oracle.forward(cfg, p0, x, count)).reshape(count, dims[-1])
+    out = yb.read(np.float32).reshape(count, dims[-1])
+    return got, grads, loss, ref, out, want, gb.read(np.float32).reshape(count, dims[0])
+
+
+def _check(cfg, result, bar):
+    got, grads, loss, ref, out, want, _ = result
+    assert max(layer_rel_errs(cfg, got, grads)) < bar
+    assert abs(loss[0] - ref[0]) <= bar * ref[0] and abs(loss[1] - ref[1]) <= bar * ref[1]
+    assert rel_err(out, want) < bar
+
+
+@pytest.mark.parametrize("count", [1023, 1024, 1025, 1151, 4095, 4096, 4097, 148 * 128 * 3 + 1])
+@pytest.mark.parametrize("dims", [[4, 32, 32, 32, 32, 4], [32, 64, 64, 64, 3], [64, 64, 64, 64, 64], [9, 17, 1]], ids=lambda d: "-".join(map(str, d)))
+def test_counts_around_a_tile(device, dims, count):
+    cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
+    _check(cfg, _run(device, cfg, count), 1e-2)
+
+
+@pytest.mark.parametrize("dtype,act", [(C.F16, C.ACT_RELU), (C.BF16, C.ACT_RELU), (C.F16, C.ACT_LEAKY_RELU), (C.BF16, C.ACT_LEAKY_RELU)],
+                         ids=["f16-relu", "bf16-relu", "f16-leaky", "bf16-leaky"])
+@pytest.mark.parametrize("dims,input_dtype", [([1, 2, 1], C.F32), ([16, 32, 16], C.F32), ([31, 33, 33, 17], C.F32), ([12, 20, 20, 20, 20, 5], C.F32),
+                                              ([24, 64, 64, 64, 16], None), ([40, 48, 48, 48, 64], None), ([33, 64, 64, 9], None),
+                                              ([20, 50, 50, 50, 50, 8], C.F32), ([8, 32, 32, 32, 32], None), ([7, 40, 4], None)],
+                         ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else "f32" if v == C.F32 else "own")
+def test_shapes_and_formats(device, dims, input_dtype, dtype, act):
+    """Every build; rows that are read as values, as whole pieces and converted one by one.  In bf16 a sum that rounds the other
+    way is 2^-8 of its value, and a few of them meet in a gradient."""
+    cfg = C.make_config(dims, dtype, act, input_dtype=dtype if input_dtype is None else input_dtype, target_dtype=C.F32 if dims[-1] % 2 else dtype, adam_master=1)
+    _check(cfg, _run(device, cfg, 5003), 2e-2 if dtype == C.BF16 else 1e-2)
+
+
+@pytest.mark.parametrize("out", [3, 20])
+def test_frequency_encoding(device, out):
+    cfg = C.make_config([32, 64, 64, out], C.F16, C.ACT_RELU, output_act=C.ACT_SIGMOID, loss=C.LOSS_L2_SUM, encoding=C.ENC_FREQ2D, input_dtype=C.F32,
+                        target_dtype=C.F32, adam_master=1)
+    _check(cfg, _run(device, cfg, 6001), 1e-2)
+
+
+@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [32, 64, 64, 3], [36, 64, 64, 20]], ids=lambda d: "-".join(map(str, d)))
+def test_zero_preactivations_pass_half_of_the_gradient(device, dims):
+    """Samples whose inputs are all zero meet zero biases: their pre-activations are zero in every layer."""
+    cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
+    rng = np.random.default_rng(1)
+    x = rng.uniform(-1, 1, (3000, dims[0])) * (rng.random((3000, 1)) < 0.5)
+    p0 = C.from_storage(C.init_params(cfg, seed=3, scheme="xavier"), C.F16)
+    _, b_off, _ = C.param_layout(cfg)
+    for l in range(cfg.n_layers):
+        p0[b_off[l]:b_off[l] + dims[l + 1]] = 0.0
+    _check(cfg, _run(device, cfg, 3000, C.to_storage(p0, C.F16), x), 1e-2)
+
+
+@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [32, 64, 64, 3], [40, 64, 64, 20], [7, 24, 3]], ids=lambda d: "-".join(map(str, d)))
+def test_input_gradients(device, dims):
+    """Against the chain rule in fp64 over the stored weights.  Roundings to half (2^-11) leave a row within a few 1e-3, except
+    where a pre-activation lies so close to zero that they carry it over the kink: 2^-11 of a unit's range, some 192 units
+    a sample, so one or two rows in a hundred differ by a whole slope."""
+    cfg = C.make_config(dims, C.F16, C.ACT_LEAKY_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
+    count = 2049
+    p0 = C.init_params(cfg, seed=3, scheme="xavier")
+    rng = np.random.default_rng(sum(dims) + count)
+    x = rng.uniform(-1, 1, (count, dims[0])).astype(np.float32)
+    t = rng.uniform(-1, 1, (count, dims[-1])).astype(np.float32)
+    p = C.from_storage(p0, C.F16).astype(np.float64)
+    w_off, b_off, _ = C.param_layout(cfg)
+    a, zs = x.astype(np.float16).astype(np.float64), []
+    for l in range(cfg.n_layers):
+        w = p[w_off[l]:w_off[l] + dims[l] * dims[l + 1]].reshape(dims[l + 1], dims[l])
+        z = a @ w.T + p[b_off[l]:b_off[l] + dims[l + 1]]
+        zs.append(z)
+        a = np.where(z < 0, cfg.act_alpha * z, z) if l < cfg.n_layers - 1 else z
+    g = 2.0 / dims[-1] * (a - t)
+    for l in reversed(range(cfg.n_layers)):
+        w = p[w_off[l]:w_off[l] + dims[l] * dims[l + 1]].reshape(dims[l + 1], dims[l])
+        g = g @ w
+        if l > 0:
+            g = g * np.where(zs[l - 1] < 0, cfg.act_alpha, 1.0)
+    got = _run(device, cfg, count, p0, x, t, input_grads=True)[6]
+    rows = np.linalg.norm(got - g, axis=1) / np.linalg.norm(g, axis=1)
+    assert np.mean(rows > 1e-2) < 0.05, np.mean(rows > 1e-2)
+    assert np.linalg.norm(got - g) / np.linalg.norm(g) < 0.1
