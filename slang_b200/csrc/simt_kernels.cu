@@ -57,6 +57,23 @@ __device__ __forceinline__ void encode_input(const MlpConfig& c, const void* inp
     }
 }
 
+// Activations with one copy of the switch behind a call: inlined at every use it made the tile kernel 11.9 k instructions long, most
+// of whose time at small batches went into fetching them.
+static __device__ __noinline__ float other_act_value(int act, float alpha, float x) { return act_value(act, alpha, x); }
+static __device__ __noinline__ float other_act_deriv(int act, float alpha, float x) { return act_deriv(act, alpha, x); }
+__device__ __forceinline__ float tile_act_value(int act, float alpha, float x)
+{
+    if (act == MLP_ACT_RELU) return act_value(MLP_ACT_RELU, alpha, x);
+    if (act == MLP_ACT_IDENTITY) return x;
+    return other_act_value(act, alpha, x);
+}
+__device__ __forceinline__ float tile_act_deriv(int act, float alpha, float x)
+{
+    if (act == MLP_ACT_RELU) return act_deriv(MLP_ACT_RELU, alpha, x);
+    if (act == MLP_ACT_IDENTITY) return 1.0f;
+    return other_act_deriv(act, alpha, x);
+}
+
 // One term of a scalar sum in the order MlpConfig.sum_order names: a fused multiply-add, or a rounded
 // product followed by a rounded add (this file is compiled with -fmad=false, so `acc + a * b` is two
 // roundings).
@@ -189,7 +206,7 @@ __device__ __forceinline__ void tile_layer_forward(const MlpConfig& c, const Wei
     for (int u = 0; u < J; ++u) {
         if (j0 + u >= w.out) break;
         const float zs = round_to(c.dtype, fused ? r[u] : r[u] + s_bias[j0 + u]);
-        const float v = act_value(act, c.act_alpha, zs);
+        const float v = tile_act_value(act, c.act_alpha, zs);
         z[(j0 + u) * kRow] = zs;
         aout[(j0 + u) * kRow] = round_act ? round_to(operand_type(c), v) : v;
     }
@@ -312,7 +329,7 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
                 float g = 0.0f;
                 if (valid) {
                     const float diff = o[j * kRow] - (j == warp ? target : load_as_f32(c.target_dtype, targets, int64_t(s0 + lane) * od + j));
-                    g = round_to(opd, ((2.0f * scale) * diff) * act_deriv(c.output_act, c.act_alpha, dz[j * kRow]));
+                    g = round_to(opd, ((2.0f * scale) * diff) * tile_act_deriv(c.output_act, c.act_alpha, dz[j * kRow]));
                 }
                 dz[j * kRow] = g;
             }
@@ -338,7 +355,7 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     if (i0 + u >= w.in) break;
-                    const float d = round_to(opd, act_deriv(c.hidden_act, c.act_alpha, zprev[(i0 + u) * kRow]));
+                    const float d = round_to(opd, tile_act_deriv(c.hidden_act, c.act_alpha, zprev[(i0 + u) * kRow]));
                     zprev[(i0 + u) * kRow] = valid ? round_to(opd, r[u] * d) : 0.0f;
                 }
             }
@@ -425,6 +442,209 @@ learn_gradient_simt_kernel(const __grid_constant__ SimtNet net, const __grid_con
     }
     // Loss words: the largest per-sample loss, and the sum added once per CTA.
     if (warp == 0) {
+        for (int o = 16; o > 0; o >>= 1) {
+            run_max = fmaxf(run_max, __shfl_xor_sync(0xffffffffu, run_max, o));
+            run_sum += __shfl_xor_sync(0xffffffffu, run_sum, o);
+        }
+        if (lane == 0) {
+            atomicMax(lossBuffer, __float_as_uint(run_max));
+            atomicAdd((float*)(lossBuffer + 1), run_sum);
+        }
+    }
+}
+
+// learnGradient of small plain fp32 networks: ReLU, linear outputs, fp32 rows, widths up to 32.  The same tiles, rows and sums
+// as the general kernel's, a layer's outputs two to a warp, without its choices: some 850 instructions instead of twelve thousand.  A
+// step of 4096 samples runs every instruction once or twice, so fetching them was what it waited for (2-16-16-16-1: 14.3 us a
+// step, 22.5 with the general kernel; 2^20 samples 684 and 1306).
+constexpr int kSmallWidth = 32;
+
+struct SmallNet {
+    int nl, od;
+    int dims[MLP_MAX_LAYERS + 1];
+    int a_row[MLP_MAX_LAYERS + 1];          // first row of the vector entering layer l (the last: the outputs)
+    int z_row[MLP_MAX_LAYERS + 1];          // first row of z_l, later dz_l (l from 1)
+    int w_at[MLP_MAX_LAYERS], b_at[MLP_MAX_LAYERS], g_at[MLP_MAX_LAYERS];   // floats: weights (rows of a multiple of four), biases, gradient sums
+    uint32_t per_row[MLP_MAX_LAYERS];       // 65536 / (in + 1), rounded up: (i * per_row) >> 16 is i / (in + 1) below 33 * 32
+    uint32_t per_input;                     // the same of the input width
+    int total;
+    float scale;
+};
+
+__device__ __forceinline__ void copy_float(float* dst, const float* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+template <bool FUSED>
+__global__ void __launch_bounds__(kSimtThreads)
+learn_gradient_small_kernel(const __grid_constant__ SmallNet net, const MlpLayerPointers* __restrict__ lp, uint32_t* lossBuffer,
+                            const float* __restrict__ inputs, const float* __restrict__ targets, uint32_t count, uint32_t n_tiles)
+{
+    extern __shared__ __align__(16) float smem[];
+    __shared__ MlpLayerPointers s_net[MLP_MAX_LAYERS];
+    const int nl = net.nl, od = net.od, tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    grid_release();
+    grid_wait();
+    if (tid < nl * 4) reinterpret_cast<uint64_t*>(s_net)[tid] = reinterpret_cast<const uint64_t*>(lp)[tid];
+    const bool once = gridDim.x == n_tiles;
+    float run_max = 0.0f, run_sum = 0.0f;
+    bool staged = false;
+#pragma unroll 1
+    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const uint32_t s0 = tile * kTile;
+        const uint32_t n_here = min((uint32_t)kTile, count - s0);
+        const bool valid = lane < n_here;
+        {
+            const int in = net.dims[0];
+            const float* x = inputs + uint64_t(s0) * in;
+#pragma unroll 1
+            for (int i = tid; i < kTile * in; i += kSimtThreads) {
+                const int s = (int)(((uint32_t)i * net.per_input) >> 16);
+                float* dst = smem + (i - s * in) * kRow + s;
+                if (s < n_here) copy_float(dst, x + i);
+                else *dst = 0.0f;
+            }
+        }
+        float target = 0.0f;
+        if (warp < od && valid) target = __ldg(targets + uint64_t(s0 + lane) * od + warp);
+        if (!staged) {
+            staged = true;
+            __syncthreads();
+#pragma unroll 1
+            for (int l = 0; l < nl; ++l) {
+                const int in = net.dims[l], out = net.dims[l + 1], stride = (in + 3) & ~3;
+                const float* w = (const float*)s_net[l].weights;
+#pragma unroll 1
+                for (int j = warp; j < out; j += kSimtWarps) {
+                    if (lane < in) copy_float(smem + net.w_at[l] + j * stride + lane, w + j * in + lane);
+                    else if (lane < stride) smem[net.w_at[l] + j * stride + lane] = 0.0f;
+                }
+                if (tid < out) copy_float(smem + net.b_at[l] + tid, (const float*)s_net[l].biases + tid);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        // ---- forward ----
+#pragma unroll 1
+        for (int l = 0; l < nl; ++l) {
+            const int in = net.dims[l], out = net.dims[l + 1], stride = (in + 3) & ~3;
+            if (2 * warp < out) {
+                const int j0 = 2 * warp, j1 = min(j0 + 1, out - 1);
+                const float* a = smem + net.a_row[l] * kRow + lane;
+                const float* w0 = smem + net.w_at[l] + j0 * stride;
+                const float* w1 = smem + net.w_at[l] + j1 * stride;
+                const float b0 = smem[net.b_at[l] + j0], b1 = smem[net.b_at[l] + j1];
+                float r0 = FUSED ? b0 : 0.0f, r1 = FUSED ? b1 : 0.0f;
+                int i = 0;
+#pragma unroll 1
+                for (; i + 4 <= in; i += 4) {
+                    const float4 u = *reinterpret_cast<const float4*>(w0 + i), v = *reinterpret_cast<const float4*>(w1 + i);
+                    const float a0 = a[i * kRow], a1 = a[(i + 1) * kRow], a2 = a[(i + 2) * kRow], a3 = a[(i + 3) * kRow];
+                    r0 = mac(u.w, a3, mac(u.z, a2, mac(u.y, a1, mac(u.x, a0, r0, FUSED), FUSED), FUSED), FUSED);
+                    r1 = mac(v.w, a3, mac(v.z, a2, mac(v.y, a1, mac(v.x, a0, r1, FUSED), FUSED), FUSED), FUSED);
+                }
+#pragma unroll 1
+                for (; i < in; ++i) {
+                    r0 = mac(w0[i], a[i * kRow], r0, FUSED);
+                    r1 = mac(w1[i], a[i * kRow], r1, FUSED);
+                }
+                if (!FUSED) { r0 += b0; r1 += b1; }
+                const bool hidden = l < nl - 1;
+                float* z = smem + net.z_row[l + 1] * kRow + lane;
+                float* o = smem + net.a_row[l + 1] * kRow + lane;
+                // rows past the batch are zero throughout, whatever the biases are
+                const float v0 = hidden && !(r0 > 0.0f) ? 0.0f : r0, v1 = hidden && !(r1 > 0.0f) ? 0.0f : r1;
+                z[j0 * kRow] = r0;
+                o[j0 * kRow] = valid ? v0 : 0.0f;
+                if (j1 != j0) {
+                    z[j1 * kRow] = r1;
+                    o[j1 * kRow] = valid ? v1 : 0.0f;
+                }
+            }
+            __syncthreads();
+        }
+        // ---- loss (warp 0, a sample per lane, outputs in ascending order) and dz of the last layer (every warp) ----
+        {
+            const float* o = smem + net.a_row[nl] * kRow + lane;
+            const float* t = targets + uint64_t(s0 + lane) * od;
+            float* dz = smem + net.z_row[nl] * kRow + lane;
+#pragma unroll 1
+            for (int j = warp; j < od; j += kSimtWarps)
+                dz[j * kRow] = valid ? (2.0f * net.scale) * (o[j * kRow] - (j == warp ? target : __ldg(t + j))) : 0.0f;
+            if (warp == 0 && valid) {
+                float loss = 0.0f;
+#pragma unroll 1
+                for (int j = 0; j < od; ++j) {
+                    const float diff = o[j * kRow] - (j == 0 ? target : __ldg(t + j));
+                    loss = fmaf(diff * net.scale, diff, loss);
+                }
+                run_max = fmaxf(run_max, loss);
+                run_sum += loss;
+            }
+        }
+        __syncthreads();
+        // ---- backward: dz of the layer before replaces its z ----
+#pragma unroll 1
+        for (int l = nl - 1; l >= 1; --l) {
+            const int in = net.dims[l], out = net.dims[l + 1], stride = (in + 3) & ~3, i0 = 2 * warp;
+            if (i0 < in) {
+                const float* dz = smem + net.z_row[l + 1] * kRow + lane;
+                const float* w = smem + net.w_at[l] + i0;
+                float r0 = 0.0f, r1 = 0.0f;
+#pragma unroll 4
+                for (int j = 0; j < out; ++j) {
+                    const float d = dz[j * kRow];
+                    const float2 u = *reinterpret_cast<const float2*>(w + j * stride);
+                    r0 = mac(u.x, d, r0, FUSED);
+                    r1 = mac(u.y, d, r1, FUSED);
+                }
+                float* z = smem + (net.z_row[l] + i0) * kRow + lane;
+                z[0] = valid ? r0 * act_deriv(MLP_ACT_RELU, 0.0f, z[0]) : 0.0f;
+                if (i0 + 1 < in) z[kRow] = valid ? r1 * act_deriv(MLP_ACT_RELU, 0.0f, z[kRow]) : 0.0f;
+            }
+            __syncthreads();
+        }
+        // ---- parameter sums of the tile, a parameter at a time (the bias is a row's last), in ascending sample order ----
+#pragma unroll 1
+        for (int l = 0; l < nl; ++l) {
+            const int in = net.dims[l], out = net.dims[l + 1];
+            float* dW = (float*)s_net[l].weightsGrad;
+            float* dB = (float*)s_net[l].biasesGrad;
+#pragma unroll 1
+            for (int item = tid; item < out * (in + 1); item += kSimtThreads) {
+                const int j = (int)(((uint32_t)item * net.per_row[l]) >> 16), i = item - j * (in + 1);
+                const float* d = smem + (net.z_row[l + 1] + j) * kRow;
+                const float* a = smem + (net.a_row[l] + min(i, in - 1)) * kRow;
+                float acc = 0.0f;
+#pragma unroll 2
+                for (int s = 0; s < kTile; s += 4) {
+                    const float4 u = *reinterpret_cast<const float4*>(d + s);
+                    float4 v = *reinterpret_cast<const float4*>(a + s);
+                    if (i == in) v = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+                    acc = mac(u.w, v.w, mac(u.z, v.z, mac(u.y, v.y, mac(u.x, v.x, acc, FUSED), FUSED), FUSED), FUSED);
+                }
+                float* g = smem + net.g_at[l] + item;
+                if (once) atomicAdd(i == in ? dB + j : dW + j * in + i, acc);
+                else *g = tile == blockIdx.x ? acc : *g + acc;
+            }
+        }
+        __syncthreads();   // the next tile overwrites the rows
+    }
+    if (!once) {
+#pragma unroll 1
+        for (int l = 0; l < nl; ++l) {
+            const int in = net.dims[l], out = net.dims[l + 1];
+#pragma unroll 1
+            for (int item = tid; item < out * (in + 1); item += kSimtThreads) {
+                const int j = (int)(((uint32_t)item * net.per_row[l]) >> 16), i = item - j * (in + 1);
+                atomicAdd(i == in ? (float*)s_net[l].biasesGrad + j : (float*)s_net[l].weightsGrad + j * in + i, smem[net.g_at[l] + item]);
+            }
+        }
+    }
+    if (warp == 0) {
+#pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             run_max = fmaxf(run_max, __shfl_xor_sync(0xffffffffu, run_max, o));
             run_sum += __shfl_xor_sync(0xffffffffu, run_sum, o);
@@ -573,6 +793,51 @@ cudaError_t launch_forward_simt(cudaStream_t st, const MlpConfig& c, const MlpFo
     return cudaGetLastError();
 }
 
+static bool small_network(const MlpConfig& c)
+{
+    if (c.dtype != MLP_F32 || (c.operand_dtype && c.operand_dtype != MLP_F32) || c.input_dtype != MLP_F32 || c.target_dtype != MLP_F32) return false;
+    if (c.encoding != MLP_ENC_NONE || c.param_layout != MLP_PARAMS_ROW_MAJOR || c.hidden_act != MLP_ACT_RELU || c.output_act != MLP_ACT_IDENTITY) return false;
+    for (int l = 0; l <= c.n_layers; ++l)
+        if (c.dims[l] > kSmallWidth) return false;
+    return true;
+}
+
+static cudaError_t launch_learn_gradient_small(cudaStream_t st, const MlpConfig& c, const MlpLearnGradParamsEx& a, int* launches)
+{
+    SmallNet net = {};
+    net.nl = c.n_layers;
+    net.od = c.dims[c.n_layers];
+    net.scale = c.loss == MLP_LOSS_MSE_MEAN ? 1.0f / float(net.od) : 1.0f;
+    net.per_input = (65536u + (uint32_t)c.dims[0] - 1u) / (uint32_t)c.dims[0];
+    int rows = 0;
+    for (int l = 0; l <= c.n_layers; ++l) { net.dims[l] = c.dims[l]; net.a_row[l] = rows; rows += c.dims[l]; }
+    for (int l = 1; l <= c.n_layers; ++l) { net.z_row[l] = rows; rows += c.dims[l]; }
+    int floats = rows * kRow;
+    for (int l = 0; l < c.n_layers; ++l) {
+        net.w_at[l] = floats; floats += c.dims[l + 1] * ((c.dims[l] + 3) & ~3);
+        net.per_row[l] = (65536u + (uint32_t)c.dims[l]) / ((uint32_t)c.dims[l] + 1u);
+    }
+    for (int l = 0; l < c.n_layers; ++l) { net.b_at[l] = floats; floats += c.dims[l + 1]; }
+    for (int l = 0; l < c.n_layers; ++l) { net.g_at[l] = floats; floats += c.dims[l + 1] * (c.dims[l] + 1); }
+    net.total = floats;
+    const size_t smem = size_t(floats) * 4;
+    constexpr size_t kLargest = ((2 * MLP_MAX_LAYERS + 1) * kSmallWidth * kRow + MLP_MAX_LAYERS * kSmallWidth * (2 * kSmallWidth + 2)) * 4;
+    static_assert(kLargest <= kSimtSmemMax, "the largest small network fits");
+    const bool fused = c.sum_order == MLP_SUM_BIAS_FIRST_FUSED;
+    auto kern = fused ? learn_gradient_small_kernel<true> : learn_gradient_small_kernel<false>;
+    int device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    static SmemLimit limit[2];   // one per build
+    if (e == cudaSuccess) e = limit[fused].raise((const void*)kern, device, kLargest);
+    if (e != cudaSuccess) return e;
+    const uint32_t tiles = (uint32_t)((uint64_t(a.count) + kTile - 1) / kTile);
+    const uint32_t per_sm = uint32_t(std::max<size_t>(1, std::min<size_t>(4, kSimtSmemMax / (smem + 2048))));
+    *launches += 1;
+    return launch_after(st, kern, std::min(tiles, per_sm * uint32_t(sms)), kSimtThreads, smem, net, (const MlpLayerPointers*)a.networkBuffer,
+                        (uint32_t*)a.lossBuffer, (const float*)a.inputs, (const float*)a.targets, a.count, tiles);
+}
+
 cudaError_t launch_learn_gradient_simt(cudaStream_t st, const MlpConfig& c, const MlpLearnGradParamsEx& a,
                                        float* seq_scratch, int* launches, std::string* err, float* input_grads)
 {
@@ -580,6 +845,7 @@ cudaError_t launch_learn_gradient_simt(cudaStream_t st, const MlpConfig& c, cons
     if (!make_simt_net(c, &net, err)) return cudaErrorInvalidValue;
     if (a.count == 0) return cudaSuccess;
     const bool seq = (a.flags & MLP_FLAG_SEQUENTIAL_SUM) != 0;
+    if (!seq && !input_grads && small_network(c)) return launch_learn_gradient_small(st, c, a, launches);
     SimtSmem map{};
     int floats = net.a_off[c.n_layers + 1] * kRow;
     map.z = floats;
