@@ -239,7 +239,9 @@ int32_t mlp_buffer_clear(MlpDevice* d, MlpBuffer* b, size_t offset, size_t size)
     if (!d || !b) return fail(MLP_E_INVALID_ARG, "null argument");
     if (offset > b->size || size > b->size - offset) return fail(MLP_E_INVALID_ARG, "clear range outside the buffer");
     CUDA_TRY(cudaSetDevice(d->ordinal));
-    CUDA_TRY(cudaMemsetAsync((char*)b->ptr + offset, 0, size, d->stream));
+    if (size == 0) return MLP_OK;
+    if (size <= kClearBytes) CUDA_TRY(launch_clear_bytes(d->stream, (char*)b->ptr + offset, (uint32_t)size));
+    else CUDA_TRY(cudaMemsetAsync((char*)b->ptr + offset, 0, size, d->stream));
     return MLP_OK;
 }
 
