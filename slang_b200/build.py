@@ -34,7 +34,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
 # (object name, source, extra flags).  The general kernels must not contract a*b+c into
 # an fma on their own: their fp32 results are compared bit for bit with a sequential CPU.  The
 # tensor-core kernels are instantiated some two hundred times; the narrow ones' source is compiled in ten parts, the
-# tile chains' in six, the wide kernel's in three (training builds, forward-only builds, training builds with the optional outputs).
+# tile chains' in seven, the wide kernel's in three (training builds, forward-only builds, training builds with the optional outputs).
 UNITS = [
     ("abi", "abi.cu", []),
     ("simt_kernels", "simt_kernels.cu", ["-fmad=false"]),
@@ -49,7 +49,7 @@ UNITS = [
     ("selftest", "selftest.cu", []),
     ("tile_mma", "tile_mma.cu", []),
 ] + [("tc_narrow_%d" % i, "tc_narrow.cu", ["-DMLPB200_NARROW_PART=%d" % i]) for i in range(10)
-] + [("tc_chain_%d" % i, "tc_chain.cu", ["-DMLPB200_CHAIN_PART=%d" % i]) for i in range(6)]
+] + [("tc_chain_%d" % i, "tc_chain.cu", ["-DMLPB200_CHAIN_PART=%d" % i]) for i in range(7)]
 
 
 def _nvcc():

@@ -62,6 +62,7 @@ cudaError_t launch_forward_narrow(cudaStream_t st, TcWorkspace* ws, const MlpCon
                                   int* launches, std::string* err);
 // The same for the networks and batches that whole tiles of 128 samples on tcgen05 suit better (tc_chain.cu).
 bool chain_train_suits(const MlpConfig& c, uint32_t count);
+bool chain_train_wide_suits(const MlpConfig& c, uint32_t count);   // networks of launch_learn_gradient_tc
 bool chain_forward_suits(const MlpConfig& c, uint32_t count);
 cudaError_t launch_learn_gradient_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpLearnGradParamsEx& a,
                                         int* launches, std::string* err, float* input_grads = nullptr);

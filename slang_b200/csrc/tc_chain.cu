@@ -42,11 +42,12 @@ template <int H, int NL, int IW, int OW, int NCH>
 struct TrainMap {
     static constexpr int kWarps = 4 * NCH;                // with samples; one more per chain issues its layer products, one or two the gradient products
     static constexpr int kGradWarps = grad_warps(NCH);
+    static constexpr bool kWide = H == 128;
     static constexpr int kThreads = 32 * (kWarps + NCH + kGradWarps);
-    static constexpr int kDzW = OW == 16 ? 32 : H;             // row width of the last layer's dZ
+    static constexpr int kDzW = OW == 16 ? 32 : OW;            // row width of the last layer's dZ
     __host__ __device__ static constexpr int in_w(int l) { return l == 0 ? IW : H; }
     __host__ __device__ static constexpr int out_w(int l) { return l == NL - 1 ? OW : H; }
-    static constexpr uint32_t kRowsIn = kTile * IW * 2, kRows = kTile * H * 2;
+    static constexpr uint32_t kRowsIn = kTile * IW * 2, kRows = kTile * H * 2, kPanel = kTile * 128;   // (of 64 features)
     // a chain's tiles: A_0, A_1 .. A_{NL-1} (dZ_{l-1} replaces A_l), dZ_{NL-1}
     __host__ __device__ static constexpr uint32_t a_off(int l) { return l == 0 ? 0u : kRowsIn + (uint32_t)(l - 1) * kRows; }
     static constexpr uint32_t kDz = a_off(NL);
@@ -55,8 +56,9 @@ struct TrainMap {
     static constexpr uint32_t kWeights = 0;
     static constexpr uint32_t kChains = (w_off(NL - 1) + (uint32_t)OW * H * 2 + 1023) & ~1023u;
     static constexpr uint32_t kOnesIn = kChains + NCH * kChainBytes;   // 16 rows whose first element is one, in the layout of A_0
-    static constexpr uint32_t kOnes = kOnesIn + (IW == H ? 0 : 16 * IW * 2);
-    static constexpr uint32_t kUnit = kOnes + 16 * H * 2;
+    static constexpr int kOnesW = H == 32 ? 32 : 64;
+    static constexpr uint32_t kOnes = kOnesIn + (IW == kOnesW ? 0 : 16 * IW * 2);
+    static constexpr uint32_t kUnit = kOnes + 16 * kOnesW * 2;
     static constexpr uint32_t kHiddenBias = kUnit + kUnitBytes;        // [NL - 1][H rows][16]
     static constexpr uint32_t kBias = kHiddenBias + (NL - 1) * H * 32; // the output layer's, fp32 [OW]
     static constexpr uint32_t kLoss = kBias + OW * 4;              // fp32 [kWarps][2]
@@ -65,13 +67,22 @@ struct TrainMap {
     static constexpr uint32_t kAbort = kTmemPtr + 4;
     static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;
     static constexpr uint32_t kSmemBytes = kNet + NL * 32 + 1024;
-    static constexpr uint32_t kSumRow = H + 1;                         // the outgoing gradients: fp32 [NL][H][H + 1], over the chains' tiles
-    static_assert(NL * H * kSumRow * 4 <= kOnesIn, "room for the sums");
+    // the outgoing gradients: fp32 [layers at a time][H][H + 1], over the chains' tiles
+    static constexpr uint32_t kSumRow = H + 1;
+    static constexpr int kSumLayers = kWide ? 1 : NL;
+    static_assert(kSumLayers * H * kSumRow * 4 <= kOnesIn, "room for the sums");
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
-    // tensor memory: an accumulator per chain, then the gradients, which the chains share
+    // Tensor memory: an accumulator per chain, then the gradients, which the chains share.  Up to width 64 dW_l | db_l is one
+    // product of 64 rows; at 128 dW_l has 128 rows (and the last layer's lies the other way round, in features by outputs)
+    // and db_l is a product of its own.
     __host__ __device__ static constexpr uint32_t dw_cols(int l) { return (uint32_t)in_w(l) + 16; }
-    __host__ __device__ static constexpr uint32_t dw_col(int l) { return NCH * (uint32_t)H + (l == 0 ? 0u : dw_cols(0) + (uint32_t)(l - 1) * (H + 16)); }
-    static_assert(dw_col(NL) <= 512, "tensor memory budget");
+    __host__ __device__ static constexpr uint32_t dw_col(int l)
+    {
+        if (kWide) return NCH * (uint32_t)H + (l == 0 ? (NL - 2) * 128u + (OW > IW ? OW : 0u) : l < NL - 1 ? (l - 1) * 128u : (NL - 2) * 128u + (OW > IW ? 0u : IW));
+        return NCH * (uint32_t)H + (l == 0 ? 0u : dw_cols(0) + (uint32_t)(l - 1) * (H + 16));
+    }
+    __host__ __device__ static constexpr uint32_t db_col(int l) { return NCH * (uint32_t)H + (NL - 2) * 128u + IW + OW + 16u * (uint32_t)l; }
+    static_assert((kWide ? db_col(NL) : dw_col(NL)) <= 512, "tensor memory budget");
 };
 
 template <int H, int NL, int IW, int OW, int NCH, int FMT, int HACT>
@@ -105,11 +116,12 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         *abort_flag = 0u;
         fence_mbar_init();
     }
-    for (int i = threadIdx.x; i < 16 * H / 2; i += kThreads) {
-        const int row = i / (H / 2), word = i % (H / 2);
-        ((uint32_t*)(smem + M::kOnes))[i] = (uint32_t)(word * 4) == row_at<H>(row) - (uint32_t)row * H * 2 ? (C::kOnes & 0xffffu) : 0u;
+    constexpr int OH = M::kOnesW;
+    for (int i = threadIdx.x; i < 16 * OH / 2; i += kThreads) {
+        const int row = i / (OH / 2), word = i % (OH / 2);
+        ((uint32_t*)(smem + M::kOnes))[i] = (uint32_t)(word * 4) == row_at<OH>(row) - (uint32_t)row * OH * 2 ? (C::kOnes & 0xffffu) : 0u;
     }
-    if constexpr (IW != H) {
+    if constexpr (IW != OH) {
         for (int i = threadIdx.x; i < 16 * IW / 2; i += kThreads) {
             const int row = i / (IW / 2), word = i % (IW / 2);
             ((uint32_t*)(smem + M::kOnesIn))[i] = (uint32_t)(word * 4) == row_at<IW>(row) - (uint32_t)row * IW * 2 ? (C::kOnes & 0xffffu) : 0u;
@@ -137,6 +149,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     });
     for (int i = threadIdx.x; i < OW; i += kThreads)
         ((float*)(smem + M::kBias))[i] = i < od ? load_as_f32(cfg.dtype, (const void*)s_net[NL - 1].biases, i) : 0.0f;
+    cp_async_wait_all();
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -214,14 +227,13 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 if (!ok) break;
                 const uint32_t dst = own_row + (uint32_t)l * M::kRows;   // A_{l + 1}
                 float least = 1.0f;
-                uint32_t v[H / 32][32];
+                uint32_t v[H == 32 ? 1 : 2][32];
                 tmem_ld_32x32(t_acc, v[0]);
-                wait_ld(v[0]);
-                if constexpr (H == 64) tmem_ld_32x32(t_acc + 32u, v[H / 32 - 1]);
-                hidden_columns<FMT, HACT>(v[0], dst, alpha, least);
-                if constexpr (H == 64) {
-                    wait_ld(v[H / 32 - 1]);
-                    hidden_columns<FMT, HACT>(v[H / 32 - 1], dst ^ 64u, alpha, least);
+#pragma unroll
+                for (int b = 0; b < H / 32; ++b) {   // the next block's read runs under this one's arithmetic
+                    wait_ld(v[b & 1]);
+                    if (b + 1 < H / 32) tmem_ld_32x32(t_acc + (uint32_t)(32 * b + 32), v[(b + 1) & (H == 32 ? 0 : 1)]);
+                    hidden_columns<FMT, HACT>(v[b & 1], block_at<H>(dst, b), alpha, least);
                 }
                 if (HACT == MLP_ACT_RELU && __any_sync(0xffffffffu, least <= 0.5f * C::kSmallest)) {   // one that rounds to zero
                     zero_seen = true;
@@ -272,21 +284,20 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     if (!ok) break;
                     reverse_marked_columns<FMT, H>(t_acc, at);
                 } else {
-                    uint32_t v[H / 32][32], z[H / 32][16];
+                    uint32_t v[H == 32 ? 1 : 2][32], z[H / 32][16];
                     tmem_ld_32x32(t_acc, v[0]);
-                    wait_ld(v[0]);
-                    if constexpr (H == 64) tmem_ld_32x32(t_acc + 32u, v[H / 32 - 1]);
-                    reverse_columns<FMT, HACT>(z[0], v[0], at, alpha_op);
-                    if constexpr (H == 64) {
-                        wait_ld(v[H / 32 - 1]);
-                        reverse_columns<FMT, HACT>(z[H / 32 - 1], v[H / 32 - 1], at ^ 64u, alpha_op);
+#pragma unroll
+                    for (int b = 0; b < H / 32; ++b) {
+                        wait_ld(v[b & 1]);
+                        if (b + 1 < H / 32) tmem_ld_32x32(t_acc + (uint32_t)(32 * b + 32), v[(b + 1) & (H == 32 ? 0 : 1)]);
+                        reverse_columns<FMT, HACT>(z[b], v[b & 1], block_at<H>(at, b), alpha_op);
                     }
                     wait_done(l);
                     if (!ok) break;
 #pragma unroll
                     for (int j = 0; j < H / 8; ++j) {
                         const uint32_t* w = &z[j >> 2][4 * (j & 3)];
-                        sts128(at ^ (uint32_t)(16 * j), w[0], w[1], w[2], w[3]);
+                        sts128(block_at<H>(at, j >> 2) ^ (uint32_t)(16 * (j & 3)), w[0], w[1], w[2], w[3]);
                     }
                 }
                 release(l > 1 || p.input_grads, l - 1);
@@ -357,7 +368,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     } else {
 #pragma unroll
                         for (int k = 0; k < H / 16; ++k)
-                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l), k), desc_k<H>(lo, M::kWeights + M::w_off(l), k), umma_idesc(F, 0, 0, 128, M::out_w(l)),
+                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l), k, M::kPanel), desc_k<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)M::out_w(l) * 128u), umma_idesc(F, 0, 0, 128, M::out_w(l)),
                                      l < NL - 1 || k > 0);
                     }
                     umma_commit(&acc_full[ch]);
@@ -373,15 +384,15 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
 #pragma unroll
                         for (int k = 0; k < OW / 16; ++k)
                             if (k < out_steps)
-                                umma_f16(acc, desc_k<M::kDzW>(lo, cb + M::kDz, k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k), umma_idesc(F, 0, 1, 128, H), k > 0);
+                                umma_f16(acc, desc_k<M::kDzW>(lo, cb + M::kDz, k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)OW * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
                     } else if (l > 0) {
 #pragma unroll
                         for (int k = 0; k < H / 16; ++k)
-                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l + 1), k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k), umma_idesc(F, 0, 1, 128, H), k > 0);
+                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l + 1), k, M::kPanel), desc_mn<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)H * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
                     } else {
 #pragma unroll
                         for (int k = 0; k < H / 16; ++k)
-                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(1), k), desc_mn<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 1, 128, IW), k > 0);
+                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(1), k, M::kPanel), desc_mn<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 1, 128, IW), k > 0);
                     }
                     umma_commit(&acc_full[ch]);
                 }
@@ -411,21 +422,51 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 const uint32_t l = (layers >> (4 * c)) & 15u, cb = M::kChains + c * M::kChainBytes;
                 const uint32_t a = l == 0 ? cb : cb + M::kRowsIn + (l - 1) * M::kRows;           // A_l
                 const uint32_t z = l == NL - 1 ? cb + M::kDz : cb + M::kRowsIn + l * M::kRows;   // dZ_l
-                const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16));
                 const uint32_t begun = (started >> l) & 1u;
-                auto gradient = [&](auto z_width, auto a_width, uint32_t ones) {
-                    constexpr int ZW = decltype(z_width)::value, AW = decltype(a_width)::value;
+                if constexpr (M::kWide) {
+                    const uint32_t db = tmem_base + M::db_col(0) + 16u * l;
+                    if (elect_one()) {
+                        if (l == NL - 1) {
+                            // A^T . dZ, and dZ^T . 1 of 64 rows (those past the outputs are never read)
 #pragma unroll
-                    for (int k = 0; k < kTile / 16; ++k)
-                        umma_f16(d, desc_mn<ZW>(lo, z, k), desc_mn<AW>(lo, a, k, ones - a - (uint32_t)k * 16u * (uint32_t)layout::row_bytes(AW)),
-                                 umma_idesc(F, 1, 1, 64, AW + 8), k > 0 ? 1u : begun);
-                };
-                using WideT = std::integral_constant<int, H>;
-                if (elect_one()) {
-                    if (l == 0 && IW != H) gradient(WideT{}, std::integral_constant<int, IW>{}, M::kOnesIn);
-                    else if (l == NL - 1 && M::kDzW != H) gradient(std::integral_constant<int, M::kDzW>{}, WideT{}, M::kOnes);
-                    else gradient(WideT{}, WideT{}, M::kOnes);
-                    umma_commit(&dw_done[G * c + g]);
+                            for (int k = 0; k < kTile / 16; ++k)
+                                umma_f16(tmem_base + M::dw_col(NL - 1), desc_mn<H>(lo, a, k, M::kPanel), desc_mn<M::kDzW>(lo, z, k), umma_idesc(F, 1, 1, 128, OW), k > 0 ? 1u : begun);
+#pragma unroll
+                            for (int k = 0; k < kTile / 16; ++k)
+                                umma_f16(db, desc_mn<M::kDzW>(lo, z, k), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 64, 8), k > 0 ? 1u : begun);
+                        } else {
+                            const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * 128u);
+                            if (l == 0) {
+#pragma unroll
+                                for (int k = 0; k < kTile / 16; ++k)
+                                    umma_f16(d, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<IW>(lo, a, k), umma_idesc(F, 1, 1, 128, IW), k > 0 ? 1u : begun);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < kTile / 16; ++k)
+                                    umma_f16(d, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<H>(lo, a, k, M::kPanel), umma_idesc(F, 1, 1, 128, 128), k > 0 ? 1u : begun);
+                            }
+#pragma unroll
+                            for (int k = 0; k < kTile / 16; ++k)
+                                umma_f16(db, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 128, 16), k > 0 ? 1u : begun);
+                        }
+                        umma_commit(&dw_done[G * c + g]);
+                    }
+                } else {
+                    const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16));
+                    auto gradient = [&](auto z_width, auto a_width, uint32_t ones) {
+                        constexpr int ZW = decltype(z_width)::value, AW = decltype(a_width)::value;
+#pragma unroll
+                        for (int k = 0; k < kTile / 16; ++k)
+                            umma_f16(d, desc_mn<ZW>(lo, z, k), desc_mn<AW>(lo, a, k, ones - a - (uint32_t)k * 16u * (uint32_t)layout::row_bytes(AW)),
+                                     umma_idesc(F, 1, 1, 64, AW + 8), k > 0 ? 1u : begun);
+                    };
+                    using WideT = std::integral_constant<int, H>;
+                    if (elect_one()) {
+                        if (l == 0 && IW != H) gradient(WideT{}, std::integral_constant<int, IW>{}, M::kOnesIn);
+                        else if (l == NL - 1 && M::kDzW != H) gradient(std::integral_constant<int, M::kDzW>{}, WideT{}, M::kOnes);
+                        else gradient(WideT{}, WideT{}, M::kOnes);
+                        umma_commit(&dw_done[G * c + g]);
+                    }
                 }
                 __syncwarp();
                 started |= 1u << l;
@@ -448,39 +489,53 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     tc_fence_after();
     const bool good = !*abort_flag;
     float* sums = (float*)smem;
-    if (good && warp < NW) {
-        // Row r of a 64-row accumulator sits on lane 32 (r / 16) + r % 16: the first 16 lanes of this warp's quarter hold rows
-        // 16 quarter + lane.  The warps of a quarter take the 16-column pieces in turn.
-        const int quarter = warp & 3, row = quarter * 16 + lane;
 #pragma unroll 1
-        for (int l = 0; l < NL; ++l) {
-            const int w = l == 0 ? IW : H;
+    for (int l0 = 0; l0 < NL; l0 += M::kSumLayers) {
+        if (l0 > 0) __syncthreads();
+        if (good && warp < NW) {
+            // Row r of a 64-row accumulator sits on lane 32 (r / 16) + r % 16, of one of 128 rows on lane r.  The warps of a lane
+            // quarter take the 16-column pieces in turn.
+            const int quarter = warp & 3;
+            const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int piece = warp >> 2; piece <= w / 16; piece += NCH) {
-                uint32_t v[16];
-                tmem_ld_32x16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (uint32_t)(l - 1) * (H + 16)) + (uint32_t)piece * 16u, v);
-                wait_ld(v);
-                if (lane < 16 && row < H) {
-                    float* at = sums + (l * H + row) * (int)M::kSumRow;
-                    if (piece == w / 16) at[H] = __uint_as_float(v[0]);
-                    else
+            for (int l = l0; l < l0 + M::kSumLayers; ++l) {
+                const int w = M::kWide && l == NL - 1 ? OW : l == 0 ? IW : H;
+                float* layer = sums + (l - l0) * H * (int)M::kSumRow;
+#pragma unroll 1
+                for (int piece = warp >> 2; piece <= w / 16; piece += NCH) {
+                    const bool bias = piece == w / 16;
+                    uint32_t col;
+                    if constexpr (M::kWide) col = bias ? M::db_col(0) + 16u * l : (l == 0 ? M::dw_col(0) : l < NL - 1 ? M::dw_col(1) + (l - 1) * 128u : M::dw_col(NL - 1)) + piece * 16u;
+                    else col = (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16)) + piece * 16u;
+                    uint32_t v[16];
+                    tmem_ld_32x16(lanes + col, v);
+                    wait_ld(v);
+                    const bool half = !M::kWide || (bias && l == NL - 1);   // 64 rows
+                    const int row = half ? quarter * 16 + lane : quarter * 32 + lane;
+                    if ((!half || lane < 16) && row < H) {
+                        // the last layer of width 128 lies in features by outputs
+                        const bool across = M::kWide && l == NL - 1;
+                        float* at = bias ? layer + row * (int)M::kSumRow + H : across ? layer + piece * 16 * (int)M::kSumRow + row : layer + row * (int)M::kSumRow + piece * 16;
+                        const int step = across ? (int)M::kSumRow : 1;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) at[piece * 16 + i] = __uint_as_float(v[i]);
+                        for (int i = 0; i < 16; ++i)
+                            if (i == 0 || !bias) at[i * step] = __uint_as_float(v[i]);
+                    }
+                    __syncwarp();
                 }
             }
+            tc_fence_before();
         }
-        tc_fence_before();
-    }
-    __syncthreads();
-    if (good) {
+        __syncthreads();
+        if (!good) continue;
         // real parameters in the order they are stored, four to a reduction where rows are whole 16-byte pieces
         int i = threadIdx.x;
 #pragma unroll 1
-        for (int l = 0; l < NL; ++l) {
+        for (int l = l0; l < l0 + M::kSumLayers; ++l) {
             const int in = cfg.dims[l], out = cfg.dims[l + 1];
             float* dW = (float*)s_net[l].weightsGrad;
             float* dB = (float*)s_net[l].biasesGrad;
-            const float* s = sums + l * H * (int)M::kSumRow;
+            const float* s = sums + (l - l0) * H * (int)M::kSumRow;
             const bool fours = (in & 3) == 0 && cfg.param_layout == MLP_PARAMS_ROW_MAJOR && ((uint64_t)dW & 15u) == 0;
             const int per_row = fours ? in >> 2 : in;
             for (; i < out * per_row; i += kThreads) {
@@ -493,6 +548,8 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             for (; i < out; i += kThreads) atomicAdd(dB + i, s[i * (int)M::kSumRow + H]);
             i -= out;
         }
+    }
+    if (good) {
         if (threadIdx.x == 0) {
             const float* part = (const float*)(smem + M::kLoss);
             float mx = part[0], sm = part[1];
@@ -572,6 +629,7 @@ __global__ void __launch_bounds__(32 * 5 * NCH, 1) forward_chain_kernel(const __
     });
     for (int i = threadIdx.x; i < OW; i += kThreads)
         ((float*)(smem + M::kBias))[i] = i < od ? load_as_f32(cfg.dtype, (const void*)s_net[nl - 1].biases, i) : 0.0f;
+    cp_async_wait_all();
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -709,16 +767,18 @@ __global__ void __launch_bounds__(32 * 5 * NCH, 1) forward_chain_kernel(const __
 
 // ------------------------------------------------------------------------------------------------
 // Host side.  Compiled once per MLPB200_CHAIN_PART: 0 the entry points, 1 .. 4 the training builds of 2 .. 5 layers, 5 the
-// forward builds.
+// forward builds, 6 the training builds of widths up to 128.
 // ------------------------------------------------------------------------------------------------
 #ifndef MLPB200_CHAIN_PART
-#error "compile with -DMLPB200_CHAIN_PART=0..5 (slang_b200/build.py does)"
+#error "compile with -DMLPB200_CHAIN_PART=0..6 (slang_b200/build.py does)"
 #endif
 
 template <int NL> cudaError_t launch_chain_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p);
 cudaError_t launch_chain_forward(cudaStream_t st, TcWorkspace* ws, narrow::Params& p);
 
-#if MLPB200_CHAIN_PART >= 1 && MLPB200_CHAIN_PART <= 4
+cudaError_t launch_chain_train_wide(cudaStream_t st, TcWorkspace* ws, narrow::Params& p);
+
+#if (MLPB200_CHAIN_PART >= 1 && MLPB200_CHAIN_PART <= 4) || MLPB200_CHAIN_PART == 6
 template <int H, int NL, int IW, int OW, int NCH, int FMT, int HACT>
 static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
 {
@@ -727,7 +787,11 @@ static cudaError_t launch_train(cudaStream_t st, TcWorkspace* ws, narrow::Params
     static SmemLimit limit;
     const cudaError_t e = limit.raise((const void*)kern, ws->ordinal, M::kSmemBytes);
     if (e != cudaSuccess) return e;
-    const uint32_t grid = p.n_tiles < (uint32_t)ws->sm_count ? p.n_tiles : (uint32_t)ws->sm_count;
+    // A CTA per tile as far as the SMs go; beyond, as few CTAs as finish in the same number of tiles a chain: each brings a set of
+    // gradients to add (20011 samples, 157 tiles, one CTA per SM against 79: 32-128-128-3 26.1 / 23.2 us a step, texture network 21.4 /
+    // 20.6; 16384 samples, 128 tiles, packed 23.4 against 22.3 and 20.5 against 17.9).
+    const uint32_t sms = (uint32_t)ws->sm_count, rounds = (p.n_tiles + sms * NCH - 1) / (sms * NCH);
+    const uint32_t grid = p.n_tiles <= sms ? p.n_tiles : (p.n_tiles + rounds * NCH - 1) / (rounds * NCH);
     return launch_after(st, kern, grid, M::kThreads, M::kSmemBytes, p);
 }
 
@@ -739,6 +803,7 @@ static cudaError_t launch_shape(cudaStream_t st, TcWorkspace* ws, narrow::Params
     return relu ? launch_train<H, NL, IW, OW, NCH, MLP_F16, MLP_ACT_RELU>(st, ws, p) : launch_train<H, NL, IW, OW, NCH, MLP_F16, MLP_ACT_LEAKY_RELU>(st, ws, p);
 }
 
+#if MLPB200_CHAIN_PART <= 4
 template <int NL>
 cudaError_t launch_chain_train(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
 {
@@ -751,6 +816,25 @@ cudaError_t launch_chain_train(cudaStream_t st, TcWorkspace* ws, narrow::Params&
     return cudaErrorInvalidValue;
 }
 template cudaError_t launch_chain_train<1 + MLPB200_CHAIN_PART>(cudaStream_t, TcWorkspace*, narrow::Params&);
+#else
+// Two chains where shared memory (the tiles and all weights) and tensor memory hold them.
+cudaError_t launch_chain_train_wide(cudaStream_t st, TcWorkspace* ws, narrow::Params& p)
+{
+    const bool few_in = p.cfg.dims[0] <= 32, few_out = p.cfg.dims[p.cfg.n_layers] <= 16;
+    switch (p.cfg.n_layers) {
+    case 2:
+        if (few_in && few_out) return launch_shape<128, 2, 32, 16, 2>(st, ws, p);
+        return launch_shape<128, 2, 64, 64, 2>(st, ws, p);
+    case 3:
+        if (few_in && few_out) return launch_shape<128, 3, 32, 16, 2>(st, ws, p);
+        return launch_shape<128, 3, 64, 64, 1>(st, ws, p);
+    case 4:
+        if (few_in && few_out) return launch_shape<128, 4, 32, 16, 1>(st, ws, p);
+        break;
+    }
+    return cudaErrorInvalidValue;
+}
+#endif
 #endif
 
 #if MLPB200_CHAIN_PART == 5
@@ -830,13 +914,35 @@ static bool chain_train_network(const MlpConfig& c)
     return c.dims[0] <= 32 && c.dims[c.n_layers] <= 16;
 }
 
+// Networks of widths up to 128 (those that launch_learn_gradient_tc takes).
+static bool chain_wide_network(const MlpConfig& c)
+{
+    if (c.n_layers < 2 || c.n_layers > 4 || (c.dtype != MLP_BF16 && c.dtype != MLP_F16) || (c.operand_dtype && c.operand_dtype != c.dtype)) return false;
+    const int act = narrow::built_activation(c);
+    if ((act != MLP_ACT_RELU && act != MLP_ACT_LEAKY_RELU) || c.encoding != MLP_ENC_NONE) return false;
+    if (c.dims[0] > 64 || c.dims[c.n_layers] > 64) return false;
+    for (int l = 1; l < c.n_layers; ++l)
+        if (c.dims[l] > 128) return false;
+    return c.n_layers < 4 || (c.dims[0] <= 32 && c.dims[c.n_layers] <= 16);
+}
+// Against the kernels of tc_kernels.cu, us a step: 32-128-128-3, 1024 samples 20.5 / 19.3, 2^20: 581 / 235; 16-128-3 14.3 / 12.6, 379 / 124;
+// 64-96-96-40 33 / 25, 1433 / 578; 64-128-64 16.4 / 19.9, 65536 samples 36.9 / 36.9, 2^20: 369 / 321; 32-128-128-128-3 25.1 / 27.0,
+// 16384 samples 34.8 / 31.5, 2^20: 772 / 457.
+bool chain_train_wide_suits(const MlpConfig& c, uint32_t count)
+{
+    const bool few = c.dims[0] <= 32 && c.dims[c.n_layers] <= 16;
+    const uint32_t from = c.n_layers == 4 ? 16384u : c.n_layers == 2 && !few ? 131072u : kTrainFrom;
+    return count >= from && chain_wide_network(c);
+}
+
 bool chain_train_suits(const MlpConfig& c, uint32_t count) { return count >= kTrainFrom && chain_train_network(c); }
 bool chain_forward_suits(const MlpConfig& c, uint32_t count) { return count >= kForwardFrom && chain_network(c); }
 
 cudaError_t launch_learn_gradient_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpLearnGradParamsEx& a,
                                         int* launches, std::string* err, float* input_grads)
 {
-    if (!chain_train_network(c)) { if (err) *err = "shape not built for tiles of samples"; return cudaErrorInvalidValue; }
+    const bool wide = !chain_train_network(c);
+    if (wide && !chain_wide_network(c)) { if (err) *err = "shape not built for tiles of samples"; return cudaErrorInvalidValue; }
     narrow::Params p = chain_params(ws, c, a.networkBuffer, a.inputs, a.count);
     p.loss_words = (uint32_t*)a.lossBuffer;
     p.targets = (const void*)a.targets;
@@ -845,6 +951,7 @@ cudaError_t launch_learn_gradient_chain(cudaStream_t st, TcWorkspace* ws, const 
     p.vec_tgt = pieces(a.targets, c.dims[c.n_layers], tgt, 4 * tgt);
     p.vec_dx = pieces((uint64_t)input_grads, c.dims[0], 4, 32);
     *launches += 1;
+    if (wide) return launch_chain_train_wide(st, ws, p);
     switch (c.n_layers) {
     case 2: return launch_chain_train<2>(st, ws, p);
     case 3: return launch_chain_train<3>(st, ws, p);

@@ -49,8 +49,8 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
-// Byte offset of the first 16-byte chunk of row r of a [rows][W] operand tile (W 16, 32 or 64); chunk j is there ^ (16 j), as
-// tiles start on 1024-byte boundaries.
+// Byte offset of the first 16-byte chunk of row r of a [rows][W] operand tile (W 16, 32, 64 or 128); chunk j is there ^ (16 j), as
+// tiles start on 1024-byte boundaries.  128 features are two panels of 64, one after the other: chunk 8 + j is a panel further.
 template <int W>
 __device__ __forceinline__ uint32_t row_at(int r)
 {
@@ -58,19 +58,25 @@ __device__ __forceinline__ uint32_t row_at(int r)
 }
 
 // Operand descriptors of a [rows][W] tile at byte offset `at` (lo: the base's address field).  K-major: step k is 16
-// features, 32 bytes inside the row.  MN-major: step k is 16 rows; `lbo` bytes lead from one row-wide block of the other
-// dimension to the next.
+// features, 32 bytes inside the row (of panel k / 4; `panel`: bytes of one).  MN-major: step k is 16 rows; `lbo` bytes lead
+// from one row-wide block of the other dimension to the next.
 template <int W>
-__device__ __forceinline__ uint64_t desc_k(uint32_t lo, uint32_t at, int k)
+__device__ __forceinline__ uint64_t desc_k(uint32_t lo, uint32_t at, int k, uint32_t panel = 0u)
 {
     constexpr uint32_t hi = ((8u * (uint32_t)layout::row_bytes(W)) >> 4) | (1u << 14) | (layout::layout_type(W) << 29);
-    return ((uint64_t)hi << 32) | (lo + ((at + (uint32_t)k * 32u) >> 4) + (1u << 16));
+    return ((uint64_t)hi << 32) | (lo + ((at + (uint32_t)(k >> 2) * panel + (uint32_t)(W > 64 ? k & 3 : k) * 32u) >> 4) + (1u << 16));
 }
 template <int W>
 __device__ __forceinline__ uint64_t desc_mn(uint32_t lo, uint32_t at, int k, uint32_t lbo = 16u)
 {
     constexpr uint32_t hi = ((8u * (uint32_t)layout::row_bytes(W)) >> 4) | (1u << 14) | (layout::layout_type(W) << 29);
     return ((uint64_t)hi << 32) | (lo + ((at + (uint32_t)k * 16u * (uint32_t)layout::row_bytes(W)) >> 4) + ((lbo >> 4) << 16));
+}
+// Where the block of 32 features b of a row lies (row: row_at() of it).
+template <int W>
+__device__ __forceinline__ uint32_t block_at(uint32_t row, int b)
+{
+    return W == 128 ? (row ^ (uint32_t)(64 * (b & 1))) + (uint32_t)(b >> 1) * (kTile * 128u) : row ^ (uint32_t)(64 * b);
 }
 
 // The biases of hidden layers enter as one more K step of the layer product, the first: a tile of rows (1, 0, .. 0) times rows
@@ -86,13 +92,14 @@ __device__ __forceinline__ uint64_t desc_unit(uint32_t lo, uint32_t at)
 template <class F>
 __device__ __forceinline__ void first_column(uint8_t* dst, int rows, int tid, int nthreads, F value)
 {
-    for (int i = tid; i < rows * 2; i += nthreads) {
-        const int row = i >> 1, chunk = i & 1;
-        *(uint4*)(dst + (row_at<16>(row) ^ (uint32_t)(16 * chunk))) = make_uint4(chunk == 0 ? value(row) & 0xffffu : 0u, 0u, 0u, 0u);
+    for (int row = tid; row < rows; row += nthreads) {
+        uint8_t* at = dst + row_at<16>(row);
+        *(uint4*)at = make_uint4(value(row) & 0xffffu, 0u, 0u, 0u);
+        *(uint4*)(dst + (row_at<16>(row) ^ 16u)) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
-// A layer's weights as a zero-padded [rows][W] tile (rows: outputs), 16-bit storage.
+// A layer's weights as a zero-padded [rows][W] tile (rows: outputs), 16-bit storage.  cp_async_wait_all() is still to come.
 template <int W>
 __device__ __forceinline__ void stage_weights(uint8_t* dst, const MlpConfig& c, const void* weights, int rows, int in, int out, int tid, int nthreads)
 {
@@ -101,18 +108,15 @@ __device__ __forceinline__ void stage_weights(uint8_t* dst, const MlpConfig& c, 
 #pragma unroll 1
     for (int i = tid; i < rows * (W / 8); i += nthreads) {
         const int o = i / (W / 8), j = i % (W / 8);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (o < out && 8 * j < in) {
-            if (whole) {
-                v = *(const uint4*)(w + o * in + 8 * j);
-            } else {
-                uint16_t h[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) h[e] = 8 * j + e < in ? w[weight_index(c.param_layout, in, out, o, 8 * j + e)] : (uint16_t)0;
-                v = make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
-            }
+        uint8_t* at = dst + (row_at<W>(o) ^ (uint32_t)(16 * (j & 7))) + (uint32_t)(j >> 3) * (uint32_t)rows * 128u;
+        if (whole && o < out && 8 * j < in) {   // all copies of all layers in flight together
+            cp_async_16(smem_u32(at), w + o * in + 8 * j);
+            continue;
         }
-        *(uint4*)(dst + (row_at<W>(o) ^ (uint32_t)(16 * j))) = v;
+        uint16_t h[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) h[e] = o < out && 8 * j + e < in ? w[weight_index(c.param_layout, in, out, o, 8 * j + e)] : (uint16_t)0;
+        *(uint4*)at = make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
     }
 }
 
@@ -344,7 +348,7 @@ __device__ __forceinline__ void marked_columns(uint32_t t_acc, uint32_t row)
             const float z0 = __uint_as_float(v[2 * i]), z1 = __uint_as_float(v[2 * i + 1]);
             a[i] = C::relu2(C::pack2(z0, z1)) | (fabsf(z0) <= kTiny ? 0x8000u : 0u) | (fabsf(z1) <= kTiny ? 0x80000000u : 0u);
         }
-        sts128(row ^ (uint32_t)(16 * j), a[0], a[1], a[2], a[3]);
+        sts128(block_at<H>(row, j >> 2) ^ (uint32_t)(16 * (j & 3)), a[0], a[1], a[2], a[3]);
     }
 }
 
@@ -380,7 +384,8 @@ __device__ __forceinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t 
     for (int j = 0; j < H / 8; ++j) {
         uint32_t v[8], z[4];
         tmem_ld_32x8(t_acc + (uint32_t)(8 * j), v);
-        const uint4 act = narrow::lds128(row ^ (uint32_t)(16 * j));
+        const uint32_t at = block_at<H>(row, j >> 2) ^ (uint32_t)(16 * (j & 3));
+        const uint4 act = narrow::lds128(at);
         const uint32_t a[4] = {act.x, act.y, act.z, act.w};
         tmem_ld_wait();
 #pragma unroll
@@ -388,7 +393,7 @@ __device__ __forceinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t 
             const float g0 = __uint_as_float(v[2 * i]), g1 = __uint_as_float(v[2 * i + 1]);
             z[i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | (C::pack2(0.5f * g0, 0.5f * g1) & narrow::sign_mask(a[i]));
         }
-        sts128(row ^ (uint32_t)(16 * j), z[0], z[1], z[2], z[3]);
+        sts128(at, z[0], z[1], z[2], z[3]);
     }
 }
 

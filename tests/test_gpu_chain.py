@@ -52,7 +52,7 @@ def _check(cfg, result, bar):
 
 
 @pytest.mark.parametrize("count", [1023, 1024, 1025, 1151, 4095, 4096, 4097, 148 * 128 * 3 + 1])
-@pytest.mark.parametrize("dims", [[4, 32, 32, 32, 32, 4], [32, 64, 64, 64, 3], [64, 64, 64, 64, 64], [9, 17, 1]], ids=lambda d: "-".join(map(str, d)))
+@pytest.mark.parametrize("dims", [[4, 32, 32, 32, 32, 4], [32, 64, 64, 64, 3], [64, 64, 64, 64, 64], [9, 17, 1], [32, 128, 128, 3]], ids=lambda d: "-".join(map(str, d)))
 def test_counts_around_a_tile(device, dims, count):
     cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
     _check(cfg, _run(device, cfg, count), 1e-2)
@@ -62,7 +62,9 @@ def test_counts_around_a_tile(device, dims, count):
                          ids=["f16-relu", "bf16-relu", "f16-leaky", "bf16-leaky"])
 @pytest.mark.parametrize("dims,input_dtype", [([1, 2, 1], C.F32), ([16, 32, 16], C.F32), ([31, 33, 33, 17], C.F32), ([12, 20, 20, 20, 20, 5], C.F32),
                                               ([24, 64, 64, 64, 16], None), ([40, 48, 48, 48, 64], None), ([33, 64, 64, 9], None),
-                                              ([20, 50, 50, 50, 50, 8], C.F32), ([8, 32, 32, 32, 32], None), ([7, 40, 4], None)],
+                                              ([20, 50, 50, 50, 50, 8], C.F32), ([8, 32, 32, 32, 32], None), ([7, 40, 4], None), ([32, 128, 128, 3], None),
+                                              ([64, 128, 64], None), ([24, 100, 66, 20], None), ([16, 65, 1], C.F32), ([40, 128, 128, 16], C.F32),
+                                              ([8, 90, 128, 100, 16], None)],
                          ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else "f32" if v == C.F32 else "own")
 def test_shapes_and_formats(device, dims, input_dtype, dtype, act):
     """Every build; rows that are read as values, as whole pieces and converted one by one.  In bf16 a sum that rounds the other
@@ -78,7 +80,7 @@ def test_frequency_encoding(device, out):
     _check(cfg, _run(device, cfg, 6001), 1e-2)
 
 
-@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [32, 64, 64, 3], [36, 64, 64, 20]], ids=lambda d: "-".join(map(str, d)))
+@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [32, 64, 64, 3], [36, 64, 64, 20], [32, 128, 128, 3]], ids=lambda d: "-".join(map(str, d)))
 def test_zero_preactivations_pass_half_of_the_gradient(device, dims):
     """Samples whose inputs are all zero meet zero biases: their pre-activations are zero in every layer."""
     cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
@@ -91,7 +93,7 @@ def test_zero_preactivations_pass_half_of_the_gradient(device, dims):
     _check(cfg, _run(device, cfg, 3000, C.to_storage(p0, C.F16), x), 1e-2)
 
 
-@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [32, 64, 64, 3], [40, 64, 64, 20], [7, 24, 3]], ids=lambda d: "-".join(map(str, d)))
+@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [32, 64, 64, 3], [40, 64, 64, 20], [7, 24, 3], [32, 128, 128, 3]], ids=lambda d: "-".join(map(str, d)))
 def test_input_gradients(device, dims):
     """Against the chain rule in fp64 over the stored weights.  Roundings to half (2^-11) leave a row within a few 1e-3, except
     where a pre-activation lies so close to zero that they carry it over the kink: 2^-11 of a unit's range, some 192 units
