@@ -44,6 +44,7 @@ UNITS = [
     ("tc_kernels_2", "tc_kernels.cu", ["-DMLPB200_WIDE_PART=2"]),
     ("tc_forward", "tc_forward.cu", []),
     ("comm", "comm.cu", []),
+    ("clear", "clear.cu", []),
     ("matrix_convert", "matrix_convert.cu", []),
     ("permuto", "permuto.cu", ["-fmad=false"]),
     ("selftest", "selftest.cu", []),

@@ -656,19 +656,6 @@ learn_gradient_small_kernel(const __grid_constant__ SmallNet net, const MlpLayer
     }
 }
 
-// Clears a few words (a loss buffer, an example's gradients).  A kernel, because a kernel overlaps its neighbours on the stream and
-// a memset does not: example step 8.2 -> 7.7 us, 4096 samples of 2-16-16-16-1 14.3 -> 13.0.
-__global__ void __launch_bounds__(256) clear_bytes_kernel(uint8_t* p, uint32_t size)
-{
-    grid_release();
-    grid_wait();
-    if ((((uint64_t)p | size) & 3u) == 0) {
-        for (uint32_t i = threadIdx.x; i < size / 4; i += 256) ((uint32_t*)p)[i] = 0u;
-    } else {
-        for (uint32_t i = threadIdx.x; i < size; i += 256) p[i] = 0;
-    }
-}
-
 // Second pass of the sequential mode: one thread per parameter walks the samples in ascending order,
 // exactly the adds a sequential machine performs (load, fused multiply-add, store).
 __global__ void __launch_bounds__(256)
@@ -792,8 +779,6 @@ cudaError_t launch_example_adjust_parameters(cudaStream_t st, const MlpAdjustPar
 {
     return launch_after(st, adjustParameters, grid, 256, 0, (MlpExampleAdamState*)a.adamStates, (__half*)a.params, (__half*)a.gradients, a.count);
 }
-
-cudaError_t launch_clear_bytes(cudaStream_t st, void* p, uint32_t size) { return launch_after(st, clear_bytes_kernel, 1, 256, 0, (uint8_t*)p, size); }
 
 cudaError_t launch_forward_simt(cudaStream_t st, const MlpConfig& c, const MlpForwardParams& a, int* launches,
                                 std::string* err)

@@ -42,7 +42,7 @@ def test_small_fp32_networks(device, dims, count, order):
     assert abs(largest - ref[0]) <= 1e-6 * ref[0] and abs(total - ref[1]) <= 1e-5 * ref[1]
 
 
-@pytest.mark.parametrize("offset,size", [(0, 8), (4, 4), (1, 3), (3, 1024), (8, 4096), (16, 4097), (5, 0)])
+@pytest.mark.parametrize("offset,size", [(0, 8), (4, 4), (1, 3), (8, 64), (3, 61), (16, 65), (5, 1024), (5, 0)])
 def test_clears_touch_their_range_only(device, offset, size):
     b = device.create_buffer(8192, np.full(8192, 0xa5, dtype=np.uint8))
     b.clear(offset, size)
