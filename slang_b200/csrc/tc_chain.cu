@@ -8,8 +8,8 @@
 //
 // Bound by instruction issue and by the hand-offs between a chain's four warps and the tensor pipe; the chains' tiles fill
 // shared memory, so there are no more of them.  Against the register-chained kernels of tc_narrow.cu, us: texture network
-// (32-64-64-64-3) 2^24 samples a step 3830 -> 2400, width 32 (4-32-32-32-32-4, leaky ReLU) 2^20 samples 160 -> 132, 1920 x 1080 view of the
-// texture network 142 -> 96.  Counters of 2^20 samples of the texture network: issue slots 41 %, tensor pipe 31 %, LSU wavefronts 43 %.
+// (32-64-64-64-3) 2^24 samples a step 3830 -> 2160, width 32 (4-32-32-32-32-4, leaky ReLU) 2^20 samples 160 -> 124, 1920 x 1080 view of the
+// texture network 142 -> 94.  Counters of 2^20 samples of the texture network: issue slots 43 %, tensor pipe 36 %, LSU wavefronts 39 %.
 //
 // What the reference does instead: one thread per sample with per-element global atomics
 // (examples/mlp-training/mlp_sw.slang:28-58) or CoopVec calls whose CPU/CUDA fallback is scalar loops
@@ -48,7 +48,9 @@ struct TrainMap {
     __host__ __device__ static constexpr int in_w(int l) { return l == 0 ? IW : H; }
     __host__ __device__ static constexpr int out_w(int l) { return l == NL - 1 ? OW : H; }
     static constexpr uint32_t kRowsIn = kTile * IW * 2, kRows = kTile * H * 2, kPanel = kTile * 128;   // (of 64 features)
-    // a chain's tiles: A_0, A_1 .. A_{NL-1} (dZ_{l-1} replaces A_l), dZ_{NL-1}
+    // A chain's tiles: A_0, A_1 .. A_{NL-1} (dZ_{l-1} replaces A_l), dZ_{NL-1}.  The first and the last change places with every
+    // tile, so that a tile's inputs need not wait for the gradient product that still reads the last one's.
+    static_assert(IW == kDzW, "inputs and the last layer's dZ share their layout");
     __host__ __device__ static constexpr uint32_t a_off(int l) { return l == 0 ? 0u : kRowsIn + (uint32_t)(l - 1) * kRows; }
     static constexpr uint32_t kDz = a_off(NL);
     static constexpr uint32_t kChainBytes = kDz + kTile * kDzW * 2;
@@ -163,7 +165,8 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         const int ch = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
         const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ch * H);
         const uint32_t cb = sbase + M::kChains + (uint32_t)ch * M::kChainBytes;
-        const uint32_t in_row = cb + row_at<IW>(r), own_row = cb + M::kRowsIn + row_at<H>(r), dz_row = cb + M::kDz + row_at<M::kDzW>(r);
+        uint32_t in_row = cb + row_at<IW>(r), dz_row = cb + M::kDz + row_at<M::kDzW>(r);   // change places with every tile
+        const uint32_t own_row = cb + M::kRowsIn + row_at<H>(r);
         const uint32_t s_bias = sbase + M::kBias;
         const float scale = cfg.loss == MLP_LOSS_MSE_MEAN ? 1.0f / (float)od : 1.0f;
         const float alpha = cfg.act_alpha, alpha_op = C::round(alpha);
@@ -171,12 +174,12 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         float run_max = 0.0f, run_sum = 0.0f;
         uint32_t full = 0, done = 0;                   // phases seen of acc_full; bit g: parity of dw_done's g
         auto wait_full = [&]() {
-            ok = ok && mbar_wait(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
+            ok = ok && wait_for(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
             ++full;
             tc_fence_after();
         };
         auto wait_done = [&](int l) {
-            ok = ok && mbar_wait(&dw_done[G * ch + l % G], (done >> (l % G)) & 1u, abort_flag, p.status, kStatusRow);
+            ok = ok && wait_for(&dw_done[G * ch + l % G], (done >> (l % G)) & 1u, abort_flag, p.status, kStatusRow);
             done ^= 1u << (l % G);
         };
         // hands A_l over (gradient < 0), or dZ of layer `gradient`
@@ -199,10 +202,8 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         for (; tile < p.n_tiles && ok; tile += stride) {
             const bool valid = sample < p.count;
             bool zero_seen = false;
-            // ---- input row; stored when the gradient product of the chain's last tile has read A_0 ----
-            write_row<FMT, IW>(in_row, p, raw, in.at, valid, [&]() { if (!first) wait_done(0); });
-            first = false;
-            if (!ok) break;
+            // ---- input row ----
+            write_row<FMT, IW>(in_row, p, raw, in.at, valid);
             release(true, -1);
             // few targets are fetched a forward pass ahead of their use; the next tile's rows are started on their way
             uint32_t t4[4];
@@ -224,6 +225,10 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
 #pragma unroll 1
             for (int l = 0; l < NL - 1; ++l) {
                 wait_full();
+                if (l == 0) {   // the last tile's dZ_0 lies where A_1 goes, its A_0 where dZ_{NL-1} will
+                    if (!first) wait_done(0);
+                    first = false;
+                }
                 if (!ok) break;
                 const uint32_t dst = own_row + (uint32_t)l * M::kRows;   // A_{l + 1}
                 float least = 1.0f;
@@ -246,30 +251,28 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             if (!ok) break;
             float loss = 0.0f;
 #pragma unroll 1
-            for (int f = 0; f < ((od + 15) & ~15); f += 4) {
-                uint32_t z0 = 0u, z1 = 0u;
-                if (f < od) {
-                    float o[4], d[4], t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, g[4];
-                    output_columns<FMT>(o, t_acc, s_bias, f);
-                    if (od <= 4) {
+            for (int f = 0; f < od; f += 4) {
+                float o[4], d[4], t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, g[4];
+                output_columns<FMT>(o, t_acc, s_bias, f);
+                if (od <= 4) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) t[i] = bits_value(cfg.target_dtype, t4[i]);
-                    } else if (valid) {
-                        load_targets(t, p, targets, od, f);
-                    }
-                    activate_outputs(cfg.output_act, alpha, o, d);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const bool real = valid && f + i < od;
-                        const float diff = real ? o[i] - t[i] : 0.0f;
-                        loss = fmaf(diff * scale, diff, loss);
-                        g[i] = real ? ((2.0f * scale) * diff) * d[i] : 0.0f;
-                    }
-                    z0 = C::pack2(g[0], g[1]);
-                    z1 = C::pack2(g[2], g[3]);
+                    for (int i = 0; i < 4; ++i) t[i] = bits_value(cfg.target_dtype, t4[i]);
+                } else if (valid) {
+                    load_targets(t, p, targets, od, f);
                 }
-                sts64((dz_row ^ (uint32_t)(16 * (f >> 3))) + (uint32_t)(2 * (f & 4)), z0, z1);
+                activate_outputs(cfg.output_act, alpha, o, d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bool real = valid && f + i < od;
+                    const float diff = real ? o[i] - t[i] : 0.0f;
+                    loss = fmaf(diff * scale, diff, loss);
+                    g[i] = real ? ((2.0f * scale) * diff) * d[i] : 0.0f;
+                }
+                sts64((dz_row ^ (uint32_t)(16 * (f >> 3))) + (uint32_t)(2 * (f & 4)), C::pack2(g[0], g[1]), C::pack2(g[2], g[3]));
             }
+#pragma unroll 1
+            for (int f = (od + 3) & ~3; f < ((od + 15) & ~15); f += 4)   // the rest of the K step
+                sts64((dz_row ^ (uint32_t)(16 * (f >> 3))) + (uint32_t)(2 * (f & 4)), 0u, 0u);
             run_max = fmaxf(run_max, loss);
             run_sum += loss;
             release(true, NL - 1);
@@ -329,6 +332,9 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 }
                 tc_fence_before();
             }
+            const uint32_t swap = in_row;
+            in_row = dz_row;
+            dz_row = swap;
         }
         if (!first) wait_done(0);
 #pragma unroll
@@ -348,56 +354,107 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         const uint32_t acc = tmem_base + (uint32_t)(ch * H);
         const int in_steps = (cfg.dims[0] + 15) / 16, out_steps = (od + 15) / 16;
         constexpr uint32_t F = C::kUmmaFmt;
-        uint32_t seen = 0;
+        // A copy of the code per layer up to width 64 (width 32, 2^20 samples: 123.5 us, 128.5 with one for all layers), one at 128 (229
+        // us for 2^20 samples of 32-128-128-3, 237 with a copy each).
+        uint32_t seen = 0, x = cb, y = cb + M::kDz;   // A_0 and the last dZ
         auto wait_ready = [&]() {
-            ok = ok && mbar_wait(&ready[ch], seen & 1u, abort_flag, p.status, kStatusIssue);
+            ok = ok && wait_for(&ready[ch], seen & 1u, abort_flag, p.status, kStatusIssue);
             ok = __all_sync(0xffffffffu, ok);
             ++seen;
             tc_fence_after();
         };
         for (uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch; tile < p.n_tiles && ok; tile += stride) {
+            if constexpr (M::kWide) {
+#pragma unroll 1
+                for (int l = 0; l < NL; ++l) {
+                    wait_ready();
+                    if (ok && elect_one()) {
+                        if (l < NL - 1) umma_f16(acc, desc_unit(lo, M::kUnit), desc_k<16>(lo, M::kHiddenBias + (uint32_t)l * (H * 32), 0), umma_idesc(F, 0, 0, 128, H), 0u);
+                        if (l == 0) {
 #pragma unroll
-            for (int l = 0; l < NL; ++l) {
-                wait_ready();
-                if (ok && elect_one()) {
-                    if (l < NL - 1) umma_f16(acc, desc_unit(lo, M::kUnit), desc_k<16>(lo, M::kHiddenBias + (uint32_t)l * H * 32, 0), umma_idesc(F, 0, 0, 128, H), 0u);
-                    if (l == 0) {
+                            for (int k = 0; k < IW / 16; ++k)
+                                if (k < in_steps) umma_f16(acc, desc_k<IW>(lo, x, k), desc_k<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 0, 128, H), 1u);
+                        } else {
+                            const uint32_t a = cb + M::kRowsIn + (uint32_t)(l - 1) * M::kRows, w = M::kWeights + M::w_off(1) + (uint32_t)(l - 1) * (H * H * 2);
+                            const uint32_t id = l < NL - 1 ? umma_idesc(F, 0, 0, 128, H) : umma_idesc(F, 0, 0, 128, OW), panel = l < NL - 1 ? H * 128u : OW * 128u;
 #pragma unroll
-                        for (int k = 0; k < IW / 16; ++k)
-                            if (k < in_steps) umma_f16(acc, desc_k<IW>(lo, cb, k), desc_k<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 0, 128, H), 1u);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < H / 16; ++k)
-                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l), k, M::kPanel), desc_k<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)M::out_w(l) * 128u), umma_idesc(F, 0, 0, 128, M::out_w(l)),
-                                     l < NL - 1 || k > 0);
+                            for (int k = 0; k < H / 16; ++k)
+                                umma_f16(acc, desc_k<H>(lo, a, k, M::kPanel), desc_k<H>(lo, w, k, panel), id, l < NL - 1 || k > 0);
+                        }
+                        umma_commit(&acc_full[ch]);
                     }
-                    umma_commit(&acc_full[ch]);
+                    __syncwarp();
                 }
-                __syncwarp();
-            }
+#pragma unroll 1
+                for (int l = NL - 1; l >= (p.input_grads ? 0 : 1); --l) {
+                    wait_ready();
+                    if (ok && elect_one()) {
+                        const uint32_t w = M::kWeights + M::w_off(1) + (uint32_t)(l - 1) * (H * H * 2), z = cb + M::kRowsIn + (uint32_t)l * M::kRows;
+                        if (l == NL - 1) {
 #pragma unroll
-            for (int l = NL - 1; l >= 0; --l) {
-                if (l == 0 && !p.input_grads) break;
-                wait_ready();
-                if (ok && elect_one()) {
-                    if (l == NL - 1) {
+                            for (int k = 0; k < OW / 16; ++k)
+                                if (k < out_steps)
+                                    umma_f16(acc, desc_k<M::kDzW>(lo, y, k), desc_mn<H>(lo, w, k, (uint32_t)OW * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
+                        } else if (l > 0) {
 #pragma unroll
-                        for (int k = 0; k < OW / 16; ++k)
-                            if (k < out_steps)
-                                umma_f16(acc, desc_k<M::kDzW>(lo, cb + M::kDz, k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)OW * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
-                    } else if (l > 0) {
+                            for (int k = 0; k < H / 16; ++k)
+                                umma_f16(acc, desc_k<H>(lo, z, k, M::kPanel), desc_mn<H>(lo, w, k, (uint32_t)H * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
+                        } else {
 #pragma unroll
-                        for (int k = 0; k < H / 16; ++k)
-                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l + 1), k, M::kPanel), desc_mn<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)H * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < H / 16; ++k)
-                            umma_f16(acc, desc_k<H>(lo, cb + M::a_off(1), k, M::kPanel), desc_mn<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 1, 128, IW), k > 0);
+                            for (int k = 0; k < H / 16; ++k)
+                                umma_f16(acc, desc_k<H>(lo, z, k, M::kPanel), desc_mn<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 1, 128, IW), k > 0);
+                        }
+                        umma_commit(&acc_full[ch]);
                     }
-                    umma_commit(&acc_full[ch]);
+                    __syncwarp();
                 }
-                __syncwarp();
+            } else {
+#pragma unroll
+                for (int l = 0; l < NL; ++l) {
+                    wait_ready();
+                    if (ok && elect_one()) {
+                        if (l < NL - 1) umma_f16(acc, desc_unit(lo, M::kUnit), desc_k<16>(lo, M::kHiddenBias + (uint32_t)l * H * 32, 0), umma_idesc(F, 0, 0, 128, H), 0u);
+                        if (l == 0) {
+#pragma unroll
+                            for (int k = 0; k < IW / 16; ++k)
+                                if (k < in_steps) umma_f16(acc, desc_k<IW>(lo, x, k), desc_k<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 0, 128, H), 1u);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < H / 16; ++k)
+                                umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l), k, M::kPanel), desc_k<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)M::out_w(l) * 128u), umma_idesc(F, 0, 0, 128, M::out_w(l)),
+                                         l < NL - 1 || k > 0);
+                        }
+                        umma_commit(&acc_full[ch]);
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int l = NL - 1; l >= 0; --l) {
+                    if (l == 0 && !p.input_grads) break;
+                    wait_ready();
+                    if (ok && elect_one()) {
+                        if (l == NL - 1) {
+#pragma unroll
+                            for (int k = 0; k < OW / 16; ++k)
+                                if (k < out_steps)
+                                    umma_f16(acc, desc_k<M::kDzW>(lo, y, k), desc_mn<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)OW * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
+                        } else if (l > 0) {
+#pragma unroll
+                            for (int k = 0; k < H / 16; ++k)
+                                umma_f16(acc, desc_k<H>(lo, cb + M::a_off(l + 1), k, M::kPanel), desc_mn<H>(lo, M::kWeights + M::w_off(l), k, (uint32_t)H * 128u), umma_idesc(F, 0, 1, 128, H), k > 0);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < H / 16; ++k)
+                                umma_f16(acc, desc_k<H>(lo, cb + M::a_off(1), k, M::kPanel), desc_mn<IW>(lo, M::kWeights, k), umma_idesc(F, 0, 1, 128, IW), k > 0);
+                        }
+                        umma_commit(&acc_full[ch]);
+                    }
+                    __syncwarp();
+                }
             }
+            const uint32_t swap = x;
+            x = y;
+            y = swap;
         }
     } else {
         // =================================== gradient products of all chains =======================
@@ -408,7 +465,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         const uint32_t lo = (sbase & 0x3FFFFu) >> 4;
         constexpr uint32_t F = C::kUmmaFmt;
         const uint32_t top = (uint32_t)(NL - 1 - (NL - 1 - g) % G);        // this warp's last layer; its first is g
-        uint32_t total = 0, idle = 0, started = 0, phase = 0, layers = 0;   // hand-overs to come; layers begun; four bits a chain: its layer
+        uint32_t total = 0, idle = 0, started = 0, phase = 0, layers = 0, flip = 0;   // hand-overs to come; layers begun; four bits a chain: its layer; whether A_0 and the last dZ have changed places
         for (int c = 0; c < NCH; ++c) {
             const uint32_t first = blockIdx.x + gridDim.x * (uint32_t)c;
             layers |= top << (4 * c);
@@ -420,32 +477,33 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             if (__all_sync(0xffffffffu, mbar_test_wait(&dz_ready[G * c + g], (phase >> c) & 1u))) {
                 tc_fence_after();
                 const uint32_t l = (layers >> (4 * c)) & 15u, cb = M::kChains + c * M::kChainBytes;
-                const uint32_t a = l == 0 ? cb : cb + M::kRowsIn + (l - 1) * M::kRows;           // A_l
-                const uint32_t z = l == NL - 1 ? cb + M::kDz : cb + M::kRowsIn + l * M::kRows;   // dZ_l
+                const bool flipped = (flip >> c) & 1u;
+                const uint32_t a = l == 0 ? cb + (flipped ? M::kDz : 0u) : cb + M::kRowsIn + (l - 1) * M::kRows;           // A_l
+                const uint32_t z = l == NL - 1 ? cb + (flipped ? 0u : M::kDz) : cb + M::kRowsIn + l * M::kRows;   // dZ_l
                 const uint32_t begun = (started >> l) & 1u;
                 if constexpr (M::kWide) {
                     const uint32_t db = tmem_base + M::db_col(0) + 16u * l;
                     if (elect_one()) {
                         if (l == NL - 1) {
                             // A^T . dZ, and dZ^T . 1 of 64 rows (those past the outputs are never read)
-#pragma unroll
+#pragma unroll 2
                             for (int k = 0; k < kTile / 16; ++k)
                                 umma_f16(tmem_base + M::dw_col(NL - 1), desc_mn<H>(lo, a, k, M::kPanel), desc_mn<M::kDzW>(lo, z, k), umma_idesc(F, 1, 1, 128, OW), k > 0 ? 1u : begun);
-#pragma unroll
+#pragma unroll 2
                             for (int k = 0; k < kTile / 16; ++k)
                                 umma_f16(db, desc_mn<M::kDzW>(lo, z, k), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 64, 8), k > 0 ? 1u : begun);
                         } else {
                             const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * 128u);
                             if (l == 0) {
-#pragma unroll
+#pragma unroll 2
                                 for (int k = 0; k < kTile / 16; ++k)
                                     umma_f16(d, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<IW>(lo, a, k), umma_idesc(F, 1, 1, 128, IW), k > 0 ? 1u : begun);
                             } else {
-#pragma unroll
+#pragma unroll 2
                                 for (int k = 0; k < kTile / 16; ++k)
                                     umma_f16(d, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<H>(lo, a, k, M::kPanel), umma_idesc(F, 1, 1, 128, 128), k > 0 ? 1u : begun);
                             }
-#pragma unroll
+#pragma unroll 2
                             for (int k = 0; k < kTile / 16; ++k)
                                 umma_f16(db, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 128, 16), k > 0 ? 1u : begun);
                         }
@@ -455,7 +513,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16));
                     auto gradient = [&](auto z_width, auto a_width, uint32_t ones) {
                         constexpr int ZW = decltype(z_width)::value, AW = decltype(a_width)::value;
-#pragma unroll
+#pragma unroll 2
                         for (int k = 0; k < kTile / 16; ++k)
                             umma_f16(d, desc_mn<ZW>(lo, z, k), desc_mn<AW>(lo, a, k, ones - a - (uint32_t)k * 16u * (uint32_t)layout::row_bytes(AW)),
                                      umma_idesc(F, 1, 1, 64, AW + 8), k > 0 ? 1u : begun);
@@ -471,6 +529,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 __syncwarp();
                 started |= 1u << l;
                 layers += (l < G ? top - l : 0u - G) << (4 * c);
+                if (l < G) flip ^= 1u << c;
                 phase ^= 1u << c;
                 --total;
                 idle = 0;
@@ -646,7 +705,7 @@ __global__ void __launch_bounds__(32 * 5 * NCH, 1) forward_chain_kernel(const __
         const float alpha = cfg.act_alpha;
         uint32_t full = 0;
         auto wait_full = [&]() {
-            ok = ok && mbar_wait(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
+            ok = ok && wait_for(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
             ++full;
             tc_fence_after();
         };
@@ -670,7 +729,7 @@ __global__ void __launch_bounds__(32 * 5 * NCH, 1) forward_chain_kernel(const __
         for (; tile < p.n_tiles && ok; tile += stride) {
             const bool valid = sample < p.count;
             float* dst = (float*)out.at;
-            write_row<FMT, IW>(in_row, p, raw, in.at, valid, []() {});
+            write_row<FMT, IW>(in_row, p, raw, in.at, valid);
             release();
             sample += (uint64_t)stride * kTile;
             in.at += in.step;
@@ -735,7 +794,7 @@ __global__ void __launch_bounds__(32 * 5 * NCH, 1) forward_chain_kernel(const __
         for (uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch; tile < p.n_tiles && ok; tile += stride) {
 #pragma unroll 1
             for (int l = 0; l < nl; ++l) {
-                ok = ok && mbar_wait(&ready[ch], seen & 1u, abort_flag, p.status, kStatusIssue);
+                ok = ok && wait_for(&ready[ch], seen & 1u, abort_flag, p.status, kStatusIssue);
                 ok = __all_sync(0xffffffffu, ok);
                 ++seen;
                 tc_fence_after();
@@ -925,14 +984,18 @@ static bool chain_wide_network(const MlpConfig& c)
         if (c.dims[l] > 128) return false;
     return c.n_layers < 4 || (c.dims[0] <= 32 && c.dims[c.n_layers] <= 16);
 }
-// Against the kernels of tc_kernels.cu, us a step: 32-128-128-3, 1024 samples 20.5 / 19.3, 2^20: 581 / 235; 16-128-3 14.3 / 12.6, 379 / 124;
-// 64-96-96-40 33 / 25, 1433 / 578; 64-128-64 16.4 / 19.9, 65536 samples 36.9 / 36.9, 2^20: 369 / 321; 32-128-128-128-3 25.1 / 27.0,
-// 16384 samples 34.8 / 31.5, 2^20: 772 / 457.
+// Against the kernels of tc_kernels.cu, us a step.  Two chains: 32-128-128-3, 1024 samples 20.5 / 19.3, 2^20: 581 / 229; 16-128-3 14.3 /
+// 12.6, 379 / 124; 64-128-64 16.4 / 19.9, 65536 samples 36.9 / 36.9, 2^20: 369 / 321.  One chain: 32-128-128-128-3 25.1 / 27.0, 65536
+// samples 67.6 / 53.1, 2^20: 772 / 457; 56-103-103-3, 25505 samples (two tiles one after the other) 32.8 / 35.6, 65536: 53.0 / 47.2, 2^20: 597 /
+// 336; 64-128-128-64 51 / 61, 567 / 606.  Leaky ReLU has no build of its own there below five layers: 64-96-96-40 33 / 25, 1433 / 578;
+// 64-128-64, 1024 samples 19.3 / 19.9, 16384: 26.6 / 21.2.
 bool chain_train_wide_suits(const MlpConfig& c, uint32_t count)
 {
-    const bool few = c.dims[0] <= 32 && c.dims[c.n_layers] <= 16;
-    const uint32_t from = c.n_layers == 4 ? 16384u : c.n_layers == 2 && !few ? 131072u : kTrainFrom;
-    return count >= from && chain_wide_network(c);
+    if (!chain_wide_network(c)) return false;
+    const bool few_out = c.dims[c.n_layers] <= 16, few = c.dims[0] <= 32 && few_out;
+    if (c.hidden_act == MLP_ACT_LEAKY_RELU) return count >= (few || c.n_layers > 2 ? kTrainFrom : 4u * kTrainFrom);
+    if (c.n_layers == 4 || (c.n_layers == 3 && !few)) return few_out && count >= 65536u;   // one chain
+    return count >= (few ? kTrainFrom : 131072u);
 }
 
 bool chain_train_suits(const MlpConfig& c, uint32_t count) { return count >= kTrainFrom && chain_train_network(c); }

@@ -5,9 +5,10 @@
 // operand of the next layer's product and the MN-major operand of the weight-gradient product, and dZ_l replaces A_{l+1} where
 // it lay.  A fifth warp per chain issues its layer products and two warps the gradient products of all chains, so nothing
 // waits for another chain, and a chain's hand-offs (some 500 cycles each) are covered by the others' work.
-// Code that runs once per tile is kept small: the kernel is bound by instruction issue, and its loops have to stay in the
-// instruction cache (texture network, 2^24 texels: 2.5 ms a step with one copy of the gradient products' code, 2.6 with one
-// per layer and chain).
+// The kernels are bound by instruction issue and by instruction fetches: what a tile runs through is some 2300 instructions,
+// about as much as the instruction cache holds, so what runs once per tile or rarely is kept small or behind a call (texture
+// network, 2^24 texels: 2.64 ms a step with a copy of the gradient products' code per layer and chain, 2.51 with one; later 2.42
+// with the waits' polling loops and the marked zeros' code in line, 2.16 without).
 #pragma once
 
 #include "tc_layout.cuh"
@@ -38,6 +39,16 @@ __device__ __forceinline__ void wait_ld(uint32_t (&r)[16])
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
                    "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                  ::"memory");
+}
+
+// mbar_wait() with all but the first poll behind a call.
+static __device__ __noinline__ bool wait_on(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status, uint32_t code)
+{
+    return mbar_wait(bar, parity, abort_flag, status, code);
+}
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status, uint32_t code)
+{
+    return mbar_try_wait(bar, parity) || wait_on(bar, parity, abort_flag, status, code);
 }
 
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b)
@@ -189,9 +200,9 @@ static __device__ __noinline__ void convert_row(uint32_t at, int dtype, const ch
     }
 }
 
-// A thread's input row in operand format, up to the end of its last K step; `free()` is called before the first store.
-template <int FMT, int IW, class F>
-__device__ __forceinline__ void write_row(uint32_t at, const Params& p, const RawRow& raw, const char* src_row, bool real, F free)
+// A thread's input row in operand format, up to the end of its last K step.
+template <int FMT, int IW>
+__device__ __forceinline__ void write_row(uint32_t at, const Params& p, const RawRow& raw, const char* src_row, bool real)
 {
     using C = Cvt<FMT>;
     const MlpConfig& c = p.cfg;
@@ -203,7 +214,6 @@ __device__ __forceinline__ void write_row(uint32_t at, const Params& p, const Ra
         for (int k = 0; k < 2; ++k) {
             float2 x[8];
             narrow::encode_octaves(u, v, 4 * k, x);
-            if (k == 0) free();
             sts128(at ^ (uint32_t)(16 * k), C::pack2(x[0].x, x[1].x), C::pack2(x[2].x, x[3].x), C::pack2(x[4].x, x[5].x), C::pack2(x[6].x, x[7].x));
             sts128(at ^ (uint32_t)(32 + 16 * k), C::pack2(x[0].y, x[1].y), C::pack2(x[2].y, x[3].y), C::pack2(x[4].y, x[5].y), C::pack2(x[6].y, x[7].y));
         }
@@ -211,7 +221,6 @@ __device__ __forceinline__ void write_row(uint32_t at, const Params& p, const Ra
         float x[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = i < width ? bits_value(type, raw.v[i]) : 0.0f;
-        free();
         sts128(at, C::pack2(x[0], x[1]), C::pack2(x[2], x[3]), C::pack2(x[4], x[5]), C::pack2(x[6], x[7]));
         sts128(at ^ 16u, 0u, 0u, 0u, 0u);
     } else if (p.vec_in && type == MLP_F32) {
@@ -222,7 +231,6 @@ __device__ __forceinline__ void write_row(uint32_t at, const Params& p, const Ra
             float4 x[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = real && h + 4 * j < width ? __ldg(src + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (h == 0) free();
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 sts128(at ^ (uint32_t)(2 * h + 16 * j), C::pack2(x[2 * j].x, x[2 * j].y), C::pack2(x[2 * j].z, x[2 * j].w), C::pack2(x[2 * j + 1].x, x[2 * j + 1].y),
@@ -233,11 +241,9 @@ __device__ __forceinline__ void write_row(uint32_t at, const Params& p, const Ra
         uint4 x[IW / 8];
 #pragma unroll
         for (int j = 0; j < IW / 8; ++j) x[j] = real && 8 * j < width ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
-        free();
 #pragma unroll
         for (int j = 0; j < IW / 8; ++j) sts128(at ^ (uint32_t)(16 * j), x[j].x, x[j].y, x[j].z, x[j].w);
     } else {
-        free();
         convert_row<FMT>(at, type, src_row, width, real);
     }
 }
@@ -334,7 +340,7 @@ __device__ __forceinline__ void hidden_columns(const uint32_t (&v)[32], uint32_t
 // ReLU activations of a row in which a pre-activation rounds to zero, once more from the accumulator: those zeros are marked
 // by the sign.  Rare, so kept small.
 template <int FMT, int H>
-__device__ __forceinline__ void marked_columns(uint32_t t_acc, uint32_t row)
+__device__ __noinline__ void marked_columns(uint32_t t_acc, uint32_t row)
 {
     using C = Cvt<FMT>;
     constexpr float kTiny = 0.5f * C::kSmallest;   // the largest magnitude that rounds to zero
@@ -377,7 +383,7 @@ __device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_
 
 // The same over a whole row with marked zeros, where half of the gradient passes, in place.
 template <int FMT, int H>
-__device__ __forceinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row)
+__device__ __noinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row)
 {
     using C = Cvt<FMT>;
 #pragma unroll 1
