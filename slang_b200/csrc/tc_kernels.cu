@@ -1208,7 +1208,8 @@ cudaError_t launch_learn_gradient_tc(cudaStream_t st, TcWorkspace* ws, const Mlp
 {
     if (!wide_supported(c)) return launch_learn_gradient_narrow(st, ws, c, a, launches, err, input_grads);
     if (a.count == 0) return cudaSuccess;
-    if (chain_train_wide_suits(c, a.count)) return launch_learn_gradient_chain(st, ws, c, a, launches, err, input_grads);
+    // (input rows off a 16-byte boundary are refused below, whatever the batch)
+    if (chain_train_wide_suits(c, a.count) && (a.inputs & 15u) == 0) return launch_learn_gradient_chain(st, ws, c, a, launches, err, input_grads);
     const int nl = c.n_layers;
     const int d0 = c.dims[0], dout = c.dims[nl];
     CUtensorMap mx, mt;

@@ -3,6 +3,7 @@ width and layer count, input rows of each kind, outputs that leave in each way, 
 import numpy as np
 import pytest
 
+from oracle import layout_oracle as LO
 from oracle import oracle
 from slang_b200 import config as C
 
@@ -122,3 +123,36 @@ def test_input_gradients(device, dims):
     rows = np.linalg.norm(got - g, axis=1) / np.linalg.norm(g, axis=1)
     assert np.mean(rows > 1e-2) < 0.05, np.mean(rows > 1e-2)
     assert np.linalg.norm(got - g) / np.linalg.norm(g) < 0.1
+
+
+@pytest.mark.parametrize("dims", [[20, 48, 64, 3], [4, 32, 32, 32, 32, 4], [32, 96, 128, 10]], ids=lambda d: "-".join(map(str, d)))
+def test_optimal_layout_parameters(device, dims):
+    """Parameters and gradients in 16x16 tiles: the outputs are those of the same parameters by rows, the gradients too (to the
+    order of the CTAs' fp32 sums), each at its weight's place."""
+    results = []
+    for tiled in (False, True):
+        cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F16, target_dtype=C.F32, adam_master=1)
+        p0 = C.init_params(cfg, seed=5, scheme="xavier")
+        w_off, b_off, total = C.param_layout(cfg)
+        at = np.full(total, -1, dtype=np.int64)   # where each parameter lies
+        if tiled:
+            cfg.param_layout = C.PARAMS_OPTIMAL
+            ow, ob, ototal = C.param_layout(cfg)
+            for l in range(cfg.n_layers):
+                out16 = LO.align16(dims[l + 1])
+                for o in range(dims[l + 1]):
+                    for i in range(dims[l]):
+                        at[w_off[l] + o * dims[l] + i] = ow[l] + ((i // 16) * (out16 // 16) + o // 16) * 256 + LO.native_tile_pos(i % 16, o % 16)
+                    at[b_off[l] + o] = ob[l] + o
+            tp = np.zeros(ototal, dtype=p0.dtype)
+            tp[at[at >= 0]] = p0[at >= 0]
+            p0 = tp
+        got, _, loss, _, out, _, _ = _run(device, cfg, 4100, p0)
+        if tiled:
+            rows = np.zeros(total, dtype=got.dtype)
+            rows[at >= 0] = got[at[at >= 0]]
+            got = rows
+        results.append((got, loss, out))
+    assert rel_err(results[1][0], results[0][0]) < 1e-5
+    assert abs(results[1][1][1] - results[0][1][1]) <= 1e-5 * results[0][1][1]
+    assert np.array_equal(results[1][2], results[0][2])
