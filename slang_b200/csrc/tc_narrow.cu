@@ -1,5 +1,6 @@
-// learnGradient and forward for networks of widths up to 64 (the fp16 CoopVec-style network 4-32-32-32-32-4, the
-// neural-texture network enc(2->32)-64-64-64-3, anything in between), 16-bit operands.
+// learnGradient and forward for networks of widths up to 64, 16-bit operands: those that tc_chain.cu does not take (fp32
+// storage, other activations than ReLU and leaky ReLU) and the smallest batches.  Times of larger batches below are this file's
+// kernels' own.
 //
 // A warp carries 16 samples (training) or 32 (forward) through every layer in registers (tc_narrow.cuh) and never waits
 // for another warp on the way down or back up.  What contracts over samples, the weight and bias gradients, is done
