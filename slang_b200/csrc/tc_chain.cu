@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             wait_full();
             if (!ok) break;
             float loss = 0.0f;
+            uint32_t nan = 0u;   // width 128: a dZ that is not a number stays one past ReLUs that are off, as in the kernels of tc_kernels.cu
 #pragma unroll 1
             for (int f = 0; f < od; f += 4) {
                 float o[4], d[4], t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, g[4];
@@ -267,6 +268,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     const float diff = real ? o[i] - t[i] : 0.0f;
                     loss = fmaf(diff * scale, diff, loss);
                     g[i] = real ? ((2.0f * scale) * diff) * d[i] : 0.0f;
+                    if (M::kWide && g[i] != g[i]) nan = 0x7fff7fffu;
                 }
                 sts64((dz_row ^ (uint32_t)(16 * (f >> 3))) + (uint32_t)(2 * (f & 4)), C::pack2(g[0], g[1]), C::pack2(g[2], g[3]));
             }
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 if (HACT == MLP_ACT_RELU && zero_seen) {
                     wait_done(l);
                     if (!ok) break;
-                    reverse_marked_columns<FMT, H>(t_acc, at);
+                    reverse_marked_columns<FMT, H>(t_acc, at, M::kWide ? nan : 0u);
                 } else {
                     uint32_t v[H == 32 ? 1 : 2][32], z[H / 32][16];
                     tmem_ld_32x32(t_acc, v[0]);
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     for (int b = 0; b < H / 32; ++b) {
                         wait_ld(v[b & 1]);
                         if (b + 1 < H / 32) tmem_ld_32x32(t_acc + (uint32_t)(32 * b + 32), v[(b + 1) & (H == 32 ? 0 : 1)]);
-                        reverse_columns<FMT, HACT>(z[b], v[b & 1], block_at<H>(at, b), alpha_op);
+                        reverse_columns<FMT, HACT>(z[b], v[b & 1], block_at<H>(at, b), alpha_op, M::kWide ? nan : 0u);
                     }
                     wait_done(l);
                     if (!ok) break;

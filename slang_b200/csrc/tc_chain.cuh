@@ -358,9 +358,10 @@ __device__ __noinline__ void marked_columns(uint32_t t_acc, uint32_t row)
     }
 }
 
-// dZ = dA times the derivative, of the activations in the four chunks from `at` on.
+// dZ = dA times the derivative, of the activations in the four chunks from `at` on.  ReLU: `nan` is zero, or the bits that make a
+// pair NaN.
 template <int FMT, int HACT>
-__device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_t (&v)[32], uint32_t at, float alpha_op)
+__device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_t (&v)[32], uint32_t at, float alpha_op, uint32_t nan)
 {
     using C = Cvt<FMT>;
 #pragma unroll
@@ -371,7 +372,7 @@ __device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_
         for (int i = 0; i < 4; ++i) {
             const float g0 = __uint_as_float(v[8 * j + 2 * i]), g1 = __uint_as_float(v[8 * j + 2 * i + 1]);
             if constexpr (HACT == MLP_ACT_RELU) {
-                z[4 * j + i] = C::pack2(g0, g1) & C::positive_mask(a[i]);
+                z[4 * j + i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | nan;
             } else {
                 const uint32_t neg = narrow::sign_mask(a[i]);
                 const float2 ag = __fmul2_rn(make_float2(g0, g1), make_float2(alpha_op, alpha_op));
@@ -383,7 +384,7 @@ __device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_
 
 // The same over a whole row with marked zeros, where half of the gradient passes, in place.
 template <int FMT, int H>
-__device__ __noinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row)
+__device__ __noinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row, uint32_t nan)
 {
     using C = Cvt<FMT>;
 #pragma unroll 1
@@ -397,7 +398,7 @@ __device__ __noinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float g0 = __uint_as_float(v[2 * i]), g1 = __uint_as_float(v[2 * i + 1]);
-            z[i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | (C::pack2(0.5f * g0, 0.5f * g1) & narrow::sign_mask(a[i]));
+            z[i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | (C::pack2(0.5f * g0, 0.5f * g1) & narrow::sign_mask(a[i])) | nan;
         }
         sts128(at, z[0], z[1], z[2], z[3]);
     }

@@ -156,3 +156,14 @@ def test_optimal_layout_parameters(device, dims):
     assert rel_err(results[1][0], results[0][0]) < 1e-5
     assert abs(results[1][1][1] - results[0][1][1]) <= 1e-5 * results[0][1][1]
     assert np.array_equal(results[1][2], results[0][2])
+
+
+@pytest.mark.parametrize("count", [1024, 3000])
+def test_a_sample_that_overflows_reaches_every_gradient(device, count):
+    """Width 128: one sample's output is not a number, so no gradient it enters is, whichever ReLUs are off."""
+    cfg = C.make_config([32, 128, 128, 3], C.F16, C.ACT_RELU, input_dtype=C.F16, target_dtype=C.F32, adam_master=1)
+    x = np.random.default_rng(1).normal(size=(count, 32))
+    x[77] = 6e4
+    got, grads, loss, ref, _, _, _ = _run(device, cfg, count, None, x)
+    assert np.isnan(ref[1]) and np.isnan(loss[1])
+    assert np.array_equal(np.isnan(got), np.isnan(grads))
