@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     using M = TrainMap<H, NL, IW, OW, NCH>;
     using C = Cvt<FMT>;
     constexpr int kThreads = M::kThreads, NW = M::kWarps, G = M::kGradWarps;
+    constexpr bool kOverflow = M::kWide && HACT == MLP_ACT_RELU;   // reverse_whole_row() where a dA is not finite
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem);
@@ -250,7 +251,6 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             wait_full();
             if (!ok) break;
             float loss = 0.0f;
-            uint32_t nan = 0u;   // width 128: a dZ that is not a number stays one past ReLUs that are off, as in the kernels of tc_kernels.cu
 #pragma unroll 1
             for (int f = 0; f < od; f += 4) {
                 float o[4], d[4], t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, g[4];
@@ -268,7 +268,6 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     const float diff = real ? o[i] - t[i] : 0.0f;
                     loss = fmaf(diff * scale, diff, loss);
                     g[i] = real ? ((2.0f * scale) * diff) * d[i] : 0.0f;
-                    if (M::kWide && g[i] != g[i]) nan = 0x7fff7fffu;
                 }
                 sts64((dz_row ^ (uint32_t)(16 * (f >> 3))) + (uint32_t)(2 * (f & 4)), C::pack2(g[0], g[1]), C::pack2(g[2], g[3]));
             }
@@ -284,25 +283,36 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 wait_full();
                 if (!ok) break;
                 const uint32_t at = own_row + (uint32_t)(l - 1) * M::kRows;   // A_l
-                if (HACT == MLP_ACT_RELU && zero_seen) {
+                uint32_t v[H == 32 ? 1 : 2][32];
+                bool whole = HACT == MLP_ACT_RELU && zero_seen;
+                tmem_ld_32x32(t_acc, v[0]);
+                wait_ld(v[0]);
+                if constexpr (kOverflow && FMT == MLP_F16) whole = whole || __any_sync(0xffffffffu, not_finite<FMT>(v[0]));
+                if (whole) {
                     wait_done(l);
                     if (!ok) break;
-                    reverse_marked_columns<FMT, H>(t_acc, at, M::kWide ? nan : 0u);
+                    reverse_whole_row<FMT, H>(t_acc, at);
                 } else {
-                    uint32_t v[H == 32 ? 1 : 2][32], z[H / 32][16];
-                    tmem_ld_32x32(t_acc, v[0]);
+                    uint32_t z[H / 32][16];
+                    bool odd = false;
 #pragma unroll
                     for (int b = 0; b < H / 32; ++b) {
-                        wait_ld(v[b & 1]);
+                        if (b > 0) wait_ld(v[b & 1]);
                         if (b + 1 < H / 32) tmem_ld_32x32(t_acc + (uint32_t)(32 * b + 32), v[(b + 1) & (H == 32 ? 0 : 1)]);
-                        reverse_columns<FMT, HACT>(z[b], v[b & 1], block_at<H>(at, b), alpha_op, M::kWide ? nan : 0u);
+                        reverse_columns<FMT, HACT>(z[b], v[b & 1], block_at<H>(at, b), alpha_op);
+                        if constexpr (kOverflow && FMT == MLP_BF16) odd = odd || not_finite<FMT>(v[b & 1]);
                     }
+                    if constexpr (kOverflow && FMT == MLP_BF16) odd = __any_sync(0xffffffffu, odd);
                     wait_done(l);
                     if (!ok) break;
+                    if (odd) {
+                        reverse_whole_row<FMT, H>(t_acc, at);
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < H / 8; ++j) {
-                        const uint32_t* w = &z[j >> 2][4 * (j & 3)];
-                        sts128(block_at<H>(at, j >> 2) ^ (uint32_t)(16 * (j & 3)), w[0], w[1], w[2], w[3]);
+                        for (int j = 0; j < H / 8; ++j) {
+                            const uint32_t* w = &z[j >> 2][4 * (j & 3)];
+                            sts128(block_at<H>(at, j >> 2) ^ (uint32_t)(16 * (j & 3)), w[0], w[1], w[2], w[3]);
+                        }
                     }
                 }
                 release(l > 1 || p.input_grads, l - 1);

@@ -358,10 +358,9 @@ __device__ __noinline__ void marked_columns(uint32_t t_acc, uint32_t row)
     }
 }
 
-// dZ = dA times the derivative, of the activations in the four chunks from `at` on.  ReLU: `nan` is zero, or the bits that make a
-// pair NaN.
+// dZ = dA times the derivative, of the activations in the four chunks from `at` on.
 template <int FMT, int HACT>
-__device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_t (&v)[32], uint32_t at, float alpha_op, uint32_t nan)
+__device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_t (&v)[32], uint32_t at, float alpha_op)
 {
     using C = Cvt<FMT>;
 #pragma unroll
@@ -372,7 +371,7 @@ __device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_
         for (int i = 0; i < 4; ++i) {
             const float g0 = __uint_as_float(v[8 * j + 2 * i]), g1 = __uint_as_float(v[8 * j + 2 * i + 1]);
             if constexpr (HACT == MLP_ACT_RELU) {
-                z[4 * j + i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | nan;
+                z[4 * j + i] = C::pack2(g0, g1) & C::positive_mask(a[i]);
             } else {
                 const uint32_t neg = narrow::sign_mask(a[i]);
                 const float2 ag = __fmul2_rn(make_float2(g0, g1), make_float2(alpha_op, alpha_op));
@@ -382,9 +381,27 @@ __device__ __forceinline__ void reverse_columns(uint32_t (&z)[16], const uint32_
     }
 }
 
-// The same over a whole row with marked zeros, where half of the gradient passes, in place.
+// Whether a row's dA holds an infinity or a NaN, from the first 32 features (halves) or of 32 features (bfloat16s).  An infinite or NaN
+// dZ of the layer behind makes every feature so (times any weight, zero included, it is not finite), so the first one tells;
+// from finite halves a sum of 128 products stays finite, of bfloat16s it can overflow, feature by feature.
+template <int FMT>
+__device__ __forceinline__ bool not_finite(const uint32_t (&v)[32])
+{
+    if constexpr (FMT == MLP_F16) {
+        return (v[0] & 0x7f800000u) == 0x7f800000u;
+    } else {
+        float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) s = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), make_float2(0.0f, 0.0f), s);
+        return !(s.x + s.y == 0.0f);
+    }
+}
+
+// The same over a whole row, in place, where half of the gradient passes at marked zeros.  Width 128: as a product with the derivative, like the kernels
+// of tc_kernels.cu, so that a dA that is not finite is NaN past a ReLU that is off; below that a ReLU that is off gives zero
+// whatever comes, like the kernels of tc_narrow.cu.
 template <int FMT, int H>
-__device__ __noinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row, uint32_t nan)
+__device__ __noinline__ void reverse_whole_row(uint32_t t_acc, uint32_t row)
 {
     using C = Cvt<FMT>;
 #pragma unroll 1
@@ -398,7 +415,13 @@ __device__ __noinline__ void reverse_marked_columns(uint32_t t_acc, uint32_t row
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float g0 = __uint_as_float(v[2 * i]), g1 = __uint_as_float(v[2 * i + 1]);
-            z[i] = (C::pack2(g0, g1) & C::positive_mask(a[i])) | (C::pack2(0.5f * g0, 0.5f * g1) & narrow::sign_mask(a[i])) | nan;
+            const uint32_t on = C::positive_mask(a[i]), zero = narrow::sign_mask(a[i]);
+            if constexpr (H == 128) {
+                const float d0 = (on & 1u) ? 1.0f : (zero & 1u) ? 0.5f : 0.0f, d1 = (on >> 31) ? 1.0f : (zero >> 31) ? 0.5f : 0.0f;
+                z[i] = C::pack2(g0 * d0, g1 * d1);
+            } else {
+                z[i] = (C::pack2(g0, g1) & on) | (C::pack2(0.5f * g0, 0.5f * g1) & zero);
+            }
         }
         sts128(at, z[0], z[1], z[2], z[3]);
     }

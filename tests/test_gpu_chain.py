@@ -167,3 +167,38 @@ def test_a_sample_that_overflows_reaches_every_gradient(device, count):
     got, grads, loss, ref, _, _, _ = _run(device, cfg, count, None, x)
     assert np.isnan(ref[1]) and np.isnan(loss[1])
     assert np.array_equal(np.isnan(got), np.isnan(grads))
+
+
+@pytest.mark.parametrize("where", ["output", "hidden"])
+@pytest.mark.parametrize("dtype", [C.F16, C.BF16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("dims,count", [([32, 128, 128, 3], 1024), ([16, 96, 100, 3], 1100), ([64, 128, 64], 131072 + 77), ([40, 128, 128, 16], 65536 + 77),
+                                        ([8, 90, 128, 100, 16], 65536 + 77)], ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else str(v))
+def test_an_overflow_reaches_the_gradients_that_the_oracle_says(device, dims, count, dtype, where):
+    """Width 128: one sample's dZ overflows, in the output layer (whose loss is finite in half), or first in the layer below, where weights of 1/2 keep
+    a dA in range and weights of 30 do not.  A ReLU that is off turns an infinite dA into a NaN, a finite one into zero: the same
+    entries as the oracle's are NaN, infinite and finite."""
+    from slang_b200.api import Trainer
+    cfg = C.make_config(dims, dtype, C.ACT_RELU, loss=C.LOSS_L2_SUM, input_dtype=dtype, target_dtype=C.F32, adam_master=1)
+    rng = np.random.default_rng(count)
+    p = C.from_storage(C.init_params(cfg, seed=3, scheme="xavier"), dtype).copy()
+    x = C.to_storage(rng.uniform(-1, 1, (count, dims[0])), dtype)
+    t = rng.uniform(-1, 1, (count, dims[-1])).astype(np.float32)
+    w_off, _, total = C.param_layout(cfg)
+    if where == "output":
+        t[77, 0] = 5e4 if dtype == C.F16 else 3e38
+    else:
+        t[77, 0] = 1.5e4 if dtype == C.F16 else 5e37
+        p[w_off[-1]:w_off[-1] + dims[-2]] = rng.choice([0.5, 30.0], dims[-2])
+    params = C.to_storage(p, dtype)
+    tr = Trainer(device, cfg, params)
+    xb, tb, gb = device.create_buffer(x.nbytes, x), device.create_buffer(t.nbytes, t), device.create_buffer(4 * count * dims[0])
+    tr.learn_gradient(xb.address, tb.address, count, input_grads_address=gb.address)
+    want = np.zeros(total, dtype=np.float32)
+    loss = oracle.learn_gradient(cfg, params, want, x, t, count, n_threads=8).view(np.float32)
+    if where == "output" and dtype == C.F16:
+        assert np.isfinite(loss).all()
+    assert not np.isfinite(want).all() and np.isfinite(want).any()
+    want_dx = oracle.learn_gradient_inputs(cfg, params, np.zeros(total, dtype=np.float32), x, t, 200, np.zeros(2, dtype=np.uint32)).ravel()
+    for got, ref in ((tr.read_grads(), want), (gb.read(np.float32)[:want_dx.size], want_dx)):
+        assert np.array_equal(np.isnan(got), np.isnan(ref))
+        assert np.array_equal(np.isposinf(got), np.isposinf(ref)) and np.array_equal(np.isneginf(got), np.isneginf(ref))
