@@ -35,6 +35,8 @@ enum : uint32_t { kStatusIssue = 0x4000u, kStatusRow = 0x8000u, kStatusGrad = 0x
 // Warps that issue gradient products: two (even and odd layers) beside four chains; with three, sixteen warps in all leave
 // each thread 128 registers and seventeen 96.
 __host__ __device__ constexpr int grad_warps(int chains) { return chains == 3 ? 1 : 2; }
+// Width 32: warps that take the windows' sums, one for each quarter of the lanes that has rows (registers are dealt four warps at a time, so they cost none).
+__host__ __device__ constexpr int sum_warps(int h) { return h == 32 ? 2 : 0; }
 
 // Shared-memory map of the training kernel (bytes from a 1024-aligned base).  H: padded hidden width; IW: padded input
 // width; OW: padded output width; NCH: chains.
@@ -43,7 +45,22 @@ struct TrainMap {
     static constexpr int kWarps = 4 * NCH;                // with samples; one more per chain issues its layer products, one or two the gradient products
     static constexpr int kGradWarps = grad_warps(NCH);
     static constexpr bool kWide = H == 128;
-    static constexpr int kThreads = 32 * (kWarps + NCH + kGradWarps);
+    // An accumulator in tensor memory is not rounded but cut off: every addition loses up to a unit in the last place, always toward zero.  Where all samples pull
+    // one way, a gradient summed there over all of a CTA's tiles is 1e-7 short for every 16 samples: 4.5e-5 at 2^20 samples, 7e-4 at 2^24.  So what the kernels
+    // of tc_narrow.cu and tc_kernels.cu sum in registers (all of width 32; dW_0 and the biases of width 128) is summed there over windows of a few tiles, and the windows
+    // in fp32.  (What they sum in tensor memory too, all of width 64 and the hidden layers' dW at 128, is summed there over all tiles.)
+    static constexpr bool kWindows = H != 64;
+    // Width 32: windows of four tiles, one for each chain, are 2.9e-6 short at any batch (the register sums 5.3e-6 at 2^20, 9e-5 at 2^24).  Warps of their own take
+    // them: a step of 2^20 samples of 4-32-32-32-32-4 takes 129.9 us, 141.6 with the tiles' warps taking them between two layers, 124.2
+    // without windows; windows of eight tiles 129.1.
+    static constexpr uint32_t kWindow = 4;
+    // Width 128: dW_0 and db_0 are taken with every tile (1.3e-6, the register sums 1.0e-6), the other biases with some 32 (sums of 16-bit values are
+    // exact for about as long), by the chain's warps: 2^20 samples of 32-128-128-3 231.8 -> 233.9 us, of 32-128-128-128-3 437.7 -> 448.5.
+    // Whether tile `turn` of chain c (of its own count, at least modulo 16) ends a window of layer l.
+    __host__ __device__ static constexpr bool ends_window(int l, uint32_t c, uint32_t turn) { return kWide && (l == 0 || (c == 0u && (turn & 15u) == 15u)); }
+    static constexpr int kSumWarps = sum_warps(H);
+    static_assert(kSumWarps == 0 || (kWarps + NCH) % 4 == 0, "the sums' warps reach the quarters 0 and 1");
+    static constexpr int kThreads = 32 * (kWarps + NCH + kSumWarps + kGradWarps);
     static constexpr int kDzW = OW == 16 ? 32 : OW;            // row width of the last layer's dZ
     __host__ __device__ static constexpr int in_w(int l) { return l == 0 ? IW : H; }
     __host__ __device__ static constexpr int out_w(int l) { return l == NL - 1 ? OW : H; }
@@ -65,10 +82,19 @@ struct TrainMap {
     static constexpr uint32_t kBias = kHiddenBias + (NL - 1) * H * 32; // the output layer's, fp32 [OW]
     static constexpr uint32_t kLoss = kBias + OW * 4;              // fp32 [kWarps][2]
     static constexpr uint32_t kBars = kLoss + kWarps * 8;              // per chain: ready, acc_full, and for each gradient warp dz_ready, dw_done
-    static constexpr uint32_t kTmemPtr = kBars + (2 + 2 * kGradWarps) * NCH * 8;
+    static constexpr uint32_t kTaken = kBars + (2 + 2 * kGradWarps) * NCH * 8;   // more barriers, one a layer: a window's sums are taken
+    static constexpr uint32_t kEnded = kTaken + (kWindows ? NL * 8 : 0);         // width 32, one a layer: a window's last product has completed
+    static constexpr uint32_t kTmemPtr = kEnded + (kSumWarps ? NL * 8 : 0);
     static constexpr uint32_t kAbort = kTmemPtr + 4;
-    static constexpr uint32_t kNet = (kAbort + 4 + 15) & ~15u;
-    static constexpr uint32_t kSmemBytes = kNet + NL * 32 + 1024;
+    static constexpr uint32_t kOpen = kAbort + 4;                      // bit l: layer l has products in tensor memory that no window took
+    static constexpr uint32_t kNet = (kOpen + 4 + 15) & ~15u;
+    // Sums of whole windows, fp32: biases [layer][H], then weights [layer][rows][32] with 16-byte chunks ^ (row % 8).  (Of width 128 only dW_0,
+    // and only where tensor memory has no room for it.)
+    static constexpr uint32_t kBiasSums = (kNet + NL * 32 + 15) & ~15u;
+    static constexpr uint32_t kSums = (kBiasSums + (kWindows ? NL * H * 4 : 0) + 127) & ~127u;
+    static constexpr bool kSumsInTmem = kWide && NL < 4;
+    static constexpr uint32_t kSumsBytes = !kWindows || kSumsInTmem ? 0 : kWide ? H * 128 : ((NL - 1) * H + OW) * 128;
+    static constexpr uint32_t kSmemBytes = kSums + kSumsBytes + 1024;
     // the outgoing gradients: fp32 [layers at a time][H][H + 1], over the chains' tiles
     static constexpr uint32_t kSumRow = H + 1;
     static constexpr int kSumLayers = kWide ? 1 : NL;
@@ -84,11 +110,65 @@ struct TrainMap {
         return NCH * (uint32_t)H + (l == 0 ? 0u : dw_cols(0) + (uint32_t)(l - 1) * (H + 16));
     }
     __host__ __device__ static constexpr uint32_t db_col(int l) { return NCH * (uint32_t)H + (NL - 2) * 128u + IW + OW + 16u * (uint32_t)l; }
-    static_assert((kWide ? db_col(NL) : dw_col(NL)) <= 512, "tensor memory budget");
+    __host__ __device__ static constexpr uint32_t sum_col() { return db_col(NL); }   // kSumsInTmem
+    static_assert((kWide ? db_col(NL) + (kSumsInTmem ? IW : 0) : dw_col(NL)) <= 512, "tensor memory budget");
 };
 
+// Adds what layer l's products have summed in tensor memory since its last window to the sums of windows: dW and db, of width 128 only dW_0 and
+// db.  By one warp for each lane quarter with rows (width 32: 0 and 1); `lanes` is the tensor-memory address of the warp's.
+template <class M, int H, int NL, int IW>
+static __device__ __noinline__ void take_window(uint32_t lanes, uint32_t sbase, int l)
+{
+    const int lane = threadIdx.x & 31, quarter = (int)(threadIdx.x >> 5) & 3;
+    const bool half = !M::kWide || l == NL - 1;   // 64 rows: on lanes 0 to 15 of each quarter
+    const int row = half ? quarter * 16 + lane : quarter * 32 + lane;
+    const bool real = (!half || lane < 16) && row < (l == NL - 1 ? M::out_w(NL - 1) : H);
+    const uint32_t bias = sbase + M::kBiasSums + 4u * (uint32_t)(l * H + row);
+    tc_fence_after();
+    uint32_t b;
+    if constexpr (M::kWide) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(b) : "r"(lanes + M::db_col(0) + 16u * (uint32_t)l) : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(b)::"memory");
+        if (l == 0) {
+            const uint32_t at = sbase + M::kSums + (uint32_t)row * 128u;
+#pragma unroll 1
+            for (int c = 0; c < IW; c += 16) {
+                uint32_t v[16], s[16];
+                tmem_ld_32x16(lanes + M::dw_col(0) + (uint32_t)c, v);
+                if constexpr (M::kSumsInTmem) {
+                    tmem_ld_32x16(lanes + M::sum_col() + (uint32_t)c, s);
+                    wait_ld(v);
+                    wait_ld(s);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) + __uint_as_float(v[i]));
+                    tmem_st_32x16(lanes + M::sum_col() + (uint32_t)c, s);
+                } else {
+                    wait_ld(v);
+                    add_chunks<4>(at, row, c / 4, v);
+                }
+            }
+            if constexpr (M::kSumsInTmem) tmem_st_wait();
+        }
+    } else {
+        const uint32_t col = lanes + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (uint32_t)(l - 1) * (H + 16));
+        uint32_t v[32];
+        tmem_ld_32x32(col, v);
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(b) : "r"(col + (uint32_t)H) : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(b)::"memory");
+        wait_ld(v);
+        if (real) add_chunks<8>(sbase + M::kSums + (uint32_t)(l * H + row) * 128u, row, 0, v);
+    }
+    if (real) {
+        float x;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(bias) : "memory");
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias), "f"(x + __uint_as_float(b)) : "memory");
+    }
+    tc_fence_before();
+    __syncwarp();
+}
+
 template <int H, int NL, int IW, int OW, int NCH, int FMT, int HACT>
-__global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gradient_chain_kernel(const __grid_constant__ Params p)
+__global__ void __launch_bounds__(32 * (5 * NCH + sum_warps(H) + grad_warps(NCH)), 1) learn_gradient_chain_kernel(const __grid_constant__ Params p)
 {
     using M = TrainMap<H, NL, IW, OW, NCH>;
     using C = Cvt<FMT>;
@@ -103,6 +183,8 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     uint64_t* acc_full = ready + NCH;                 // a layer product has completed
     uint64_t* dz_ready = acc_full + NCH;              // [chain][layer % G]: a dZ is written
     uint64_t* dw_done = dz_ready + G * NCH;           // [chain][layer % G]: a gradient product has completed
+    uint64_t* taken = (uint64_t*)(smem + M::kTaken);  // [layer]: a window's sums have left tensor memory
+    uint64_t* ended = (uint64_t*)(smem + M::kEnded);  // [layer], width 32: a window's last product has completed
     volatile uint32_t* abort_flag = (volatile uint32_t*)(smem + M::kAbort);
     const int od = cfg.dims[NL];
 
@@ -116,8 +198,18 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 mbar_init(&dw_done[G * c + g], 1);
             }
         }
+        if constexpr (M::kWindows) {
+            for (int l = 0; l < NL; ++l) {
+                mbar_init(&taken[l], M::kWide ? 4 : 2);
+                if (M::kSumWarps) mbar_init(&ended[l], 1);
+            }
+            *(uint32_t*)(smem + M::kOpen) = 0u;
+        }
         *abort_flag = 0u;
         fence_mbar_init();
+    }
+    if constexpr (M::kWindows) {
+        for (uint32_t i = M::kBiasSums + 16u * threadIdx.x; i < M::kSums + M::kSumsBytes; i += 16u * kThreads) *(uint4*)(smem + i) = make_uint4(0u, 0u, 0u, 0u);
     }
     constexpr int OH = M::kOnesW;
     for (int i = threadIdx.x; i < 16 * OH / 2; i += kThreads) {
@@ -139,6 +231,15 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     const MlpLayerPointers* s_net = (const MlpLayerPointers*)(smem + M::kNet);
     if (threadIdx.x < NL * 4) ((uint64_t*)(smem + M::kNet))[threadIdx.x] = ((const uint64_t*)p.net)[threadIdx.x];
     __syncthreads();
+    if constexpr (M::kSumsInTmem) {
+        if (warp < 4) {
+            const uint32_t zero[16] = {};
+            const uint32_t at = *(volatile uint32_t*)(smem + M::kTmemPtr) + ((uint32_t)(warp * 32) << 16) + M::sum_col();
+#pragma unroll
+            for (int c = 0; c < IW; c += 16) tmem_st_32x16(at + (uint32_t)c, zero);
+            tmem_st_wait();
+        }
+    }
     stage_weights<IW>(smem + M::kWeights, cfg, (const void*)s_net[0].weights, H, cfg.dims[0], cfg.dims[1], threadIdx.x, kThreads);
 #pragma unroll 1
     for (int l = 1; l < NL; ++l)
@@ -160,6 +261,14 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     const uint32_t tmem_base = *(volatile uint32_t*)(smem + M::kTmemPtr);
     const uint32_t stride = gridDim.x * NCH;
     bool ok = true;
+    auto tiles_here = [&]() {   // the CTA's
+        uint32_t n = 0;
+        for (int c = 0; c < NCH; ++c) {
+            const uint32_t first = blockIdx.x + gridDim.x * (uint32_t)c;
+            n += first < p.n_tiles ? (p.n_tiles - first + stride - 1) / stride : 0u;
+        }
+        return n;
+    };
 
     if (warp < NW) {
         // =================================== samples ===============================================
@@ -173,7 +282,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
         const float alpha = cfg.act_alpha, alpha_op = C::round(alpha);
         constexpr float kTiny = 0.5f * C::kSmallest;   // the largest magnitude that rounds to zero
         float run_max = 0.0f, run_sum = 0.0f;
-        uint32_t full = 0, done = 0;                   // phases seen of acc_full; bit g: parity of dw_done's g
+        uint32_t full = 0, done = 0;                   // phases seen of acc_full; bit g: parity of dw_done's g, from bit 2 on the chain's tiles so far
         auto wait_full = [&]() {
             ok = ok && wait_for(&acc_full[ch], full & 1u, abort_flag, p.status, kStatusRow);
             ++full;
@@ -193,13 +302,20 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                 if (gradient >= 0) mbar_arrive(&dz_ready[G * ch + gradient % G]);
             }
         };
+        // width 128: takes layer l's sums if this chain's tile `of`, whose product has completed, ends a window
+        auto take = [&](int l, uint32_t of) {
+            if constexpr (M::kWide) {
+                if (!M::ends_window(l, (uint32_t)ch, of)) return;
+                take_window<M, H, NL, IW>(t_acc - (uint32_t)(ch * H), sbase, l);
+                if (lane == 0) mbar_arrive(&taken[l]);
+            }
+        };
         RawRow raw;
         uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)ch;
         uint64_t sample = (uint64_t)tile * kTile + (uint64_t)r;
         Rows in(p.inputs, stored_inputs(cfg), cfg.input_dtype, sample, stride * kTile), tgt(p.targets, od, cfg.target_dtype, sample, stride * kTile);
         const bool wide_target = cfg.target_dtype == MLP_F32;
         fetch_row(raw, p, in.at, sample < p.count);
-        bool first = true;
         for (; tile < p.n_tiles && ok; tile += stride) {
             const bool valid = sample < p.count;
             bool zero_seen = false;
@@ -227,8 +343,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             for (int l = 0; l < NL - 1; ++l) {
                 wait_full();
                 if (l == 0) {   // the last tile's dZ_0 lies where A_1 goes, its A_0 where dZ_{NL-1} will
-                    if (!first) wait_done(0);
-                    first = false;
+                    if (done > 3u) wait_done(0);
                 }
                 if (!ok) break;
                 const uint32_t dst = own_row + (uint32_t)l * M::kRows;   // A_{l + 1}
@@ -246,6 +361,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     marked_columns<FMT, H>(t_acc, dst);
                 }
                 release(true, -1);
+                if (l == 0 && done > 3u) take(0, (done >> 2) - 1u);
             }
             // ---- output layer, loss, dZ of the last layer ----
             wait_full();
@@ -316,7 +432,9 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                     }
                 }
                 release(l > 1 || p.input_grads, l - 1);
+                take(l, done >> 2);
             }
+            done += 4u;
             // ---- optional: the input gradients dZ_0 . W_0, rounded to the storage type ----
             if (p.input_grads) {
                 wait_full();
@@ -348,7 +466,10 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             in_row = dz_row;
             dz_row = swap;
         }
-        if (!first) wait_done(0);
+        if (done > 3u) {
+            wait_done(0);
+            if (ok) take(0, (done >> 2) - 1u);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             run_max = fmaxf(run_max, __shfl_xor_sync(0xffffffffu, run_max, o));
@@ -468,33 +589,60 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             x = y;
             y = swap;
         }
+    } else if (warp < NW + NCH + M::kSumWarps) {
+        // =================================== the windows' sums =====================================
+        // The n-th product of a layer comes before the n-th of the layer before it, so windows end in this order.
+        if constexpr (M::kSumWarps > 0) {
+            const uint32_t windows = tiles_here() / M::kWindow;
+#pragma unroll 1
+            for (uint32_t n = 0; n < windows && ok; ++n) {
+#pragma unroll 1
+                for (int l = NL - 1; l >= 0; --l) {
+                    ok = ok && wait_for(&ended[l], n & 1u, abort_flag, p.status, kStatusGrad);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    take_window<M, H, NL, IW>(tmem_base + ((uint32_t)((warp & 3) * 32) << 16), sbase, l);
+                    if (lane == 0) mbar_arrive(&taken[l]);
+                }
+            }
+        }
     } else {
         // =================================== gradient products of all chains =======================
         // Warp g takes the layers g, g + G, .. of whichever chain has a dZ ready; one thread issues all
         // products into one accumulator, so those are in order.  (The loop is kept small: with a copy of the code per chain and
         // layer, its instructions were fetched anew each time.)
-        const int g = warp - NW - NCH;
+        const int g = warp - NW - NCH - M::kSumWarps;
         const uint32_t lo = (sbase & 0x3FFFFu) >> 4;
         constexpr uint32_t F = C::kUmmaFmt;
         const uint32_t top = (uint32_t)(NL - 1 - (NL - 1 - g) % G);        // this warp's last layer; its first is g
-        uint32_t total = 0, idle = 0, started = 0, phase = 0, layers = 0, flip = 0;   // hand-overs to come; layers begun; four bits a chain: its layer; whether A_0 and the last dZ have changed places
-        for (int c = 0; c < NCH; ++c) {
-            const uint32_t first = blockIdx.x + gridDim.x * (uint32_t)c;
-            layers |= top << (4 * c);
-            total += first < p.n_tiles ? ((p.n_tiles - first + stride - 1) / stride) * (top / G + 1) : 0u;
-        }
+        uint32_t total = tiles_here() * (top / G + 1), idle = 0;   // hand-overs to come
+        uint32_t started = 0, phase = 0, layers = 0;               // layers begun; four bits a chain: its layer
+        uint32_t turns = 0;                                        // eight bits a chain: its tiles so far, modulo 16
+        uint32_t over = 0, parity = 0;                             // layers whose window has ended and may not be taken yet; their parities of `taken`
+        uint32_t summed = 0, filled = 0;                           // width 128: layers whose db's window has begun; width 32, four bits a layer: tiles in its window
+        for (int c = 0; c < NCH; ++c) layers |= top << (4 * c);
         uint32_t c = 0;
 #pragma unroll 1
         while (total > 0 && ok) {
-            if (__all_sync(0xffffffffu, mbar_test_wait(&dz_ready[G * c + g], (phase >> c) & 1u))) {
+            const uint32_t l = (layers >> (4 * c)) & 15u;
+            bool go = __all_sync(0xffffffffu, mbar_test_wait(&dz_ready[G * c + g], (phase >> c) & 1u));
+            if (M::kWindows && go && (over >> l) & 1u) go = __all_sync(0xffffffffu, mbar_test_wait(&taken[l], (parity >> l) & 1u));
+            if (go) {
                 tc_fence_after();
-                const uint32_t l = (layers >> (4 * c)) & 15u, cb = M::kChains + c * M::kChainBytes;
-                const bool flipped = (flip >> c) & 1u;
+                const uint32_t cb = M::kChains + c * M::kChainBytes;
+                const uint32_t turn = turns >> (8 * c);
+                const bool flipped = turn & 1u;   // A_0 and the last dZ change places with every tile
+                if (M::kWindows && (over >> l) & 1u) {
+                    parity ^= 1u << l;
+                    over ^= 1u << l;
+                    if (M::kWide) summed ^= 1u << l;
+                    if (!M::kWide || l == 0) started ^= 1u << l;
+                }
                 const uint32_t a = l == 0 ? cb + (flipped ? M::kDz : 0u) : cb + M::kRowsIn + (l - 1) * M::kRows;           // A_l
                 const uint32_t z = l == NL - 1 ? cb + (flipped ? 0u : M::kDz) : cb + M::kRowsIn + l * M::kRows;   // dZ_l
                 const uint32_t begun = (started >> l) & 1u;
                 if constexpr (M::kWide) {
-                    const uint32_t db = tmem_base + M::db_col(0) + 16u * l;
+                    const uint32_t db = tmem_base + M::db_col(0) + 16u * l, window = (summed >> l) & 1u;
                     if (elect_one()) {
                         if (l == NL - 1) {
                             // A^T . dZ, and dZ^T . 1 of 64 rows (those past the outputs are never read)
@@ -503,7 +651,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                                 umma_f16(tmem_base + M::dw_col(NL - 1), desc_mn<H>(lo, a, k, M::kPanel), desc_mn<M::kDzW>(lo, z, k), umma_idesc(F, 1, 1, 128, OW), k > 0 ? 1u : begun);
 #pragma unroll 2
                             for (int k = 0; k < kTile / 16; ++k)
-                                umma_f16(db, desc_mn<M::kDzW>(lo, z, k), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 64, 8), k > 0 ? 1u : begun);
+                                umma_f16(db, desc_mn<M::kDzW>(lo, z, k), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 64, 8), k > 0 ? 1u : window);
                         } else {
                             const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * 128u);
                             if (l == 0) {
@@ -517,12 +665,13 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                             }
 #pragma unroll 2
                             for (int k = 0; k < kTile / 16; ++k)
-                                umma_f16(db, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 128, 16), k > 0 ? 1u : begun);
+                                umma_f16(db, desc_mn<H>(lo, z, k, M::kPanel), desc_mn<M::kOnesW>(lo, M::kOnes, 0), umma_idesc(F, 1, 1, 128, 16), k > 0 ? 1u : window);
                         }
                         umma_commit(&dw_done[G * c + g]);
                     }
                 } else {
                     const uint32_t d = tmem_base + (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16));
+                    const bool ends = M::kWindows && ((filled >> (4 * l)) & (M::kWindow - 1u)) == M::kWindow - 1u;
                     auto gradient = [&](auto z_width, auto a_width, uint32_t ones) {
                         constexpr int ZW = decltype(z_width)::value, AW = decltype(a_width)::value;
 #pragma unroll 2
@@ -536,12 +685,19 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
                         else if (l == NL - 1 && M::kDzW != H) gradient(std::integral_constant<int, M::kDzW>{}, WideT{}, M::kOnes);
                         else gradient(WideT{}, WideT{}, M::kOnes);
                         umma_commit(&dw_done[G * c + g]);
+                        if (ends) umma_commit(&ended[l]);
                     }
+                    if (M::kWindows) filled = (filled + (1u << (4 * l))) & (0x11111u * (M::kWindow - 1u));
+                    if (ends) over |= 1u << l;
                 }
                 __syncwarp();
                 started |= 1u << l;
+                if constexpr (M::kWide) {
+                    summed |= 1u << l;
+                    if (M::ends_window((int)l, c, turn)) over |= 1u << l;
+                }
                 layers += (l < G ? top - l : 0u - G) << (4 * c);
-                if (l < G) flip ^= 1u << c;
+                if (l < G) turns = (turns + (1u << (8 * c))) & 0x0f0f0f0fu;
                 phase ^= 1u << c;
                 --total;
                 idle = 0;
@@ -552,6 +708,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             }
             c = c + 1 == NCH ? 0u : c + 1;
         }
+        if (M::kWindows && lane == 0) atomicOr((uint32_t*)(smem + M::kOpen), (M::kWide ? summed : started) & ~over);
     }
 
     // ---- one add per parameter per CTA ----
@@ -559,31 +716,42 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
     __syncthreads();   // every chain has seen its last gradient product completed (or the CTA is aborting)
     tc_fence_after();
     const bool good = !*abort_flag;
+    if constexpr (M::kWindows) {   // the windows that are open, a chain's warps each
+        if (good && warp < NW && (M::kWide || (warp & 3) < 2)) {
+            const uint32_t open = *(const volatile uint32_t*)(smem + M::kOpen);
+#pragma unroll 1
+            for (int l = warp >> 2; l < NL; l += NCH)
+                if ((open >> l) & 1u) take_window<M, H, NL, IW>(tmem_base + ((uint32_t)((warp & 3) * 32) << 16), sbase, l);
+        }
+        __syncthreads();
+        tc_fence_after();
+    }
     float* sums = (float*)smem;
+    constexpr bool kStaged = H != 32;   // through shared memory, from tensor memory; width 32 has its sums there
 #pragma unroll 1
     for (int l0 = 0; l0 < NL; l0 += M::kSumLayers) {
         if (l0 > 0) __syncthreads();
-        if (good && warp < NW) {
+        if (kStaged && good && warp < NW) {
             // Row r of a 64-row accumulator sits on lane 32 (r / 16) + r % 16, of one of 128 rows on lane r.  The warps of a lane
             // quarter take the 16-column pieces in turn.
             const int quarter = warp & 3;
             const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
             for (int l = l0; l < l0 + M::kSumLayers; ++l) {
+                if (M::kWide && l == 0 && !M::kSumsInTmem) break;
                 const int w = M::kWide && l == NL - 1 ? OW : l == 0 ? IW : H;
                 float* layer = sums + (l - l0) * H * (int)M::kSumRow;
 #pragma unroll 1
-                for (int piece = warp >> 2; piece <= w / 16; piece += NCH) {
+                for (int piece = warp >> 2; piece < w / 16 + (M::kWide ? 0 : 1); piece += NCH) {
                     const bool bias = piece == w / 16;
                     uint32_t col;
-                    if constexpr (M::kWide) col = bias ? M::db_col(0) + 16u * l : (l == 0 ? M::dw_col(0) : l < NL - 1 ? M::dw_col(1) + (l - 1) * 128u : M::dw_col(NL - 1)) + piece * 16u;
+                    if constexpr (M::kWide) col = (l == 0 ? M::sum_col() : l < NL - 1 ? M::dw_col(1) + (l - 1) * 128u : M::dw_col(NL - 1)) + piece * 16u;
                     else col = (l == 0 ? M::dw_col(0) : M::dw_col(1) + (l - 1) * (H + 16)) + piece * 16u;
                     uint32_t v[16];
                     tmem_ld_32x16(lanes + col, v);
                     wait_ld(v);
-                    const bool half = !M::kWide || (bias && l == NL - 1);   // 64 rows
-                    const int row = half ? quarter * 16 + lane : quarter * 32 + lane;
-                    if ((!half || lane < 16) && row < H) {
+                    const int row = M::kWide ? quarter * 32 + lane : quarter * 16 + lane;
+                    if (M::kWide || (lane < 16 && row < H)) {
                         // the last layer of width 128 lies in features by outputs
                         const bool across = M::kWide && l == NL - 1;
                         float* at = bias ? layer + row * (int)M::kSumRow + H : across ? layer + piece * 16 * (int)M::kSumRow + row : layer + row * (int)M::kSumRow + piece * 16;
@@ -597,7 +765,7 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             }
             tc_fence_before();
         }
-        __syncthreads();
+        if (kStaged) __syncthreads();
         if (!good) continue;
         // real parameters in the order they are stored, four to a reduction where rows are whole 16-byte pieces
         int i = threadIdx.x;
@@ -606,17 +774,25 @@ __global__ void __launch_bounds__(32 * (5 * NCH + grad_warps(NCH)), 1) learn_gra
             const int in = cfg.dims[l], out = cfg.dims[l + 1];
             float* dW = (float*)s_net[l].weightsGrad;
             float* dB = (float*)s_net[l].biasesGrad;
-            const float* s = sums + (l - l0) * H * (int)M::kSumRow;
+            const bool swizzled = !kStaged || (M::kWide && l == 0 && !M::kSumsInTmem);   // rows of the windows' sums
+            const float* s = swizzled ? (const float*)(smem + M::kSums) + (kStaged ? 0 : l * H * 32) : sums + (l - l0) * H * (int)M::kSumRow;
+            const float* b = M::kWindows ? (const float*)(smem + M::kBiasSums) + l * H : s + H;
             const bool fours = (in & 3) == 0 && cfg.param_layout == MLP_PARAMS_ROW_MAJOR && ((uint64_t)dW & 15u) == 0;
             const int per_row = fours ? in >> 2 : in;
             for (; i < out * per_row; i += kThreads) {
                 const int o = i / per_row, k = i - o * per_row;
+                if (swizzled) {
+                    const float* at = s + o * 32;
+                    if (fours) atomicAdd((float4*)dW + i, *(const float4*)(at + 4 * (k ^ (o & 7))));
+                    else atomicAdd(dW + weight_index(cfg.param_layout, in, out, o, k), at[(k ^ (4 * (o & 7)))]);
+                    continue;
+                }
                 const float* at = s + o * (int)M::kSumRow;
                 if (fours) atomicAdd((float4*)dW + i, make_float4(at[4 * k], at[4 * k + 1], at[4 * k + 2], at[4 * k + 3]));
                 else atomicAdd(dW + weight_index(cfg.param_layout, in, out, o, k), at[k]);
             }
             i -= out * per_row;
-            for (; i < out; i += kThreads) atomicAdd(dB + i, s[i * (int)M::kSumRow + H]);
+            for (; i < out; i += kThreads) atomicAdd(dB + i, b[M::kWindows ? i : i * (int)M::kSumRow]);
             i -= out;
         }
     }

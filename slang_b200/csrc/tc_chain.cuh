@@ -427,5 +427,18 @@ __device__ __noinline__ void reverse_whole_row(uint32_t t_acc, uint32_t row)
     }
 }
 
+// Adds 4 N values to chunks first .. first + N - 1 of a row of fp32 sums at `at`, whose 16-byte chunks lie ^ (row % 8).
+template <int N>
+__device__ __forceinline__ void add_chunks(uint32_t at, int row, int first, const uint32_t* v)
+{
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t chunk = at + (uint32_t)(16 * ((first + j) ^ (row & 7)));
+        const float4 x = narrow::lds_float4(chunk);
+        sts128(chunk, __float_as_uint(x.x + __uint_as_float(v[4 * j])), __float_as_uint(x.y + __uint_as_float(v[4 * j + 1])),
+               __float_as_uint(x.z + __uint_as_float(v[4 * j + 2])), __float_as_uint(x.w + __uint_as_float(v[4 * j + 3])));
+    }
+}
+
 }  // namespace chain
 }  // namespace mlpb200

@@ -202,3 +202,40 @@ def test_an_overflow_reaches_the_gradients_that_the_oracle_says(device, dims, co
     for got, ref in ((tr.read_grads(), want), (gb.read(np.float32)[:want_dx.size], want_dx)):
         assert np.array_equal(np.isnan(got), np.isnan(ref))
         assert np.array_equal(np.isposinf(got), np.isposinf(ref)) and np.array_equal(np.isneginf(got), np.isneginf(ref))
+
+
+@pytest.mark.parametrize("dims,dtype", [([16, 32, 3], C.F16), ([4, 32, 32, 32, 32, 4], C.F16), ([20, 24, 30, 16], C.BF16), ([32, 128, 128, 3], C.F16),
+                                        ([64, 128, 64], C.F16), ([32, 128, 128, 128, 3], C.F16)], ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else {C.F16: "f16", C.BF16: "bf16"}[v])
+def test_long_sums_are_not_cut_off(device, dims, dtype):
+    """A sample over and over: the sums are one sample's gradients times the count.  (Values and weights are small multiples of powers of
+    two, so one sample's arithmetic is the same in every kernel.)  Tensor memory drops what does not fit, at every addition and inside it: over four
+    tiles of eight additions, to a sum that is half the final one on average, 32 / 2 * 2 * 2^-23 = 3.8e-6.  A CTA's 14 windows and 148 CTAs are added in fp32,
+    (14 + 148) / 2 * 2^-24 = 4.8e-6 if every rounding goes the same way: 9e-6 in all.  Cut off over a CTA's 55 tiles the sums are 4e-5 short.
+    Width 128: of dW_0 and the biases (the other dW are summed over all tiles)."""
+    from slang_b200.api import Trainer
+    cfg = C.make_config(dims, dtype, C.ACT_RELU, input_dtype=dtype, target_dtype=C.F32, adam_master=1)
+    rng = np.random.default_rng(7)
+    w_off, b_off, total = C.param_layout(cfg)
+    p = np.zeros(total, dtype=np.float32)
+    for l in range(cfg.n_layers):
+        p[w_off[l]:w_off[l] + dims[l] * dims[l + 1]] = rng.integers(1, 8, dims[l] * dims[l + 1]) / 256.0
+        p[b_off[l]:b_off[l] + dims[l + 1]] = rng.integers(1, 8, dims[l + 1]) / 16.0
+    params = C.to_storage(p, dtype)
+    count = (1 << 20) + 77
+    x = np.tile(C.to_storage(rng.integers(1, 8, (1, dims[0])) / 8.0, dtype), (count, 1))
+    t = np.tile(-rng.integers(8, 16, (1, dims[-1])).astype(np.float32) / 8, (count, 1))
+    grads = []
+    for n in (1, count):
+        tr = Trainer(device, cfg, params)
+        xb, tb = device.create_buffer(x[:n].nbytes, x[:n]), device.create_buffer(t[:n].nbytes, t[:n])
+        tr.learn_gradient(xb.address, tb.address, n)
+        grads.append(tr.read_grads().astype(np.float64))
+        xb.destroy(); tb.destroy()
+    want, got = grads[0] * count, grads[1]
+    for l in range(cfg.n_layers):
+        parts = [slice(b_off[l], b_off[l] + dims[l + 1])]
+        if max(dims) <= 32 or l == 0:
+            parts.append(slice(w_off[l], w_off[l] + dims[l] * dims[l + 1]))
+        for part in parts:
+            assert np.all(want[part] != 0)
+            assert np.max(np.abs(got[part] / want[part] - 1)) < 9e-6
