@@ -30,7 +30,7 @@ using namespace ptx;
 
 namespace chain {
 
-enum : uint32_t { kStatusIssue = 0x4000u, kStatusRow = 0x8000u, kStatusGrad = 0x10000u };
+enum : uint32_t { kStatusIssue = 0x20000u, kStatusRow = 0x40000u, kStatusGrad = 0x80000u };
 
 // Warps that issue gradient products: two (even and odd layers) beside four chains; with three, sixteen warps in all leave
 // each thread 128 registers and seventeen 96.

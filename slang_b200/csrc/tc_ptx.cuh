@@ -12,6 +12,8 @@ namespace mlpb200 {
 namespace ptx {
 
 constexpr uint32_t kMaxPolls = 4000000u;
+// The status word's bits, which all kernels of a device share: 0x1 to 0x20 tc_kernels.cu, 0x100 to 0x800 tc_forward.cu, 0x2000 tc_narrow.cu,
+// 0x4000 tile_mma.cu, 0x20000 to 0x80000 tc_chain.cu, 0x20000000 and 0x40000000 selftest.cu.
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

@@ -8,7 +8,9 @@ the kernel normally and surfaces as MLP_E_DEVICE_STATUS from mlp_wait exactly on
 library reports an asynchronous error, or that does not finish in time, surfaces as MLP_E_COMM from
 mlp_comm_wait (checked against a stand-in collective library built by the test).
 """
+import glob
 import os
+import re
 import socket
 import subprocess
 import sys
@@ -78,6 +80,18 @@ def test_survivor_learns_of_a_missing_rank_before_the_next_collective(tmp_path, 
     else:
         assert outcome == "timeout:1:step2"
         assert float(seconds) < 10.0
+
+
+def test_every_wait_has_a_status_bit_of_its_own():
+    """All kernels of a device share one status word, so no two of their codes may share a bit (read from the sources)."""
+    owner = {}
+    for path in sorted(glob.glob(os.path.join(ROOT, "slang_b200", "csrc", "*.cu*"))):
+        for name, value in re.findall(r"\b(kStatus\w+)\s*=\s*(0x[0-9a-fA-F]+|\d+)u", open(path).read()):
+            v = int(value, 0)
+            assert v and v & (v - 1) == 0, (path, name)
+            assert v not in owner, (owner[v], (path, name))
+            owner[v] = (path, name)
+    assert len(owner) >= 17
 
 
 # ---- GPU --------------------------------------------------------------------------------------
