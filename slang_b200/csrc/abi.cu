@@ -240,7 +240,8 @@ int32_t mlp_buffer_clear(MlpDevice* d, MlpBuffer* b, size_t offset, size_t size)
     if (offset > b->size || size > b->size - offset) return fail(MLP_E_INVALID_ARG, "clear range outside the buffer");
     CUDA_TRY(cudaSetDevice(d->ordinal));
     if (size == 0) return MLP_OK;
-    if (size <= kClearBytes) CUDA_TRY(launch_clear_bytes(d->stream, (char*)b->ptr + offset, (uint32_t)size));
+    // (wrapped memory, and buffers of another device, may be where a kernel of this one faults and a memset works or is refused)
+    if (size <= kClearBytes && b->owned && b->ordinal == d->ordinal) CUDA_TRY(launch_clear_bytes(d->stream, (char*)b->ptr + offset, (uint32_t)size));
     else CUDA_TRY(cudaMemsetAsync((char*)b->ptr + offset, 0, size, d->stream));
     return MLP_OK;
 }

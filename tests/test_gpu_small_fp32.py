@@ -49,3 +49,30 @@ def test_clears_touch_their_range_only(device, offset, size):
     want = np.full(8192, 0xa5, dtype=np.uint8)
     want[offset:offset + size] = 0
     assert np.array_equal(b.read(np.uint8), want)
+
+
+def test_clears_of_wrapped_memory_stay_memsets(device):
+    """A small clear is a kernel where the library owns the memory.  Memory that was wrapped may be anywhere (another device's, or an address that
+    only a memset refuses), so no kernel writes there: read from what a capture records, without running it."""
+    from cuda.bindings import runtime as rt
+    from slang_b200.api import Device
+
+    def ok(result):
+        assert result[0] == rt.cudaError_t.cudaSuccess, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    stream = ok(rt.cudaStreamCreate())
+    d = Device(0, int(stream))
+    owned = d.create_buffer(64)
+    kinds = []
+    for b in (owned, d.wrap_buffer(owned.address, 64)):
+        ok(rt.cudaStreamBeginCapture(stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
+        b.clear(0, 8)
+        graph = ok(rt.cudaStreamEndCapture(stream))
+        nodes, n = ok(rt.cudaGraphGetNodes(graph, 4))
+        assert n == 1
+        kinds.append(ok(rt.cudaGraphNodeGetType(nodes[0])))
+        rt.cudaGraphDestroy(graph)
+    assert kinds == [rt.cudaGraphNodeType.cudaGraphNodeTypeKernel, rt.cudaGraphNodeType.cudaGraphNodeTypeMemset]
+    d.destroy()
+    rt.cudaStreamDestroy(stream)
