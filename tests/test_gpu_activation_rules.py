@@ -129,3 +129,28 @@ def test_output_sigmoid_is_as_exact_as_one_thread_per_sample(device, dims):
         tr.forward(xb.address, yb.address, x.size)
         outputs.append(yb.read(np.float32).copy())
     assert np.array_equal(outputs[0], outputs[1])
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16"])
+@pytest.mark.parametrize("dims", [[1, 32, 3], [1, 32, 9], [1, 24, 16], [1, 40, 20], [1, 64, 64]], ids=lambda d: "-".join(map(str, d)))
+def test_output_sigmoid_of_every_value(device, dims, storage):
+    """The same for every finite pre-activation of the storage type, for few outputs and many."""
+    from slang_b200.api import Trainer
+    cfg = _config(dims, storage, C.ACT_RELU, output_act=C.ACT_SIGMOID)
+    w_off, _, total = C.param_layout(cfg)
+    p = np.zeros(total, dtype=np.float32)
+    p[w_off[0]], p[w_off[0] + 1] = 1.0, -1.0
+    for o in range(dims[2]):
+        p[w_off[1] + o * dims[1]:w_off[1] + o * dims[1] + 2] = [1.0, -1.0]
+    params = C.to_storage(p, cfg.dtype)
+    bits = np.arange(1 << 16, dtype=np.uint32)
+    x = bits.astype(np.uint16).view(np.float16).astype(np.float32) if storage == "f16" else (bits << 16).view(np.float32)
+    x = np.ascontiguousarray(x[np.isfinite(x)]).reshape(-1, 1)
+    xb, yb = device.create_buffer(x.nbytes, x), device.create_buffer(4 * x.size * dims[2])
+    outputs = []
+    for entry in ("forward", "forward_simt"):
+        tr = Trainer(device, cfg, params, forward_entry=entry)
+        tr.forward(xb.address, yb.address, x.size)
+        outputs.append(yb.read(np.float32).copy().reshape(x.size, dims[2]))
+    differ = outputs[0] != outputs[1]
+    assert not differ.any(), (int(differ.sum()), x[differ.any(1)][:4], outputs[0][differ][:4], outputs[1][differ][:4])
