@@ -57,12 +57,11 @@ def test_leaky_relu_takes_the_rounded_preactivation(device, width, storage, alph
     assert np.array_equal(tr.read_grads(), want)
 
 
-def _around_zero(device, dims, storage, act):
+def _around_zero(device, dims, storage, act, count=500):
     """Three samples in four have one input, the smallest half above zero: every first-layer pre-activation is a product
     of less than half of it (biases are zero), of either sign.  Gradients, input gradients and loss against the oracle."""
     from slang_b200.api import Trainer
     cfg = _config(dims, storage, act, act_alpha=0.02)
-    count = 500
     rng = np.random.default_rng(sum(dims))
     params = C.init_params(cfg, seed=4, scheme="xavier")
     p = C.from_storage(params, cfg.dtype).copy()
@@ -107,6 +106,47 @@ def test_leaky_relu_around_zero(device, dims, storage):
 def test_relu_around_zero(device, dims, storage):
     """The derivative at zero is one half, from whichever side the pre-activation was rounded."""
     _around_zero(device, dims, storage, C.ACT_RELU)
+
+
+# Batches from 1024 samples on (forward 4096) run in whole tiles of 128, networks up to width 128 among them.
+@pytest.mark.parametrize("alpha", [0.01, 0.3])
+@pytest.mark.parametrize("storage", ["f16", "bf16"])
+@pytest.mark.parametrize("dims", [[2, 12, 12], [2, 24, 24], [2, 40, 40], [8, 100, 64]], ids=lambda d: "-".join(map(str, d)))
+def test_leaky_relu_takes_the_rounded_preactivation_in_tiles(device, dims, storage, alpha):
+    """The sample of the test above inside a batch of samples that are zero and have no gradient: still bit for bit."""
+    from slang_b200.api import Trainer
+    cfg = _config(dims, storage, C.ACT_LEAKY_RELU, act_alpha=alpha)
+    count, width, out = 5001, dims[1], dims[2]
+    rng = np.random.default_rng(width)
+    w_off, b_off, total = C.param_layout(cfg)
+    p = np.zeros(total, dtype=np.float32)
+    w0 = np.zeros((width, dims[0]), dtype=np.float32)
+    w0[:, 0] = -rng.integers(64, 128, width) / 128.0
+    w0[:, 1] = rng.integers(-7, 8, width) / 8192.0
+    p[w_off[0]:w_off[0] + w0.size] = w0.ravel()
+    p[w_off[1]:w_off[1] + width * out] = np.eye(out, width, dtype=np.float32).ravel()
+    params = C.to_storage(p, cfg.dtype)
+    x, t = np.zeros((count, dims[0]), dtype=np.float32), np.zeros((count, out), dtype=np.float32)
+    x[777, :2] = [13.0 / 16.0, 1.0]
+    t[777] = rng.uniform(-1, 1, out)
+    tr = Trainer(device, cfg, params)
+    xb, tb, yb = device.create_buffer(x.nbytes, x), device.create_buffer(t.nbytes, t), device.create_buffer(4 * count * out)
+    dxb = device.create_buffer(x.nbytes)
+    tr.forward(xb.address, yb.address, count)
+    assert np.array_equal(yb.read(np.float32), np.asarray(oracle.forward(cfg, params, x, count), dtype=np.float32).ravel())
+    want, words = np.zeros(total, dtype=np.float32), np.zeros(2, dtype=np.uint32)
+    oracle.learn_gradient_inputs(cfg, params, want, x, t, count, words)
+    tr.learn_gradient(xb.address, tb.address, count, input_grads_address=dxb.address)
+    assert np.array_equal(tr.read_grads(), want)
+    dx = dxb.read(np.float32).reshape(x.shape)
+    assert np.all(dx[777, :2] != 0) and np.count_nonzero(dx) == np.count_nonzero(dx[777])
+
+
+@pytest.mark.parametrize("dims,act", [(d, a) for d in AROUND_ZERO + [[32, 128, 128, 3]] for a in (C.ACT_LEAKY_RELU, C.ACT_RELU)] + [([8, 100, 64], C.ACT_LEAKY_RELU)],
+                         ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else {C.ACT_LEAKY_RELU: "leaky", C.ACT_RELU: "relu"}[v])
+def test_around_zero_in_tiles(device, dims, act):
+    """(ReLU through 8-100-64 runs in tiles from 131072 samples on: test_gpu_chain.py.)"""
+    _around_zero(device, dims, "f16", act, count=5000)
 
 
 @pytest.mark.parametrize("dims", [[1, 32, 3], [1, 40, 8], [1, 16, 1], [1, 24, 2], [1, 64, 4], [1, 33, 5]], ids=lambda d: "-".join(map(str, d)))

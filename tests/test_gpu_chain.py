@@ -68,8 +68,8 @@ def test_counts_around_a_tile(device, dims, count):
                                               ([8, 90, 128, 100, 16], None)],
                          ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else "f32" if v == C.F32 else "own")
 def test_shapes_and_formats(device, dims, input_dtype, dtype, act):
-    """Every build; rows that are read as values, as whole pieces and converted one by one.  In bf16 a sum that rounds the other
-    way is 2^-8 of its value, and a few of them meet in a gradient."""
+    """Rows that are read as values, as whole pieces and converted one by one; every build but those of ReLU at width 128 that take larger batches
+    only (test_relu_builds_of_large_batches).  In bf16 a sum that rounds the other way is 2^-8 of its value, and a few of them meet in a gradient."""
     cfg = C.make_config(dims, dtype, act, input_dtype=dtype if input_dtype is None else input_dtype, target_dtype=C.F32 if dims[-1] % 2 else dtype, adam_master=1)
     _check(cfg, _run(device, cfg, 5003), 2e-2 if dtype == C.BF16 else 1e-2)
 
@@ -239,3 +239,99 @@ def test_long_sums_are_not_cut_off(device, dims, dtype):
         for part in parts:
             assert np.all(want[part] != 0)
             assert np.max(np.abs(got[part] / want[part] - 1)) < 9e-6
+
+
+@pytest.mark.parametrize("dtype", [C.F16, C.BF16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("dims,count", [([64, 128, 64], 131072 + 77), ([24, 70, 40], 131072), ([40, 128, 128, 16], 65536 + 77), ([8, 90, 128, 100, 16], 65536 + 77),
+                                        ([32, 128, 128, 128, 3], 65536)], ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else str(v))
+def test_relu_builds_of_large_batches(device, dims, count, dtype):
+    """Width 128, with input gradients; a third of the samples are zero and meet zero biases, so their pre-activations are zero in every layer."""
+    cfg = C.make_config(dims, dtype, C.ACT_RELU, input_dtype=dtype, target_dtype=C.F32, adam_master=1)
+    rng = np.random.default_rng(count)
+    x = rng.uniform(-1, 1, (count, dims[0])) * (rng.random((count, 1)) < 0.7)
+    t = rng.uniform(-1, 1, (count, dims[-1]))
+    p0 = C.from_storage(C.init_params(cfg, seed=3, scheme="xavier"), dtype)
+    w_off, b_off, total = C.param_layout(cfg)
+    for l in range(cfg.n_layers):
+        p0[b_off[l]:b_off[l] + dims[l + 1]] = 0.0
+    p0 = C.to_storage(p0, dtype)
+    bar = 2e-2 if dtype == C.BF16 else 1e-2
+    result = _run(device, cfg, count, p0, x, t, input_grads=True)
+    _check(cfg, result, bar)
+    n = 300
+    dx = oracle.learn_gradient_inputs(cfg, p0, np.zeros(total, dtype=np.float32), C.to_storage(x, dtype), C.to_storage(t, C.F32), n, np.zeros(2, dtype=np.uint32))
+    assert rel_err(result[6][:n], dx[:n]) < bar
+
+
+@pytest.mark.parametrize("dtype,act", [(C.F16, C.ACT_RELU), (C.BF16, C.ACT_RELU), (C.BF16, C.ACT_LEAKY_RELU)], ids=["f16-relu", "bf16-relu", "bf16-leaky"])
+@pytest.mark.parametrize("dims", [[8, 32, 32, 4], [7, 24, 3], [32, 64, 64, 3], [40, 64, 64, 20], [32, 128, 128, 3]], ids=lambda d: "-".join(map(str, d)))
+def test_input_gradients_against_the_oracle(device, dims, dtype, act):
+    """The other formats and activations; the oracle rounds where the kernels do, so what is left is the order of sums of 16-bit values."""
+    cfg = C.make_config(dims, dtype, act, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
+    count = 1100
+    rng = np.random.default_rng(sum(dims))
+    x, t = rng.uniform(-1, 1, (count, dims[0])).astype(np.float32), rng.uniform(-1, 1, (count, dims[-1])).astype(np.float32)
+    p0 = C.init_params(cfg, seed=3, scheme="xavier")
+    want = oracle.learn_gradient_inputs(cfg, p0, np.zeros(C.param_layout(cfg)[2], dtype=np.float32), x, t, count, np.zeros(2, dtype=np.uint32))
+    got = _run(device, cfg, count, p0, x, t, input_grads=True)[6]
+    assert rel_err(got, want) < (2e-2 if dtype == C.BF16 else 1e-2)
+
+
+@pytest.mark.parametrize("dims,input_dtype", [([8, 24, 8], C.F32), ([8, 24, 8], C.F16), ([16, 32, 16], C.F32), ([24, 32, 32, 4], C.F16), ([40, 64, 64, 20], C.F32),
+                                              ([32, 64, 64, 64, 4], C.F16), ([32, 128, 128, 4], C.F16), ([32, 128, 128, 4], C.F32)],
+                         ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else {C.F32: "f32", C.F16: "f16"}[v])
+def test_memory_off_its_boundary(device, dims, input_dtype):
+    """Rows, outputs, parameters and gradients one element past a 16-byte boundary (width 128: not its input rows): the values of aligned ones, the sums of
+    gradients in another order."""
+    from slang_b200.api import Trainer
+    cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=input_dtype, target_dtype=C.F32, adam_master=1)
+    count = 4500
+    rng = np.random.default_rng(sum(dims))
+    x, t = C.to_storage(rng.uniform(-1, 1, (count, dims[0])), input_dtype), rng.uniform(-1, 1, (count, dims[-1])).astype(np.float32)
+    p0 = C.init_params(cfg, seed=3, scheme="xavier")
+    results = []
+    for off in (0, 1):
+        buffers = []
+
+        def memory(nbytes, shift, data=None):
+            b = device.create_buffer(nbytes + 64)
+            buffers.append(b)
+            if data is not None:
+                b.write(data, offset=shift)
+            return b.address + shift
+
+        params, grads = memory(p0.nbytes, 2 * off), memory(4 * p0.size, 4 * off)
+        tr = Trainer(device, cfg, p0, param_memory=(params, grads))
+        xa = memory(x.nbytes, x.itemsize * off if max(dims) <= 64 else 0, x)
+        ta = memory(t.nbytes, 4 * off, t)
+        dx, y = memory(4 * count * dims[0], 4 * off), memory(4 * count * dims[-1], 4 * off)
+        tr.learn_gradient(xa, ta, count, input_grads_address=dx)
+        if max(dims) <= 64:   # (the other forward kernels want their memory aligned)
+            tr.forward(xa, y, count)
+        results.append([device.wrap_buffer(dx, 4 * count * dims[0]).read(np.float32), device.wrap_buffer(y, 4 * count * dims[-1]).read(np.float32), tr.read_grads(), tr.read_loss()])
+    assert np.array_equal(results[0][0], results[1][0]) and np.array_equal(results[0][1], results[1][1])
+    assert np.any(results[0][0]) and rel_err(results[1][2], results[0][2]) < 1e-5
+    assert results[0][3][0] == results[1][3][0] and abs(results[0][3][1] - results[1][3][1]) <= 1e-5 * results[0][3][1]
+
+
+@pytest.mark.parametrize("count", [500, 5000])
+def test_misaligned_input_rows_of_wide_networks_are_refused(device, count):
+    """By the host, in every batch."""
+    from slang_b200.api import Trainer
+    from slang_b200.lib import MlpError
+    for input_dtype, shift in ((C.F16, 2), (C.F32, 4)):
+        cfg = C.make_config([32, 128, 128, 3], C.F16, C.ACT_RELU, input_dtype=input_dtype, target_dtype=C.F32, adam_master=1)
+        tr = Trainer(device, cfg, C.init_params(cfg, seed=3, scheme="xavier"))
+        xb, tb = device.create_buffer(4 * 32 * count + 64), device.create_buffer(12 * count)
+        with pytest.raises(MlpError):
+            tr.learn_gradient(xb.address + shift, tb.address, count)
+        tr.learn_gradient(xb.address, tb.address, count)
+    device.wait()
+
+
+@pytest.mark.parametrize("tiles", [4 * 148, 5 * 148, 8 * 148 - 1, 33 * 148 + 1])
+@pytest.mark.parametrize("dims", [[9, 17, 1], [4, 32, 32, 32, 32, 4], [16, 100, 3]], ids=lambda d: "-".join(map(str, d)))
+def test_windows_of_tiles(device, dims, tiles):
+    """Gradients leave tensor memory every four tiles (width 32), every tile and every 16th (width 128): batches that end with a window, behind one, or before."""
+    cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F16, target_dtype=C.F32, adam_master=1)
+    _check(cfg, _run(device, cfg, 128 * tiles - 5), 1e-2)

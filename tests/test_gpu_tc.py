@@ -161,6 +161,26 @@ def test_narrow_kernel_two_tiles_in_flight(device, dims, dtype):
     assert abs(l_gpu[0][0] - l_ref[0][0]) <= 1e-2 * abs(l_ref[0][0])
 
 
+@pytest.mark.parametrize("act", [C.ACT_RELU, C.ACT_LEAKY_RELU], ids=["relu", "leaky"])
+@pytest.mark.parametrize("dims,operand", [([32, 64, 64, 3], C.F16), ([10, 40, 12], C.BF16), ([8, 32, 32, 4], C.F16)])
+def test_register_kernels_over_many_units(device, dims, operand, act):
+    """The same over fp32 storage, which whole tiles of 128 samples do not take: the kernels that carry 16 samples a warp in registers, with many units
+    of work for every warp."""
+    rng = np.random.default_rng(len(dims) * 7 + dims[0])
+    cfg = C.make_config(dims, dtype=C.F32, hidden_act=act, output_act=C.ACT_IDENTITY, operand_dtype=operand)
+    p0 = C.init_params(cfg, seed=8, scheme="kaiming")
+    count = 128 * 148 * 2 + 77
+    x = rng.uniform(-1, 1, (count, dims[0])).astype(np.float32)
+    x[::5] = 0.0
+    t = rng.uniform(-1, 1, (count, dims[-1])).astype(np.float32)
+    _, l_ref, g_ref, _ = oracle_trajectory(cfg, p0, [(x, t)], n_threads=8)
+    _, l_gpu, g_gpu, _, tr = gpu_trajectory(device, cfg, p0, [(x, t)])
+    assert tr.k_learn.implementation == "tcgen05"
+    assert _grad_layer_errs(cfg, g_gpu, g_ref) < (2e-2 if operand == C.BF16 else 1e-2)
+    assert abs(l_gpu[0][1] - l_ref[0][1]) <= 1e-2 * abs(l_ref[0][1])
+    assert abs(l_gpu[0][0] - l_ref[0][0]) <= 1e-2 * abs(l_ref[0][0])
+
+
 @pytest.mark.parametrize("name,count,steps", [("c2", 2048, 10), ("c3", 1024, 10)])
 def test_narrow_network_trajectories(device, name, count, steps):
     cfg, p0, batches = make_problem(name, count, seed=3, steps=steps)
