@@ -187,17 +187,62 @@ __device__ __forceinline__ void fetch_row(RawRow& raw, const Params& p, const ch
     }
 }
 
-// Rows that are neither short nor whole 16-byte pieces of fp32 or operand-type values.
+// Rows of nine to sixteen values that are not whole 16-byte pieces of fp32 or operand-type values.
 template <int FMT>
 static __device__ __noinline__ void convert_row(uint32_t at, int dtype, const char* row, int width, bool real)
 {
-    for (int j = 0; j < (width + 15) / 16 * 2; ++j) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
         float x[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = real && 8 * j + i < width ? load_as_f32(dtype, row, 8 * j + i) : 0.0f;
         using C = Cvt<FMT>;
         sts128(at ^ (uint32_t)(16 * j), C::pack2(x[0], x[1]), C::pack2(x[2], x[3]), C::pack2(x[4], x[5]), C::pack2(x[6], x[7]));
     }
+}
+
+// Wider ones: the warp reads its rows as the one run of memory they are, values or pairs of them side by side, and puts each where
+// it belongs.  (A row a thread, value by value, every load touched 32 rows: forward of 600000 samples of 59-62-62-62-27, fp32 rows, 382 us, 123 so; a step of
+// 33-63-63-63-9, halves, 217 and 161.)  `tile`: the tile's address; `rows`: how many of the warp's are real.
+template <int FMT, int IW>
+static __device__ __noinline__ void scatter_rows(uint32_t tile, int dtype, const char* src, int width, int rows)
+{
+    using C = Cvt<FMT>;
+    const int lane = threadIdx.x & 31, r0 = (int)(threadIdx.x & 96u), n = rows * width;
+    const uint32_t inverse = ((1u << 20) + (uint32_t)width - 1u) / (uint32_t)width;   // (i * inverse) >> 20 is i / width for i < 32 width <= 2048
+    const auto place = [&](int i) {
+        const int r = (int)(((uint32_t)i * inverse) >> 20), f = i - r * width;
+        return (tile + row_at<IW>(r0 + r)) ^ (uint32_t)(2 * f);   // (inside its row of 64 or 128 bytes a row's address has only the swizzle's bits)
+    };
+    // the rest of the last K step, and rows past the batch
+    for (int f = rows > lane ? width & ~15 : 0; f < ((width + 15) & ~15); f += 8) sts128((tile + row_at<IW>(r0 + lane)) ^ (uint32_t)(2 * f), 0u, 0u, 0u, 0u);
+    __syncwarp();
+    if (dtype == FMT && ((width & 1) | (int)((uint64_t)src & 3u)) == 0) {
+#pragma unroll 8
+        for (int i = 2 * lane; i < n; i += 64) {
+            const uint32_t v = __ldg((const uint32_t*)src + i / 2);
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(place(i)), "r"(v) : "memory");
+        }
+    } else if (dtype == MLP_F32 && ((width & 1) | (int)((uint64_t)src & 7u)) == 0) {
+#pragma unroll 8
+        for (int i = 2 * lane; i < n; i += 64) {
+            const float2 v = __ldg((const float2*)src + i / 2);
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(place(i)), "r"(C::pack2(v.x, v.y)) : "memory");
+        }
+    } else if (dtype == MLP_F32) {
+#pragma unroll 8
+        for (int i = lane; i < n; i += 32) {
+            const float v = __ldg((const float*)src + i);
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(place(i)), "h"((uint16_t)C::pack2(v, 0.0f)) : "memory");
+        }
+    } else {
+#pragma unroll 8
+        for (int i = lane; i < n; i += 32) {
+            const uint32_t v = __ldg((const unsigned short*)src + i);
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(place(i)), "h"((uint16_t)(dtype == FMT ? v : C::pack2(bits_value(dtype, v), 0.0f))) : "memory");
+        }
+    }
+    __syncwarp();
 }
 
 // A thread's input row in operand format, up to the end of its last K step.
@@ -243,8 +288,11 @@ __device__ __forceinline__ void write_row(uint32_t at, const Params& p, const Ra
         for (int j = 0; j < IW / 8; ++j) x[j] = real && 8 * j < width ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int j = 0; j < IW / 8; ++j) sts128(at ^ (uint32_t)(16 * j), x[j].x, x[j].y, x[j].z, x[j].w);
-    } else {
+    } else if (width <= 16) {
         convert_row<FMT>(at, type, src_row, width, real);
+    } else {
+        const char* first = src_row - (size_t)(threadIdx.x & 31u) * (size_t)(width * (type == MLP_F32 ? 4 : 2));
+        scatter_rows<FMT, IW>(at - row_at<IW>((int)(threadIdx.x & 127u)), type, first, width, __popc(__ballot_sync(0xffffffffu, real)));
     }
 }
 

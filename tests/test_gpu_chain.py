@@ -335,3 +335,13 @@ def test_windows_of_tiles(device, dims, tiles):
     """Gradients leave tensor memory every four tiles (width 32), every tile and every 16th (width 128): batches that end with a window, behind one, or before."""
     cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F16, target_dtype=C.F32, adam_master=1)
     _check(cfg, _run(device, cfg, 128 * tiles - 5), 1e-2)
+
+
+@pytest.mark.parametrize("count", [4096 + 61, 20000])
+@pytest.mark.parametrize("dims,dtype,input_dtype", [([20, 30, 30, 16], C.F16, C.F16), ([50, 44, 44, 40], C.F16, C.F32), ([50, 64, 48], C.BF16, C.BF16), ([37, 54, 6], C.BF16, C.F32), ([63, 40, 8], C.F16, C.F16),
+                                                    ([18, 24, 5], C.F16, C.F32), ([25, 40, 8], C.F16, C.BF16), ([30, 40, 40, 8], C.F16, C.BF16), ([13, 41, 12], C.F16, C.F16), ([11, 20, 5], C.BF16, C.F32)],
+                         ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else {C.F16: "f16", C.BF16: "bf16", C.F32: "f32"}[v])
+def test_ragged_input_rows(device, dims, dtype, input_dtype, count):
+    """Input rows that are no whole 16-byte pieces: even and odd widths, each number format, last tiles with few rows."""
+    cfg = C.make_config(dims, dtype, C.ACT_RELU, input_dtype=input_dtype, target_dtype=C.F32, adam_master=1)
+    _check(cfg, _run(device, cfg, count), 2e-2 if dtype == C.BF16 else 1e-2)
