@@ -1161,6 +1161,20 @@ static bool chain_train_network(const MlpConfig& c)
     return c.dims[0] <= 32 && c.dims[c.n_layers] <= 16;
 }
 
+// Rows that the chains read or write less well than the register kernels, which deal 16 or 32 samples to a warp and their columns to its lanes.
+// Targets of no whole pieces of four: a thread reads its own row value by value.
+static bool ragged_targets(const MlpConfig& c) { return c.dims[c.n_layers] > 40 && (c.dims[c.n_layers] & 3) != 0; }
+// Odd input rows go to shared memory value by value (scatter_rows()).
+static bool odd_inputs(const MlpConfig& c) { return c.encoding != MLP_ENC_FREQ2D && c.dims[0] > 32 && (c.dims[0] & 1) != 0; }
+// Samples that a B200's 148 SMs have in flight at once, a tile in each of so many chains.  Just above it few SMs have a second round.
+static constexpr uint32_t one_round(uint32_t chains) { return 148u * chains * (uint32_t)chain::kTile; }
+static int widest_of(const MlpConfig& c)
+{
+    int w = 0;
+    for (int l = 0; l <= c.n_layers; ++l) w = c.dims[l] > w ? c.dims[l] : w;
+    return w;
+}
+
 // Networks of widths up to 128 (those that launch_learn_gradient_tc takes).
 static bool chain_wide_network(const MlpConfig& c)
 {
@@ -1180,14 +1194,54 @@ static bool chain_wide_network(const MlpConfig& c)
 bool chain_train_wide_suits(const MlpConfig& c, uint32_t count)
 {
     if (!chain_wide_network(c)) return false;
+    // Weight rows of hidden layers in no whole 16-byte pieces are staged value by value: 32-70-70-3, 4096 samples 18.7 / 20.7, 10000: 23.2 / 20.5; 8-109-109-15: 22.6 /
+    // 25.9, 9000: 24.7 / 26.4, 20000: 32.9 / 29.7.  (Two layers, 16-100-3: 14.4 / 12.4 at 2048; leaky ReLU, 32-127-127-16: 35.0 / 27.7; but 24-99-99-62 34.9 / 42.4,
+    // 20000: 64.6 / 59.2, whose targets are read so too.)
+    bool pieces = c.param_layout == MLP_PARAMS_ROW_MAJOR;
+    for (int l = 1; l < c.n_layers; ++l) pieces = pieces && (c.dims[l] & 7) == 0;
+    if (count < 12288u && c.n_layers > 2 && !pieces && (c.hidden_act == MLP_ACT_RELU || ragged_targets(c))) return false;
     const bool few_out = c.dims[c.n_layers] <= 16, few = c.dims[0] <= 32 && few_out;
     if (c.hidden_act == MLP_ACT_LEAKY_RELU) return count >= (few || c.n_layers > 2 ? kTrainFrom : 4u * kTrainFrom);
     if (c.n_layers == 4 || (c.n_layers == 3 && !few)) return few_out && count >= 65536u;   // one chain
     return count >= (few ? kTrainFrom : 131072u);
 }
 
-bool chain_train_suits(const MlpConfig& c, uint32_t count) { return count >= kTrainFrom && chain_train_network(c); }
-bool chain_forward_suits(const MlpConfig& c, uint32_t count) { return count >= kForwardFrom && chain_network(c); }
+bool chain_train_suits(const MlpConfig& c, uint32_t count)
+{
+    if (count < kTrainFrom || !chain_train_network(c)) return false;
+    // us against tc_narrow.cu: 38-36-55, 4096 samples 18.5 / 22.3, 20000: 22.7 / 26.0, 50000: 31.2 / 26.5, 65536: 34.8 / 42.3, 600000: 175 / 266; 13-24-47: 18.5 /
+    // 20.2, 20.7 / 23.3, 28.9 / 23.8, 31.3 / 37.2, 156 / 208; 50-44-44-44-61 (two chains): 28.3 / 30.9, 32.9 / 36.8, 48.2 / 60.6, 288 / 406.
+    if (ragged_targets(c)) return count >= 32768u && count <= one_round(c.n_layers == 4 ? 2 : 3);
+    // 37-54-6 of fp32 rows, 131072 samples 32.4 / 30.3, 600000: 90.8 / 107
+    if (odd_inputs(c) && c.input_dtype == MLP_F32 && c.n_layers == 2) return count <= 262144u;
+    return true;
+}
+
+bool chain_forward_suits(const MlpConfig& c, uint32_t count)
+{
+    if (count < kForwardFrom || !chain_network(c)) return false;
+    const int nl = c.n_layers, in = c.dims[0], out = c.dims[nl], widest = widest_of(c);
+    if (widest <= 32) {
+        // Networks of a few products of 16 x 8 with fp32 rows, or with rows of nine to sixteen values in no whole pieces: 3-8-8-8-1, 131072 samples 8.1 / 9.3, 600000:
+        // 19.3 / 22.0; 5-32-7: 7.5 / 8.3, 17.6 / 19.4; 10-8-8 of halves: 8.5 / 9.9, 22.9 / 24.2.  (2-16-16-2: 600000 within 3 %; 4-16-4 of halves: 8.4 / 6.8, 21.9 / 14.4.)
+        int products = 0;
+        for (int l = 0; l < nl; ++l) products += (c.dims[l] + 15) / 16 * ((c.dims[l + 1] + 7) / 8);
+        const bool by_value = c.input_dtype == MLP_F32 ? in <= 8 : in > 8 && in < 16;
+        if (by_value && c.encoding != MLP_ENC_FREQ2D && products <= (nl == 2 ? 6 : 4)) return false;
+        // odd fp32 rows, which scatter_rows() takes value by value: 21-31-3, 65536 samples 6.5 / 7.6, 600000: 25.0 / 28.6; 21-28-28-28-28-3: 8.9 / 10.7, 32.8 / 38.8
+        if (c.input_dtype == MLP_F32 && in > 16 && (in & 1) != 0) return false;
+        return count >= 16384u || out <= 16;   // 10-32-32-20, 9000 samples 6.6 / 7.2, 50000: 9.5 / 8.1
+    }
+    if (in <= 32 && out <= 16) return true;    // six chains; three below
+    // 37-54-6, 50000 samples 9.8 / 8.8, 65536: 9.8 / 12.5, 600000: 51.1 / 78.2; 53-41-41-41-41-54: 28.7 / 19.6, 30.6 / 31.2, 141 / 206
+    if (odd_inputs(c)) return count <= one_round(3);
+    // 64-64-64-64, 56832 samples 16.5 / 12.4, 65536: 16.8 / 18.0, 75000: 17.0 / 17.9, 80000: 21.6 / 18.7; 64-48-3: 8.7 / 7.6, 8.7 / 9.5, 8.8 / 9.2, 12.4 / 9.9.
+    // (Narrower inputs or outputs of more layers, and outputs in no whole pieces, are faster here in between too.)  56-20-40, 131072: 22.7 / 23.5, 600000: 80.4 / 103.
+    const bool whole = (out & 3) == 0 && out >= 40;
+    if (whole && nl == 2 && c.dims[1] <= 32) return count <= one_round(3);
+    if ((whole && nl > 2 && in > 32) || (out <= 4 && nl == 2)) return count <= one_round(3) || count > one_round(4);
+    return true;
+}
 
 cudaError_t launch_learn_gradient_chain(cudaStream_t st, TcWorkspace* ws, const MlpConfig& c, const MlpLearnGradParamsEx& a,
                                         int* launches, std::string* err, float* input_grads)
