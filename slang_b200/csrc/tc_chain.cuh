@@ -1,14 +1,14 @@
-// Networks of widths up to 64 on tcgen05 with whole tiles of 128 samples: what the kernels of tc_chain.cu share.
+// Networks of widths up to 128 on tcgen05 with whole tiles of 128 samples: what the kernels of tc_chain.cu share.
 //
 // A "chain" is four warps that carry one tile through the network: a thread owns one sample (one tensor-memory lane).  The
 // layer inputs A_l lie in shared memory as [128 samples][features] tiles, 16-bit, swizzled, so that one copy is the K-major
 // operand of the next layer's product and the MN-major operand of the weight-gradient product, and dZ_l replaces A_{l+1} where
-// it lay.  A fifth warp per chain issues its layer products and two warps the gradient products of all chains, so nothing
+// it lay.  A fifth warp per chain issues its layer products and one or two warps the gradient products of all chains, so nothing
 // waits for another chain, and a chain's hand-offs (some 500 cycles each) are covered by the others' work.
 // The kernels are bound by instruction issue and by instruction fetches: what a tile runs through is some 2300 instructions,
 // about as much as the instruction cache holds, so what runs once per tile or rarely is kept small or behind a call (texture
 // network, 2^24 texels: 2.64 ms a step with a copy of the gradient products' code per layer and chain, 2.51 with one; later 2.42
-// with the waits' polling loops and the marked zeros' code in line, 2.16 without).
+// with the waits' polling loops and the marked zeros' code in line, 2.16 without; 2.11 with the least polling between gradient products).
 #pragma once
 
 #include "tc_layout.cuh"
@@ -189,7 +189,7 @@ __device__ __forceinline__ void fetch_row(RawRow& raw, const Params& p, const ch
 
 // Rows of nine to sixteen values that are not whole 16-byte pieces of fp32 or operand-type values.
 template <int FMT>
-static __device__ __noinline__ void convert_row(uint32_t at, int dtype, const char* row, int width, bool real)
+static __device__ __forceinline__ void convert_row(uint32_t at, int dtype, const char* row, int width, bool real)
 {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -205,7 +205,7 @@ static __device__ __noinline__ void convert_row(uint32_t at, int dtype, const ch
 // it belongs.  (A row a thread, value by value, every load touched 32 rows: forward of 600000 samples of 59-62-62-62-27, fp32 rows, 382 us, 123 so; a step of
 // 33-63-63-63-9, halves, 217 and 161.)  `tile`: the tile's address; `rows`: how many of the warp's are real.
 template <int FMT, int IW>
-static __device__ __noinline__ void scatter_rows(uint32_t tile, int dtype, const char* src, int width, int rows)
+static __device__ __forceinline__ void scatter_rows(uint32_t tile, int dtype, const char* src, int width, int rows)
 {
     using C = Cvt<FMT>;
     const int lane = threadIdx.x & 31, r0 = (int)(threadIdx.x & 96u), n = rows * width;
@@ -243,6 +243,18 @@ static __device__ __noinline__ void scatter_rows(uint32_t tile, int dtype, const
         }
     }
     __syncwarp();
+}
+
+// Either, behind one call with the arguments that are at hand, so that the other kinds of rows do not fetch it.
+template <int FMT, int IW>
+static __device__ __noinline__ void ragged_row(uint32_t at, int dtype, const char* row, int width, bool real)
+{
+    if (width <= 16) {
+        convert_row<FMT>(at, dtype, row, width, real);
+    } else {
+        const char* first = row - (size_t)(threadIdx.x & 31u) * (size_t)(width * (dtype == MLP_F32 ? 4 : 2));
+        scatter_rows<FMT, IW>(at - row_at<IW>((int)(threadIdx.x & 127u)), dtype, first, width, __popc(__ballot_sync(0xffffffffu, real)));
+    }
 }
 
 // A thread's input row in operand format, up to the end of its last K step.
@@ -288,11 +300,8 @@ __device__ __forceinline__ void write_row(uint32_t at, const Params& p, const Ra
         for (int j = 0; j < IW / 8; ++j) x[j] = real && 8 * j < width ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int j = 0; j < IW / 8; ++j) sts128(at ^ (uint32_t)(16 * j), x[j].x, x[j].y, x[j].z, x[j].w);
-    } else if (width <= 16) {
-        convert_row<FMT>(at, type, src_row, width, real);
     } else {
-        const char* first = src_row - (size_t)(threadIdx.x & 31u) * (size_t)(width * (type == MLP_F32 ? 4 : 2));
-        scatter_rows<FMT, IW>(at - row_at<IW>((int)(threadIdx.x & 127u)), type, first, width, __popc(__ballot_sync(0xffffffffu, real)));
+        ragged_row<FMT, IW>(at, type, src_row, width, real);
     }
 }
 
