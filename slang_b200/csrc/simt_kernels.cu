@@ -467,7 +467,6 @@ struct SmallNet {
     int w_at[MLP_MAX_LAYERS], b_at[MLP_MAX_LAYERS], g_at[MLP_MAX_LAYERS];   // floats: weights (rows of a multiple of four), biases, gradient sums
     uint32_t per_row[MLP_MAX_LAYERS];       // 65536 / (in + 1), rounded up: (i * per_row) >> 16 is i / (in + 1) below 33 * 32
     uint32_t per_input;                     // the same of the input width
-    int total;
     float scale;
 };
 
@@ -819,7 +818,6 @@ static cudaError_t launch_learn_gradient_small(cudaStream_t st, const MlpConfig&
     }
     for (int l = 0; l < c.n_layers; ++l) { net.b_at[l] = floats; floats += c.dims[l + 1]; }
     for (int l = 0; l < c.n_layers; ++l) { net.g_at[l] = floats; floats += c.dims[l + 1] * (c.dims[l] + 1); }
-    net.total = floats;
     const size_t smem = size_t(floats) * 4;
     constexpr size_t kLargest = ((2 * MLP_MAX_LAYERS + 1) * kSmallWidth * kRow + MLP_MAX_LAYERS * kSmallWidth * (2 * kSmallWidth + 2)) * 4;
     static_assert(kLargest <= kSimtSmemMax, "the largest small network fits");

@@ -1,6 +1,6 @@
-// learnGradient and forward for networks of widths up to 64, 16-bit storage, ReLU or leaky ReLU hidden layers: tcgen05
-// products over whole tiles of 128 samples, several tiles in flight per SM (tc_chain.cuh).  tc_narrow.cu has the other
-// networks and the smallest batches.
+// learnGradient for networks of widths up to 128 and forward for widths up to 64, 16-bit storage, ReLU or leaky ReLU hidden layers: tcgen05
+// products over whole tiles of 128 samples, up to six tiles in flight per SM (tc_chain.cuh).  tc_narrow.cu and tc_kernels.cu have the other
+// networks, the smallest batches and what the rules below leave them.
 //
 //   forward   Z_l [128 x H]    = 1 . b_l^T + A_l [128 x W] . W_l^T   A: A_l, K-major      B: W_l [out][in], K-major
 //   input     dA_l [128 x H]   = dZ_l [128 x H] . W_l                A: dZ_l, K-major     B: W_l, MN-major
@@ -8,8 +8,8 @@
 //
 // Bound by instruction issue and by the hand-offs between a chain's four warps and the tensor pipe; the chains' tiles fill
 // shared memory, so there are no more of them.  Against the register-chained kernels of tc_narrow.cu, us: texture network
-// (32-64-64-64-3) 2^24 samples a step 3830 -> 2160, width 32 (4-32-32-32-32-4, leaky ReLU) 2^20 samples 160 -> 124, 1920 x 1080 view of the
-// texture network 142 -> 94.  Counters of 2^20 samples of the texture network: issue slots 43 %, tensor pipe 36 %, LSU wavefronts 39 %.
+// (32-64-64-64-3) 2^24 samples a step 3830 -> 2110, width 32 (4-32-32-32-32-4, leaky ReLU) 2^20 samples 160 -> 130, 1920 x 1080 view of the
+// texture network 142 -> 94.  Counters of 2^20 samples of the texture network: issue slots 44 %, tensor pipe 37 %, LSU wavefronts 40 %.
 //
 // What the reference does instead: one thread per sample with per-element global atomics
 // (examples/mlp-training/mlp_sw.slang:28-58) or CoopVec calls whose CPU/CUDA fallback is scalar loops
@@ -55,7 +55,7 @@ struct TrainMap {
     // without windows; windows of eight tiles 129.1.
     static constexpr uint32_t kWindow = 4;
     // Width 128: dW_0 and db_0 are taken with every tile (1.3e-6, the register sums 1.0e-6), the other biases with some 32 (sums of 16-bit values are
-    // exact for about as long), by the chain's warps: 2^20 samples of 32-128-128-3 231.8 -> 233.9 us, of 32-128-128-128-3 437.7 -> 448.5.
+    // exact for about as long), by the chain's warps: 2^20 samples of 32-128-128-3 231.8 -> 233.9 us, of 32-128-128-128-3 437.7 -> 452.
     // Whether tile `turn` of chain c (of its own count, at least modulo 16) ends a window of layer l.
     __host__ __device__ static constexpr bool ends_window(int l, uint32_t c, uint32_t turn) { return kWide && (l == 0 || (c == 0u && (turn & 15u) == 15u)); }
     static constexpr int kSumWarps = sum_warps(H);
@@ -106,7 +106,7 @@ struct TrainMap {
     __host__ __device__ static constexpr uint32_t dw_cols(int l) { return (uint32_t)in_w(l) + 16; }
     __host__ __device__ static constexpr uint32_t dw_col(int l)
     {
-        if (kWide) return NCH * (uint32_t)H + (l == 0 ? (NL - 2) * 128u + (OW > IW ? OW : 0u) : l < NL - 1 ? (l - 1) * 128u : (NL - 2) * 128u + (OW > IW ? 0u : IW));
+        if (kWide) return NCH * (uint32_t)H + (l == 0 ? (NL - 2) * 128u : l < NL - 1 ? (l - 1) * 128u : (NL - 2) * 128u + IW);
         return NCH * (uint32_t)H + (l == 0 ? 0u : dw_cols(0) + (uint32_t)(l - 1) * (H + 16));
     }
     __host__ __device__ static constexpr uint32_t db_col(int l) { return NCH * (uint32_t)H + (NL - 2) * 128u + IW + OW + 16u * (uint32_t)l; }
@@ -280,7 +280,6 @@ __global__ void __launch_bounds__(32 * (5 * NCH + sum_warps(H) + grad_warps(NCH)
         const uint32_t s_bias = sbase + M::kBias;
         const float scale = cfg.loss == MLP_LOSS_MSE_MEAN ? 1.0f / (float)od : 1.0f;
         const float alpha = cfg.act_alpha, alpha_op = C::round(alpha);
-        constexpr float kTiny = 0.5f * C::kSmallest;   // the largest magnitude that rounds to zero
         float run_max = 0.0f, run_sum = 0.0f;
         uint32_t full = 0, done = 0;                   // phases seen of acc_full; bit g: parity of dw_done's g, from bit 2 on the chain's tiles so far
         auto wait_full = [&]() {
@@ -1147,7 +1146,7 @@ static bool chain_network(const MlpConfig& c)
 
 // Batches from which the tiles are the better way, us against the kernels of tc_narrow.cu (which deal 16 samples at a time):
 // learnGradient and adjustParameters of the texture network, 600 samples 22.5 / 20.5, 16384: 26.7 / 20.6, 2^20: 267 / 174; width
-// 32, 16 samples 17.5 / 18.4, 600: 18.5 / 18.4, 2^20: 160 / 132; 16-32-3, 600: 12.9 / 12.6, 2^20: 113 / 55.
+// 32, 16 samples 17.5 / 18.4, 600: 18.5 / 18.4, 2^20: 160 / 130; 16-32-3, 600: 12.9 / 12.6, 2^20: 113 / 54.
 constexpr uint32_t kTrainFrom = 1024;
 // forward, 20-48-48-3: 100 samples 6.5 / 9.3, 8192: 7.2 / 6.6, 2^20: 73.6 / 42.5; 4-32-32-32-32-4, 2000 samples 6.5 / 6.7, 16384: 9.3 /
 // 6.8, 2^20: 45.6 / 41.6; 64-64-64-50, 2^20: 214 / 134.
@@ -1186,8 +1185,8 @@ static bool chain_wide_network(const MlpConfig& c)
         if (c.dims[l] > 128) return false;
     return c.n_layers < 4 || (c.dims[0] <= 32 && c.dims[c.n_layers] <= 16);
 }
-// Against the kernels of tc_kernels.cu, us a step.  Two chains: 32-128-128-3, 1024 samples 20.5 / 19.3, 2^20: 581 / 229; 16-128-3 14.3 /
-// 12.6, 379 / 124; 64-128-64 16.4 / 19.9, 65536 samples 36.9 / 36.9, 2^20: 369 / 321.  One chain: 32-128-128-128-3 25.1 / 27.0, 65536
+// Against the kernels of tc_kernels.cu, us a step.  Two chains: 32-128-128-3, 1024 samples 20.5 / 19.3, 2^20: 581 / 234; 16-128-3 14.3 /
+// 12.0, 379 / 122; 64-128-64 16.4 / 19.9, 65536 samples 36.9 / 36.9, 2^20: 369 / 321.  One chain: 32-128-128-128-3 25.1 / 27.0, 65536
 // samples 67.6 / 53.1, 2^20: 772 / 457; 56-103-103-3, 25505 samples (two tiles one after the other) 32.8 / 35.6, 65536: 53.0 / 47.2, 2^20: 597 /
 // 336; 64-128-128-64 51 / 61, 567 / 606.  Leaky ReLU has no build of its own there below five layers: 64-96-96-40 33 / 25, 1433 / 578;
 // 64-128-64, 1024 samples 19.3 / 19.9, 16384: 26.6 / 21.2.
