@@ -236,8 +236,8 @@ __device__ __noinline__ void wide_write_out(const WideTrainParams& p, bool ok)
                 const int o = i / in, k = i - o * in;
                 atomicAdd(g + weight_index(p.param_layout, in, out, o, k), s[o * stride + k]);
             }
-        } else if ((in & 3) == 0) {
-            const int n = in >> 2;   // four parameters per reduction (16-byte aligned: rows are multiples of 16 bytes)
+        } else if ((in & 3) == 0 && ((uint64_t)g & 15u) == 0) {
+            const int n = in >> 2;   // four parameters per reduction (rows are multiples of 16 bytes)
             for (int i = t; i < out * n; i += kEpiThreads) {
                 const int o = i / n, k = i - o * n;
                 atomicAdd((float4*)g + i, *(const float4*)(s + o * stride + 4 * k));
@@ -357,7 +357,7 @@ learn_gradient_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
         constexpr bool fp32_storage = F32S;
         const int chunks_per_row = inp / 8;  // 16-byte chunks: 8 elements
         const uint32_t panel_stride = (uint32_t)outp * 128u;
-        const bool rows_aligned = (in & 7) == 0 && p.param_layout == MLP_PARAMS_ROW_MAJOR && !fp32_storage;
+        const bool rows_aligned = (in & 7) == 0 && p.param_layout == MLP_PARAMS_ROW_MAJOR && !fp32_storage && ((uint64_t)w16 & 15u) == 0;
         for (int idx = threadIdx.x; idx < outp * chunks_per_row; idx += kThreads) {
             const int o = idx / chunks_per_row, c = idx % chunks_per_row;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
