@@ -1198,7 +1198,8 @@ bool chain_train_wide_suits(const MlpConfig& c, uint32_t count)
     // 20000: 64.6 / 59.2, whose targets are read so too.)
     bool pieces = c.param_layout == MLP_PARAMS_ROW_MAJOR;
     for (int l = 1; l < c.n_layers; ++l) pieces = pieces && (c.dims[l] & 7) == 0;
-    if (count < 12288u && c.n_layers > 2 && !pieces && (c.hidden_act == MLP_ACT_RELU || ragged_targets(c))) return false;
+    // Rows that the other kernel would convert first (fp32) stay here: no launch in front, nothing allocated.
+    if (count < 12288u && c.n_layers > 2 && !pieces && c.input_dtype == c.dtype && (c.hidden_act == MLP_ACT_RELU || ragged_targets(c))) return false;
     const bool few_out = c.dims[c.n_layers] <= 16, few = c.dims[0] <= 32 && few_out;
     if (c.hidden_act == MLP_ACT_LEAKY_RELU) return count >= (few || c.n_layers > 2 ? kTrainFrom : 4u * kTrainFrom);
     if (c.n_layers == 4 || (c.n_layers == 3 && !few)) return few_out && count >= 65536u;   // one chain

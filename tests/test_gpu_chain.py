@@ -345,3 +345,26 @@ def test_ragged_input_rows(device, dims, dtype, input_dtype, count):
     """Input rows that are no whole 16-byte pieces: even and odd widths, each number format, last tiles with few rows."""
     cfg = C.make_config(dims, dtype, C.ACT_RELU, input_dtype=input_dtype, target_dtype=C.F32, adam_master=1)
     _check(cfg, _run(device, cfg, count), 2e-2 if dtype == C.BF16 else 1e-2)
+
+
+def test_a_first_call_with_fp32_rows_can_be_captured():
+    """Width 128, fp32 input rows: nothing is converted in front and nothing allocated, so the first call of a device may be recorded."""
+    from cuda.bindings import runtime as rt
+    from slang_b200.api import Device, Trainer
+    err, stream = rt.cudaStreamCreate()
+    assert err == rt.cudaError_t.cudaSuccess
+    for dims in ([32, 128, 128, 3], [32, 70, 70, 3]):
+        d = Device(0, int(stream))
+        cfg = C.make_config(dims, C.F16, C.ACT_RELU, input_dtype=C.F32, target_dtype=C.F32, adam_master=1)
+        tr = Trainer(d, cfg, C.init_params(cfg, seed=3, scheme="xavier"))
+        xb, tb = d.create_buffer(4 * 32 * 4096), d.create_buffer(4 * 3 * 4096)
+        d.wait()
+        assert rt.cudaStreamBeginCapture(stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)[0] == rt.cudaError_t.cudaSuccess
+        try:
+            tr.learn_gradient(xb.address, tb.address, 4096)
+        finally:
+            err, graph = rt.cudaStreamEndCapture(stream)
+        assert err == rt.cudaError_t.cudaSuccess
+        rt.cudaGraphDestroy(graph)
+        d.destroy()
+    rt.cudaStreamDestroy(stream)
